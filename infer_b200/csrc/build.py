@@ -29,6 +29,7 @@ NVCC_FLAGS = ["-gencode", "arch=compute_100a,code=sm_100a", "-lineinfo", "-O3", 
 # module name -> source file; headers that every module depends on
 MODULES: Dict[str, str] = {
     "plain": "plain_ops.cu",
+    "lin32": "linear_f32.cu",    # the matrix product of the 32-bit path
     "seq": "seq_ops.cu",         # filters over time, pair rotation, gated recurrence, side-by-side sublayers
     "mix": "mix_ops.cu",         # norms on sublayer results, decayed and delta-rule recurrences, routers, row norms of q and k
     "latent": "latent_ops.cu",   # attention through low-rank latents, layer norm, sigmoid router, capped logits

@@ -139,7 +139,8 @@ rmsnorm_vec_kernel(const float* __restrict__ x, const float* __restrict__ w, flo
 }
 
 // ------------------------------------------------------------------------------------------------
-// Linear: out[m, n] = sum_k x[m, k] * w[n, k] (+ bias[n]) (+ residual[m, n]).
+// Linear over bfloat16 operands: out[m, n] = sum_k x[m, k] * w[n, k] (+ bias[n]) (+ residual[m, n]). (Float operands have
+// kernels of their own: linear_f32.cu.)
 // 64x64 output tile, 16-wide k steps, 4x4 outputs per thread. Each output's sum runs over k in
 // ascending order in float, whatever M is.
 constexpr int LT = 64, LK = 16;
@@ -671,9 +672,7 @@ IB_EXPORT int ib_linear_plain(const void* x, const void* w, const float* bias, c
     if (K <= 0) return ib::fail(IB_ERR_ARG, "ib_linear_plain: K must be positive");
     const dim3 grid{unsigned((N + LT - 1) / LT), unsigned((M + LT - 1) / LT), 1u};
     if (grid.y > 65535) return ib::fail(IB_ERR_ARG, "ib_linear_plain: too many rows (%lld)", (long long)M);
-    if (in_dtype == IB_F32 && out_dtype == IB_F32)
-        IB_LAUNCH((linear_kernel<float, float>), grid, 256, 0, (const float*)x, (const float*)w, bias, residual, (float*)out, M, N, K);
-    else if (in_dtype == IB_BF16 && out_dtype == IB_BF16)
+    if (in_dtype == IB_BF16 && out_dtype == IB_BF16)
         IB_LAUNCH((linear_kernel<bf16, bf16>), grid, 256, 0, (const bf16*)x, (const bf16*)w, bias, residual, (bf16*)out, M, N, K);
     else if (in_dtype == IB_BF16 && out_dtype == IB_F32)
         IB_LAUNCH((linear_kernel<bf16, float>), grid, 256, 0, (const bf16*)x, (const bf16*)w, bias, residual, (float*)out, M, N, K);

@@ -130,8 +130,9 @@ def rmsnorm(x: torch.Tensor, weight: torch.Tensor, eps: float, out_dtype: torch.
 
 def linear_plain(x: torch.Tensor, w: torch.Tensor, bias: Optional[torch.Tensor] = None,
                  residual: Optional[torch.Tensor] = None, out_dtype: Optional[torch.dtype] = None,
-                 out: Optional[torch.Tensor] = None) -> torch.Tensor:
-    """out = x @ w.T (+ bias) (+ residual) with float accumulation in ascending k."""
+                 out: Optional[torch.Tensor] = None, kind: int = 0) -> torch.Tensor:
+    """out = x @ w.T (+ bias) (+ residual) with float accumulation in an order that K alone fixes. kind: which of the
+    float32 kernels (0 = by the sizes; every one gives the same bits)."""
     _check(x, "x")
     _check(w, "w", x.dtype)
     M, K = x.shape
@@ -147,6 +148,10 @@ def linear_plain(x: torch.Tensor, w: torch.Tensor, bias: Optional[torch.Tensor] 
         out = torch.empty((M, N), dtype=out_dtype, device=x.device)
     else:
         _check(out, "out", out_dtype, (M, N))
+    if x.dtype == torch.float32 and out_dtype == torch.float32:
+        f = _fn("lin32", "ib_linear_f32", [c_void_p] * 5 + [c_int64] * 3 + [c_int, c_int, c_void_p])
+        _call(f, x.data_ptr(), w.data_ptr(), _ptr(bias), _ptr(residual), out.data_ptr(), M, N, K, int(kind), 0, _stream())
+        return out
     f = _fn("plain", "ib_linear_plain", [c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_int64, c_int64, c_int64,
                                          c_int, c_int, c_void_p])
     _call(f, x.data_ptr(), w.data_ptr(), _ptr(bias), _ptr(residual), out.data_ptr(), M, N, K,
