@@ -12,7 +12,8 @@ wanted rows) travel to the device in ONE packed int32 buffer and one copy.
 """
 from __future__ import annotations
 
-import os
+import gc
+import time
 from dataclasses import dataclass, field
 from typing import Dict, Hashable, List, Mapping, Optional, Sequence
 
@@ -66,6 +67,7 @@ class StepContext:
     extras: Dict[str, object] = field(default_factory=dict)   # per-step scratch that fast kernels share
     # sampling at the wanted rows inside the step (None: the step returns logits)
     sampling: Optional["SamplingInputs"] = None
+    measured: Optional["_PortionRun"] = None                  # where an eager run of this shape writes down its times
 
 
 @dataclass
@@ -95,16 +97,24 @@ def _round_up(x: int, m: int) -> int:
 
 FEEDBACK_TOKEN = -1           # as a decode entry's token: "what the sampler produced last for this request"
 GRAPH_WIDTH_PAGES = 32        # decode-only block tables are padded to a multiple of this many pages (512 positions)
-GRAPH_WARMUP_STEPS = 2        # eager steps of a shape before its graph is captured
+GRAPH_WARMUP_STEPS = 1        # eager steps of a shape before its graph is captured (libraries, workspaces, attributes)
 MAX_GRAPHS = 48
 GRAPH_COPIES = 2              # executable copies per decode shape, launched in turn
 # Steps that hold prompt portions are captured too when their exact shape (segment lengths, wanted rows, table widths)
 # comes a second time, as it does when prompts are cut into portions of the token budget or a short prompt joins a full
-# batch of decoding requests: the first step of a shape runs eagerly (about 10 microseconds of host time per launch, two
-# hundred launches), the second is captured, later ones are replayed. One executable each; a graph keeps its
-# activations allocated, so only steps of at most PORTION_GRAPH_MAX_TOKENS tokens are captured and the captured shapes
-# together hold at most PORTION_GRAPH_TOKEN_POOL tokens (the oldest goes first).
-PORTION_GRAPH_AFTER = 1
+# batch of decoding requests: the first step of a shape runs eagerly (about 20 microseconds of host time per launch, two
+# hundred launches), the second is captured, later ones are replayed. Only steps whose launches take longer on the host
+# than on the device are captured that early, that is: the eager step's span on the device (two events) is at most
+# PORTION_GRAPH_BOUND times the host's time for its launches. A longer one gains little by a replay (1.5 % for 512 tokens at
+# 7B sizes), and its capture costs: at 1.5B sizes a step of 2,048 tokens takes 7.1 ms on the device and 4.3 on the host, its
+# capture 12; eight such shapes in turn did not fit the pool below and were captured anew each time (eight prompts of 2,048
+# tokens: 96 ms instead of 61). It is captured when it comes for the PORTION_GRAPH_LATERth time, if the pool has room for it
+# without another shape's leaving. One executable each; a
+# graph keeps its activations allocated, so only steps of at most PORTION_GRAPH_MAX_TOKENS tokens are captured and the
+# captured shapes together hold at most PORTION_GRAPH_TOKEN_POOL tokens (the oldest goes first).
+PORTION_GRAPH_BOUND = 1.15
+PORTION_GRAPH_LATER = 5
+PORTION_GRAPH_COLD = 1.5      # an eager run this much slower per launch than the fastest one is measured again
 MAX_PORTION_GRAPHS = 32
 PORTION_GRAPH_MAX_TOKENS = 8192
 PORTION_GRAPH_TOKEN_POOL = 16384
@@ -116,6 +126,21 @@ class _GraphEntry:
         self.pinned, self.flip = None, 0
         self.copied = None                 # per pinned buffer: the event recorded after the copy that read it last
         self.copies = GRAPH_COPIES
+
+
+class _PortionRun:
+    """What is known of a shape with prompt portions: its last eager run's host time, launches and span on the device."""
+
+    def __init__(self):
+        self.begin = torch.cuda.Event(enable_timing=True)
+        self.end = torch.cuda.Event(enable_timing=True)
+        self.host_ms, self.launches, self.worth, self.came = 0.0, 0, None, 0
+
+    def decide(self, ms_per_launch: float) -> bool:
+        """True if the shape is worth a graph; ``worth`` stays None until its run has ended on the device and was a warm one."""
+        if self.worth is None and self.launches and self.end.query() and self.host_ms <= PORTION_GRAPH_COLD * ms_per_launch * self.launches:
+            self.worth = self.begin.elapsed_time(self.end) <= PORTION_GRAPH_BOUND * self.host_ms
+        return bool(self.worth)
 
 
 class Engine:
@@ -156,8 +181,10 @@ class Engine:
         # steps with prompt portions once their exact shape has repeated.
         self.use_graphs = bool(cuda_graphs) and dtype == torch.bfloat16 and self.model.graph_safe()
         self._graphs: Dict[tuple, _GraphEntry] = {}
-        self._portion_seen: Dict[tuple, int] = {}         # how often a shape with prompt portions has come
+        self._portion_runs: Dict[tuple, _PortionRun] = {}
+        self._ms_per_launch = float("inf")                # the fastest eager run's host time per launch
         self._graph_pool = torch.cuda.graph_pool_handle() if self.use_graphs else None
+        self._capture_stream = torch.cuda.Stream(self.rt.device) if self.use_graphs else None
 
     # ------------------------------------------------------------------ construction helpers
 
@@ -286,7 +313,7 @@ class Engine:
                 if temp[i] > 0 and (topk[i] > 0 or topp[i] < 1.0):
                     filtered = True
         mode = 0 if sample is None else (2 if filtered else 1)
-        entry = None
+        entry = run = None
         key = None
         if graphs and T == S:
             key = (S, n_want, tuple(widths), mode)
@@ -295,11 +322,16 @@ class Engine:
             if pkey in self._graphs:
                 key = pkey
             else:
-                if len(self._portion_seen) > 256:
-                    self._portion_seen.clear()
-                seen = self._portion_seen[pkey] = self._portion_seen.get(pkey, 0) + 1
-                if seen > PORTION_GRAPH_AFTER:
+                if len(self._portion_runs) > 256:
+                    self._portion_runs.clear()
+                seen = self._portion_runs.setdefault(pkey, _PortionRun())
+                seen.came += 1
+                held = [sum(k[1]) for k in self._graphs if k[0] == "portions"]
+                if seen.decide(self._ms_per_launch) or (seen.worth is False and seen.came >= PORTION_GRAPH_LATER
+                                                        and len(held) < MAX_PORTION_GRAPHS and sum(held) + T <= PORTION_GRAPH_TOKEN_POOL):
                     key = pkey
+                elif seen.worth is None:
+                    run = seen                                # (a shape that is not worth a graph is not measured again)
         if key is not None:
             entry = self._graphs.get(key)
             if entry is None:
@@ -348,6 +380,7 @@ class Engine:
         if entry is not None:
             # a graph's launch shapes must not depend on the step: bound the context by the table width
             ctx.max_ctx_len = max(widths) * cache.page_size if widths else ctx.max_ctx_len
+        ctx.measured = run
         return ctx, entry
 
     def _run_model(self, ctx: StepContext) -> torch.Tensor:
@@ -361,6 +394,39 @@ class Engine:
             return ops.sample_filtered(logits, sp.temperature, sp.seed, sp.position, sp.top_k, sp.top_p,
                                        self.next_tokens, sp.slot)
         return ops.sample(logits, sp.temperature, sp.seed, sp.position, self.next_tokens, sp.slot)
+
+    def _run_measured(self, ctx: StepContext, run: _PortionRun) -> torch.Tensor:
+        n0, t0 = ops.kernel_launches(), time.perf_counter()
+        run.begin.record()
+        out = self._run_model(ctx)
+        run.end.record()
+        run.host_ms, run.launches = 1e3 * (time.perf_counter() - t0), ops.kernel_launches() - n0
+        self._ms_per_launch = min(self._ms_per_launch, run.host_ms / max(1, run.launches))
+        return out
+
+    def _capture(self, ctx: StepContext):
+        """The step as a CUDA graph: (graph, its output). Capturing only records, so nothing needs to have ended on the
+        device; ``torch.cuda.graph`` waits for it, collects garbage and gives the allocator's free memory back to the
+        driver, which costs milliseconds to hundreds of them. That is the second way, where memory is short."""
+        graph, collecting = torch.cuda.CUDAGraph(), gc.isenabled()
+        gc.disable()                              # (a graph that a collection finds must not be destroyed meanwhile)
+        try:
+            with torch.cuda.stream(self._capture_stream):
+                graph.capture_begin(pool=self._graph_pool)
+                try:
+                    out = self._run_model(ctx)
+                finally:
+                    graph.capture_end()
+            return graph, out
+        except torch.cuda.OutOfMemoryError:
+            pass
+        finally:
+            if collecting:
+                gc.enable()
+        graph = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(graph, pool=self._graph_pool):
+            out = self._run_model(ctx)
+        return graph, out
 
     def step(self, entries: Sequence[StepEntry], sample=None) -> torch.Tensor:
         """Runs one batch; returns float32 logits [wanted places, vocab] on the device. With ``sample`` (one
@@ -422,7 +488,7 @@ class Engine:
             raise
         with torch.cuda.device(self.rt.device):
             if entry is None:
-                out = self._run_model(ctx)
+                out = self._run_model(ctx) if ctx.measured is None else self._run_measured(ctx, ctx.measured)
             elif len(entry.graphs) == entry.copies:
                 # Copies of the graph take turns: launching an executable graph again while its previous launch is
                 # still running is serialised by the driver, which would put the launch cost between two steps.
@@ -435,10 +501,8 @@ class Engine:
                 entry.warm += 1
                 out = self._run_model(ctx)
             else:
-                graph = torch.cuda.CUDAGraph()
                 n0 = ops.kernel_launches()
-                with torch.cuda.graph(graph, pool=self._graph_pool):
-                    out = self._run_model(ctx)
+                graph, out = self._capture(ctx)
                 entry.n_launches = ops.kernel_launches() - n0        # kernels of this package inside the graph
                 ops._LAUNCHES[0] = n0
                 entry.graphs.append((graph, out))
