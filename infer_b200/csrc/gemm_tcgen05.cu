@@ -52,7 +52,7 @@ constexpr int BM = 128;            // tile rows on the A side = TMEM lanes
 constexpr int BK = 64;             // bf16 elements per stage row = one 128-byte swizzle line
 constexpr int UMMA_K = 16;
 constexpr int NUM_THREADS = 192;
-constexpr uint32_t SPIN_LIMIT = 1u << 22;
+constexpr uint32_t WAIT_LIMIT = 1u << 20;
 
 constexpr int STATUS_TIMEOUT_PRODUCER = 101, STATUS_TIMEOUT_MMA = 102, STATUS_TIMEOUT_EPILOGUE = 103;
 
@@ -66,23 +66,31 @@ __device__ __forceinline__ void mbar_init(uint32_t bar, uint32_t count) {
 __device__ __forceinline__ void mbar_expect_tx(uint32_t bar, uint32_t bytes) {
     asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(bytes) : "memory");
 }
-__device__ __forceinline__ bool mbar_test(uint32_t bar, uint32_t parity) {
-    uint32_t ok;
-    asm volatile(
-        "{\n\t.reg .pred p;\n\t"
-        "mbarrier.test_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
-        "selp.u32 %0, 1, 0, p;\n\t}"
-        : "=r"(ok) : "r"(bar), "r"(parity) : "memory");
-    return ok != 0;
-}
-// Bounded wait (non-blocking probes, short sleeps after the first thousand): false if the phase did not complete
-// within the limit, which is of the order of a second.
+// Bounded wait: the thread sleeps in hardware until the phase completes or about a microsecond has passed, again and again
+// (of the order of a second altogether); false if the phase did not complete. Probing in a loop instead kept the shared
+// memory's port busy: with 128 epilogue threads at it a chain of MMAs ran a tenth slower.
 __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity) {
-    for (uint32_t i = 0; i < SPIN_LIMIT; i++) {
-        if (mbar_test(bar, parity)) return true;
-        if (i > 1024) __nanosleep(64);
+    for (uint32_t i = 0; i < WAIT_LIMIT; i++) {
+        uint32_t ok;
+        asm volatile(
+            "{\n\t.reg .pred p;\n\t"
+            "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2, %3;\n\t"
+            "selp.u32 %0, 1, 0, p;\n\t}"
+            : "=r"(ok) : "r"(bar), "r"(parity), "r"(1000u) : "memory");
+        if (ok) return true;
     }
     return false;
+}
+// The same for a whole warp, of which one lane waits.
+__device__ __forceinline__ bool warp_mbar_wait(uint32_t bar, uint32_t parity) {
+    int ok = 1;
+    if ((threadIdx.x & 31) == 0) ok = mbar_wait(bar, parity) ? 1 : 0;
+    return __shfl_sync(0xffffffffu, ok, 0) != 0;
+}
+__device__ __forceinline__ bool elect_one() {
+    uint32_t p;
+    asm volatile("{\n\t.reg .pred P;\n\telect.sync _|P, 0xffffffff;\n\tselp.u32 %0, 1, 0, P;\n\t}" : "=r"(p));
+    return p != 0;
 }
 __device__ __forceinline__ void fence_barrier_init() { asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory"); }
 __device__ __forceinline__ void fence_proxy_async() { asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); }
@@ -378,7 +386,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant__
     volatile uint32_t* slots = reinterpret_cast<volatile uint32_t*>(base_ptr + S * C::STAGE_BYTES + (2 * S + 1) * 8);
     // slots[0] = TMEM base address, slots[1] = abort flag, slots[2] = "this CTA reduces the split-K slices"
 
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int warp = __shfl_sync(0xffffffffu, int(threadIdx.x >> 5), 0), lane = threadIdx.x & 31;    // (uniform, for the compiler too)
     if (threadIdx.x == 0) IB_MT(0);
     // grid (tiles a, tiles b, slices), or with the slices as one cluster: (slices, tiles a, tiles b)
     const int tile_a = p.cluster_split ? blockIdx.y : blockIdx.x, tile_b = p.cluster_split ? blockIdx.z : blockIdx.y;
@@ -505,19 +513,20 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant__
         }
     } else if (warp == 1) {
         // ---------------------------------------------------------------- MMA issuer
-        if (lane == 0) {
-            constexpr uint32_t idesc = make_idesc(BN);
-            int s = 0;
-            uint32_t round = 0;
-            for (int i = 0; i < n_kb; i++, s = (s + 1 == S ? 0 : s + 1), round += (s == 0)) {
-                if (!mbar_wait(full_bar(s), round & 1)) {
-                    atomicExch(p.status, STATUS_TIMEOUT_MMA); slots[1] = 1; break;
-                }
-                tc_fence_after();
-                if (i == 0) IB_MT(5);
-                if (i == n_kb / 2) IB_MT(6);
-                const uint32_t a_addr = base + s * C::STAGE_BYTES, b_addr = a_addr + C::A_BYTES;
-                const uint64_t a_desc = make_desc(a_addr), b_desc = make_desc(b_addr);
+        // The whole warp walks through the loop and one elected lane issues: addresses and descriptors stay in uniform
+        // registers. (Issued from inside a branch of one lane: 64 rows against 17920 x 1536 12.7 us, like this 12.1.)
+        constexpr uint32_t idesc = make_idesc(BN);
+        const bool leader = elect_one();
+        int s = 0;
+        uint32_t parity = 0;
+        bool ok = true;
+        for (int i = 0; i < n_kb; i++) {
+            if (!mbar_wait(full_bar(s), parity)) { ok = false; break; }
+            if (lane == 0 && i == 0) IB_MT(5);
+            if (lane == 0 && i == n_kb / 2) IB_MT(6);
+            const uint32_t a_addr = base + s * C::STAGE_BYTES;
+            const uint64_t a_desc = make_desc(a_addr), b_desc = make_desc(a_addr + C::A_BYTES);
+            if (leader) {
 #pragma unroll
                 for (int k = 0; k < BK / UMMA_K; k++) {
                     // 16 elements along K = 32 bytes = 2 units of the descriptor's 16-byte address field
@@ -525,9 +534,13 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant__
                 }
                 umma_commit(empty_bar(s));
             }
-            umma_commit(tmem_full_bar);
-            IB_MT(7);
+            __syncwarp();
+            if (++s == S) { s = 0; parity ^= 1u; }
         }
+        if (!ok && lane == 0) { atomicExch(p.status, STATUS_TIMEOUT_MMA); slots[1] = 1; }
+        if (leader) umma_commit(tmem_full_bar);
+        __syncwarp();
+        if (lane == 0) IB_MT(7);
         ib::pdl_launch_dependents();
     } else {
         // ---------------------------------------------------------------- epilogue (warps 2..5)
@@ -546,9 +559,8 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant__
                 }
             }
         }
-        bool ok = mbar_wait(tmem_full_bar, 0);
+        const bool ok = warp_mbar_wait(tmem_full_bar, 0);
         if (!ok) { atomicExch(p.status, STATUS_TIMEOUT_EPILOGUE); slots[1] = 1; }
-        ok = __all_sync(0xffffffffu, ok);
         tc_fence_after();
         if (threadIdx.x == 64) IB_MT(8);
         if (ok) {
@@ -777,7 +789,7 @@ gemm_tc_persistent_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid
     const uint32_t bars = base + S * P_STAGE_BYTES;               // full[S], empty[S], acc_full[2], acc_empty[2]
     volatile uint32_t* slots = reinterpret_cast<volatile uint32_t*>(base_ptr + S * P_STAGE_BYTES + (2 * S + 4) * 8);
     // slots[0] = TMEM base address, slots[1] = abort flag
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int warp = __shfl_sync(0xffffffffu, int(threadIdx.x >> 5), 0), lane = threadIdx.x & 31;    // (uniform, for the compiler too)
     int tiles_m = int((p.rows_a + TM - 1) / TM);
     const int tiles_n = GROUPED ? p.g_tiles_n : int((p.rows_b + TN - 1) / TN);
     int n_tiles = tiles_m * tiles_n;
@@ -817,7 +829,8 @@ gemm_tc_persistent_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid
         if (lane == 0) {
             ib::pdl_wait();
             tiles_in_use();
-            int it = 0, issued = 0;
+            int it = 0, issued = 0, s = 0;
+            uint32_t parity = 1;                                  // of the wait for the slot's use before
             const uint64_t once = policy_evict_first();
             for (int tile = blockIdx.x; tile < n_tiles && !slots[1]; tile += gridDim.x) {
                 const int tm = tile % tiles_m, tn = tile / tiles_m;    // neighbouring CTAs share the weight tile
@@ -828,8 +841,7 @@ gemm_tc_persistent_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid
                     b_k = e * p.g_k;
                 }
                 for (int kb = 0; kb < n_kb; kb++, it++) {
-                    const int s = it % S;
-                    if (it >= S && !mbar_wait(empty_bar(s), ((it / S) - 1) & 1)) {
+                    if (it >= S && !mbar_wait(empty_bar(s), parity)) {
                         atomicExch(p.status, STATUS_TIMEOUT_PRODUCER); slots[1] = 1; break;
                     }
                     if (slots[1]) break;
@@ -839,6 +851,7 @@ gemm_tc_persistent_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid
                     if (p.weights_once) tma_load_2d_once(b_dst, &tm_b, full_bar(s), b_k + kb * BK, b_row, once);
                     else tma_load_2d(b_dst, &tm_b, full_bar(s), b_k + kb * BK, b_row);
                     issued = it + 1;
+                    if (++s == S) { s = 0; parity ^= 1u; }
                 }
             }
             if (slots[1]) {
@@ -848,42 +861,38 @@ gemm_tc_persistent_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid
         }
     } else if (warp == 1) {
         // ---------------------------------------------------------------- MMA issuer
-        if (lane == 0) {
-            constexpr uint32_t idesc = make_idesc(TN);
-            int it = 0, lt = 0;
-            if constexpr (GROUPED) ib::pdl_wait();
-            tiles_in_use();
-            for (int tile = blockIdx.x; tile < n_tiles && !slots[1]; tile += gridDim.x, lt++) {
-                const int b = lt & 1;
-                if (lt >= 2 && !mbar_wait(acc_empty_bar(b), ((lt >> 1) - 1) & 1)) {      // the epilogue has drained it
-                    atomicExch(p.status, STATUS_TIMEOUT_MMA); slots[1] = 1; break;
-                }
-                tc_fence_after();
-                const uint32_t d0 = tmem_base + uint32_t(b * 256), d1 = d0 + 128u;
-                for (int kb = 0; kb < n_kb; kb++, it++) {
-                    const int s = it % S;
-                    if (!mbar_wait(full_bar(s), (it / S) & 1)) {
-                        atomicExch(p.status, STATUS_TIMEOUT_MMA); slots[1] = 1; break;
-                    }
-                    tc_fence_after();
-                    const uint32_t a_addr = base + s * P_STAGE_BYTES;
-                    const uint64_t a0 = make_desc(a_addr), a1 = make_desc(a_addr + 128 * BK * 2), bd = make_desc(a_addr + A_BYTES);
+        // (the whole warp walks, one elected lane issues: as in the one-tile kernel)
+        constexpr uint32_t idesc = make_idesc(TN);
+        const bool leader = elect_one();
+        int s = 0, lt = 0;
+        uint32_t parity = 0;
+        bool ok = true;
+        if constexpr (GROUPED) ib::pdl_wait();
+        tiles_in_use();
+        for (int tile = blockIdx.x; tile < n_tiles && ok; tile += gridDim.x, lt++) {
+            const int b = lt & 1;
+            if (lt >= 2 && !mbar_wait(acc_empty_bar(b), ((lt >> 1) - 1) & 1)) { ok = false; break; }      // the epilogue has drained it
+            tc_fence_after();
+            const uint32_t d0 = tmem_base + uint32_t(b * 256), d1 = d0 + 128u;
+            for (int kb = 0; kb < n_kb; kb++) {
+                if (!mbar_wait(full_bar(s), parity)) { ok = false; break; }
+                const uint32_t a_addr = base + s * P_STAGE_BYTES;
+                const uint64_t a0 = make_desc(a_addr), a1 = make_desc(a_addr + 128 * BK * 2), bd = make_desc(a_addr + A_BYTES);
+                if (leader) {
 #pragma unroll
                     for (int k = 0; k < BK / UMMA_K; k++) {
                         const uint32_t acc = (kb > 0 || k > 0) ? 1u : 0u;
-                        if constexpr (WIDE) {
-                            umma_f16(d0, a0 + uint64_t(2 * k), bd + uint64_t(2 * k), idesc, acc);
-                        } else {
-                            umma_f16(d0, a0 + uint64_t(2 * k), bd + uint64_t(2 * k), idesc, acc);
-                            umma_f16(d1, a1 + uint64_t(2 * k), bd + uint64_t(2 * k), idesc, acc);
-                        }
+                        umma_f16(d0, a0 + uint64_t(2 * k), bd + uint64_t(2 * k), idesc, acc);
+                        if constexpr (!WIDE) umma_f16(d1, a1 + uint64_t(2 * k), bd + uint64_t(2 * k), idesc, acc);
                     }
                     umma_commit(empty_bar(s));
+                    if (kb == n_kb - 1) umma_commit(acc_full_bar(b));
                 }
-                if (slots[1]) break;
-                umma_commit(acc_full_bar(b));
+                __syncwarp();
+                if (++s == S) { s = 0; parity ^= 1u; }
             }
         }
+        if (!ok && lane == 0) { atomicExch(p.status, STATUS_TIMEOUT_MMA); slots[1] = 1; }
         ib::pdl_launch_dependents();                     // (unless that happened at the start)
     } else {
         // ---------------------------------------------------------------- epilogue (warps 2..5)
@@ -899,9 +908,8 @@ gemm_tc_persistent_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid
             // the first 64 residual values of this thread's row travel while the tile's last MMAs still run
             ra.on = p.epi == 0 && p.residual != nullptr && (p.N & 7) == 0 && row0 < p.M;
             residual_request<TN>(p, ra, row0, n_base, 0);
-            bool ok = !slots[1] && mbar_wait(acc_full_bar(b), (lt >> 1) & 1);
-            if (!ok && !slots[1]) { atomicExch(p.status, STATUS_TIMEOUT_EPILOGUE); slots[1] = 1; }
-            ok = __all_sync(0xffffffffu, ok);
+            bool ok = __all_sync(0xffffffffu, !slots[1]);
+            if (ok && !warp_mbar_wait(acc_full_bar(b), (lt >> 1) & 1)) { atomicExch(p.status, STATUS_TIMEOUT_EPILOGUE); slots[1] = 1; ok = false; }
             if (!ok) break;
             tc_fence_after();
             const uint32_t taddr = tmem_base + (uint32_t(quad * 32) << 16) + uint32_t(b * 256);
