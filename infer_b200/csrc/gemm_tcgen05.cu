@@ -935,6 +935,181 @@ gemm_tc_persistent_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid
     }
 }
 
+// ------------------------------------------------------------------------------------------------ pairs of SMs
+// The persistent kernel's tiles of 128 x 256 read 48 KB of operands per k-block and SM; at its rate that is 59 bytes a
+// cycle, what the way from L2 to an SM gives, and the tensor cores wait a third of their time (gate/up of a 2,048-token
+// step at 1,536 features: 0.44 us a k-block, its MMAs alone 0.27). Here two SMs (a cluster of two CTAs) work on one tile of
+// 256 tokens x PN features with tcgen05.mma.cta_group::2: each loads 128 token rows and HALF of the features' rows, 32 KB a
+// k-block for PN = 256, and keeps the result rows of its own tokens in its tensor memory.
+//   Both CTAs' producers load their halves; all copies of a stage are counted on the first CTA's barrier, whose MMA warp
+//   issues for both and hands the stage back to both (tcgen05.commit, multicast). Both CTAs' epilogues drain their own
+//   rows; the first CTA's MMA warp waits for all eight epilogue warps before it writes an accumulator again.
+constexpr int PAIR_STAGES = 6, PAIR_STAGE_BYTES = 2 * 128 * BK * 2;
+constexpr int PAIR_SMEM_BYTES = PAIR_STAGES * PAIR_STAGE_BYTES + 1024 + 256;
+
+__device__ __forceinline__ uint32_t cluster_rank() {
+    uint32_t r;
+    asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
+    return r;
+}
+__device__ __forceinline__ void mbar_arrive_cluster(uint32_t remote_bar) {
+    asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(remote_bar) : "memory");
+}
+// A copy into this CTA's shared memory, counted on a barrier of either CTA of the pair.
+__device__ __forceinline__ void tma_load_2d_pair(uint32_t dst, const CUtensorMap* map, uint32_t cluster_bar, int x, int y) {
+    asm volatile(
+        "cp.async.bulk.tensor.2d.cta_group::2.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4}], [%2];"
+        ::"r"(dst), "l"(map), "r"(cluster_bar), "r"(x), "r"(y) : "memory");
+}
+__device__ __forceinline__ void tma_load_2d_pair_once(uint32_t dst, const CUtensorMap* map, uint32_t cluster_bar, int x, int y, uint64_t policy) {
+    asm volatile(
+        "cp.async.bulk.tensor.2d.cta_group::2.shared::cluster.global.mbarrier::complete_tx::bytes.L2::cache_hint [%0], [%1, {%3, %4}], [%2], %5;"
+        ::"r"(dst), "l"(map), "r"(cluster_bar), "r"(x), "r"(y), "l"(policy) : "memory");
+}
+__device__ __forceinline__ void umma_f16_pair(uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc, uint32_t idesc, uint32_t accumulate) {
+    asm volatile(
+        "{\n\t.reg .pred p;\n\t"
+        "setp.ne.b32 p, %4, 0;\n\t"
+        "tcgen05.mma.cta_group::2.kind::f16 [%0], %1, %2, %3, p;\n\t}"
+        ::"r"(d_tmem), "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(accumulate) : "memory");
+}
+// Arrives on the barrier at this place in both CTAs once every MMA issued so far has finished.
+__device__ __forceinline__ void umma_commit_pair(uint32_t bar) {
+    asm volatile("tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;"
+                 ::"r"(bar), "h"(uint16_t(3)) : "memory");
+}
+
+template <int PN, typename TOut>
+__global__ void __launch_bounds__(NUM_THREADS)
+gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant__ CUtensorMap tm_b, const GemmParams p) {
+    static_assert(PN % 32 == 0 && PN >= 32 && PN <= 256, "tile width of a pair");
+    extern __shared__ uint8_t smem_raw[];
+    const uint32_t base = (smem_u32(smem_raw) + 1023u) & ~1023u;
+    uint8_t* base_ptr = smem_raw + (base - smem_u32(smem_raw));
+    constexpr int S = PAIR_STAGES;
+    constexpr int A_BYTES = 128 * BK * 2, B_BYTES = PN / 2 * BK * 2;
+    const uint32_t bars = base + S * PAIR_STAGE_BYTES;            // full[S], empty[S], acc_full[2], acc_empty[2]
+    volatile uint32_t* slots = reinterpret_cast<volatile uint32_t*>(base_ptr + S * PAIR_STAGE_BYTES + (2 * S + 4) * 8);
+    // slots[0] = TMEM base address, slots[1] = abort flag (of this CTA)
+    const int warp = __shfl_sync(0xffffffffu, int(threadIdx.x >> 5), 0), lane = threadIdx.x & 31;
+    const uint32_t rank = cluster_rank();
+    const int pair = blockIdx.x >> 1, pairs = gridDim.x >> 1;
+    const int tiles_m = int((p.rows_a + 255) / 256), tiles_n = int((p.rows_b + PN - 1) / PN), n_tiles = tiles_m * tiles_n;
+    const int n_kb = p.kb_total;
+    auto full_bar = [&](int s) { return bars + 8u * s; };
+    auto empty_bar = [&](int s) { return bars + 8u * (S + s); };
+    auto acc_full_bar = [&](int b) { return bars + 8u * (2 * S + b); };
+    auto acc_empty_bar = [&](int b) { return bars + 8u * (2 * S + 2 + b); };
+
+    if (threadIdx.x == 0) {
+        for (int s = 0; s < S; s++) { mbar_init(full_bar(s), 1); mbar_init(empty_bar(s), 1); }
+        for (int b = 0; b < 2; b++) { mbar_init(acc_full_bar(b), 1); mbar_init(acc_empty_bar(b), 8); }
+        slots[1] = 0;
+        fence_barrier_init();
+        prefetch_tensormap(&tm_a);
+        prefetch_tensormap(&tm_b);
+    }
+    if (warp == 1) {
+        asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;"
+                     ::"r"(smem_u32(const_cast<uint32_t*>(&slots[0]))), "r"(uint32_t(P_TMEM_COLS)) : "memory");
+        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;" ::: "memory");
+    }
+    tc_fence_before();
+    __syncthreads();
+    cluster_sync();                                               // the other CTA's barriers are initialised
+    tc_fence_after();
+    const uint32_t tmem_base = slots[0];
+
+    if (warp == 0) {
+        // ---------------------------------------------------------------- TMA producer (of each CTA)
+        if (p.early_release && lane != 0) ib::pdl_launch_dependents();
+        if (lane == 0) {
+            ib::pdl_wait();
+            int it = 0, s = 0;
+            uint32_t parity = 1;                                  // of the wait for the slot's use before
+            const uint64_t once = policy_evict_first();
+            for (int tile = pair; tile < n_tiles && !slots[1]; tile += pairs) {
+                const int a_row = (tile % tiles_m) * 256 + int(rank) * 128, b_row = (tile / tiles_m) * PN + int(rank) * (PN / 2);
+                for (int kb = 0; kb < n_kb; kb++, it++) {
+                    if (it >= S && !mbar_wait(empty_bar(s), parity)) {
+                        atomicExch(p.status, STATUS_TIMEOUT_PRODUCER); slots[1] = 1; break;
+                    }
+                    if (slots[1]) break;
+                    const uint32_t a_dst = base + s * PAIR_STAGE_BYTES, b_dst = a_dst + A_BYTES;
+                    const uint32_t bar = map_cluster(full_bar(s), 0u);
+                    if (rank == 0) mbar_expect_tx(full_bar(s), 2 * (A_BYTES + B_BYTES));
+                    tma_load_2d_pair(a_dst, &tm_a, bar, kb * BK, a_row);
+                    if (p.weights_once) tma_load_2d_pair_once(b_dst, &tm_b, bar, kb * BK, b_row, once);
+                    else tma_load_2d_pair(b_dst, &tm_b, bar, kb * BK, b_row);
+                    if (++s == S) { s = 0; parity ^= 1u; }
+                }
+            }
+            // No copy may land after the CTA is gone: the first CTA waits for every stage it was told of. (Without a failure
+            // the MMAs, which waited for them, have ended before the cluster's last barrier below.)
+            if (slots[1] && rank == 0)
+                for (int i = it > S ? it - S : 0; i < it; i++) mbar_wait(full_bar(i % S), (i / S) & 1);
+        }
+    } else if (warp == 1) {
+        if (rank == 0) {
+            // ---------------------------------------------------------------- MMA issuer (of the pair)
+            constexpr uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | (uint32_t(PN >> 3) << 17) | (uint32_t(256 >> 4) << 24);
+            const bool leader = elect_one();
+            int s = 0, lt = 0;
+            uint32_t parity = 0;
+            bool ok = true;
+            for (int tile = pair; tile < n_tiles && ok; tile += pairs, lt++) {
+                const int b = lt & 1;
+                if (lt >= 2 && !mbar_wait(acc_empty_bar(b), ((lt >> 1) - 1) & 1)) { ok = false; break; }      // both epilogues have drained it
+                tc_fence_after();
+                const uint32_t d = tmem_base + uint32_t(b * 256);
+                for (int kb = 0; kb < n_kb; kb++) {
+                    if (!mbar_wait(full_bar(s), parity)) { ok = false; break; }
+                    const uint32_t a_addr = base + s * PAIR_STAGE_BYTES;
+                    const uint64_t ad = make_desc(a_addr), bd = make_desc(a_addr + A_BYTES);
+                    if (leader) {
+#pragma unroll
+                        for (int k = 0; k < BK / UMMA_K; k++)
+                            umma_f16_pair(d, ad + uint64_t(2 * k), bd + uint64_t(2 * k), idesc, (kb > 0 || k > 0) ? 1u : 0u);
+                        umma_commit_pair(empty_bar(s));
+                        if (kb == n_kb - 1) umma_commit_pair(acc_full_bar(b));
+                    }
+                    __syncwarp();
+                    if (++s == S) { s = 0; parity ^= 1u; }
+                }
+            }
+            if (!ok && lane == 0) { atomicExch(p.status, STATUS_TIMEOUT_MMA); slots[1] = 1; }
+        }
+        ib::pdl_launch_dependents();                     // (unless that happened at the start)
+    } else {
+        // ---------------------------------------------------------------- epilogue (warps 2..5 of each CTA, its 128 rows)
+        const int quad = warp & 3;
+        ib::pdl_wait();
+        int lt = 0;
+        ResidualAhead ra;
+        for (int tile = pair; tile < n_tiles; tile += pairs, lt++) {
+            const int b = lt & 1;
+            const int64_t row = int64_t(tile % tiles_m) * 256 + int(rank) * 128 + quad * 32 + lane, n_base = int64_t(tile / tiles_m) * PN;
+            ra.on = p.epi == 0 && p.residual != nullptr && (p.N & 7) == 0 && row < p.M;
+            residual_request<PN>(p, ra, row, n_base, 0);
+            bool ok = __all_sync(0xffffffffu, !slots[1]);
+            if (ok && !warp_mbar_wait(acc_full_bar(b), (lt >> 1) & 1)) { atomicExch(p.status, STATUS_TIMEOUT_EPILOGUE); slots[1] = 1; ok = false; }
+            if (!ok) break;
+            tc_fence_after();
+            drain_row<TOut, PN>(p, tmem_base + (uint32_t(quad * 32) << 16) + uint32_t(b * 256), row, n_base, ra);
+            tc_fence_before();
+            __syncwarp();
+            if (lane == 0) mbar_arrive_cluster(map_cluster(acc_empty_bar(b), 0u));
+        }
+    }
+    tc_fence_before();
+    __syncthreads();
+    cluster_sync();                                      // neither CTA's shared memory is needed by the other any more
+    if (warp == 1) {
+        tc_fence_after();
+        asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(uint32_t(P_TMEM_COLS)) : "memory");
+    }
+}
+
 // ------------------------------------------------------------------------------------------------ host side
 
 using ib::get_map;
@@ -953,6 +1128,31 @@ int launch(const CUtensorMap& ma, const CUtensorMap& mb, const GemmParams& p, di
     if (smem > size_t(C::SMEM_BYTES)) return ib::fail(IB_ERR_ARG, "gemm_tc: %d stages and the receive area do not fit", p.stages);
     return ib::launch("gemm_tc", gemm_tc_kernel<BN, TOut>, grid, dim3(NUM_THREADS), smem, stream,
                       p.cluster_split ? unsigned(p.splits) : 1u, ma, mb, p);
+}
+
+// CTAs of the pair kernel that run at once: as many clusters of two as the device places, at most one CTA per SM.
+template <int PN, typename TOut>
+int launch_pair(const CUtensorMap& ma, const CUtensorMap& mb, const GemmParams& p, int sm_count, cudaStream_t stream) {
+    static int room = 0;
+    if (!room) {
+        cudaError_t e = cudaFuncSetAttribute(gemm_tc_pair_kernel<PN, TOut>, cudaFuncAttributeMaxDynamicSharedMemorySize, PAIR_SMEM_BYTES);
+        cudaLaunchConfig_t cfg = {};
+        cfg.gridDim = dim3(unsigned(sm_count & ~1));
+        cfg.blockDim = dim3(NUM_THREADS);
+        cfg.dynamicSmemBytes = PAIR_SMEM_BYTES;
+        cudaLaunchAttribute attr;
+        attr.id = cudaLaunchAttributeClusterDimension;
+        attr.val.clusterDim.x = 2; attr.val.clusterDim.y = 1; attr.val.clusterDim.z = 1;
+        cfg.attrs = &attr;
+        cfg.numAttrs = 1;
+        int clusters = 0;
+        if (e == cudaSuccess) e = cudaOccupancyMaxActiveClusters(&clusters, gemm_tc_pair_kernel<PN, TOut>, &cfg);
+        if (e != cudaSuccess || clusters < 1) return ib::fail(IB_ERR_CUDA, "gemm_tc: no room for a pair of CTAs: %s", cudaGetErrorString(e));
+        room = clusters < sm_count / 2 ? clusters : sm_count / 2;
+    }
+    const int64_t tiles = ((p.rows_a + 255) / 256) * ((p.rows_b + PN - 1) / PN);
+    const unsigned ctas = 2u * unsigned(tiles < room ? tiles : room);
+    return ib::launch("gemm_tc_pair", gemm_tc_pair_kernel<PN, TOut>, dim3(ctas), dim3(NUM_THREADS), size_t(PAIR_SMEM_BYTES), stream, 2u, ma, mb, p);
 }
 
 template <int PBN, bool WIDE, typename TOut>
@@ -1099,8 +1299,8 @@ IB_EXPORT int ib_gemm_tc(const void* x, const void* w, const float* bias, const 
     if (M <= 0 || N <= 0) return IB_OK;
     if (K <= 0 || K % 8) return ib::fail(IB_ERR_ARG, "gemm_tc: K = %lld must be a positive multiple of 8", (long long)K);
     if ((uintptr_t(x) & 15) || (uintptr_t(w) & 15)) return ib::fail(IB_ERR_ARG, "gemm_tc: operand bases must be 16-byte aligned");
-    if (bn != 16 && bn != 32 && bn != 64 && bn != 128 && bn != 256 && bn != 352 && bn != 384 && bn != 512 && bn != 768)
-        return ib::fail(IB_ERR_ARG, "gemm_tc: bn must be 16, 32, 64, 128, or 256 (the persistent kernel on 256 x 128 tiles), 352, 384, 512 (on 128 x 176, 128 x 192, 128 x 256 with one MMA per k-step) or 768 (one 128 x 256 tile per CTA, K slices as a cluster)");
+    if (bn != 16 && bn != 32 && bn != 64 && bn != 128 && bn != 256 && bn != 352 && bn != 384 && bn != 512 && bn != 768 && !(bn >= 1280 && bn <= 1536 && bn % 64 == 0))
+        return ib::fail(IB_ERR_ARG, "gemm_tc: bn must be 16, 32, 64, 128, or 256 (the persistent kernel on 256 x 128 tiles), 352, 384, 512 (on 128 x 176, 128 x 192, 128 x 256 with one MMA per k-step), 768 (one 128 x 256 tile per CTA, K slices as a cluster) or 1024 + 2 x width (pairs of SMs on tiles of 256 x 128, 160, 192, 224, 256)");
     const bool sliced_wide = bn == 768;
     if (sliced_wide) {
         if (swap || workspace || (splits != 2 && splits != 4 && splits != 8)) return ib::fail(IB_ERR_ARG, "gemm_tc: 128 x 256 tiles with K slices take the plain mapping, 2, 4 or 8 slices and no workspace");
@@ -1136,10 +1336,11 @@ IB_EXPORT int ib_gemm_tc(const void* x, const void* w, const float* bias, const 
     if (!f32 && out_dtype != IB_BF16) return ib::fail(IB_ERR_ARG, "gemm_tc: unknown output dtype %d", out_dtype);
     CUtensorMap ma, mb;
     if (bn >= 256 && !sliced_wide) {
-        const bool wide = bn >= 352 && bn <= 512;
-        int rc = get_map(x, p.rows_a, K, wide ? 128 : PBM, &ma);
+        const bool wide = bn >= 352 && bn <= 512, paired = bn >= 1280;
+        const int width = paired ? (bn - 1024) / 2 : wide ? bn / 2 : 128;
+        int rc = get_map(x, p.rows_a, K, wide || paired ? 128 : PBM, &ma);
         if (rc) return rc;
-        rc = get_map(w, p.rows_b, K, wide ? bn / 2 : 128, &mb);
+        rc = get_map(w, p.rows_b, K, paired ? width / 2 : width, &mb);
         if (rc) return rc;
         static int sms = 0;
         if (!sms) {
@@ -1151,10 +1352,13 @@ IB_EXPORT int ib_gemm_tc(const void* x, const void* w, const float* bias, const 
         p.weights_once = N * K * 2 <= (64LL << 20) ? 1 : 0;
         {
             // k-blocks a CTA goes through: up to about 300 (120 us) the successor is released at once
-            const int64_t tm_rows = wide ? 128 : PBM, tn_cols = wide ? bn / 2 : 128;
-            const int64_t n_tiles = ((M + tm_rows - 1) / tm_rows) * ((N + tn_cols - 1) / tn_cols);
-            p.early_release = ((n_tiles + sms - 1) / sms) * p.kb_total * (wide ? 1 : 2) <= 300 ? 1 : 0;
+            const int64_t tm_rows = wide ? 128 : PBM, walkers = paired ? sms / 2 : sms;
+            const int64_t n_tiles = ((M + tm_rows - 1) / tm_rows) * ((N + width - 1) / width);
+            p.early_release = ((n_tiles + walkers - 1) / walkers) * p.kb_total * (wide || paired ? 1 : 2) <= 300 ? 1 : 0;
         }
+#define IB_PAIR(WW) if (width == WW) return f32 ? launch_pair<WW, float>(ma, mb, p, sms, stream) : launch_pair<WW, bf16>(ma, mb, p, sms, stream)
+        if (paired) { IB_PAIR(256); IB_PAIR(224); IB_PAIR(192); IB_PAIR(160); IB_PAIR(128); }
+#undef IB_PAIR
         if (bn == 512) return f32 ? launch_persistent<256, true, float>(ma, mb, p, sms, stream) : launch_persistent<256, true, bf16>(ma, mb, p, sms, stream);
         if (bn == 384) return f32 ? launch_persistent<192, true, float>(ma, mb, p, sms, stream) : launch_persistent<192, true, bf16>(ma, mb, p, sms, stream);
         if (bn == 352) return f32 ? launch_persistent<176, true, float>(ma, mb, p, sms, stream) : launch_persistent<176, true, bf16>(ma, mb, p, sms, stream);
