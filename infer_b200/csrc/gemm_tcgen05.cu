@@ -944,8 +944,12 @@ gemm_tc_persistent_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid
 //   Both CTAs' producers load their halves; all copies of a stage are counted on the first CTA's barrier, whose MMA warp
 //   issues for both and hands the stage back to both (tcgen05.commit, multicast). Both CTAs' epilogues drain their own
 //   rows; the first CTA's MMA warp waits for all eight epilogue warps before it writes an accumulator again.
-constexpr int PAIR_STAGES = 6, PAIR_STAGE_BYTES = 2 * 128 * BK * 2;
-constexpr int PAIR_SMEM_BYTES = PAIR_STAGES * PAIR_STAGE_BYTES + 1024 + 256;
+//   A stage holds two k-blocks: with one, the producer's round (wait, count, copies) took longer than the copies for narrow
+//   tiles (512 rows, 3,584 features, K = 18944: widths 128, 192 and 256 94.3, 95.9 and 102.9 us; with two 84.0, 93.8, 105.6).
+template <int PN> struct PairCfg {
+    static constexpr int A_BYTES = 128 * BK * 2, B_BYTES = PN / 2 * BK * 2, STAGE_BYTES = 2 * (A_BYTES + B_BYTES);
+    static constexpr int STAGES = PN <= 192 ? 4 : 3, SMEM_BYTES = STAGES * STAGE_BYTES + 1024 + 256;
+};
 
 __device__ __forceinline__ uint32_t cluster_rank() {
     uint32_t r;
@@ -986,10 +990,10 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_const
     extern __shared__ uint8_t smem_raw[];
     const uint32_t base = (smem_u32(smem_raw) + 1023u) & ~1023u;
     uint8_t* base_ptr = smem_raw + (base - smem_u32(smem_raw));
-    constexpr int S = PAIR_STAGES;
-    constexpr int A_BYTES = 128 * BK * 2, B_BYTES = PN / 2 * BK * 2;
-    const uint32_t bars = base + S * PAIR_STAGE_BYTES;            // full[S], empty[S], acc_full[2], acc_empty[2]
-    volatile uint32_t* slots = reinterpret_cast<volatile uint32_t*>(base_ptr + S * PAIR_STAGE_BYTES + (2 * S + 4) * 8);
+    using C = PairCfg<PN>;
+    constexpr int S = C::STAGES, A_BYTES = C::A_BYTES, B_BYTES = C::B_BYTES;
+    const uint32_t bars = base + S * C::STAGE_BYTES;            // full[S], empty[S], acc_full[2], acc_empty[2]
+    volatile uint32_t* slots = reinterpret_cast<volatile uint32_t*>(base_ptr + S * C::STAGE_BYTES + (2 * S + 4) * 8);
     // slots[0] = TMEM base address, slots[1] = abort flag (of this CTA)
     const int warp = __shfl_sync(0xffffffffu, int(threadIdx.x >> 5), 0), lane = threadIdx.x & 31;
     const uint32_t rank = cluster_rank();
@@ -1030,17 +1034,23 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_const
             const uint64_t once = policy_evict_first();
             for (int tile = pair; tile < n_tiles && !slots[1]; tile += pairs) {
                 const int a_row = (tile % tiles_m) * 256 + int(rank) * 128, b_row = (tile / tiles_m) * PN + int(rank) * (PN / 2);
-                for (int kb = 0; kb < n_kb; kb++, it++) {
+                for (int kb = 0; kb < n_kb; kb += 2, it++) {
+                    const int n = min(2, n_kb - kb);
                     if (it >= S && !mbar_wait(empty_bar(s), parity)) {
                         atomicExch(p.status, STATUS_TIMEOUT_PRODUCER); slots[1] = 1; break;
                     }
                     if (slots[1]) break;
-                    const uint32_t a_dst = base + s * PAIR_STAGE_BYTES, b_dst = a_dst + A_BYTES;
+                    const uint32_t a_dst = base + s * C::STAGE_BYTES, b_dst = a_dst + 2 * A_BYTES;
                     const uint32_t bar = map_cluster(full_bar(s), 0u);
-                    if (rank == 0) mbar_expect_tx(full_bar(s), 2 * (A_BYTES + B_BYTES));
-                    tma_load_2d_pair(a_dst, &tm_a, bar, kb * BK, a_row);
-                    if (p.weights_once) tma_load_2d_pair_once(b_dst, &tm_b, bar, kb * BK, b_row, once);
-                    else tma_load_2d_pair(b_dst, &tm_b, bar, kb * BK, b_row);
+                    if (rank == 0) mbar_expect_tx(full_bar(s), 2 * n * (A_BYTES + B_BYTES));
+#pragma unroll
+                    for (int j = 0; j < 2; j++) {
+                        if (j < n) {
+                            tma_load_2d_pair(a_dst + j * A_BYTES, &tm_a, bar, (kb + j) * BK, a_row);
+                            if (p.weights_once) tma_load_2d_pair_once(b_dst + j * B_BYTES, &tm_b, bar, (kb + j) * BK, b_row, once);
+                            else tma_load_2d_pair(b_dst + j * B_BYTES, &tm_b, bar, (kb + j) * BK, b_row);
+                        }
+                    }
                     if (++s == S) { s = 0; parity ^= 1u; }
                 }
             }
@@ -1062,16 +1072,21 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_const
                 if (lt >= 2 && !mbar_wait(acc_empty_bar(b), ((lt >> 1) - 1) & 1)) { ok = false; break; }      // both epilogues have drained it
                 tc_fence_after();
                 const uint32_t d = tmem_base + uint32_t(b * 256);
-                for (int kb = 0; kb < n_kb; kb++) {
+                for (int kb = 0; kb < n_kb; kb += 2) {
                     if (!mbar_wait(full_bar(s), parity)) { ok = false; break; }
-                    const uint32_t a_addr = base + s * PAIR_STAGE_BYTES;
-                    const uint64_t ad = make_desc(a_addr), bd = make_desc(a_addr + A_BYTES);
+                    const uint32_t a_addr = base + s * C::STAGE_BYTES;
+                    const uint64_t ad = make_desc(a_addr), bd = make_desc(a_addr + 2 * A_BYTES);
                     if (leader) {
 #pragma unroll
                         for (int k = 0; k < BK / UMMA_K; k++)
                             umma_f16_pair(d, ad + uint64_t(2 * k), bd + uint64_t(2 * k), idesc, (kb > 0 || k > 0) ? 1u : 0u);
+                        if (kb + 1 < n_kb) {
+#pragma unroll
+                            for (int k = 0; k < BK / UMMA_K; k++)
+                                umma_f16_pair(d, ad + uint64_t((A_BYTES >> 4) + 2 * k), bd + uint64_t((B_BYTES >> 4) + 2 * k), idesc, 1u);
+                        }
                         umma_commit_pair(empty_bar(s));
-                        if (kb == n_kb - 1) umma_commit_pair(acc_full_bar(b));
+                        if (kb + 2 >= n_kb) umma_commit_pair(acc_full_bar(b));
                     }
                     __syncwarp();
                     if (++s == S) { s = 0; parity ^= 1u; }
@@ -1135,11 +1150,11 @@ template <int PN, typename TOut>
 int launch_pair(const CUtensorMap& ma, const CUtensorMap& mb, const GemmParams& p, int sm_count, cudaStream_t stream) {
     static int room = 0;
     if (!room) {
-        cudaError_t e = cudaFuncSetAttribute(gemm_tc_pair_kernel<PN, TOut>, cudaFuncAttributeMaxDynamicSharedMemorySize, PAIR_SMEM_BYTES);
+        cudaError_t e = cudaFuncSetAttribute(gemm_tc_pair_kernel<PN, TOut>, cudaFuncAttributeMaxDynamicSharedMemorySize, PairCfg<PN>::SMEM_BYTES);
         cudaLaunchConfig_t cfg = {};
         cfg.gridDim = dim3(unsigned(sm_count & ~1));
         cfg.blockDim = dim3(NUM_THREADS);
-        cfg.dynamicSmemBytes = PAIR_SMEM_BYTES;
+        cfg.dynamicSmemBytes = PairCfg<PN>::SMEM_BYTES;
         cudaLaunchAttribute attr;
         attr.id = cudaLaunchAttributeClusterDimension;
         attr.val.clusterDim.x = 2; attr.val.clusterDim.y = 1; attr.val.clusterDim.z = 1;
@@ -1152,7 +1167,7 @@ int launch_pair(const CUtensorMap& ma, const CUtensorMap& mb, const GemmParams& 
     }
     const int64_t tiles = ((p.rows_a + 255) / 256) * ((p.rows_b + PN - 1) / PN);
     const unsigned ctas = 2u * unsigned(tiles < room ? tiles : room);
-    return ib::launch("gemm_tc_pair", gemm_tc_pair_kernel<PN, TOut>, dim3(ctas), dim3(NUM_THREADS), size_t(PAIR_SMEM_BYTES), stream, 2u, ma, mb, p);
+    return ib::launch("gemm_tc_pair", gemm_tc_pair_kernel<PN, TOut>, dim3(ctas), dim3(NUM_THREADS), size_t(PairCfg<PN>::SMEM_BYTES), stream, 2u, ma, mb, p);
 }
 
 template <int PBN, bool WIDE, typename TOut>
@@ -1282,6 +1297,34 @@ IB_EXPORT int ib_gemm_tc_plan(int64_t M, int64_t N, int64_t K, int sm_count, int
             }
             if (sliced * 23 < other * 20) { *bn = 768; s = slices; *splits = s; cluster = true; }
         }
+    }
+    // Pairs of SMs on tiles of 256 rows (codes 1024 + 2 x width), where the same kind of model says so. In the unit above a
+    // k-block takes a pair 0.50 + width / 655 (0.264 us at width 128, 0.338 at 256) and an SM by itself 0.74 + width / 790 (0.364 at
+    // 176, 0.403 at 256: the way from L2 is the bound, and a pair's tile takes a third less through it), beside 20 units a launch
+    // for the pairs, 16 alone. Measured against the choices above at 2,048 rows: gate/up 78 and 86 us, down 49 and 56 at 1,536
+    // features, 363 and 395, 213 and 258 (or 306) at 3,584; one round of short tiles (2048 features, K = 1536: 14.1 and 13.8) stays.
+    static const bool pairs_on = [] { const char* e = getenv("INFER_B200_GEMM_PAIRS"); return !(e && e[0] == '0'); }();
+    if (!*swap && pairs_on && sm_count >= 2) {
+        auto unit = [](int64_t rounds, int64_t kb, int64_t at0, int64_t slope, int64_t width) { return rounds * kb * (at0 + 100 * width / slope); };
+        int64_t now;                                              // in hundredths of a unit
+        if (*bn == 768) now = 100 * (int64_t(kb_total + s - 1) / s) + (s == 8 ? 4000 : 3400);
+        else if (*bn >= 256) {
+            const int64_t width = *bn == 256 ? 256 : *bn / 2, tm = *bn == 256 ? (M + 255) / 256 : (M + 127) / 128;
+            const int64_t t = tm * ((N + (*bn == 256 ? 128 : width) - 1) / (*bn == 256 ? 128 : width));
+            now = unit((t + sm_count - 1) / sm_count, kb_total, 74, 790, width) + 1600;
+        } else {
+            const int64_t ctas = tiles * s, cap = cluster ? (s == 2 ? sm_count - 4 : sm_count - sm_count / 7) : 2 * int64_t(sm_count);
+            now = ((ctas + cap - 1) / cap) * 100 * (int64_t(kb_total + s - 1) / s) + 2000;
+        }
+        const int64_t tm = (M + 255) / 256, pairs = sm_count / 2;
+        int64_t best = -1;
+        int width = 0;
+        for (int w : {256, 224, 192, 160, 128}) {
+            const int64_t t = tm * ((N + w - 1) / w);
+            const int64_t est = unit((t + pairs - 1) / pairs, kb_total, 50, 655, w) + 2000;
+            if (best < 0 || est < best) { best = est; width = w; }
+        }
+        if (best * 100 < now * 98) { *bn = 1024 + 2 * width; s = 1; *splits = 1; cluster = false; }
     }
     *workspace_floats = (s > 1 && !*swap && !cluster) ? int64_t(s) * tiles * BM * (*bn) : 0;
     *n_counters = (s > 1 && !*swap && !cluster) ? tiles : 0;
