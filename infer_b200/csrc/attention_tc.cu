@@ -3,14 +3,14 @@
 // -DIB_HEAD_DIM=64 or 128. Pages hold 16 positions; a (page, kv head) block of the cache is 16 rows of head_dim.
 //
 // One CTA (192 threads) serves 128 consecutive queries of one head of one segment and walks over its keys in tiles
-// of 128 (8 pages), aligned to absolute multiples of 128:
+// of 64 (4 pages; 128 in the second form, below), aligned to absolute multiples of that:
 //   warp 0      lane i issues the TMA loads of page i of a tile (a box of 16 positions x 64 elements per page and half
-//               of the head), each into its place of a 128-byte-swizzled operand tile; the page ids of the CTA's key
-//               range sit in shared memory. K and V tiles are double-buffered: tile j + 2 is requested as soon as the
+//               of the head), each into its place of a 128-byte-swizzled operand tile; the page ids are read a tile
+//               ahead. K and V tiles are double-buffered: tile j + 2 is requested as soon as the
 //               MMA that read tile j has finished;
-//   warp 1      allocates tensor memory; one lane issues S(j) = Q K(j)^T (M=128 queries, N=128 keys, K over the head)
+//   warp 1      allocates tensor memory; one lane issues S(j) = Q K(j)^T (M=128 queries, N=64 keys, K over the head)
 //               two tiles ahead into one of two S buffers, and, when the probabilities of tile j are in shared memory,
-//               O += P(j) V(j) (N = head size, K = 128 keys; V is the operand whose contiguous dimension is N,
+//               O += P(j) V(j) (N = head size, K = 64 keys; V is the operand whose contiguous dimension is N,
 //               "MN-major": it is used as the cache stores it);
 //   warps 2-5   thread r owns query row r: reads its row of S from tensor memory, masks on the diagonal and at the
 //               window's edge (select, never arithmetic: unwritten cache rows may hold anything), keeps the running
@@ -27,10 +27,13 @@
 // in a workspace, and the one that arrives last at the tile's counter adds the parts in index order and writes the
 // output (the host shares only while all CTAs still run at once: a CTA's start and end cost about three key tiles).
 //
-// One CTA per SM (193 KB of shared memory, all 512 tensor-memory columns). Query tiles start heaviest first. Measured
-// at 2,048 tokens, 12/2 heads of 128: 38 us against 88 us for the mma.sync kernel. A key tile takes about 3,700 cycles,
-// the softmax thread's own sequence (wait for S, read it, maximum, 128 exponentials, wait for the previous P V, store P):
-// neither two threads per row nor a second MMA-issuing thread shortened it.
+// A key tile's time is the softmax thread's own sequence (wait for S, read it, maximum, exponentials, wait for the previous
+// P V, store P): neither two threads per row nor a second MMA-issuing thread shortened it, and with one CTA an SM the tensor
+// cores wait meanwhile. So two CTAs share an SM (112 KB of shared memory and half of the tensor memory each), which is what
+// tiles of 64 keys are for. One CTA alone walks faster in tiles of 128 (-DIB_ATTN_BN=128; 2.3 us against 3.2 per 128 keys):
+// where few long query tiles all run at once, the host takes that form. Measured, 128 -> 64 keys, heads of 128: 12 heads,
+// ten segments of 200 tokens 21.4 -> 12.5 us, 4,096 tokens behind 11,777 687 -> 635; 28 heads, 2,048 tokens 77.5 -> 62.3, 4,096
+// behind 11,777 1,593 -> 1,265 (644 TFLOP/s). Query tiles start heaviest first.
 // Every mbarrier wait is bounded; one that runs out raises the status word, and the CTA drains its copies,
 // frees its tensor memory and returns.
 #include <algorithm>
@@ -54,20 +57,19 @@ static_assert(HD == 64 || HD == 128, "the tensor-memory attention kernel takes h
 constexpr int DB = HD / 64;                 // 64-element (128-byte) blocks of the head dimension
 constexpr int PAGE = 16;
 #ifndef IB_ATTN_BN
-#define IB_ATTN_BN 128
+#define IB_ATTN_BN 64
 #endif
-constexpr int BM = 128, BN = IB_ATTN_BN;    // queries per CTA, keys per tile (64 or 128)
+constexpr int BM = 128, BN = IB_ATTN_BN;    // queries per CTA; keys per tile: 64 (two CTAs an SM) or 128 (one, for few long query tiles)
 static_assert(BN == 64 || BN == 128, "key tiles of 64 or 128");
 constexpr int PB = BN / 64;                 // 64-key (128-byte) blocks of a row of P
 constexpr int PAGES_PER_TILE = BN / PAGE;
 constexpr int NUM_THREADS = 192;
 constexpr float LOG2E = 1.4426950408889634f;
 constexpr float RESCALE_STEP = 8.0f;        // O's reference maximum follows the running maximum in steps of this (log2)
-constexpr int STATUS_TIMEOUT = 106, STATUS_BAD_PAGE = 3;
-constexpr int TAB_MAX = 2048;               // page ids kept in shared memory: 32,768 positions
+constexpr int STATUS_TIMEOUT = 106, STATUS_ALIGNMENT = 108, STATUS_BAD_PAGE = 3;
 
 constexpr int Q_BYTES = DB * BM * 128, K_BYTES = DB * BN * 128, V_BYTES = DB * BN * 128, P_BYTES = PB * BM * 128;
-constexpr int SMEM_BYTES = Q_BYTES + 2 * K_BYTES + 2 * V_BYTES + P_BYTES + 1024 /*alignment*/ + 128 /*barriers*/;
+constexpr int SMEM_BYTES = Q_BYTES + 2 * K_BYTES + 2 * V_BYTES + P_BYTES + 128 /*barriers*/;
 constexpr int TMEM_COLS = (2 * BN + HD) > 256 ? 512 : ((2 * BN + HD) > 128 ? 256 : 128);
 constexpr int S_COL = 0, O_COL = 2 * BN;    // two S tiles of BN columns each, then O's HD columns
 
@@ -117,12 +119,18 @@ constexpr int MAX_SPLIT = 4;
 constexpr int PART_MIN_TILES = 4;
 constexpr int PART_FLOATS = BM * HD + 2 * BM;   // O as [HD][BM] (a warp's rows side by side), then the maxima, then the sums
 
-__global__ void __launch_bounds__(NUM_THREADS)
+__global__ void __launch_bounds__(NUM_THREADS, BN == 64 ? 2 : 1)
 attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUtensorMap tm_k,
                        const __grid_constant__ CUtensorMap tm_v, const Params p) {
-    extern __shared__ uint8_t smem_raw[];
-    const uint32_t base = (smem_u32(smem_raw) + 1023u) & ~1023u;
-    uint8_t* base_ptr = smem_raw + (base - smem_u32(smem_raw));
+    // The swizzled tiles start on 1024-byte boundaries. The array is the kernel's only shared memory and starts on one; room
+    // to round its start up would keep the second CTA off the SM.
+    extern __shared__ __align__(1024) uint8_t smem_raw[];
+    const uint32_t base = smem_u32(smem_raw);
+    uint8_t* base_ptr = smem_raw;
+    if (base & 1023u) {
+        if (threadIdx.x == 0) atomicExch(p.status, STATUS_ALIGNMENT);
+        return;
+    }
     const uint32_t q_s = base, k_s = q_s + Q_BYTES, v_s = k_s + 2 * K_BYTES, p_s = v_s + 2 * V_BYTES, bars = p_s + P_BYTES;
     uint8_t* v_ptr = base_ptr + Q_BYTES + 2 * K_BYTES;
     uint8_t* p_ptr = v_ptr + 2 * V_BYTES;
@@ -131,7 +139,7 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_co
     // tensor memory): tile j uses member j & 1, for the (j >> 1)-th time
     const uint32_t q_full = bars, k_full = bars + 8, k_empty = bars + 24, s_full = bars + 40, v_full = bars + 56,
                    v_empty = bars + 72, p_full = bars + 88, o_full = bars + 96;
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int warp = __shfl_sync(0xffffffffu, int(threadIdx.x >> 5), 0), lane = threadIdx.x & 31;      // (uniform, for the compiler too)
 
     // The last query tiles have the most keys: they start first, for every head.
     const int n_qt = gridDim.y / p.split;
@@ -165,21 +173,7 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_co
         tile_id = (before * p.n_heads + h) * n_qt + qt;
     }
     const int* table = p.block_table + int64_t(seg) * p.max_blocks;
-    // The page ids of this CTA's key range, checked, in shared memory (a read of the table in global memory costs the
-    // producer a round trip to L2 per page otherwise); ranges longer than the array fall back to the table itself.
-    __shared__ int page_tab[TAB_MAX];
-    const int tab_n = n_tiles * PAGES_PER_TILE;
-    const bool tab_ok = tab_n <= TAB_MAX;
-    if (tab_ok) {
-        for (int i = threadIdx.x; i < tab_n; i += NUM_THREADS) {
-            const int idx = tile_of(i / PAGES_PER_TILE) * PAGES_PER_TILE + i % PAGES_PER_TILE;
-            const int page = idx < p.max_blocks ? table[idx] : -1;
-            page_tab[i] = (page < 0 || page >= p.n_pages) ? -1 : page;
-        }
-    }
-    auto page_of = [&](int j, int key) -> int {          // page id of the page that holds `key` of this CTA's tile j, or -1
-        const int idx = key / PAGE;
-        if (tab_ok) return page_tab[j * PAGES_PER_TILE + idx % PAGES_PER_TILE];
+    auto page_at = [&](int idx) -> int {                 // entry idx of the segment's table, or -1
         if (idx >= p.max_blocks) return -1;
         const int page = table[idx];
         return (page < 0 || page >= p.n_pages) ? -1 : page;
@@ -216,14 +210,16 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_co
         int pend_k[2] = {-1, -1}, pend_v[2] = {-1, -1};  // tiles whose copies were issued into each buffer last
         // Loads the K (which = 0) or V (which = 1) pages of tile j. Pages that hold nothing this step may read are
         // skipped (their rows are masked, and zeroed for V).
-        auto load_tile = [&](int j, int which) {
+        // (`id`: the table's entry of this lane's page, read a tile ahead: a trip to L2 otherwise stands before every copy)
+        auto page_id = [&](int j) -> int { return j < n_tiles && lane < PAGES_PER_TILE ? page_at(tile_of(j) * PAGES_PER_TILE + lane) : -1; };
+        auto load_tile = [&](int j, int which, int id) {
             const int key0 = tile_of(j) * BN;
             const uint32_t full = (which ? v_full : k_full) + 8 * (j & 1);
             const uint32_t dst0 = which ? v_s + (j & 1) * V_BYTES : k_s + (j & 1) * K_BYTES;
             int page = -1;
             if (lane < PAGES_PER_TILE) {
                 const int key = key0 + lane * PAGE;
-                page = key <= last_written ? page_of(j, key) : -1;
+                page = key <= last_written ? id : -1;
                 if (key <= last_written && (key + PAGE - 1 >= lo_key || key < keep_end) && page < 0) atomicExch(p.status, STATUS_BAD_PAGE);
             }
             const int valid = __popc(__ballot_sync(0xffffffffu, page >= 0));
@@ -244,19 +240,23 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_co
             if (lane == 0) got = mbar_wait(bar, parity) ? 1 : 0;
             return __shfl_sync(0xffffffffu, got, 0) != 0;
         };
-        load_tile(0, 0);
-        load_tile(0, 1);
-        if (n_tiles > 1) { load_tile(1, 0); load_tile(1, 1); }
+        const int id0 = page_id(0), id1 = page_id(1);
+        int ahead = page_id(2);
+        load_tile(0, 0, id0);
+        load_tile(0, 1, id0);
+        if (n_tiles > 1) { load_tile(1, 0, id1); load_tile(1, 1, id1); }
         bool failed = false;
         for (int j = 0; j < n_tiles && !failed; j++) {
             if (__shfl_sync(0xffffffffu, int(slots[1]), 0)) { failed = true; break; }
+            const int id = ahead;
+            ahead = page_id(j + 3);
             if (j + 2 < n_tiles) {                       // S(j) is complete: its K buffer takes tile j + 2
                 if (!wait_all(k_empty + 8 * (j & 1), (j >> 1) & 1)) { failed = true; break; }
-                load_tile(j + 2, 0);
+                load_tile(j + 2, 0, id);
             }
             if (j + 2 < n_tiles) {                       // P(j) V(j) is complete: its V buffer takes tile j + 2
                 if (!wait_all(v_empty + 8 * (j & 1), (j >> 1) & 1)) { failed = true; break; }
-                load_tile(j + 2, 1);
+                load_tile(j + 2, 1, id);
             }
         }
         if (failed && lane == 0) {
@@ -270,14 +270,16 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_co
         }
     } else if (warp == 1) {
         // ---------------------------------------------------------------- MMA issuer
-        if (lane == 0) {
-            constexpr uint32_t idesc_s = make_idesc(BN, false), idesc_o = make_idesc(HD, true);
-            const uint32_t o_tmem = tmem_base + O_COL;
-            // S(j) = Q K(j)^T into S buffer j & 1
-            auto issue_qk = [&](int j) -> bool {
-                if (!mbar_wait(k_full + 8 * (j & 1), (j >> 1) & 1)) return false;
-                tc_fence_after();
-                const uint32_t s_tmem = tmem_base + S_COL + (j & 1) * BN, kb = k_s + (j & 1) * K_BYTES;
+        // (The whole warp walks, one elected lane issues: addresses and descriptors stay in uniform registers.)
+        constexpr uint32_t idesc_s = make_idesc(BN, false), idesc_o = make_idesc(HD, true);
+        const uint32_t o_tmem = tmem_base + O_COL;
+        const bool leader = elect_one();
+        // S(j) = Q K(j)^T into S buffer j & 1
+        auto issue_qk = [&](int j) -> bool {
+            if (!mbar_wait(k_full + 8 * (j & 1), (j >> 1) & 1)) return false;
+            tc_fence_after();
+            const uint32_t s_tmem = tmem_base + S_COL + (j & 1) * BN, kb = k_s + (j & 1) * K_BYTES;
+            if (leader) {
 #pragma unroll
                 for (int db = 0; db < DB; db++) {
                     const uint64_t qd = make_desc(q_s + db * (BM * 128), 16, 1024), kd = make_desc(kb + db * (BN * 128), 16, 1024);
@@ -287,14 +289,17 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_co
                 }
                 umma_commit(s_full + 8 * (j & 1));
                 umma_commit(k_empty + 8 * (j & 1));
-                IB_T(j, 6);
-                return true;
-            };
-            bool ok = mbar_wait(q_full, 0) && issue_qk(0) && (n_tiles < 2 || issue_qk(1));
-            for (int j = 0; j < n_tiles && ok && !slots[1]; j++) {
-                ok = mbar_wait(p_full, j & 1) && mbar_wait(v_full + 8 * (j & 1), (j >> 1) & 1);
-                if (!ok) break;
-                tc_fence_after();
+            }
+            __syncwarp();
+            IB_T(j, 6);
+            return true;
+        };
+        bool ok = mbar_wait(q_full, 0) && issue_qk(0) && (n_tiles < 2 || issue_qk(1));
+        for (int j = 0; j < n_tiles && ok; j++) {
+            ok = mbar_wait(p_full, j & 1) && mbar_wait(v_full + 8 * (j & 1), (j >> 1) & 1);
+            if (!ok) break;
+            tc_fence_after();
+            if (leader) {
 #pragma unroll
                 for (int k = 0; k < BN / 16; k++) {      // 16 keys per step: 32 bytes along P's rows, 2 groups of 8 rows of V
                     const uint64_t pd = make_desc(p_s + (k / 4) * (BM * 128), 16, 1024) + uint64_t(2 * (k % 4));
@@ -303,12 +308,13 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_co
                 }
                 umma_commit(o_full);
                 umma_commit(v_empty + 8 * (j & 1));
-                IB_T(j, 7);
-                // the softmax threads have read S(j) (they wrote P(j) from it): its buffer takes S(j + 2)
-                if (j + 2 < n_tiles) ok = issue_qk(j + 2);
             }
-            if (!ok) { atomicExch(p.status, STATUS_TIMEOUT); slots[1] = 1; }
+            __syncwarp();
+            IB_T(j, 7);
+            // the softmax threads have read S(j) (they wrote P(j) from it): its buffer takes S(j + 2)
+            if (j + 2 < n_tiles) ok = issue_qk(j + 2);
         }
+        if (!ok && lane == 0) { atomicExch(p.status, STATUS_TIMEOUT); slots[1] = 1; }
     } else {
         // ---------------------------------------------------------------- softmax and epilogue (warps 2..5)
         const int quad = warp & 3;
@@ -421,7 +427,7 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_co
                 for (int u = r; u < BN * DB; u += BM) {
                     const int key_row = u % BN, db = u / BN;
                     const int key = key0 + key_row;
-                    if (key > last_written || page_of(j, key) < 0) {
+                    if (key > last_written || page_at(key / PAGE) < 0) {
                         uint4* line = reinterpret_cast<uint4*>(v_ptr + (j & 1) * V_BYTES + db * (BN * 128) + key_row * 128);
 #pragma unroll
                         for (int e = 0; e < 8; e++) line[e] = make_uint4(0u, 0u, 0u, 0u);
@@ -508,19 +514,20 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_co
                 const float inv = l_all > 0.0f ? 1.0f / l_all : 0.0f;
 #pragma unroll
                 for (int i = 0; i < MAX_SPLIT; i++) f[i] *= inv;
+                // (32 columns of every part are requested together: with 16 the row's eight trips to L2 took 8 us)
 #pragma unroll 1
-                for (int c = 0; c < HD; c += 16) {
-                    float v[16];
+                for (int c = 0; c < HD; c += 32) {
+                    float v[32];
 #pragma unroll
-                    for (int e = 0; e < 16; e++) v[e] = 0.0f;
+                    for (int e = 0; e < 32; e++) v[e] = 0.0f;
 #pragma unroll
                     for (int i = 0; i < MAX_SPLIT; i++) {
                         if (i < n_parts) {
 #pragma unroll
-                            for (int e = 0; e < 16; e++) v[e] = fmaf(__ldcg(parts + i * PART_FLOATS + (c + e) * BM + r), f[i], v[e]);
+                            for (int e = 0; e < 32; e++) v[e] = fmaf(__ldcg(parts + i * PART_FLOATS + (c + e) * BM + r), f[i], v[e]);
                         }
                     }
-                    if (qi < q_len) store16(c, v);
+                    if (qi < q_len) { store16(c, v); store16(c + 16, v + 16); }
                 }
             }
         }

@@ -53,6 +53,10 @@ DEFAULT_DEFINES = {"attn": {"IB_HEAD_DIM": 128}, "attn_tc": {"IB_HEAD_DIM": 128}
                    "talk_pf": {"IB_HEAD_DIM": 128, "IB_V_DIM": 128, "IB_HEADS": 12}}
 
 
+# a second form of a module that a model uses beside the first (built by build_all() too)
+MORE_DEFINES = {"attn_tc": {"IB_HEAD_DIM": 128, "IB_ATTN_BN": 128}}
+
+
 class BuildError(RuntimeError):
     pass
 
@@ -199,7 +203,7 @@ def build_all(modules: Optional[Sequence[str]] = None, verbose: bool = False) ->
     """Compiles every module (in parallel); used by the build check and before GPU runs."""
     from concurrent.futures import ThreadPoolExecutor
     names = [m for m in (modules or MODULES) if os.path.isfile(os.path.join(HERE, MODULES[m]))]
-    jobs = [(m, DEFAULT_DEFINES.get(m)) for m in names]
+    jobs = [(m, DEFAULT_DEFINES.get(m)) for m in names] + [(m, MORE_DEFINES[m]) for m in names if m in MORE_DEFINES]
     with ThreadPoolExecutor(max_workers=min(8, len(jobs) or 1)) as pool:
         paths = list(pool.map(lambda j: compile_module(j[0], j[1], verbose), jobs))
     return dict(zip(names, paths))

@@ -1298,37 +1298,41 @@ IB_EXPORT int ib_gemm_tc_plan(int64_t M, int64_t N, int64_t K, int sm_count, int
             if (sliced * 23 < other * 20) { *bn = 768; s = slices; *splits = s; cluster = true; }
         }
     }
-    // Pairs of SMs on tiles of 256 rows (codes 1024 + 2 x width), where the same kind of model says so. In the unit above a
-    // k-block takes a pair 0.50 + width / 655 (0.264 us at width 128, 0.338 at 256) and an SM by itself 0.74 + width / 790 (0.364 at
-    // 176, 0.403 at 256: the way from L2 is the bound, and a pair's tile takes a third less through it), beside 20 units a launch
-    // for the pairs, 16 alone. Measured against the choices above at 2,048 rows: gate/up 78 and 86 us, down 49 and 56 at 1,536
-    // features, 363 and 395, 213 and 258 (or 306) at 3,584; one round of short tiles (2048 features, K = 1536: 14.1 and 13.8) stays.
-    static const bool pairs_on = [] { const char* e = getenv("INFER_B200_GEMM_PAIRS"); return !(e && e[0] == '0'); }();
-    if (!*swap && pairs_on && sm_count >= 2) {
-        auto unit = [](int64_t rounds, int64_t kb, int64_t at0, int64_t slope, int64_t width) { return rounds * kb * (at0 + 100 * width / slope); };
-        int64_t now;                                              // in hundredths of a unit
-        if (*bn == 768) now = 100 * (int64_t(kb_total + s - 1) / s) + (s == 8 ? 4000 : 3400);
-        else if (*bn >= 256) {
-            const int64_t width = *bn == 256 ? 256 : *bn / 2, tm = *bn == 256 ? (M + 255) / 256 : (M + 127) / 128;
-            const int64_t t = tm * ((N + (*bn == 256 ? 128 : width) - 1) / (*bn == 256 ? 128 : width));
-            now = unit((t + sm_count - 1) / sm_count, kb_total, 74, 790, width) + 1600;
-        } else {
-            const int64_t ctas = tiles * s, cap = cluster ? (s == 2 ? sm_count - 4 : sm_count - sm_count / 7) : 2 * int64_t(sm_count);
-            now = ((ctas + cap - 1) / cap) * 100 * (int64_t(kb_total + s - 1) / s) + 2000;
-        }
-        const int64_t tm = (M + 255) / 256, pairs = sm_count / 2;
-        int64_t best = -1;
-        int width = 0;
-        for (int w : {256, 224, 192, 160, 128}) {
-            const int64_t t = tm * ((N + w - 1) / w);
-            const int64_t est = unit((t + pairs - 1) / pairs, kb_total, 50, 655, w) + 2000;
-            if (best < 0 || est < best) { best = est; width = w; }
-        }
-        if (best * 100 < now * 98) { *bn = 1024 + 2 * width; s = 1; *splits = 1; cluster = false; }
-    }
     *workspace_floats = (s > 1 && !*swap && !cluster) ? int64_t(s) * tiles * BM * (*bn) : 0;
     *n_counters = (s > 1 && !*swap && !cluster) ? tiles : 0;
     return IB_OK;
+}
+
+// The pair kernel's code for a product that ib_gemm_tc_plan gave this plan, or 0: the plan stands.
+IB_EXPORT int ib_gemm_tc_pairs(int64_t M, int64_t N, int64_t K, int sm_count, int swap, int bn, int s, int64_t workspace_floats) {
+    // Pairs of SMs on tiles of 256 rows, where a model like the planner's says so. In its unit (0.38 us) a k-block takes a pair
+    // 0.50 + width / 655 (0.264 us at width 128, 0.338 at 256) and an SM by itself 0.74 + width / 790 (0.364 at 176, 0.403 at 256: the way from L2 is the bound, and a pair's tile takes a third less through it), beside 20 units a launch
+    // for the pairs, 16 alone. Measured against the other plans at 2,048 rows: gate/up 75.5 and 85.2 us, down 46.6 and 56.3 at 1,536
+    // features, 348 and 392, 210 and 270 at 3,584; one round of short tiles (2048 features, K = 1536: 14.1 and 13.8) stays as it is.
+    static const bool pairs_on = [] { const char* e = getenv("INFER_B200_GEMM_PAIRS"); return !(e && e[0] == '0'); }();
+    if (swap || !pairs_on || sm_count < 2 || workspace_floats > 0) return 0;
+    const int kb_total = int((K + BK - 1) / BK);
+    const int64_t tiles = ((M + BM - 1) / BM) * ((N + 127) / 128);
+    auto unit = [](int64_t rounds, int64_t kb, int64_t at0, int64_t slope, int64_t width) { return rounds * kb * (at0 + 100 * width / slope); };
+    int64_t now;                                              // in hundredths of a unit
+    if (bn == 768) now = 100 * (int64_t(kb_total + s - 1) / s) + (s == 8 ? 4000 : 3400);
+    else if (bn >= 256) {
+        const int64_t width = bn == 256 ? 256 : bn / 2, tm = bn == 256 ? (M + 255) / 256 : (M + 127) / 128;
+        const int64_t t = tm * ((N + (bn == 256 ? 128 : width) - 1) / (bn == 256 ? 128 : width));
+        now = unit((t + sm_count - 1) / sm_count, kb_total, 74, 790, width) + 1600;
+    } else {
+        const int64_t ctas = tiles * s, cap = s > 1 ? (s == 2 ? sm_count - 4 : sm_count - sm_count / 7) : 2 * int64_t(sm_count);
+        now = ((ctas + cap - 1) / cap) * 100 * (int64_t(kb_total + s - 1) / s) + 2000;
+    }
+    const int64_t tm = (M + 255) / 256, pairs = sm_count / 2;
+    int64_t best = -1;
+    int width = 0;
+    for (int w : {256, 224, 192, 160, 128}) {
+        const int64_t t = tm * ((N + w - 1) / w);
+        const int64_t est = unit((t + pairs - 1) / pairs, kb_total, 50, 655, w) + 2000;
+        if (best < 0 || est < best) { best = est; width = w; }
+    }
+    return best * 100 < now * 98 ? 1024 + 2 * width : 0;
 }
 
 // out[M, N] = x[M, K] . w[N, K]^T (+ bias) (+ residual), or with epi = 2 out[M, N/2] = SwiGLU of feature rows

@@ -377,8 +377,9 @@ class Engine:
             feedback=self.next_tokens, status=self.status, seg_lens=seg_lens, seg_pos0_host=pos0, max_q_len=max(seg_lens),
             max_ctx_len=max(p + n for p, n in zip(pos0, seg_lens)), decode_only=all(n == 1 for n in seg_lens),
             sampling=sampling)
-        if entry is not None:
-            # a graph's launch shapes must not depend on the step: bound the context by the table width
+        if entry is not None or run is not None:
+            # a graph's launch shapes must not depend on the step: bound the context by the table width (also in the eager run
+            # before it, which sizes the kernels' scratch)
             ctx.max_ctx_len = max(widths) * cache.page_size if widths else ctx.max_ctx_len
         ctx.measured = run
         return ctx, entry

@@ -93,6 +93,22 @@ def gemm_plan(M: int, N: int, K: int, sm_count: int):
     return _PLAN_CACHE[key]
 
 
+_CHOICE_CACHE: Dict[tuple, Optional[tuple]] = {}
+
+
+def gemm_choice(M: int, N: int, K: int, sm_count: int):
+    """What a product runs as: ``gemm_plan``'s plan, or pairs of SMs (code 1024 + 2 x width) where they take less time."""
+    key = (M, N, K, sm_count)
+    if key not in _CHOICE_CACHE:
+        plan = gemm_plan(M, N, K, sm_count)
+        if plan is not None:
+            f = _fn("gemm", "ib_gemm_tc_pairs", [c_int64] * 3 + [c_int] * 4 + [c_int64])
+            code = f(M, N, K, sm_count, *plan[:4])
+            plan = (0, code, 1, 0, 0) if code else plan
+        _CHOICE_CACHE[key] = plan
+    return _CHOICE_CACHE[key]
+
+
 def gemm_tc(x: torch.Tensor, w: torch.Tensor, bias: Optional[torch.Tensor] = None, residual: Optional[torch.Tensor] = None,
             out_dtype: torch.dtype = torch.bfloat16, out: Optional[torch.Tensor] = None, plan=None,
             swiglu: bool = False) -> Optional[torch.Tensor]:
@@ -106,7 +122,7 @@ def gemm_tc(x: torch.Tensor, w: torch.Tensor, bias: Optional[torch.Tensor] = Non
     if w.shape[1] != K:
         raise KernelError(f"gemm_tc: x is [{M},{K}] but w is {tuple(w.shape)}")
     st = device_state(x.device)
-    plan = plan or gemm_plan(M, N, K, st.sm_count)
+    plan = plan or gemm_choice(M, N, K, st.sm_count)
     if plan is None or (x.data_ptr() & 15) or (w.data_ptr() & 15) or (swiglu and N % 16):
         return None
     swap, bn, splits, ws_floats, n_counters = plan
@@ -339,11 +355,32 @@ def prefill_split(sm_count: int, n_heads: int, n_prefill: int, max_q_len: int, m
     return 1
 
 
+def prefill_plan(sm_count: int, n_heads: int, head_dim: int, seg_lens, max_ctx_len: int, window: Optional[int]):
+    """(compile-time sizes of the tcgen05 prefill kernel, into how many parts it may cut the keys of a query tile). The kernel
+    walks over keys 64 at a time with two CTAs an SM, whose softmax and products overlap, or 128 at a time with one. Alone on
+    its SM a CTA is bound by its own chain, 2.3 us per 128 keys against 3.2 per 2 x 64: 128 where the query tiles are long (512
+    keys and more) and all run at once. Measured with 12 heads (192 CTAs at 2,048 tokens): 512 tokens 13.4 us with 128 keys and
+    15.9 with 64, 2,048 tokens 40 and 42, ten segments of 200 tokens 21 and 12.5; with 28 heads 2,048 tokens 77 and 62, 4,096
+    behind 11,777 1,593 and 1,265. Keys are shared among CTAs as ``prefill_split`` says. Counted for portions that end at
+    max_ctx_len, which is all that a captured step knows; any answer is correct."""
+    lens = [n for n in seg_lens if n > 1] or [1]
+    tiles = []                                                   # of 128 keys, per query tile
+    for n in lens:
+        for q_first in range(max_ctx_len - n, max_ctx_len, 128):
+            lo = max(0, q_first - window + 1) if window else 0
+            tiles.append(min(max_ctx_len - 1, q_first + 127) // 128 - lo // 128 + 1)
+    ctas, longest = n_heads * len(tiles), max(tiles)
+    split = prefill_split(sm_count, n_heads, len(lens), max(lens), max_ctx_len, window)
+    if longest >= 4 and (ctas <= sm_count or (2 * ctas <= 3 * sm_count and longest >= 16)):
+        return {"IB_HEAD_DIM": head_dim, "IB_ATTN_BN": 128}, split
+    return {"IB_HEAD_DIM": head_dim}, split
+
+
 def attention_fast(q: torch.Tensor, k_cache: torch.Tensor, v_cache: torch.Tensor, block_table: torch.Tensor,
                    seg_start: torch.Tensor, seg_pos0: torch.Tensor, n_heads: int, n_kv: int, head_dim: int,
                    window: Optional[int], scale: float, has_decode: bool, max_q_len: int, max_ctx_len: int,
                    n_decode: Optional[int] = None, n_splits: Optional[int] = None, n_clusters: int = 1,
-                   tc_split: Optional[int] = None) -> Optional[torch.Tensor]:
+                   tc_split: Optional[int] = None, seg_lens=None) -> Optional[torch.Tensor]:
     """Tensor-core attention of a step's segments over the paged bfloat16 cache; None if the shape is refused.
     The library is compiled for this head size at first use."""
     n_pages, ckv, page_size, chd = k_cache.shape
@@ -370,10 +407,11 @@ def attention_fast(q: torch.Tensor, k_cache: torch.Tensor, v_cache: torch.Tensor
     # everything else, to the mma.sync kernels (a call with max_q_len = 1 launches no prefill kernel).
     tc = ATTENTION_TC and max_q_len > 1 and head_dim in ATTENTION_TC_HEAD_DIMS and page_size == 16
     if tc:
-        g = _fn("attn_tc", "ib_attention_prefill_tc", [c_void_p] * 5 + [c_int] + [c_void_p] * 2 + [c_int, c_int64] + [c_int] * 5 +
-                [c_float, c_int64, c_int] + [c_void_p] * 2 + [c_int, c_void_p, c_int64, c_void_p, c_int64, c_int], {"IB_HEAD_DIM": head_dim})
         n_prefill = S - (n_decode or 0)
-        split = prefill_split(st.sm_count, n_heads, n_prefill, max_q_len, max_ctx_len, window) if tc_split is None else tc_split
+        defines, split = prefill_plan(st.sm_count, n_heads, head_dim, seg_lens or [max_q_len] * n_prefill, max_ctx_len, window)
+        split = split if tc_split is None else tc_split
+        g = _fn("attn_tc", "ib_attention_prefill_tc", [c_void_p] * 5 + [c_int] + [c_void_p] * 2 + [c_int, c_int64] + [c_int] * 5 +
+                [c_float, c_int64, c_int] + [c_void_p] * 2 + [c_int, c_void_p, c_int64, c_void_p, c_int64, c_int], defines)
         tc_ws = tc_cnt = None
         if split > 1:
             tiles = max(1, n_prefill) * n_heads * -(-max_q_len // 128)
@@ -423,7 +461,7 @@ def attention_prefill_biased(q, k_cache, v_cache, block_table, step, n_heads, n_
     S = step.seg_pos0.numel()
     st = device_state(q.device)
     n_prefill = sum(1 for n in step.seg_lens if n > 1)
-    split = prefill_split(st.sm_count, n_heads, n_prefill, step.max_q_len, step.max_ctx_len, window)
+    defines, split = prefill_plan(st.sm_count, n_heads, head_dim, step.seg_lens, step.max_ctx_len, window)
     tc_ws = tc_cnt = None
     if split > 1:
         tiles = max(1, n_prefill) * n_heads * -(-step.max_q_len // 128)
@@ -434,7 +472,7 @@ def attention_prefill_biased(q, k_cache, v_cache, block_table, step, n_heads, n_
     sig = [c_void_p] * 5 + [c_int] + [c_void_p] * 2 + [c_int, c_int64] + [c_int] * 5 + [c_float, c_int64, c_int] + [c_void_p] * 2 + \
           [c_int, c_void_p, c_int64, c_void_p, c_int64, c_int, c_void_p, c_int, c_void_p]
     g = _fn("attn_tc", "ib_attention_prefill_tc_kept" if kept else "ib_attention_prefill_tc_biased", sig + ([c_int, c_void_p] if kept else []),
-            {"IB_HEAD_DIM": head_dim})
+            defines)
     args = [q.data_ptr(), k_cache.data_ptr(), v_cache.data_ptr(), out.data_ptr(), block_table.data_ptr(), block_table.shape[1],
             step.seg_start.data_ptr(), step.seg_pos0.data_ptr(), S, T, n_heads, n_kv, head_dim, page_size, int(window or 0), float(scale),
             n_pages, int(step.max_q_len), st.status.data_ptr(), _stream(), int(split), _ptr(tc_ws), 0 if tc_ws is None else tc_ws.numel(),
@@ -553,7 +591,7 @@ def attention_decode_fused(qkv: torch.Tensor, cos: torch.Tensor, sin: torch.Tens
 def attention(q, cache, table, step, n_heads, n_kv, head_dim, window, scale):
     n_decode = sum(1 for n in step.seg_lens if n == 1)
     return attention_fast(q, cache.k, cache.v, table, step.seg_start, step.seg_pos0, n_heads, n_kv, head_dim, window,
-                          scale, n_decode > 0, step.max_q_len, step.max_ctx_len, n_decode)
+                          scale, n_decode > 0, step.max_q_len, step.max_ctx_len, n_decode, seg_lens=step.seg_lens)
 
 
 def gate_up_swiglu(x, gate_up_weight):
