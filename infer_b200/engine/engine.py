@@ -184,7 +184,6 @@ class Engine:
         self._portion_runs: Dict[tuple, _PortionRun] = {}
         self._ms_per_launch = float("inf")                # the fastest eager run's host time per launch
         self._graph_pool = torch.cuda.graph_pool_handle() if self.use_graphs else None
-        self._capture_stream = torch.cuda.Stream(self.rt.device) if self.use_graphs else None
 
     # ------------------------------------------------------------------ construction helpers
 
@@ -410,9 +409,10 @@ class Engine:
         device; ``torch.cuda.graph`` waits for it, collects garbage and gives the allocator's free memory back to the
         driver, which costs milliseconds to hundreds of them. That is the second way, where memory is short."""
         graph, collecting = torch.cuda.CUDAGraph(), gc.isenabled()
+        from ..fast_ops import capture_stream
         gc.disable()                              # (a graph that a collection finds must not be destroyed meanwhile)
         try:
-            with torch.cuda.stream(self._capture_stream):
+            with torch.cuda.stream(capture_stream(self.rt.device)):
                 graph.capture_begin(pool=self._graph_pool)
                 try:
                     out = self._run_model(ctx)

@@ -50,6 +50,34 @@ _STATES: Dict[torch.device, DeviceState] = {}
 _SIDE_STATES: Dict[tuple, DeviceState] = {}        # (device, raw handle of a registered side stream) -> its scratch
 
 
+_OWN_STREAMS: set = set()                          # (device, raw handle) of the streams that ``own_stream`` has handed out
+
+
+def own_stream(device) -> "torch.cuda.Stream":
+    """A stream that no other caller of this function has on the device (torch's streams come from a pool of 32 and come round
+    again: a capture that met a registered side stream's handle would take that stream's scratch)."""
+    device = torch.device(device)
+    if device.index is None:
+        device = torch.device("cuda", torch.cuda.current_device())
+    for _ in range(64):
+        stream = torch.cuda.Stream(device)
+        if (device, stream.cuda_stream) not in _OWN_STREAMS:
+            break
+    _OWN_STREAMS.add((device, stream.cuda_stream))
+    return stream
+
+
+_CAPTURE_STREAMS: Dict[torch.device, "torch.cuda.Stream"] = {}
+
+
+def capture_stream(device) -> "torch.cuda.Stream":
+    """The stream on which steps are captured into graphs, one per device."""
+    device = torch.device(device)
+    if device not in _CAPTURE_STREAMS:
+        _CAPTURE_STREAMS[device] = own_stream(device)
+    return _CAPTURE_STREAMS[device]
+
+
 def register_side_stream(stream: "torch.cuda.Stream") -> None:
     """A stream on which a part runs kernels beside those of the step's own stream. Kernels launched while it is the
     current stream get a workspace and counters of their own (calls on ONE stream run in order and may share

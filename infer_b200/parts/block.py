@@ -48,7 +48,7 @@ def _side_streams(device):
     key = str(device)
     if key not in _SIDE_STREAMS:
         from .. import fast_ops
-        _SIDE_STREAMS[key] = (torch.cuda.Stream(device), torch.cuda.Stream(device))
+        _SIDE_STREAMS[key] = (fast_ops.own_stream(device), fast_ops.own_stream(device))
         for st in _SIDE_STREAMS[key]:
             fast_ops.register_side_stream(st)
     return _SIDE_STREAMS[key]
