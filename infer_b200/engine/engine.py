@@ -177,9 +177,12 @@ class Engine:
         # The sampler leaves every request's last token here (indexed by state slot); a decode entry whose token is
         # FEEDBACK_TOKEN reads it, so that the host need not see a token before the next step is launched.
         self.next_tokens = torch.zeros(max(1, max_requests), dtype=torch.int32, device=self.rt.device)
-        # Decode-only steps of the bfloat16 path are captured into CUDA graphs, one per (batch, wanted rows, table widths);
-        # steps with prompt portions once their exact shape has repeated.
-        self.use_graphs = bool(cuda_graphs) and dtype == torch.bfloat16 and self.model.graph_safe()
+        # Decode-only steps are captured into CUDA graphs, one per (batch, wanted rows, table widths); steps with prompt
+        # portions once their exact shape has repeated. The 32-bit path does so for models of this package's own parts (a part
+        # registered from elsewhere may count on being run eagerly there) and hands out a copy of a replay's result, so that
+        # its callers own what they get. (A tiny model's 24 greedy steps: 13.6 -> 4.8 ms, of which its launches were most.)
+        self.use_graphs = bool(cuda_graphs) and self.model.graph_safe() and (dtype == torch.bfloat16 or self.model.built_in())
+        self._copy_results = dtype == torch.float32
         self._graphs: Dict[tuple, _GraphEntry] = {}
         self._portion_runs: Dict[tuple, _PortionRun] = {}
         self._ms_per_launch = float("inf")                # the fastest eager run's host time per launch
@@ -433,7 +436,7 @@ class Engine:
         """Runs one batch; returns float32 logits [wanted places, vocab] on the device. With ``sample`` (one
         (SampleParams, position) per wanted place, in order) the step samples on the device as well and returns
         int32 token ids [wanted places] instead; each id also stays on the device for its request (FEEDBACK_TOKEN).
-        With CUDA graphs on, the tensor returned by a captured step is reused by the next step of the same shape:
+        With CUDA graphs on, the tensor returned by a captured bfloat16 step is reused by the next step of the same shape:
         read it, or enqueue its copy, before that. Steps may be issued back to back without waiting for the device.
         Raises OutOfPages (nothing changed) if the pages for all entries together are not free."""
         return self._step(entries, sample, False).output
@@ -497,6 +500,7 @@ class Engine:
                 graph, out = entry.graphs[entry.turn]
                 graph.replay()
                 ops._LAUNCHES[0] += entry.n_launches
+                out = out.clone() if self._copy_results else out
             elif entry.warm < GRAPH_WARMUP_STEPS:
                 # The first steps of a shape run eagerly: they build libraries, size workspaces, set attributes.
                 entry.warm += 1
@@ -509,6 +513,7 @@ class Engine:
                 entry.graphs.append((graph, out))
                 graph.replay()
                 ops._LAUNCHES[0] += entry.n_launches
+                out = out.clone() if self._copy_results else out
         for rid, n in wanted:
             self.cache.advance(rid, n)
         self.steps_run += 1

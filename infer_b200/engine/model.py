@@ -53,6 +53,14 @@ class Model:
         """True if every part allows its forward() to be captured into a CUDA graph."""
         return all(getattr(p, "graph_safe", True) for p in self.all_parts())
 
+    def built_in(self) -> bool:
+        """True if every part, the parts inside parts, and every block are this package's own."""
+        own = __name__.split(".")[0]
+
+        def mine(obj) -> bool:
+            return type(obj).__module__.split(".")[0] == own and all(mine(v) for v in vars(obj).values() if isinstance(v, Part))
+        return all(mine(p) for p in (*self.all_parts(), *self.blocks))
+
     def cache_needs(self) -> Dict[int, object]:
         """cache index -> what the layer that writes it needs from the cache manager."""
         needs: Dict[int, object] = {}
