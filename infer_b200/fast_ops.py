@@ -9,6 +9,8 @@ range, a bounded wait that ran out).
 from __future__ import annotations
 
 import ctypes
+import functools
+import heapq
 import os
 from typing import Dict, Optional
 
@@ -383,25 +385,63 @@ def prefill_split(sm_count: int, n_heads: int, n_prefill: int, max_q_len: int, m
     return 1
 
 
+PREFILL_PARTS_MAX_FLOATS = 24 << 20      # of scratch that sharing query tiles may take (96 MB)
+PREFILL_SIMULATED_CTAS = 1024            # beyond that many CTAs they even out by themselves
+
+
+def _makespan(jobs, slots: int) -> float:
+    """When the last of ``jobs`` (durations, started in this order) ends on ``slots`` workers."""
+    if len(jobs) <= slots:
+        return max(jobs)
+    ends = list(jobs[:slots])
+    heapq.heapify(ends)
+    for d in jobs[slots:]:
+        heapq.heapreplace(ends, ends[0] + d)
+    return max(ends)
+
+
 def prefill_plan(sm_count: int, n_heads: int, head_dim: int, seg_lens, max_ctx_len: int, window: Optional[int]):
     """(compile-time sizes of the tcgen05 prefill kernel, into how many parts it may cut the keys of a query tile). The kernel
-    walks over keys 64 at a time with two CTAs an SM, whose softmax and products overlap, or 128 at a time with one. Alone on
-    its SM a CTA is bound by its own chain, 2.3 us per 128 keys against 3.2 per 2 x 64: 128 where the query tiles are long (512
-    keys and more) and all run at once. Measured with 12 heads (192 CTAs at 2,048 tokens): 512 tokens 13.4 us with 128 keys and
-    15.9 with 64, 2,048 tokens 40 and 42, ten segments of 200 tokens 21 and 12.5; with 28 heads 2,048 tokens 77 and 62, 4,096
-    behind 11,777 1,593 and 1,265. Keys are shared among CTAs as ``prefill_split`` says. Counted for portions that end at
-    max_ctx_len, which is all that a captured step knows; any answer is correct."""
-    lens = [n for n in seg_lens if n > 1] or [1]
-    tiles = []                                                   # of 128 keys, per query tile
+    walks over keys 64 at a time with two CTAs an SM, whose softmax and products overlap, or 128 at a time with one. Counted for
+    portions that end at max_ctx_len, which is all that a captured step knows; any answer is correct."""
+    form, split = _prefill_plan(sm_count, n_heads, head_dim, tuple(n for n in seg_lens if n > 1) or (1,), max_ctx_len, window)
+    return ({"IB_HEAD_DIM": head_dim, "IB_ATTN_BN": 128} if form == 128 else {"IB_HEAD_DIM": head_dim}), split
+
+
+@functools.lru_cache(maxsize=4096)
+def _prefill_plan(sm_count: int, n_heads: int, head_dim: int, lens, max_ctx_len: int, window: Optional[int]):
+    """Alone on its SM a CTA is bound by its own chain, 2.3 us per 128 keys against 3.2 per 2 x 64: 128 keys where the query tiles
+    are long (512 keys and more) and all run at once. Measured with 12 heads (192 CTAs at 2,048 tokens): 512 tokens 13.4 us with
+    128 keys and 15.9 with 64, 2,048 tokens 36 and 42, ten segments of 200 tokens 21 and 12.5; with 28 heads 2,048 tokens 77 and 62,
+    4,096 behind 11,777 1,593 and 1,257. Then the CTAs are laid onto the SMs in the order they start, for every number of parts:
+    in units of 1.75 us a CTA takes one per 64 keys and 4 to start and end (1.3 per 128 keys and 3), 3 more where parts meet. A
+    long second round that is nearly empty is what parts avoid: 12 heads, 4,096 tokens behind 11,777 (384 CTAs on 296 places)
+    632 us whole, 471 in three parts; 1,024 behind 8,192 145 and 89; 28 heads, 2,048 behind 8,192 436 and 402."""
+    n64, n128 = [], []                                           # keys of every query tile, in tiles of 64 and 128
     for n in lens:
         for q_first in range(max_ctx_len - n, max_ctx_len, 128):
-            lo = max(0, q_first - window + 1) if window else 0
-            tiles.append(min(max_ctx_len - 1, q_first + 127) // 128 - lo // 128 + 1)
-    ctas, longest = n_heads * len(tiles), max(tiles)
-    split = prefill_split(sm_count, n_heads, len(lens), max(lens), max_ctx_len, window)
+            lo, hi = max(0, q_first - window + 1) if window else 0, min(max_ctx_len - 1, q_first + 127)
+            n64.append(hi // 64 - lo // 64 + 1)
+            n128.append(hi // 128 - lo // 128 + 1)
+    ctas, longest = n_heads * len(n128), max(n128)
+    form, split = 64, prefill_split(sm_count, n_heads, len(lens), max(lens), max_ctx_len, window)
     if longest >= 4 and (ctas <= sm_count or (2 * ctas <= 3 * sm_count and longest >= 16)):
-        return {"IB_HEAD_DIM": head_dim, "IB_ATTN_BN": 128}, split
-    return {"IB_HEAD_DIM": head_dim}, split
+        form = 128
+    if longest < 2 * ATTENTION_TC_PART_MIN_TILES or ctas > PREFILL_SIMULATED_CTAS:
+        return form, split
+
+    def estimate(tiles, parts, per_tile, start, slots):
+        jobs = []
+        for n in sorted(tiles, reverse=True):
+            k = max(1, min(parts, n // ATTENTION_TC_PART_MIN_TILES))
+            jobs += [per_tile * -(-n // k) + start + (3.0 if k > 1 else 0.0)] * (n_heads * k)
+        return _makespan(jobs, slots)
+    now = estimate(n128, split, 1.3, 3.0, sm_count) if form == 128 else estimate(n64, split, 1.0, 4.0, 2 * sm_count)
+    best = (0.96 * now, form, split)
+    for parts in range(1, ATTENTION_TC_MAX_SPLIT + 1):
+        if parts == 1 or ctas * parts * (128 * head_dim + 256) <= PREFILL_PARTS_MAX_FLOATS:
+            best = min(best, (estimate(n64, parts, 1.0, 4.0, 2 * sm_count), 64, parts))
+    return best[1], best[2]
 
 
 def attention_fast(q: torch.Tensor, k_cache: torch.Tensor, v_cache: torch.Tensor, block_table: torch.Tensor,
