@@ -11,7 +11,6 @@ SMS = 148
     (28, [2048], 2048, None, 64, (1,)),                # many CTAs: two an SM
     (12, [4096], 15873, None, 64, (3, 4)),             # a second round with 88 of 296 places filled, otherwise
     (12, [1024], 9216, None, 64, (3,)),
-    (12, [1, 1, 1], 700, None, 64, (1,)),              # single tokens only
 ])
 def test_forms_and_parts(heads, lens, ctx, window, form, parts):
     from infer_b200 import fast_ops
