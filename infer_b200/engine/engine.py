@@ -428,7 +428,7 @@ class Engine:
             if collecting:
                 gc.enable()
         graph = torch.cuda.CUDAGraph()
-        with torch.cuda.graph(graph, pool=self._graph_pool):
+        with torch.cuda.graph(graph, pool=self._graph_pool, stream=capture_stream(self.rt.device)):
             out = self._run_model(ctx)
         return graph, out
 
@@ -529,5 +529,6 @@ class Engine:
             what = {1: "a token id outside the table", 2: "a cache write through an invalid page",
                     3: "a cache read through an invalid page", 101: "a tensor-core GEMM's copy wait ran out",
                     102: "a tensor-core GEMM's operand wait ran out", 103: "a tensor-core GEMM's accumulator wait ran out",
+                    108: "the prefill attention's shared memory does not start on a 1024-byte boundary",
                     }.get(code, f"code {code}")
             raise RuntimeError(f"device status word was raised: {what}")
