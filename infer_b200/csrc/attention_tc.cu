@@ -25,7 +25,8 @@
 // Where few long query tiles would leave SMs idle (a portion of a prompt behind a long context), the key tiles of a
 // query tile are shared among up to four CTAs: each leaves its unnormalised rows of O, their reference maxima and sums
 // in a workspace, and the one that arrives last at the tile's counter adds the parts in index order and writes the
-// output (the host shares only while all CTAs still run at once: a CTA's start and end cost about three key tiles).
+// output (the host decides, by laying the CTAs onto the SMs: a CTA's start and end cost about four key tiles of 64, parts
+// that meet three more).
 //
 // A key tile's time is the softmax thread's own sequence (wait for S, read it, maximum, exponentials, wait for the previous
 // P V, store P): neither two threads per row nor a second MMA-issuing thread shortened it, and with one CTA an SM the tensor

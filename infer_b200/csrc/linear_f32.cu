@@ -12,7 +12,11 @@
 // 16-byte units are placed in an XOR pattern so that eight threads reading eight blocks side by side meet eight banks.
 // The ring's first weights are requested before the kernel waits for its predecessor.
 //
-// More rows, `tile32_kernel`: bound by the FMA units. Operands stay K-contiguous in shared memory (rows padded to 36
+// (17920 x 1536: 1 row 19 us = 5.8 TB/s, 3 rows 30, 8 rows 43, bound by the reads of x from shared memory; 1536 x 8960: 15, 25, 34.
+// A single token's step of the 1.5B sizes on tiles of 64 x 64 with scalar reads and no copies in flight took 55.6 ms, its products now 2.)
+//
+// More rows, `tile32_kernel`: bound by the FMA units, which run at 57 % (512 rows, 17920 x 1536: 670 us = 42 TFLOP/s; scalar FMAs
+// in the same order 730; the products of a 512-token step of the 1.5B sizes 37 ms, on the tiles before 88). Operands stay K-contiguous in shared memory (rows padded to 36
 // floats: eight rows read side by side meet eight banks); a 16-byte read feeds two packed FMAs without any shuffling
 // of halves, which is why a block's chains are even and odd k. Tiles of 64 x 64 (8 x 4 results a thread), or smaller ones
 // where those would leave SMs idle.
