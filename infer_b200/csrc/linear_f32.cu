@@ -10,7 +10,8 @@
 // one feature in every 256 elements of K and multiplies it with all rows of x, so w is read from HBM once, by coalesced
 // 16-byte asynchronous copies through a ring of stages, and nothing but the blocks' sums crosses threads. The copies'
 // 16-byte units are placed in an XOR pattern so that eight threads reading eight blocks side by side meet eight banks.
-// The ring's first weights are requested before the kernel waits for its predecessor.
+// Where the caller says that no kernel still running writes w (a loaded weight), the ring's first weights are requested before
+// the kernel waits for its predecessor.
 //
 // (17920 x 1536: 1 row 19 us = 5.8 TB/s, 3 rows 30, 8 rows 43, bound by the reads of x from shared memory; 1536 x 8960: 15, 25, 34.
 // A single token's step of the 1.5B sizes on tiles of 64 x 64 with scalar reads and no copies in flight took 55.6 ms, its products now 2.)
@@ -81,7 +82,7 @@ constexpr int gemv_smem() { return GSTAGES * (ROWS + MT) * GK * 4; }
 template <int ROWS, int MT, bool VEC>
 __global__ void __launch_bounds__(ROWS * GBLOCKS)
 gemv32_kernel(const float* __restrict__ x, const float* __restrict__ w, const float* __restrict__ bias, const float* residual,
-              float* out, int M, int64_t N, int64_t K) {
+              float* out, int M, int64_t N, int64_t K, int w_ready) {
     extern __shared__ __align__(128) float stages[];           // [GSTAGES][ROWS rows of w, MT rows of x][GK]
     constexpr int THREADS = ROWS * GBLOCKS, UNITS = GK / 4;
     __shared__ float sums[THREADS / 32][4][GBLOCKS][MT + 1];   // per warp: 4 features x 8 blocks x rows
@@ -108,7 +109,8 @@ gemv32_kernel(const float* __restrict__ x, const float* __restrict__ w, const fl
             copy_unit<VEC>(dst + uint32_t(r) * GK * 4u + unit_place(c), x, x + r * K, int64_t(step) * GK + 4 * c, K, r < M);
         }
     };
-    for (int s = 0; s < GSTAGES - 1 && s < steps; s++) load_w(s);        // no kernel writes the weights
+    if (!w_ready) ib::pdl_wait();
+    for (int s = 0; s < GSTAGES - 1 && s < steps; s++) load_w(s);
     ib::pdl_wait();
     for (int s = 0; s < GSTAGES - 1; s++) {
         if (s < steps) load_x(s);
@@ -239,6 +241,7 @@ struct Args {
     const float *x, *w, *bias, *residual;
     float* out;
     int64_t M, N, K;
+    int w_ready;
 };
 
 template <int ROWS, int MT, bool VEC>
@@ -246,7 +249,7 @@ int launch_gemv(const Args& a, cudaStream_t stream) {
     static const cudaError_t set = cudaFuncSetAttribute(gemv32_kernel<ROWS, MT, VEC>, cudaFuncAttributeMaxDynamicSharedMemorySize, gemv_smem<ROWS, MT>());
     if (set != cudaSuccess) return ib::fail(IB_ERR_CUDA, "linear_f32: cannot set shared memory size: %s", cudaGetErrorString(set));
     return ib::launch("linear_f32", gemv32_kernel<ROWS, MT, VEC>, dim3(unsigned((a.N + ROWS - 1) / ROWS)), dim3(ROWS * GBLOCKS),
-                      size_t(gemv_smem<ROWS, MT>()), stream, 1u, a.x, a.w, a.bias, a.residual, a.out, int(a.M), a.N, a.K);
+                      size_t(gemv_smem<ROWS, MT>()), stream, 1u, a.x, a.w, a.bias, a.residual, a.out, int(a.M), a.N, a.K, a.w_ready);
 }
 
 template <int ROWS, bool VEC>
@@ -299,14 +302,15 @@ int dispatch(const Args& a, int kind, int sms, cudaStream_t stream) {
 }  // namespace
 
 // kind: 0 = chosen from the sizes; 1, 2 = up to 8 rows with 16 / 8 features a CTA; 3, 4, 5 = tiles of 64 x 64, 32 x 64, 32 x 32.
-// Every kind gives the same bits. residual may be out.
+// Every kind gives the same bits. residual may be out. w_ready: 1 = no kernel that may still run writes w (it may be read before
+// this kernel's predecessor has ended), 0 = w may come from the predecessor.
 IB_EXPORT int ib_linear_f32(const float* x, const float* w, const float* bias, const float* residual, float* out, int64_t M, int64_t N,
-                            int64_t K, int kind, int sm_count, cudaStream_t stream) {
+                            int64_t K, int kind, int sm_count, int w_ready, cudaStream_t stream) {
     if (M <= 0 || N <= 0) return IB_OK;
     if (K <= 0) return ib::fail(IB_ERR_ARG, "linear_f32: K must be positive");
     const int64_t lim = 1LL << 31;
     if (N >= lim || K >= lim) return ib::fail(IB_ERR_ARG, "linear_f32: a size exceeds 2^31");
-    const Args a{x, w, bias, residual, out, M, N, K};
+    const Args a{x, w, bias, residual, out, M, N, K, w_ready};
     const int sms = sm_count > 0 ? sm_count : 148;
     const bool vec = K % 4 == 0 && ((uintptr_t(x) | uintptr_t(w)) & 15) == 0;
     return vec ? dispatch<true>(a, kind, sms, stream) : dispatch<false>(a, kind, sms, stream);

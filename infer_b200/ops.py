@@ -130,9 +130,10 @@ def rmsnorm(x: torch.Tensor, weight: torch.Tensor, eps: float, out_dtype: torch.
 
 def linear_plain(x: torch.Tensor, w: torch.Tensor, bias: Optional[torch.Tensor] = None,
                  residual: Optional[torch.Tensor] = None, out_dtype: Optional[torch.dtype] = None,
-                 out: Optional[torch.Tensor] = None, kind: int = 0) -> torch.Tensor:
+                 out: Optional[torch.Tensor] = None, kind: int = 0, w_ready: bool = False) -> torch.Tensor:
     """out = x @ w.T (+ bias) (+ residual) with float accumulation in an order that K alone fixes. kind: which of the
-    float32 kernels (0 = by the sizes; every one gives the same bits)."""
+    float32 kernels (0 = by the sizes; every one gives the same bits). w_ready: no kernel that may still be running writes
+    ``w`` (a loaded weight), so that it may be read while the kernels before this one drain."""
     _check(x, "x")
     _check(w, "w", x.dtype)
     M, K = x.shape
@@ -149,8 +150,8 @@ def linear_plain(x: torch.Tensor, w: torch.Tensor, bias: Optional[torch.Tensor] 
     else:
         _check(out, "out", out_dtype, (M, N))
     if x.dtype == torch.float32 and out_dtype == torch.float32:
-        f = _fn("lin32", "ib_linear_f32", [c_void_p] * 5 + [c_int64] * 3 + [c_int, c_int, c_void_p])
-        _call(f, x.data_ptr(), w.data_ptr(), _ptr(bias), _ptr(residual), out.data_ptr(), M, N, K, int(kind), 0, _stream())
+        f = _fn("lin32", "ib_linear_f32", [c_void_p] * 5 + [c_int64] * 3 + [c_int, c_int, c_int, c_void_p])
+        _call(f, x.data_ptr(), w.data_ptr(), _ptr(bias), _ptr(residual), out.data_ptr(), M, N, K, int(kind), 0, int(w_ready), _stream())
         return out
     f = _fn("plain", "ib_linear_plain", [c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_int64, c_int64, c_int64,
                                          c_int, c_int, c_void_p])

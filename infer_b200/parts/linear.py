@@ -68,4 +68,4 @@ class Linear:
                 return y
         if isinstance(x, DeferredNorm):
             x = x.materialize()
-        return ops.linear_plain(x, self.weight, self.bias, residual, out_dtype or self.rt.dtype, out)
+        return ops.linear_plain(x, self.weight, self.bias, residual, out_dtype or self.rt.dtype, out, w_ready=True)

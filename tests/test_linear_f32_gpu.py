@@ -27,3 +27,19 @@ def test_every_kernel_gives_the_same_bits(M, N, K, odd):
     assert torch.equal(ops.linear_plain(x[-1:].contiguous(), w, b, r[-1:].contiguous()), got[-1:])
     x[0, K // 2] = float("inf")
     assert not torch.isfinite(ops.linear_plain(x, w, b, r)[0]).any() and torch.equal(ops.linear_plain(x, w, b, r)[1:], got[1:])
+
+
+@pytest.mark.parametrize("M,N,K", [(1, 2048, 1536), (3, 40, 64), (8, 4096, 260), (9, 2048, 1536)])
+def test_a_matrix_that_the_kernel_before_has_just_written(M, N, K):
+    """w is itself a product: nothing of it may be read before the kernel that writes it has ended, whatever was there before."""
+    from infer_b200 import ops
+    gen = torch.Generator(device=DEV).manual_seed(M + N + K)
+    x, a, b = (torch.randn(n, k, generator=gen, device=DEV) for n, k in ((M, K), (N, 1000), (K, 1000)))
+    w = ops.linear_plain(a, b)
+    torch.cuda.synchronize()
+    want = ops.linear_plain(x, w)
+    torch.cuda.synchronize()
+    for _ in range(20):
+        again = torch.full_like(w, float("nan"))
+        assert torch.equal(ops.linear_plain(x, ops.linear_plain(a, b, out=again)), want)
+    assert torch.equal(ops.linear_plain(x, w, w_ready=True), want)
