@@ -236,11 +236,6 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_co
             }
             if (valid > 0) { if (which) pend_v[j & 1] = j; else pend_k[j & 1] = j; }
         };
-        auto wait_all = [&](uint32_t bar, uint32_t parity) -> bool {      // lane 0 waits, every lane learns the outcome
-            int got = 1;
-            if (lane == 0) got = mbar_wait(bar, parity) ? 1 : 0;
-            return __shfl_sync(0xffffffffu, got, 0) != 0;
-        };
         const int id0 = page_id(0), id1 = page_id(1);
         int ahead = page_id(2);
         load_tile(0, 0, id0);
@@ -252,11 +247,11 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_co
             const int id = ahead;
             ahead = page_id(j + 3);
             if (j + 2 < n_tiles) {                       // S(j) is complete: its K buffer takes tile j + 2
-                if (!wait_all(k_empty + 8 * (j & 1), (j >> 1) & 1)) { failed = true; break; }
+                if (!mbar_wait_warp(k_empty + 8 * (j & 1), (j >> 1) & 1)) { failed = true; break; }
                 load_tile(j + 2, 0, id);
             }
             if (j + 2 < n_tiles) {                       // P(j) V(j) is complete: its V buffer takes tile j + 2
-                if (!wait_all(v_empty + 8 * (j & 1), (j >> 1) & 1)) { failed = true; break; }
+                if (!mbar_wait_warp(v_empty + 8 * (j & 1), (j >> 1) & 1)) { failed = true; break; }
                 load_tile(j + 2, 1, id);
             }
         }
@@ -277,7 +272,7 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_co
         const bool leader = elect_one();
         // S(j) = Q K(j)^T into S buffer j & 1
         auto issue_qk = [&](int j) -> bool {
-            if (!mbar_wait(k_full + 8 * (j & 1), (j >> 1) & 1)) return false;
+            if (!mbar_wait_each(k_full + 8 * (j & 1), (j >> 1) & 1)) return false;
             tc_fence_after();
             const uint32_t s_tmem = tmem_base + S_COL + (j & 1) * BN, kb = k_s + (j & 1) * K_BYTES;
             if (leader) {
@@ -295,9 +290,9 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_co
             IB_T(j, 6);
             return true;
         };
-        bool ok = mbar_wait(q_full, 0) && issue_qk(0) && (n_tiles < 2 || issue_qk(1));
+        bool ok = mbar_wait_each(q_full, 0) && issue_qk(0) && (n_tiles < 2 || issue_qk(1));
         for (int j = 0; j < n_tiles && ok; j++) {
-            ok = mbar_wait(p_full, j & 1) && mbar_wait(v_full + 8 * (j & 1), (j >> 1) & 1);
+            ok = mbar_wait_each(p_full, j & 1) && mbar_wait_each(v_full + 8 * (j & 1), (j >> 1) & 1);
             if (!ok) break;
             tc_fence_after();
             if (leader) {

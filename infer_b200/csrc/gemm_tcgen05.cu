@@ -35,6 +35,7 @@
 // Every wait on an mbarrier is bounded; a wait that runs out raises the status word, and the CTA drains its
 // copies, frees its TMEM and returns.
 #include "common.cuh"
+#include "tc_ops.cuh"
 #include "tma_map.cuh"
 
 #include <cuda.h>
@@ -52,7 +53,6 @@ constexpr int BM = 128;            // tile rows on the A side = TMEM lanes
 constexpr int BK = 64;             // bf16 elements per stage row = one 128-byte swizzle line
 constexpr int UMMA_K = 16;
 constexpr int NUM_THREADS = 192;
-constexpr uint32_t WAIT_LIMIT = 1u << 20;
 
 constexpr int STATUS_TIMEOUT_PRODUCER = 101, STATUS_TIMEOUT_MMA = 102, STATUS_TIMEOUT_EPILOGUE = 103;
 
@@ -66,32 +66,12 @@ __device__ __forceinline__ void mbar_init(uint32_t bar, uint32_t count) {
 __device__ __forceinline__ void mbar_expect_tx(uint32_t bar, uint32_t bytes) {
     asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(bytes) : "memory");
 }
-// Bounded wait: the thread sleeps in hardware until the phase completes or about a microsecond has passed, again and again
-// (of the order of a second altogether); false if the phase did not complete. Probing in a loop instead kept the shared
-// memory's port busy: with 128 epilogue threads at it a chain of MMAs ran a tenth slower.
-__device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity) {
-    for (uint32_t i = 0; i < WAIT_LIMIT; i++) {
-        uint32_t ok;
-        asm volatile(
-            "{\n\t.reg .pred p;\n\t"
-            "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2, %3;\n\t"
-            "selp.u32 %0, 1, 0, p;\n\t}"
-            : "=r"(ok) : "r"(bar), "r"(parity), "r"(1000u) : "memory");
-        if (ok) return true;
-    }
-    return false;
-}
-// The same for a whole warp, of which one lane waits.
-__device__ __forceinline__ bool warp_mbar_wait(uint32_t bar, uint32_t parity) {
-    int ok = 1;
-    if ((threadIdx.x & 31) == 0) ok = mbar_wait(bar, parity) ? 1 : 0;
-    return __shfl_sync(0xffffffffu, ok, 0) != 0;
-}
-__device__ __forceinline__ bool elect_one() {
-    uint32_t p;
-    asm volatile("{\n\t.reg .pred P;\n\telect.sync _|P, 0xffffffff;\n\tselp.u32 %0, 1, 0, P;\n\t}" : "=r"(p));
-    return p != 0;
-}
+// Waits are bounded and sleep in hardware (tc_ops.cuh). Probing in a loop instead kept the shared memory's port busy: with 128
+// epilogue threads at it a chain of MMAs ran a tenth slower.
+using ib::tc::mbar_wait;
+using ib::tc::mbar_wait_each;
+using ib::tc::mbar_wait_warp;
+using ib::tc::elect_one;
 __device__ __forceinline__ void fence_barrier_init() { asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory"); }
 __device__ __forceinline__ void fence_proxy_async() { asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); }
 
@@ -521,7 +501,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant__
         uint32_t parity = 0;
         bool ok = true;
         for (int i = 0; i < n_kb; i++) {
-            if (!mbar_wait(full_bar(s), parity)) { ok = false; break; }
+            if (!mbar_wait_each(full_bar(s), parity)) { ok = false; break; }
             if (lane == 0 && i == 0) IB_MT(5);
             if (lane == 0 && i == n_kb / 2) IB_MT(6);
             const uint32_t a_addr = base + s * C::STAGE_BYTES;
@@ -559,7 +539,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant__
                 }
             }
         }
-        const bool ok = warp_mbar_wait(tmem_full_bar, 0);
+        const bool ok = mbar_wait_warp(tmem_full_bar, 0);
         if (!ok) { atomicExch(p.status, STATUS_TIMEOUT_EPILOGUE); slots[1] = 1; }
         tc_fence_after();
         if (threadIdx.x == 64) IB_MT(8);
@@ -871,11 +851,11 @@ gemm_tc_persistent_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid
         tiles_in_use();
         for (int tile = blockIdx.x; tile < n_tiles && ok; tile += gridDim.x, lt++) {
             const int b = lt & 1;
-            if (lt >= 2 && !mbar_wait(acc_empty_bar(b), ((lt >> 1) - 1) & 1)) { ok = false; break; }      // the epilogue has drained it
+            if (lt >= 2 && !mbar_wait_each(acc_empty_bar(b), ((lt >> 1) - 1) & 1)) { ok = false; break; }      // the epilogue has drained it
             tc_fence_after();
             const uint32_t d0 = tmem_base + uint32_t(b * 256), d1 = d0 + 128u;
             for (int kb = 0; kb < n_kb; kb++) {
-                if (!mbar_wait(full_bar(s), parity)) { ok = false; break; }
+                if (!mbar_wait_each(full_bar(s), parity)) { ok = false; break; }
                 const uint32_t a_addr = base + s * P_STAGE_BYTES;
                 const uint64_t a0 = make_desc(a_addr), a1 = make_desc(a_addr + 128 * BK * 2), bd = make_desc(a_addr + A_BYTES);
                 if (leader) {
@@ -909,7 +889,7 @@ gemm_tc_persistent_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid
             ra.on = p.epi == 0 && p.residual != nullptr && (p.N & 7) == 0 && row0 < p.M;
             residual_request<TN>(p, ra, row0, n_base, 0);
             bool ok = __all_sync(0xffffffffu, !slots[1]);
-            if (ok && !warp_mbar_wait(acc_full_bar(b), (lt >> 1) & 1)) { atomicExch(p.status, STATUS_TIMEOUT_EPILOGUE); slots[1] = 1; ok = false; }
+            if (ok && !mbar_wait_warp(acc_full_bar(b), (lt >> 1) & 1)) { atomicExch(p.status, STATUS_TIMEOUT_EPILOGUE); slots[1] = 1; ok = false; }
             if (!ok) break;
             tc_fence_after();
             const uint32_t taddr = tmem_base + (uint32_t(quad * 32) << 16) + uint32_t(b * 256);
@@ -1069,11 +1049,11 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_const
             bool ok = true;
             for (int tile = pair; tile < n_tiles && ok; tile += pairs, lt++) {
                 const int b = lt & 1;
-                if (lt >= 2 && !mbar_wait(acc_empty_bar(b), ((lt >> 1) - 1) & 1)) { ok = false; break; }      // both epilogues have drained it
+                if (lt >= 2 && !mbar_wait_each(acc_empty_bar(b), ((lt >> 1) - 1) & 1)) { ok = false; break; }      // both epilogues have drained it
                 tc_fence_after();
                 const uint32_t d = tmem_base + uint32_t(b * 256);
                 for (int kb = 0; kb < n_kb; kb += 2) {
-                    if (!mbar_wait(full_bar(s), parity)) { ok = false; break; }
+                    if (!mbar_wait_each(full_bar(s), parity)) { ok = false; break; }
                     const uint32_t a_addr = base + s * C::STAGE_BYTES;
                     const uint64_t ad = make_desc(a_addr), bd = make_desc(a_addr + 2 * A_BYTES);
                     if (leader) {
@@ -1107,7 +1087,7 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_const
             ra.on = p.epi == 0 && p.residual != nullptr && (p.N & 7) == 0 && row < p.M;
             residual_request<PN>(p, ra, row, n_base, 0);
             bool ok = __all_sync(0xffffffffu, !slots[1]);
-            if (ok && !warp_mbar_wait(acc_full_bar(b), (lt >> 1) & 1)) { atomicExch(p.status, STATUS_TIMEOUT_EPILOGUE); slots[1] = 1; ok = false; }
+            if (ok && !mbar_wait_warp(acc_full_bar(b), (lt >> 1) & 1)) { atomicExch(p.status, STATUS_TIMEOUT_EPILOGUE); slots[1] = 1; ok = false; }
             if (!ok) break;
             tc_fence_after();
             drain_row<TOut, PN>(p, tmem_base + (uint32_t(quad * 32) << 16) + uint32_t(b * 256), row, n_base, ra);

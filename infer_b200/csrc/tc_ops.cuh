@@ -22,8 +22,8 @@ __device__ __forceinline__ void mbar_arrive(uint32_t bar) {
 }
 // Bounded wait (of the order of a second): the thread sleeps in hardware until the phase completes or about a microsecond has
 // passed, again and again; false if the phase did not complete. (Probing in a loop takes the shared memory's port.)
-__device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity) {
-    for (uint32_t i = 0; i < WAIT_LIMIT; i++) {
+__device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, uint32_t limit = WAIT_LIMIT) {
+    for (uint32_t i = 0; i < limit; i++) {
         uint32_t ok;
         asm volatile(
             "{\n\t.reg .pred p;\n\t"
@@ -33,6 +33,20 @@ __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity) {
         if (ok) return true;
     }
     return false;
+}
+// Two forms for a whole warp (all 32 lanes come). Every lane learns the same outcome: a wait may run out for some lanes and not
+// for others, and lanes that leave a loop by themselves leave the rest at the warp's next barrier for good.
+// mbar_wait_each: every lane waits, so that whichever of them is elected to issue has itself seen the phase complete.
+__device__ __forceinline__ bool mbar_wait_each(uint32_t bar, uint32_t parity, uint32_t limit = WAIT_LIMIT) {
+    return __all_sync(0xffffffffu, mbar_wait(bar, parity, limit)) != 0;
+}
+// mbar_wait_warp: lane 0 waits, and the warp's barrier orders what it has seen before what the others do next (a shuffle alone
+// orders no memory).
+__device__ __forceinline__ bool mbar_wait_warp(uint32_t bar, uint32_t parity, uint32_t limit = WAIT_LIMIT) {
+    int ok = 1;
+    if ((threadIdx.x & 31) == 0) ok = mbar_wait(bar, parity, limit) ? 1 : 0;
+    __syncwarp();
+    return __shfl_sync(0xffffffffu, ok, 0) != 0;
 }
 __device__ __forceinline__ bool elect_one() {
     uint32_t p;
