@@ -103,8 +103,9 @@ struct Params {
     // that way, and the heaviest tile of a causal prompt no longer sets the kernel's time alone.
     int early_release;                       // 1: the successor is released at the kernel's start (few CTAs: a short kernel)
     int split;
-    float* workspace;                        // [segments of two or more tokens][heads][query tiles][split][PART_FLOATS]
-    unsigned int* counters;                  // [segments of two or more tokens][heads][query tiles], zero between launches
+    int64_t slots;                           // query tiles (of all heads) that the scratch has room for; one beyond stays whole
+    float* workspace;                        // [query tiles of the segments of two or more tokens, per segment heads x its own][split][PART_FLOATS]
+    unsigned int* counters;                  // one for each of those, zero between launches
     // Optional. A bias per (head, distance) added to the scaled score of query i and key j: bias[h * bias_len +
     // min(i - j, bias_len - 1)], stored divided by the scale, so that it is added to the raw score. A sink per head:
     // a logit without key or value that enters the softmax denominator once (the part that holds the first keys counts it).
@@ -159,20 +160,24 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_co
     const int keep_end = min(p.keep_first, lo_key);      // keys below it are seen although the window has passed them
     const int n_keep = min((keep_end + BN - 1) / BN, all0);   // tiles of kept keys wholly before the window's first tile
     const int n_all = n_keep + all1 - all0 + 1;
-    const int n_parts = max(1, min(p.split, n_all / PART_MIN_TILES));
+    int n_parts = max(1, min(p.split, n_all / PART_MIN_TILES));
+    // Scratch is laid out over the query tiles that exist: a step may carry dozens of one-token segments and short portions
+    // beside one long portion. Those of the segments before this one are counted from the segment table.
+    int64_t tile_id = 0;
+    if (n_parts > 1) {
+        int before = 0;
+        for (int s2 = 0; s2 < seg; s2++) {
+            const int n = p.seg_start[s2 + 1] - p.seg_start[s2];
+            before += n > 1 ? (n + BM - 1) / BM : 0;
+        }
+        tile_id = int64_t(before) * p.n_heads + h * ((q_len + BM - 1) / BM) + qt;
+        if (tile_id >= p.slots) n_parts = 1;             // (the same for every part of the tile)
+    }
     if (part >= n_parts) return;
     // a CTA's tiles are numbered along the list [kept tiles | the window's tiles]
     const int lt0 = (n_all * part) / n_parts, lt1 = (n_all * (part + 1)) / n_parts - 1;
     const int n_tiles = lt1 - lt0 + 1;                   // >= PART_MIN_TILES when the tile is shared, >= 1 otherwise
     auto tile_of = [&](int j) -> int { const int lt = lt0 + j; return lt < n_keep ? lt : all0 + lt - n_keep; };
-    // Scratch is laid out over the segments that have two or more tokens only (a step may carry dozens of one-token
-    // segments beside one portion): this segment's rank among those, counted from the segment table.
-    int tile_id = 0;
-    if (n_parts > 1) {
-        int before = 0;
-        for (int s2 = 0; s2 < seg; s2++) before += (p.seg_start[s2 + 1] - p.seg_start[s2] > 1) ? 1 : 0;
-        tile_id = (before * p.n_heads + h) * n_qt + qt;
-    }
     const int* table = p.block_table + int64_t(seg) * p.max_blocks;
     auto page_at = [&](int idx) -> int {                 // entry idx of the segment's table, or -1
         if (idx >= p.max_blocks) return -1;
@@ -471,7 +476,7 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_co
         } else {
             // Every softmax warp goes through both barriers whatever happened to it, so that a failed wait in one warp
             // (the status word is raised then) cannot leave the others waiting; the counter is always brought back to 0.
-            float* parts = p.workspace + int64_t(tile_id) * p.split * PART_FLOATS;
+            float* parts = p.workspace + tile_id * p.split * PART_FLOATS;
             float* mine = parts + part * PART_FLOATS;
             if (ok) {
                 tc_fence_after();
@@ -544,13 +549,13 @@ IB_EXPORT int ib_attention_tc_head_dim() { return HD; }
 // q, out: bfloat16 [tokens, heads * HD]; caches bfloat16 [pages, kv heads, 16, HD] holding this step's keys and values
 // already; block_table int32 [segments, max_blocks]; seg_start int32 [segments + 1]; seg_pos0 int32 [segments].
 // split: up to how many CTAs share the key tiles of one query tile (1: none); it is lowered to what the workspace
-// (floats) and the counters (zero before and after) have room for: one slot per segment of two or more tokens
-// (n_long_segments of them; 0: assume all), head and query tile.
+// (floats) and the counters (zero before and after) have room for: one slot per head and query tile of the segments of two
+// or more tokens (n_query_tiles of them altogether; 0: assume that every segment has as many as the longest).
 static int prefill_tc(const void* q, const void* k_cache, const void* v_cache, void* out, const int* block_table,
                       int max_blocks, const int* seg_start, const int* seg_pos0, int n_segments, int64_t n_tokens,
                       int n_heads, int n_kv, int head_dim, int page_size, int window, float scale, int64_t n_pages,
                       int max_q_len, int* status, cudaStream_t stream, int split, float* workspace,
-                      int64_t workspace_floats, unsigned int* counters, int64_t n_counters, int n_long_segments,
+                      int64_t workspace_floats, unsigned int* counters, int64_t n_counters, int n_query_tiles,
                       const float* bias, int bias_len, const float* sink, int keep_first = 0, const float* slopes = nullptr) {
     if (n_segments <= 0 || max_q_len <= 1) return IB_OK;
     if (slopes && !(scale > 0.0f)) return ib::fail(IB_ERR_ARG, "attention_tc: slopes need a positive scale");
@@ -582,13 +587,13 @@ static int prefill_tc(const void* q, const void* k_cache, const void* v_cache, v
     p.bias = bias; p.bias_len = bias_len; p.sink = sink;
     p.keep_first = (window > 0 && keep_first > 0) ? keep_first : 0; p.slopes = slopes;
     // Sharing query tiles needs scratch for every (segment, head, query tile); with less than that, fewer parts.
-    if (n_long_segments <= 0 || n_long_segments > n_segments) n_long_segments = n_segments;
-    const int64_t n_qt = (max_q_len + BM - 1) / BM, tiles = int64_t(n_long_segments) * n_heads * n_qt;
+    const int64_t n_qt = (max_q_len + BM - 1) / BM;
+    const int64_t tiles = (n_query_tiles > 0 && n_query_tiles < n_segments * n_qt ? n_query_tiles : n_segments * n_qt) * n_heads;
     split = std::max(1, std::min(split, MAX_SPLIT));
     if (!workspace || !counters || tiles > n_counters) split = 1;
     while (split > 1 && tiles * split * PART_FLOATS > workspace_floats) split--;
     if (n_qt * split > 65535) split = 1;
-    p.split = split; p.workspace = workspace; p.counters = counters;
+    p.split = split; p.slots = tiles; p.workspace = workspace; p.counters = counters;
     p.early_release = int64_t(n_segments) * n_heads * n_qt * split <= 296 ? 1 : 0;
     const dim3 grid{unsigned(n_heads), unsigned(n_qt * split), unsigned(n_segments)};
     return ib::launch("attention_tc", attn_prefill_tc_kernel, grid, dim3(NUM_THREADS), size_t(SMEM_BYTES), stream, 1u, mq, mk, mv, p);
@@ -598,10 +603,10 @@ IB_EXPORT int ib_attention_prefill_tc(const void* q, const void* k_cache, const 
                                       int max_blocks, const int* seg_start, const int* seg_pos0, int n_segments, int64_t n_tokens,
                                       int n_heads, int n_kv, int head_dim, int page_size, int window, float scale, int64_t n_pages,
                                       int max_q_len, int* status, cudaStream_t stream, int split, float* workspace,
-                                      int64_t workspace_floats, unsigned int* counters, int64_t n_counters, int n_long_segments) {
+                                      int64_t workspace_floats, unsigned int* counters, int64_t n_counters, int n_query_tiles) {
     return prefill_tc(q, k_cache, v_cache, out, block_table, max_blocks, seg_start, seg_pos0, n_segments, n_tokens, n_heads, n_kv,
                       head_dim, page_size, window, scale, n_pages, max_q_len, status, stream, split, workspace, workspace_floats,
-                      counters, n_counters, n_long_segments, nullptr, 0, nullptr);
+                      counters, n_counters, n_query_tiles, nullptr, 0, nullptr);
 }
 
 // The same with a bias per (head, distance), float [heads, bias_len], ALREADY DIVIDED by the scale (it is added to the
@@ -610,11 +615,11 @@ IB_EXPORT int ib_attention_prefill_tc_biased(const void* q, const void* k_cache,
                                              int max_blocks, const int* seg_start, const int* seg_pos0, int n_segments, int64_t n_tokens,
                                              int n_heads, int n_kv, int head_dim, int page_size, int window, float scale, int64_t n_pages,
                                              int max_q_len, int* status, cudaStream_t stream, int split, float* workspace,
-                                             int64_t workspace_floats, unsigned int* counters, int64_t n_counters, int n_long_segments,
+                                             int64_t workspace_floats, unsigned int* counters, int64_t n_counters, int n_query_tiles,
                                              const float* bias, int bias_len, const float* sink) {
     return prefill_tc(q, k_cache, v_cache, out, block_table, max_blocks, seg_start, seg_pos0, n_segments, n_tokens, n_heads, n_kv,
                       head_dim, page_size, window, scale, n_pages, max_q_len, status, stream, split, workspace, workspace_floats,
-                      counters, n_counters, n_long_segments, bias, bias_len, sink);
+                      counters, n_counters, n_query_tiles, bias, bias_len, sink);
 }
 
 // The same with, beside bias and sink, kept first keys (with a window: every query also sees the keys below keep_first)
@@ -623,11 +628,11 @@ IB_EXPORT int ib_attention_prefill_tc_kept(const void* q, const void* k_cache, c
                                            int max_blocks, const int* seg_start, const int* seg_pos0, int n_segments, int64_t n_tokens,
                                            int n_heads, int n_kv, int head_dim, int page_size, int window, float scale, int64_t n_pages,
                                            int max_q_len, int* status, cudaStream_t stream, int split, float* workspace,
-                                           int64_t workspace_floats, unsigned int* counters, int64_t n_counters, int n_long_segments,
+                                           int64_t workspace_floats, unsigned int* counters, int64_t n_counters, int n_query_tiles,
                                            const float* bias, int bias_len, const float* sink, int keep_first, const float* slopes) {
     return prefill_tc(q, k_cache, v_cache, out, block_table, max_blocks, seg_start, seg_pos0, n_segments, n_tokens, n_heads, n_kv,
                       head_dim, page_size, window, scale, n_pages, max_q_len, status, stream, split, workspace, workspace_floats,
-                      counters, n_counters, n_long_segments, bias, bias_len, sink, keep_first, slopes);
+                      counters, n_counters, n_query_tiles, bias, bias_len, sink, keep_first, slopes);
 }
 
 #ifdef IB_ATTN_TRACE

@@ -389,6 +389,19 @@ PREFILL_PARTS_MAX_FLOATS = 24 << 20      # of scratch that sharing query tiles m
 PREFILL_SIMULATED_CTAS = 1024            # beyond that many CTAs they even out by themselves
 
 
+def prefill_query_tiles(seg_lens) -> int:
+    """Query tiles of 128 tokens that a head has in the segments of two or more tokens."""
+    return sum(-(-n // 128) for n in seg_lens if n > 1)
+
+
+def prefill_scratch(st, n_heads: int, head_dim: int, query_tiles: int, parts: int):
+    """(workspace, counters) in which the parts of query tiles meet, for ``query_tiles`` of them per head; (None, None) for whole ones."""
+    if parts <= 1:
+        return None, None
+    tiles = max(1, query_tiles) * n_heads
+    return st.workspace(tiles * parts * (128 * head_dim + 256)), st.counters(tiles)
+
+
 def _makespan(jobs, slots: int) -> float:
     """When the last of ``jobs`` (durations, started in this order) ends on ``slots`` workers."""
     if len(jobs) <= slots:
@@ -480,16 +493,16 @@ def attention_fast(q: torch.Tensor, k_cache: torch.Tensor, v_cache: torch.Tensor
         split = split if tc_split is None else tc_split
         g = _fn("attn_tc", "ib_attention_prefill_tc", [c_void_p] * 5 + [c_int] + [c_void_p] * 2 + [c_int, c_int64] + [c_int] * 5 +
                 [c_float, c_int64, c_int] + [c_void_p] * 2 + [c_int, c_void_p, c_int64, c_void_p, c_int64, c_int], defines)
-        tc_ws = tc_cnt = None
+        # (without the lengths every segment that may have two or more tokens counts as the longest one)
+        query_tiles = prefill_query_tiles(seg_lens or [max_q_len] * max(1, n_prefill))
+        tc_ws, tc_cnt = prefill_scratch(st, n_heads, head_dim, query_tiles, split)
         if split > 1:
-            tiles = max(1, n_prefill) * n_heads * -(-max_q_len // 128)
-            tc_ws, tc_cnt = st.workspace(tiles * split * (128 * head_dim + 256)), st.counters(tiles)
             ops.note("attention_prefill_tc:shared_query_tiles")
         _call(g, q.data_ptr(), k_cache.data_ptr(), v_cache.data_ptr(), out.data_ptr(), block_table.data_ptr(),
               block_table.shape[1], seg_start.data_ptr(), seg_pos0.data_ptr(), S, T, n_heads, n_kv, head_dim, page_size,
               int(window or 0), float(scale), n_pages, int(max_q_len), st.status.data_ptr(), _stream(), int(split),
               _ptr(tc_ws), 0 if tc_ws is None else tc_ws.numel(), _ptr(tc_cnt), 0 if tc_cnt is None else tc_cnt.numel(),
-              int(n_prefill) if n_decode is not None else 0)
+              int(query_tiles))
         if max_q_len > 128:
             ops.note("attention_prefill_tc:several_query_tiles")
         if not has_decode:
@@ -528,12 +541,9 @@ def attention_prefill_biased(q, k_cache, v_cache, block_table, step, n_heads, n_
         _check(slopes, "slopes", torch.float32, (n_heads,))
     S = step.seg_pos0.numel()
     st = device_state(q.device)
-    n_prefill = sum(1 for n in step.seg_lens if n > 1)
     defines, split = prefill_plan(st.sm_count, n_heads, head_dim, step.seg_lens, step.max_ctx_len, window)
-    tc_ws = tc_cnt = None
-    if split > 1:
-        tiles = max(1, n_prefill) * n_heads * -(-step.max_q_len // 128)
-        tc_ws, tc_cnt = st.workspace(tiles * split * (128 * head_dim + 256)), st.counters(tiles)
+    query_tiles = prefill_query_tiles(step.seg_lens)
+    tc_ws, tc_cnt = prefill_scratch(st, n_heads, head_dim, query_tiles, split)
     out = torch.empty_like(q)
     keep_first = int(keep_first or 0) if window else 0
     kept = keep_first > 0 or slopes is not None                 # (the entry point that takes them; the other is unchanged)
@@ -544,7 +554,7 @@ def attention_prefill_biased(q, k_cache, v_cache, block_table, step, n_heads, n_
     args = [q.data_ptr(), k_cache.data_ptr(), v_cache.data_ptr(), out.data_ptr(), block_table.data_ptr(), block_table.shape[1],
             step.seg_start.data_ptr(), step.seg_pos0.data_ptr(), S, T, n_heads, n_kv, head_dim, page_size, int(window or 0), float(scale),
             n_pages, int(step.max_q_len), st.status.data_ptr(), _stream(), int(split), _ptr(tc_ws), 0 if tc_ws is None else tc_ws.numel(),
-            _ptr(tc_cnt), 0 if tc_cnt is None else tc_cnt.numel(), int(n_prefill), _ptr(bias_by_head),
+            _ptr(tc_cnt), 0 if tc_cnt is None else tc_cnt.numel(), int(query_tiles), _ptr(bias_by_head),
             0 if bias_by_head is None else bias_by_head.shape[1], _ptr(sink)]
     _call(g, *(args + ([keep_first, _ptr(slopes)] if kept else [])))
     return out

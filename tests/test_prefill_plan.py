@@ -34,3 +34,23 @@ def test_makespan():
     from infer_b200.fast_ops import _makespan
     assert _makespan([3.0, 2.0], 4) == 3.0
     assert _makespan([3.0, 3.0, 2.0, 2.0, 1.0], 2) == 6.0
+
+
+@pytest.mark.parametrize("heads,lens,ctx", [(12, [3346] + list(range(2, 101, 3)), 26219), (12, [3000] + [30] * 30, 16384), (12, [900] + [100] * 10, 8192),
+                                            (28, [512, 2, 2, 2], 9000), (64, [2048] + [2] * 40, 30000)])
+def test_scratch_of_ragged_portions_stays_within_its_limit(heads, lens, ctx):
+    """What the plan compares with the limit is what a launch asks for: the query tiles that exist, not every portion at the longest one's."""
+    from infer_b200 import fast_ops
+
+    class State:
+        def workspace(self, n):
+            self.floats = n
+
+        def counters(self, n):
+            self.n = n
+    _, parts = fast_ops.prefill_plan(SMS, heads, 128, lens, ctx, None)
+    st = State()
+    fast_ops.prefill_scratch(st, heads, 128, fast_ops.prefill_query_tiles(lens), max(parts, 2))
+    assert st.n == heads * sum(-(-n // 128) for n in lens)
+    assert st.floats == st.n * max(parts, 2) * (128 * 128 + 256)
+    assert parts == 1 or st.floats <= fast_ops.PREFILL_PARTS_MAX_FLOATS
