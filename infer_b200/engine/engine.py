@@ -317,9 +317,10 @@ class Engine:
         mode = 0 if sample is None else (2 if filtered else 1)
         entry = run = None
         key = None
+        may_capture = graphs and (T == S or T <= PORTION_GRAPH_MAX_TOKENS)
         if graphs and T == S:
             key = (S, n_want, tuple(widths), mode)
-        elif graphs and T <= PORTION_GRAPH_MAX_TOKENS:
+        elif may_capture:
             pkey = ("portions", tuple(seg_lens), n_want, tuple(widths), mode)
             if pkey in self._graphs:
                 key = pkey
@@ -379,9 +380,10 @@ class Engine:
             feedback=self.next_tokens, status=self.status, seg_lens=seg_lens, seg_pos0_host=pos0, max_q_len=max(seg_lens),
             max_ctx_len=max(p + n for p, n in zip(pos0, seg_lens)), decode_only=all(n == 1 for n in seg_lens),
             sampling=sampling)
-        if entry is not None or run is not None:
-            # a graph's launch shapes must not depend on the step: bound the context by the table width (also in the eager run
-            # before it, which sizes the kernels' scratch)
+        if may_capture:
+            # a graph's launch shapes must not depend on the step: bound the context by the table width. Also in the eager runs of
+            # a shape that may come as a graph: they size the kernels' scratch, and how a kernel divides its work, and so the order
+            # of its sums, follows from the bound. (When a shape is captured follows from measured times; its bits may not.)
             ctx.max_ctx_len = max(widths) * cache.page_size if widths else ctx.max_ctx_len
         ctx.measured = run
         return ctx, entry

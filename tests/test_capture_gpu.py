@@ -42,3 +42,39 @@ def test_streams_of_captures_and_side_branches_differ():
     handles = [s.cuda_stream for s in (*sides, fast_ops.capture_stream(device), fast_ops.own_stream(device))]
     assert len(set(handles)) == 4
     assert fast_ops.capture_stream(device) is fast_ops.capture_stream(device)
+
+
+# ------------------------------------------------------------------------------------------------ what decides the bits of a step
+
+def _one_layer(heads, kv):
+    return dict(architectures=["Qwen2ForCausalLM"], hidden_size=heads * 128, num_hidden_layers=1, num_attention_heads=heads,
+                num_key_value_heads=kv, intermediate_size=256, vocab_size=320, rope_theta=1000000.0, rms_norm_eps=1e-6,
+                max_position_embeddings=4096, tie_word_embeddings=True)
+
+
+# (contexts that are no multiple of a page or a tile, where the attention's form or parts for the true context are not those for the
+# table's width: (64 keys, 3 parts) and (128, 1); (128, 4) and (64, 3))
+@pytest.mark.parametrize("heads,kv,first,n", [(12, 2, 915, 2048), (28, 4, 732, 300)])
+def test_bits_of_a_portion_do_not_depend_on_what_was_captured(heads, kv, first, n, monkeypatch):
+    """Whether a shape is captured, and when, follows from measured times; the step's result may not."""
+    from infer_b200 import Engine, StepEntry
+    from infer_b200.engine import engine as module
+    cfg = _one_layer(heads, kv)
+    ids = H.random_ids(cfg, first + n, heads)
+    results = []
+    for worth in (True, False):
+        def decide(self, ms_per_launch, worth=worth):
+            if self.launches:                            # (it has run eagerly once, as every shape does first)
+                self.worth = worth
+            return bool(self.worth)
+        monkeypatch.setattr(module._PortionRun, "decide", decide)
+        eng = Engine(H.spec_of(cfg), H.make_weights(cfg, 3), max_tokens=4096, max_requests=1)
+        for _ in range(module.PORTION_GRAPH_LATER + 2):
+            eng.add_request("r")
+            eng.step([StepEntry("r", ids[:first], [])])
+            results.append(eng.step([StepEntry("r", ids[first:], [0, n // 2, n - 1])]).clone())
+            eng.end_request("r")
+        eng.check_status()
+        assert eng._graphs
+    for i, r in enumerate(results[1:]):
+        assert torch.equal(r, results[0]), f"pass {i + 1}"
