@@ -98,6 +98,7 @@ def _round_up(x: int, m: int) -> int:
 FEEDBACK_TOKEN = -1           # as a decode entry's token: "what the sampler produced last for this request"
 GRAPH_WIDTH_PAGES = 32        # decode-only block tables are padded to a multiple of this many pages (512 positions)
 GRAPH_WARMUP_STEPS = 1        # eager steps of a shape before its graph is captured (libraries, workspaces, attributes)
+GRAPH_RETRY_STEPS = 64        # eager steps of a shape after a capture that found no memory
 MAX_GRAPHS = 48
 GRAPH_COPIES = 2              # executable copies per decode shape, launched in turn
 # Steps that hold prompt portions are captured too when their exact shape (segment lengths, wanted rows, table widths)
@@ -410,7 +411,7 @@ class Engine:
         return out
 
     def _capture(self, ctx: StepContext):
-        """The step as a CUDA graph: (graph, its output). Capturing only records, so nothing needs to have ended on the
+        """The step as a CUDA graph: (graph, its output), or None if there is no memory for it. Capturing only records, so nothing needs to have ended on the
         device; ``torch.cuda.graph`` waits for it, collects garbage and gives the allocator's free memory back to the
         driver, which costs milliseconds to hundreds of them. That is the second way, where memory is short."""
         graph, collecting = torch.cuda.CUDAGraph(), gc.isenabled()
@@ -430,8 +431,11 @@ class Engine:
             if collecting:
                 gc.enable()
         graph = torch.cuda.CUDAGraph()
-        with torch.cuda.graph(graph, pool=self._graph_pool, stream=capture_stream(self.rt.device)):
-            out = self._run_model(ctx)
+        try:
+            with torch.cuda.graph(graph, pool=self._graph_pool, stream=capture_stream(self.rt.device)):
+                out = self._run_model(ctx)
+        except torch.cuda.OutOfMemoryError:
+            return None
         return graph, out
 
     def step(self, entries: Sequence[StepEntry], sample=None) -> torch.Tensor:
@@ -509,13 +513,22 @@ class Engine:
                 out = self._run_model(ctx)
             else:
                 n0 = ops.kernel_launches()
-                graph, out = self._capture(ctx)
-                entry.n_launches = ops.kernel_launches() - n0        # kernels of this package inside the graph
-                ops._LAUNCHES[0] = n0
-                entry.graphs.append((graph, out))
-                graph.replay()
-                ops._LAUNCHES[0] += entry.n_launches
-                out = out.clone() if self._copy_results else out
+                captured = self._capture(ctx)
+                n_launches, ops._LAUNCHES[0] = ops.kernel_launches() - n0, n0
+                if captured is None:
+                    # A graph keeps its activations to itself, an eager step reuses the others': it may still fit.
+                    if entry.graphs:
+                        entry.copies = len(entry.graphs)
+                    else:
+                        entry.warm -= GRAPH_RETRY_STEPS
+                    out = self._run_model(ctx)
+                else:
+                    graph, out = captured
+                    entry.n_launches = n_launches                    # kernels of this package inside the graph
+                    entry.graphs.append(captured)
+                    graph.replay()
+                    ops._LAUNCHES[0] += entry.n_launches
+                    out = out.clone() if self._copy_results else out
         for rid, n in wanted:
             self.cache.advance(rid, n)
         self.steps_run += 1

@@ -78,3 +78,27 @@ def test_bits_of_a_portion_do_not_depend_on_what_was_captured(heads, kv, first, 
         assert eng._graphs
     for i, r in enumerate(results[1:]):
         assert torch.equal(r, results[0]), f"pass {i + 1}"
+
+
+def test_a_capture_without_memory_leaves_the_step_to_the_eager_way(monkeypatch):
+    """No room for a graph's activations is no reason for a step to fail."""
+    from infer_b200 import StepEntry
+    from test_engine_gpu import _engine
+    ids = H.random_ids(H.TINY["a"], 30, 5)
+    outs = []
+    for short in (False, True):
+        eng = _engine("a", torch.float32, cuda_graphs=short)
+        run_model = eng._run_model
+
+        def none_left(ctx):
+            if torch.cuda.is_current_stream_capturing():
+                raise torch.cuda.OutOfMemoryError("no room for a graph")
+            return run_model(ctx)
+        if short:
+            monkeypatch.setattr(eng, "_run_model", none_left)
+        eng.add_request("r")
+        outs.append([eng.step([StepEntry("r", ids[:20], [19])])] + [eng.step([StepEntry("r", ids[t:t + 1], [0])]) for t in range(20, 30)])
+        eng.check_status()
+        assert not eng._graphs or not any(e.graphs for e in eng._graphs.values())
+    for a, b in zip(*outs):
+        assert torch.equal(a, b)
