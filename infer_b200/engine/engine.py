@@ -13,6 +13,7 @@ wanted rows) travel to the device in ONE packed int32 buffer and one copy.
 from __future__ import annotations
 
 import gc
+import threading
 import time
 from dataclasses import dataclass, field
 from typing import Dict, Hashable, List, Mapping, Optional, Sequence
@@ -119,6 +120,11 @@ PORTION_GRAPH_COLD = 1.5      # an eager run this much slower per launch than th
 MAX_PORTION_GRAPHS = 32
 PORTION_GRAPH_MAX_TOKENS = 8192
 PORTION_GRAPH_TOKEN_POOL = 16384
+
+
+# One capture at a time in the process: torch's generator and the stream of captures take one. What other threads do meanwhile on
+# streams of their own is not part of it (capture mode "thread_local").
+_CAPTURING = threading.Lock()
 
 
 class _GraphEntry:
@@ -414,12 +420,16 @@ class Engine:
         """The step as a CUDA graph: (graph, its output), or None if there is no memory for it. Capturing only records, so nothing needs to have ended on the
         device; ``torch.cuda.graph`` waits for it, collects garbage and gives the allocator's free memory back to the
         driver, which costs milliseconds to hundreds of them. That is the second way, where memory is short."""
+        with _CAPTURING:
+            return self._capture_alone(ctx)
+
+    def _capture_alone(self, ctx: StepContext):
         graph, collecting = torch.cuda.CUDAGraph(), gc.isenabled()
         from ..fast_ops import capture_stream
         gc.disable()                              # (a graph that a collection finds must not be destroyed meanwhile)
         try:
             with torch.cuda.stream(capture_stream(self.rt.device)):
-                graph.capture_begin(pool=self._graph_pool)
+                graph.capture_begin(pool=self._graph_pool, capture_error_mode="thread_local")
                 try:
                     out = self._run_model(ctx)
                 finally:
@@ -432,7 +442,7 @@ class Engine:
                 gc.enable()
         graph = torch.cuda.CUDAGraph()
         try:
-            with torch.cuda.graph(graph, pool=self._graph_pool, stream=capture_stream(self.rt.device)):
+            with torch.cuda.graph(graph, pool=self._graph_pool, stream=capture_stream(self.rt.device), capture_error_mode="thread_local"):
                 out = self._run_model(ctx)
         except torch.cuda.OutOfMemoryError:
             return None

@@ -102,3 +102,46 @@ def test_a_capture_without_memory_leaves_the_step_to_the_eager_way(monkeypatch):
         assert not eng._graphs or not any(e.graphs for e in eng._graphs.values())
     for a, b in zip(*outs):
         assert torch.equal(a, b)
+
+
+@pytest.mark.parametrize("own_streams", [True, False])
+def test_engines_in_two_threads_capture_their_steps(own_streams):
+    """Steps of float32 engines in threads of their own, each on its own stream or both on the default one: new shapes (and so captures) all the time in both, and
+    device memory asked for outside of a capture while the other captures."""
+    import threading
+    from infer_b200 import StepEntry
+    from test_engine_gpu import _engine
+    cfg = H.TINY["b"]
+    ids = {r: H.random_ids(cfg, 40, 30 + i) for i, r in enumerate("abcd")}
+
+    def run(eng, stream, out, keep):
+        with torch.cuda.stream(stream):
+            for batch in (1, 2, 3, 4):
+                rids = "abcd"[:batch]
+                for r in rids:
+                    eng.add_request(r)
+                out.append(eng.step([StepEntry(r, ids[r][:20], [19]) for r in rids]))
+                for t in range(20, 40):
+                    out.append(eng.step([StepEntry(r, ids[r][t:t + 1], [0]) for r in rids]))
+                    keep.append(torch.empty((1 << 20) + 4096 * len(keep), dtype=torch.uint8, device=DEV))
+                for r in rids:
+                    eng.end_request(r)
+            stream.synchronize()
+    want, results, errors = [], [[], []], []
+    run(_engine("b", torch.float32, cuda_graphs=False), torch.cuda.default_stream(), want, [])
+
+    def guarded(i, eng, stream):
+        try:
+            run(eng, stream, results[i], [])
+        except Exception as e:
+            errors.append(e)
+    engines = [_engine("b", torch.float32) for _ in range(2)]
+    torch.cuda.synchronize()
+    threads = [threading.Thread(target=guarded, args=(i, engines[i], torch.cuda.Stream() if own_streams else torch.cuda.default_stream())) for i in range(2)]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    assert not errors, errors
+    for got in results:
+        assert len(got) == len(want) and all(torch.equal(a, b) for a, b in zip(got, want))
