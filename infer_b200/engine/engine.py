@@ -193,7 +193,7 @@ class Engine:
         self._graphs: Dict[tuple, _GraphEntry] = {}
         self._portion_runs: Dict[tuple, _PortionRun] = {}
         self._ms_per_launch = float("inf")                # the fastest eager run's host time per launch
-        self._graph_pool = torch.cuda.graph_pool_handle() if self.use_graphs else None
+        self._graph_pool = None
 
     # ------------------------------------------------------------------ construction helpers
 
@@ -423,13 +423,20 @@ class Engine:
         with _CAPTURING:
             return self._capture_alone(ctx)
 
+    def _pool(self):
+        """The memory pool that this engine's graphs share. One whose last graph is gone takes no capture any more (the allocator raises,
+        and torch's generator stays with the capture that never ended): another takes its place."""
+        if not any(e.graphs for e in self._graphs.values()):
+            self._graph_pool = torch.cuda.graph_pool_handle()
+        return self._graph_pool
+
     def _capture_alone(self, ctx: StepContext):
         graph, collecting = torch.cuda.CUDAGraph(), gc.isenabled()
         from ..fast_ops import capture_stream
         gc.disable()                              # (a graph that a collection finds must not be destroyed meanwhile)
         try:
             with torch.cuda.stream(capture_stream(self.rt.device)):
-                graph.capture_begin(pool=self._graph_pool, capture_error_mode="thread_local")
+                graph.capture_begin(pool=self._pool(), capture_error_mode="thread_local")
                 try:
                     out = self._run_model(ctx)
                 finally:
@@ -442,7 +449,7 @@ class Engine:
                 gc.enable()
         graph = torch.cuda.CUDAGraph()
         try:
-            with torch.cuda.graph(graph, pool=self._graph_pool, stream=capture_stream(self.rt.device), capture_error_mode="thread_local"):
+            with torch.cuda.graph(graph, pool=self._pool(), stream=capture_stream(self.rt.device), capture_error_mode="thread_local"):
                 out = self._run_model(ctx)
         except torch.cuda.OutOfMemoryError:
             return None

@@ -145,3 +145,39 @@ def test_engines_in_two_threads_capture_their_steps(own_streams):
     assert not errors, errors
     for got in results:
         assert len(got) == len(want) and all(torch.equal(a, b) for a, b in zip(got, want))
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16], ids=["f32", "bf16"])
+def test_a_capture_after_the_last_graph_has_gone(dtype, monkeypatch):
+    """The shapes of single tokens take turns in a table of two: the only captured one leaves for shapes that have not been captured yet."""
+    from infer_b200 import StepEntry
+    from infer_b200.engine import engine as module
+    from test_engine_gpu import _engine
+    monkeypatch.setattr(module, "MAX_GRAPHS", 2)
+    cfg = H.TINY["a"]
+    ids = H.random_ids(cfg, 60, 5)
+    outs = []
+    for graphs in (False, True):
+        eng = _engine("a", dtype, cuda_graphs=graphs)
+        at = {r: 0 for r in "abc"}
+
+        def some(rids, n):
+            for _ in range(n):
+                outs[-1].append(eng.step([StepEntry(r, ids[at[r]:at[r] + 1], [0]) for r in rids]).clone())
+                for r in rids:
+                    at[r] += 1
+        outs.append([])
+        for r in "abc":
+            eng.add_request(r)
+        some("a", 4)
+        assert not graphs or [len(e.graphs) for e in eng._graphs.values()] == [2]
+        some("ab", 1)
+        some("abc", 1)
+        assert not any(e.graphs for e in eng._graphs.values())
+        some("ab", 4)
+        some("a", 4)
+        some("abc", 4)
+        torch.randn(4, device=DEV)
+        eng.check_status()
+    for i, (a, b) in enumerate(zip(*outs)):
+        assert (a - b).abs().max() < (1e-6 if dtype == torch.float32 else 0.05), f"step {i}"
