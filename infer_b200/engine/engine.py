@@ -25,6 +25,7 @@ from .. import ops
 from ..cache.manager import CacheManager
 from ..config.registry import load_config
 from ..config.specs import ModelSpec
+from ..parts.base import CHANGES
 from ..runtime import Runtime, parse_dtype
 from ..weights.binder import load_weights
 from .model import Model
@@ -186,14 +187,17 @@ class Engine:
         self.next_tokens = torch.zeros(max(1, max_requests), dtype=torch.int32, device=self.rt.device)
         # Decode-only steps are captured into CUDA graphs, one per (batch, wanted rows, table widths); steps with prompt
         # portions once their exact shape has repeated. The 32-bit path does so for models of this package's own parts (a part
-        # registered from elsewhere may count on being run eagerly there) and hands out a copy of a replay's result, so that
-        # its callers own what they get. (A tiny model's 24 greedy steps: 13.6 -> 4.8 ms, of which its launches were most.)
-        self.use_graphs = bool(cuda_graphs) and self.model.graph_safe() and (dtype == torch.bfloat16 or self.model.built_in())
+        # registered from elsewhere may count on being run eagerly there), as long as nothing of the model is replaced, and hands
+        # out a copy of a replay's result, so that its callers own what they get. (A tiny model's 24 greedy steps: 13.6 -> 4.8 ms,
+        # of which its launches were most.)
+        self.use_graphs = self._may_use_graphs = bool(cuda_graphs) and self.model.graph_safe()
         self._copy_results = dtype == torch.float32
         self._graphs: Dict[tuple, _GraphEntry] = {}
         self._portion_runs: Dict[tuple, _PortionRun] = {}
         self._ms_per_launch = float("inf")                # the fastest eager run's host time per launch
         self._graph_pool = None
+        self._made_of, self._changes_seen = None, -1
+        self._look_at_parts()
 
     # ------------------------------------------------------------------ construction helpers
 
@@ -216,6 +220,18 @@ class Engine:
         return rid in self.cache.requests
 
     # ------------------------------------------------------------------ the step
+
+    def _look_at_parts(self) -> None:
+        """32-bit path: captured steps go when an attribute of a part was replaced since they were made (a method, a matrix, a whole
+        part), and while one of the parts is not the package's own every step runs eagerly, as it would without graphs."""
+        if not (self._may_use_graphs and self._copy_results) or self._changes_seen == CHANGES[0]:
+            return
+        self._changes_seen = CHANGES[0]
+        before, self._made_of = self._made_of, self.model.made_of()
+        if before is None or len(before) != len(self._made_of) or any(x is not y for x, y in zip(before, self._made_of)):
+            self._graphs.clear()
+            self._portion_runs.clear()
+            self.use_graphs = self.model.built_in()
 
     def _build_context(self, entries: Sequence[StepEntry], graphs: bool = False, sample=None):
         """Packs the step's integers on the host and places them on the device. With ``graphs`` and a decode-only
@@ -508,6 +524,7 @@ class Engine:
             if not self.cache.reserve(rid, n):
                 raise AssertionError("reserve failed after can_reserve succeeded")
         try:
+            self._look_at_parts()
             ctx, entry = self._build_context(entries, self.use_graphs, sample)
         except Exception:
             for rid, _ in wanted:

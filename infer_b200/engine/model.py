@@ -7,12 +7,13 @@ what the spec lists and calls ``forward`` on the embedding, the blocks, the fina
 """
 from __future__ import annotations
 
+from types import FunctionType
 from typing import Dict, List, Mapping
 
 import torch
 
 from ..config.specs import LayerSpec, ModelSpec, PartSpec
-from ..parts.base import Block, Part, build_part, part_class
+from ..parts.base import Block, Part, Watched, build_part, part_class
 from ..parts.linear import Linear
 from ..runtime import Runtime
 from ..weights.binder import check_weights
@@ -53,13 +54,41 @@ class Model:
         """True if every part allows its forward() to be captured into a CUDA graph."""
         return all(getattr(p, "graph_safe", True) for p in self.all_parts())
 
+    def made_of(self) -> list:
+        """Every part, block and product of the model with its attributes, in a fixed order, whatever it sits in (attributes, lists,
+        dicts): [object, None, None, object, attribute name, value, ...] (one list: tens of thousands of tuples would be the garbage
+        collector's)."""
+        found, seen = [], set()
+
+        def visit(obj):
+            if isinstance(obj, dict):
+                obj = list(obj.values())
+            if isinstance(obj, (list, tuple)):
+                for v in obj:
+                    visit(v)
+            elif isinstance(obj, Watched) and id(obj) not in seen:
+                seen.add(id(obj))
+                found.extend((obj, None, None))
+                for name, value in vars(obj).items():
+                    found.extend((obj, name, value))
+                    visit(value)
+        visit([*self.all_parts(), *self.blocks])
+        return found
+
     def built_in(self) -> bool:
-        """True if every part, the parts inside parts, and every block are this package's own."""
+        """True if every part, the parts inside parts, every block and product are this package's own, and so are their methods: none
+        was replaced, neither on an instance nor on its class."""
         own = __name__.split(".")[0]
 
-        def mine(obj) -> bool:
-            return type(obj).__module__.split(".")[0] == own and all(mine(v) for v in vars(obj).values() if isinstance(v, Part))
-        return all(mine(p) for p in (*self.all_parts(), *self.blocks))
+        def ours(x) -> bool:
+            return str(getattr(x, "__module__", "")).split(".")[0] == own
+
+        def own_class(cls) -> bool:
+            return all(ours(c) and all(ours(f) for f in vars(c).values() if isinstance(f, FunctionType)) for c in cls.__mro__ if c is not object)
+        made_of = self.made_of()
+        return (all(own_class(c) for c in {type(o) for o in made_of[::3]})
+                and not any(callable(v) and name is not None and hasattr(type(o), name) and not ours(v)
+                            for o, name, v in zip(made_of[::3], made_of[1::3], made_of[2::3])))
 
     def cache_needs(self) -> Dict[int, object]:
         """cache index -> what the layer that writes it needs from the cache manager."""

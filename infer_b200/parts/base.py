@@ -62,7 +62,25 @@ class CompositeNeed:
 
 # ----------------------------------------------------------------------------- interfaces
 
-class Part:
+# How many attributes were set on or taken from any ``Watched`` object (in a list: an attribute of the class would empty Python's
+# method caches of all parts each time).
+CHANGES = [0]
+
+
+class Watched:
+    """What a model is made of: whoever keeps something made from such objects (a captured step) sees by ``CHANGES`` that none has
+    changed since."""
+
+    def __setattr__(self, name, value):
+        CHANGES[0] += 1
+        object.__setattr__(self, name, value)
+
+    def __delattr__(self, name):
+        CHANGES[0] += 1
+        object.__delattr__(self, name)
+
+
+class Part(Watched):
     """Common surface of every part."""
 
     def __init__(self, spec: PartSpec, runtime: "Runtime"):
@@ -235,7 +253,7 @@ class Head(Part):
         raise NotImplementedError
 
 
-class Block:
+class Block(Watched):
     """An arrangement of parts into a layer. ``parts`` maps the slot names of the layer's spec to the built and
     loaded parts, in the spec's order; each is also an attribute of the block under its slot name. A block class
     defines which slots it wants and how ``forward`` runs them."""

@@ -12,9 +12,10 @@ import torch
 
 from .. import ops
 from ..runtime import Runtime
+from .base import Watched
 
 
-class Linear:
+class Linear(Watched):
     def __init__(self, rt: Runtime, weight: torch.Tensor, bias: Optional[torch.Tensor] = None):
         self.rt = rt
         self.weight = weight.to(device=rt.device, dtype=rt.dtype).contiguous()

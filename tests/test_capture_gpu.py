@@ -181,3 +181,90 @@ def test_a_capture_after_the_last_graph_has_gone(dtype, monkeypatch):
         eng.check_status()
     for i, (a, b) in enumerate(zip(*outs)):
         assert (a - b).abs().max() < (1e-6 if dtype == torch.float32 else 0.05), f"step {i}"
+
+
+# ------------------------------------------------------------------------------------------------ parts that change after they were captured
+
+def test_float32_steps_see_what_was_replaced():
+    """A method or a matrix that is replaced between steps is in use from the next step on, as without graphs; with the package's own
+    method back in its place steps are captured again."""
+    from infer_b200 import StepEntry
+    from test_engine_gpu import _engine
+    cfg = H.TINY["b"]
+    ids = H.random_ids(cfg, 60, 9)
+    calls = []
+
+    def run(eng):
+        eng.add_request("r")
+        outs = [eng.step([StepEntry("r", ids[:10], [9])])]
+        at = 10
+
+        def some(n):
+            nonlocal at
+            for _ in range(n):
+                outs.append(eng.step([StepEntry("r", ids[at:at + 1], [0])]))
+                at += 1
+        some(6)
+        mixer = eng.model.blocks[1].mixer
+        own = type(mixer).forward
+
+        def counted(*a, **k):
+            calls.append(eng)
+            return own(mixer, *a, **k)
+        mixer.forward = counted
+        before = len(calls)
+        some(5)
+        assert len(calls) == before + 5
+        del mixer.forward
+        some(6)
+        assert len(calls) == before + 5
+        eng.model.head.linear.weight = eng.model.head.linear.weight * 2.0
+        some(6)
+        eng.end_request("r")
+        return outs
+    eager, captured = _engine("b", torch.float32, cuda_graphs=False), _engine("b", torch.float32)
+    for i, (a, b) in enumerate(zip(run(eager), run(captured))):
+        assert torch.equal(a, b), f"step {i}"
+    assert captured.use_graphs and any(e.graphs for e in captured._graphs.values())
+
+
+@pytest.mark.parametrize("cases", ["ruvenex", "notirax", "pefazen", "bolelix", "fozerax", "biravik"])
+def test_the_packages_designs_are_its_own(cases):
+    import importlib
+    from infer_b200 import Engine
+    mod = importlib.import_module(cases + "_cases")
+    for name, cfg in mod.CASES.items():
+        spec = mod.spec_of(cfg)
+        from infer_b200.weights import random_weights
+        eng = Engine(spec, random_weights(spec, 1, torch.float32), dtype=torch.float32, max_tokens=64, max_requests=1)
+        assert eng.use_graphs, name
+
+
+def test_a_mixer_from_elsewhere_beside_another_is_run_eagerly():
+    """One of two mixers side by side is registered from elsewhere: the 32-bit path runs every step."""
+    from dataclasses import replace
+    import ruvenex_cases as rc
+    from infer_b200 import Engine, StepEntry
+    from infer_b200.parts.base import part_class, register_mixer, unregister
+    from infer_b200.weights import random_weights
+    cfg = rc.CASES["p"]
+    spec = rc.spec_of(cfg)
+    second = spec.layers[0].parts["mixer"][1]["second"]
+    runs = []
+
+    class Elsewhere(part_class("mixer", second.kind)):
+        def forward(self, *a, **k):
+            runs.append(1)
+            return super().forward(*a, **k)
+    register_mixer("from_elsewhere")(Elsewhere)
+    try:
+        spec.layers[0].parts["mixer"][1].params["second"] = replace(second, kind="from_elsewhere")
+        eng = Engine(spec, random_weights(spec, 1, torch.float32), dtype=torch.float32, max_tokens=64, max_requests=1)
+        assert not eng.use_graphs
+        ids = H.random_ids({"vocab_size": cfg["vocab"]}, 20, 1)
+        eng.add_request("r")
+        for t in range(20):
+            eng.step([StepEntry("r", ids[t:t + 1], [0])])
+        assert len(runs) == 20
+    finally:
+        unregister("mixer", "from_elsewhere")
