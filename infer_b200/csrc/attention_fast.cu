@@ -930,17 +930,13 @@ int page_maps(const void* k_cache, const void* v_cache, int64_t n_pages, int n_k
 }
 
 int configure() {
-    static bool configured = false;
-    if (!configured) {
-        cudaError_t e = cudaFuncSetAttribute(attn_decode_kernel<false, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, DEC_SMEM);
-        if (e == cudaSuccess) e = cudaFuncSetAttribute(attn_decode_kernel<false, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize, DEC_SMEM);
-        if (e == cudaSuccess) e = cudaFuncSetAttribute(attn_decode_kernel<true, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, DEC_SMEM);
-        if (e == cudaSuccess) e = cudaFuncSetAttribute(attn_decode_kernel<true, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize, DEC_SMEM);
-        if (e == cudaSuccess) e = cudaFuncSetAttribute(attn_prefill_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, PF_SMEM);
-        if (e != cudaSuccess) return ib::fail(IB_ERR_CUDA, "attention_fast: cannot set shared memory size: %s", cudaGetErrorString(e));
-        configured = true;
-    }
-    return IB_OK;
+    static ib::PerDevice allowed[5];
+    int rc = ib::allow_smem(allowed[0], "attention_fast", attn_decode_kernel<false, 1>, DEC_SMEM);
+    if (!rc) rc = ib::allow_smem(allowed[1], "attention_fast", attn_decode_kernel<false, 2>, DEC_SMEM);
+    if (!rc) rc = ib::allow_smem(allowed[2], "attention_fast", attn_decode_kernel<true, 1>, DEC_SMEM);
+    if (!rc) rc = ib::allow_smem(allowed[3], "attention_fast", attn_decode_kernel<true, 2>, DEC_SMEM);
+    if (!rc) rc = ib::allow_smem(allowed[4], "attention_fast", attn_prefill_kernel, PF_SMEM);
+    return rc;
 }
 
 }  // namespace

@@ -574,12 +574,9 @@ static int prefill_tc(const void* q, const void* k_cache, const void* v_cache, v
     if (rc) return rc;
     rc = ib::get_map(v_cache, n_pages * n_kv * PAGE, HD, PAGE, &mv);
     if (rc) return rc;
-    static bool configured = false;
-    if (!configured) {
-        cudaError_t e = cudaFuncSetAttribute(attn_prefill_tc_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_BYTES);
-        if (e != cudaSuccess) return ib::fail(IB_ERR_CUDA, "attention_tc: cannot set shared memory size: %s", cudaGetErrorString(e));
-        configured = true;
-    }
+    static ib::PerDevice allowed;
+    rc = ib::allow_smem(allowed, "attention_tc", attn_prefill_tc_kernel, SMEM_BYTES);
+    if (rc) return rc;
     Params p = {};
     p.out = (bf16*)out; p.block_table = block_table; p.max_blocks = max_blocks; p.seg_start = seg_start; p.seg_pos0 = seg_pos0;
     p.n_heads = n_heads; p.n_kv = n_kv; p.group = n_heads / n_kv; p.window = window; p.scale_log2 = scale * LOG2E;

@@ -47,7 +47,7 @@ MODULES: Dict[str, str] = {
     "attn_tc": "attention_tc.cu",
     "capi": "capi.cpp",          # host code only: the C handle API over the engine (needs the interpreter's headers)
 }
-HEADERS = ["common.cuh", "gemm_static.h", "tc_ops.cuh", "tma_map.cuh"]
+HEADERS = ["common.cuh", "gemm_static.h", "per_device.h", "tc_ops.cuh", "tma_map.cuh"]
 # modules that are compiled per model size: the variant that build_all() makes (others are built at first use)
 DEFAULT_DEFINES = {"attn": {"IB_HEAD_DIM": 128}, "attn_tc": {"IB_HEAD_DIM": 128}, "latent_pf": {"IB_QK_DIM": 128, "IB_V_DIM": 128},
                    "talk_pf": {"IB_HEAD_DIM": 128, "IB_V_DIM": 128, "IB_HEADS": 12}}

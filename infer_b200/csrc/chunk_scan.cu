@@ -427,13 +427,10 @@ int launch_chunk(dim3 grid, cudaStream_t stream, const bf16* qk, const float* ro
                  int b_col, int lng_col, float* state, float* ones_state, const int* seg_start, const int* seg_slot, float* raw_out,
                  float* ones_out, const float* skip, int n_heads, int hpq, int d, int dv, int write_state, int vec_v) {
     constexpr size_t smem = sizeof(Layout<D, NB>);
-    static bool set = false;
-    if (!set) {
-        const cudaError_t e = cudaFuncSetAttribute(chunk_scan_kernel<D, NB>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem));
-        if (e != cudaSuccess) return ib::fail(IB_ERR_CUDA, "ib_chunk_scan: %s", cudaGetErrorString(e));
-        set = true;
-    }
-    const int rc = ib::launch("chunk_scan_kernel", chunk_scan_kernel<D, NB>, grid, dim3(THREADS), smem, stream, 1u, qk, rows, ld, v_col,
+    static ib::PerDevice allowed;
+    int rc = ib::allow_smem(allowed, "ib_chunk_scan", chunk_scan_kernel<D, NB>, smem);
+    if (rc) return rc;
+    rc = ib::launch("chunk_scan_kernel", chunk_scan_kernel<D, NB>, grid, dim3(THREADS), smem, stream, 1u, qk, rows, ld, v_col,
                               aux, lda, b_col, lng_col, state, ones_state, seg_start, seg_slot, raw_out, ones_out, skip, n_heads, hpq, d, dv,
                               write_state, vec_v);
     return rc ? rc : ib::check_launch("ib_chunk_scan");

@@ -12,6 +12,8 @@
 #include <cstdio>
 #include <cstdarg>
 
+#include "per_device.h"
+
 #define IB_OK 0
 #define IB_ERR_ARG -1      // a size, dtype or pointer the kernel does not accept
 #define IB_ERR_CUDA -2     // the CUDA runtime reported an error at launch
@@ -38,6 +40,23 @@ inline int fail(int code, const char* fmt, ...) {
 inline int check_launch(const char* what) {
     cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) return fail(IB_ERR_CUDA, "%s: %s", what, cudaGetErrorString(e));
+    return IB_OK;
+}
+
+inline int current_device() {
+    int device = -1;
+    return cudaGetDevice(&device) == cudaSuccess ? device : -1;
+}
+
+// Lets `kernel` take `bytes` of dynamic shared memory on the current device.
+template <typename Kernel>
+inline int allow_smem(PerDevice& done, const char* what, Kernel kernel, size_t bytes) {
+    cudaError_t e = cudaSuccess;
+    done.get(current_device(), [&] {
+        e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(bytes));
+        return e == cudaSuccess ? 1 : 0;
+    });
+    if (e != cudaSuccess) return fail(IB_ERR_CUDA, "%s: cannot set shared memory size: %s", what, cudaGetErrorString(e));
     return IB_OK;
 }
 

@@ -1112,12 +1112,8 @@ using ib::get_map;
 template <int BN, typename TOut>
 int launch(const CUtensorMap& ma, const CUtensorMap& mb, const GemmParams& p, dim3 grid, cudaStream_t stream) {
     using C = Cfg<BN>;
-    static bool configured = false;
-    if (!configured) {
-        cudaError_t e = cudaFuncSetAttribute(gemm_tc_kernel<BN, TOut>, cudaFuncAttributeMaxDynamicSharedMemorySize, C::SMEM_BYTES);
-        if (e != cudaSuccess) return ib::fail(IB_ERR_CUDA, "gemm_tc: cannot set shared memory size: %s", cudaGetErrorString(e));
-        configured = true;
-    }
+    static ib::PerDevice allowed;
+    if (const int rc = ib::allow_smem(allowed, "gemm_tc", gemm_tc_kernel<BN, TOut>, C::SMEM_BYTES)) return rc;
     if (p.stages < 1 || p.stages > C::MAX_STAGES) return ib::fail(IB_ERR_ARG, "gemm_tc: %d stages (at most %d)", p.stages, C::MAX_STAGES);
     const size_t smem = size_t(p.stages) * C::STAGE_BYTES + C::SMEM_EXTRA + (p.cluster_split && !p.recv_in_ring ? C::RECV_BYTES : 0);
     if (smem > size_t(C::SMEM_BYTES)) return ib::fail(IB_ERR_ARG, "gemm_tc: %d stages and the receive area do not fit", p.stages);
@@ -1128,9 +1124,10 @@ int launch(const CUtensorMap& ma, const CUtensorMap& mb, const GemmParams& p, di
 // CTAs of the pair kernel that run at once: as many clusters of two as the device places, at most one CTA per SM.
 template <int PN, typename TOut>
 int launch_pair(const CUtensorMap& ma, const CUtensorMap& mb, const GemmParams& p, int sm_count, cudaStream_t stream) {
-    static int room = 0;
-    if (!room) {
-        cudaError_t e = cudaFuncSetAttribute(gemm_tc_pair_kernel<PN, TOut>, cudaFuncAttributeMaxDynamicSharedMemorySize, PairCfg<PN>::SMEM_BYTES);
+    static ib::PerDevice allowed, fit;
+    if (const int rc = ib::allow_smem(allowed, "gemm_tc_pair", gemm_tc_pair_kernel<PN, TOut>, PairCfg<PN>::SMEM_BYTES)) return rc;
+    cudaError_t e = cudaSuccess;
+    const int room = fit.get(ib::current_device(), [&] {
         cudaLaunchConfig_t cfg = {};
         cfg.gridDim = dim3(unsigned(sm_count & ~1));
         cfg.blockDim = dim3(NUM_THREADS);
@@ -1141,10 +1138,10 @@ int launch_pair(const CUtensorMap& ma, const CUtensorMap& mb, const GemmParams& 
         cfg.attrs = &attr;
         cfg.numAttrs = 1;
         int clusters = 0;
-        if (e == cudaSuccess) e = cudaOccupancyMaxActiveClusters(&clusters, gemm_tc_pair_kernel<PN, TOut>, &cfg);
-        if (e != cudaSuccess || clusters < 1) return ib::fail(IB_ERR_CUDA, "gemm_tc: no room for a pair of CTAs: %s", cudaGetErrorString(e));
-        room = clusters < sm_count / 2 ? clusters : sm_count / 2;
-    }
+        e = cudaOccupancyMaxActiveClusters(&clusters, gemm_tc_pair_kernel<PN, TOut>, &cfg);
+        return e != cudaSuccess ? 0 : clusters < sm_count / 2 ? clusters : sm_count / 2;
+    });
+    if (room < 1) return ib::fail(IB_ERR_CUDA, "gemm_tc: no room for a pair of CTAs: %s", cudaGetErrorString(e));
     const int64_t tiles = ((p.rows_a + 255) / 256) * ((p.rows_b + PN - 1) / PN);
     const unsigned ctas = 2u * unsigned(tiles < room ? tiles : room);
     return ib::launch("gemm_tc_pair", gemm_tc_pair_kernel<PN, TOut>, dim3(ctas), dim3(NUM_THREADS), size_t(PairCfg<PN>::SMEM_BYTES), stream, 2u, ma, mb, p);
@@ -1152,12 +1149,8 @@ int launch_pair(const CUtensorMap& ma, const CUtensorMap& mb, const GemmParams& 
 
 template <int PBN, bool WIDE, typename TOut>
 int launch_persistent(const CUtensorMap& ma, const CUtensorMap& mb, const GemmParams& p, int sm_count, cudaStream_t stream) {
-    static bool configured = false;
-    if (!configured) {
-        cudaError_t e = cudaFuncSetAttribute(gemm_tc_persistent_kernel<PBN, WIDE, TOut>, cudaFuncAttributeMaxDynamicSharedMemorySize, P_SMEM_BYTES);
-        if (e != cudaSuccess) return ib::fail(IB_ERR_CUDA, "gemm_tc: cannot set shared memory size: %s", cudaGetErrorString(e));
-        configured = true;
-    }
+    static ib::PerDevice allowed;
+    if (const int rc = ib::allow_smem(allowed, "gemm_tc", gemm_tc_persistent_kernel<PBN, WIDE, TOut>, P_SMEM_BYTES)) return rc;
     const int64_t tiles = WIDE ? ((p.rows_a + 127) / 128) * ((p.rows_b + PBN - 1) / PBN) : ((p.rows_a + PBM - 1) / PBM) * ((p.rows_b + PBN - 1) / PBN);
     const unsigned ctas = unsigned(tiles < sm_count ? tiles : sm_count);
     return ib::launch("gemm_tc", gemm_tc_persistent_kernel<PBN, WIDE, TOut>, dim3(ctas), dim3(NUM_THREADS), size_t(P_SMEM_BYTES), stream, 1u, ma, mb, p);
@@ -1369,12 +1362,13 @@ IB_EXPORT int ib_gemm_tc(const void* x, const void* w, const float* bias, const 
         if (rc) return rc;
         rc = get_map(w, p.rows_b, K, paired ? width / 2 : width, &mb);
         if (rc) return rc;
-        static int sms = 0;
-        if (!sms) {
-            int dev = 0;
-            if (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || sms <= 0)
-                return ib::fail(IB_ERR_CUDA, "gemm_tc: cannot read the number of SMs");
-        }
+        static ib::PerDevice counted;
+        const int device = ib::current_device();
+        const int sms = counted.get(device, [&] {
+            int n = 0;
+            return device >= 0 && cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, device) == cudaSuccess ? n : 0;
+        });
+        if (sms <= 0) return ib::fail(IB_ERR_CUDA, "gemm_tc: cannot read the number of SMs");
         p.splits = 1; p.cluster_split = 0; p.stages = PSTAGES;
         p.weights_once = N * K * 2 <= (64LL << 20) ? 1 : 0;
         {
@@ -1457,12 +1451,8 @@ IB_EXPORT int ib_gemm_tc_grouped(const void* x, const void* w, void* out, int64_
     if (rc) return rc;
 #define IB_GROUPED(WW, TT)                                                                                                           \
     do {                                                                                                                             \
-        static bool configured = false;                                                                                              \
-        if (!configured) {                                                                                                           \
-            cudaError_t e = cudaFuncSetAttribute(gemm_tc_persistent_kernel<WW, true, TT, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, P_SMEM_BYTES); \
-            if (e != cudaSuccess) return ib::fail(IB_ERR_CUDA, "gemm_tc_grouped: cannot set shared memory size: %s", cudaGetErrorString(e)); \
-            configured = true;                                                                                                       \
-        }                                                                                                                            \
+        static ib::PerDevice allowed;                                                                                                \
+        if (const int e = ib::allow_smem(allowed, "gemm_tc_grouped", gemm_tc_persistent_kernel<WW, true, TT, true>, P_SMEM_BYTES)) return e; \
         const int64_t most = max_tiles * p.g_tiles_n;                                                                                \
         return ib::launch("gemm_tc_grouped", gemm_tc_persistent_kernel<WW, true, TT, true>, dim3(unsigned(most < sms ? most : sms)), \
                           dim3(NUM_THREADS), size_t(P_SMEM_BYTES), stream, 1u, ma, mb, p);                                           \

@@ -461,13 +461,8 @@ int launch(const GemvParams& p, int out_dtype, int epi, int grid_ctas, cudaStrea
     const unsigned cl = unsigned(p.cluster);
 #define IB_GEMV_LAUNCH_(EPI_, T_, NWS_)                                                                            \
     do {                                                                                                           \
-        static bool configured = false;                                                                            \
-        if (!configured) {                                                                                         \
-            cudaError_t e = cudaFuncSetAttribute(bulk_gemv_kernel<NT, EPI_, T_, NWS_>,                             \
-                                                 cudaFuncAttributeMaxDynamicSharedMemorySize, RING_BYTES + NW_BYTES); \
-            if (e != cudaSuccess) return ib::fail(IB_ERR_CUDA, "linear_skinny_bulk: cannot set shared memory size: %s", cudaGetErrorString(e)); \
-            configured = true;                                                                                     \
-        }                                                                                                          \
+        static ib::PerDevice allowed;                                                                              \
+        if (const int rc = ib::allow_smem(allowed, "linear_skinny_bulk", bulk_gemv_kernel<NT, EPI_, T_, NWS_>, RING_BYTES + NW_BYTES)) return rc; \
         return ib::launch("linear_skinny_bulk", bulk_gemv_kernel<NT, EPI_, T_, NWS_>, grid, block,                 \
                           size_t(RING_BYTES) + (NWS_ ? size_t(NW_BYTES) : 0), stream, cl, p);                      \
     } while (0)

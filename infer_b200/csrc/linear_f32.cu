@@ -246,8 +246,8 @@ struct Args {
 
 template <int ROWS, int MT, bool VEC>
 int launch_gemv(const Args& a, cudaStream_t stream) {
-    static const cudaError_t set = cudaFuncSetAttribute(gemv32_kernel<ROWS, MT, VEC>, cudaFuncAttributeMaxDynamicSharedMemorySize, gemv_smem<ROWS, MT>());
-    if (set != cudaSuccess) return ib::fail(IB_ERR_CUDA, "linear_f32: cannot set shared memory size: %s", cudaGetErrorString(set));
+    static ib::PerDevice allowed;
+    if (const int rc = ib::allow_smem(allowed, "linear_f32", gemv32_kernel<ROWS, MT, VEC>, gemv_smem<ROWS, MT>())) return rc;
     return ib::launch("linear_f32", gemv32_kernel<ROWS, MT, VEC>, dim3(unsigned((a.N + ROWS - 1) / ROWS)), dim3(ROWS * GBLOCKS),
                       size_t(gemv_smem<ROWS, MT>()), stream, 1u, a.x, a.w, a.bias, a.residual, a.out, int(a.M), a.N, a.K, a.w_ready);
 }
@@ -262,8 +262,8 @@ int launch_gemv_rows(const Args& a, cudaStream_t stream) {
 
 template <int TM, int TN, bool VEC>
 int launch_tile(const Args& a, cudaStream_t stream) {
-    static const cudaError_t set = cudaFuncSetAttribute(tile32_kernel<TM, TN, VEC>, cudaFuncAttributeMaxDynamicSharedMemorySize, tile_smem<TM, TN>());
-    if (set != cudaSuccess) return ib::fail(IB_ERR_CUDA, "linear_f32: cannot set shared memory size: %s", cudaGetErrorString(set));
+    static ib::PerDevice allowed;
+    if (const int rc = ib::allow_smem(allowed, "linear_f32", tile32_kernel<TM, TN, VEC>, tile_smem<TM, TN>())) return rc;
     const dim3 grid{unsigned((a.N + 16 * TN - 1) / (16 * TN)), unsigned((a.M + 8 * TM - 1) / (8 * TM)), 1u};
     if (grid.y > 65535) return ib::fail(IB_ERR_ARG, "linear_f32: too many rows (%lld)", (long long)a.M);
     return ib::launch("linear_f32", tile32_kernel<TM, TN, VEC>, grid, dim3(128), size_t(tile_smem<TM, TN>()), stream, 1u, a.x, a.w, a.bias,
