@@ -308,8 +308,8 @@ IB_EXPORT int ib_linear_f32(const float* x, const float* w, const float* bias, c
                             int64_t K, int kind, int sm_count, int w_ready, cudaStream_t stream) {
     if (M <= 0 || N <= 0) return IB_OK;
     if (K <= 0) return ib::fail(IB_ERR_ARG, "linear_f32: K must be positive");
-    const int64_t lim = 1LL << 31;
-    if (N >= lim || K >= lim) return ib::fail(IB_ERR_ARG, "linear_f32: a size exceeds 2^31");
+    const int64_t lim = 1LL << 31;                             // of the blocks of 32 elements of K, and of CTAs with 8 features each
+    if (N >= 8 * lim || K >= BLOCK_K * lim) return ib::fail(IB_ERR_ARG, "linear_f32: more features or columns than the kernels count");
     const Args a{x, w, bias, residual, out, M, N, K, w_ready};
     const int sms = sm_count > 0 ? sm_count : 148;
     const bool vec = K % 4 == 0 && ((uintptr_t(x) | uintptr_t(w)) & 15) == 0;
