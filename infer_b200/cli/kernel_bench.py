@@ -63,7 +63,8 @@ def main(argv=None) -> int:
     ap.add_argument("--head-dim", type=int, default=128)
     ap.add_argument("--v-dim", type=int, default=128, help="recurrence: columns of a head's state (its rows are --head-dim)")
     ap.add_argument("--splits", type=int, default=0)
-    ap.add_argument("--bn", type=int, default=0, help="tc: the tile code instead of the planner's (many tokens; 768 with --splits 2, 4 or 8: K slices as a cluster)")
+    ap.add_argument("--bn", type=int, default=0, help="tc: the tile code instead of the planner's (many tokens; 768 with --splits 2, 4 or 8: K slices as a cluster; "
+                    "1024 + 2 x width: pairs of SMs)")
     ap.add_argument("--cluster", type=int, default=0)
     ap.add_argument("--fused", action="store_true", help="attention: the decode kernel that also rotates and stores k/v")
     ap.add_argument("--norm", action="store_true", help="skinny kernel with the fused RMSNorm prologue")
@@ -89,7 +90,9 @@ def main(argv=None) -> int:
         swiglu = args.epi == "swiglu"
         odt = torch.float32 if res is not None else torch.bfloat16
 
-        plan = fast_ops.gemm_plan(M, N, K, fast_ops.device_state(dev).sm_count)
+        # what gemm_tc itself would take, unless the flags ask for another tile or another number of K slices
+        choose = fast_ops.gemm_plan if args.splits else fast_ops.gemm_choice
+        plan = choose(M, N, K, fast_ops.device_state(dev).sm_count)
         if plan is not None and args.splits:
             tiles = -(-(N if plan[0] else M) // 128) * -(-(M if plan[0] else N) // plan[1])
             plan = (plan[0], plan[1], args.splits, args.splits * tiles * 128 * plan[1], tiles)

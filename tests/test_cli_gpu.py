@@ -111,3 +111,14 @@ def test_kernel_bench_times_a_kernel():
     out = _run(["-m", "infer_b200.cli.kernel_bench", "attention", "--batch", "2", "--context", "100", "--heads", "4", "--kv-heads", "2",
                 "--head-dim", "64", "--fused", "--reps", "3"])
     assert json.loads(out.strip().splitlines()[-1])["us_median"] > 0
+
+
+def test_kernel_bench_times_the_product_that_gemm_tc_runs():
+    """Without flags that ask for another one, the tool's plan is the engine's: pairs of SMs at the sizes of a 2,048-token prompt."""
+    from infer_b200 import fast_ops
+    sms = fast_ops.device_state("cuda:0").sm_count
+    for M, N, K, flags in ((2048, 17920, 1536, ["--epi", "swiglu"]), (300, 1536, 1536, []), (64, 1536, 1536, [])):
+        out = json.loads(_run(["-m", "infer_b200.cli.kernel_bench", "linear", "--M", str(M), "--N", str(N), "--K", str(K), "--kernel", "tc", "--reps", "2"]
+                              + flags).splitlines()[-1])
+        assert tuple(out["plan"]) == fast_ops.gemm_choice(M, N, K, sms)
+    assert fast_ops.gemm_choice(2048, 17920, 1536, sms)[1] >= 1280
