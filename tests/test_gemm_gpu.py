@@ -232,22 +232,29 @@ def test_skinny_with_fused_norm(M, N, K):
 @pytest.mark.parametrize("M,N,K", [(2048, 1536, 8960), (2048, 17920, 1536), (1100, 3000, 520), (100, 1536, 8960), (300, 1000, 1536)])
 def test_gemm_tc_against_float64(M, N, K):
     """The tensor-core product against torch in float64, directly (not through the plain kernel): the persistent
-    kernel at the model's down and gate/up shapes of a 2,048-token prompt and at a ragged shape, the swapped mapping
-    and the one-tile mapping once each. Bias, and the residual added in place."""
+    kernel and pairs of SMs at the model's down and gate/up shapes of a 2,048-token prompt and at a ragged shape, the
+    swapped mapping and the one-tile mapping once each. Bias, and the residual added in place."""
     from infer_b200 import fast_ops
     g = torch.Generator(device=DEV).manual_seed(M + 3 * N + 5 * K)
     x = torch.randn(M, K, device=DEV, generator=g).bfloat16()
     w = (torch.randn(N, K, device=DEV, generator=g) * 0.05).bfloat16()
     bias = torch.randn(N, device=DEV, generator=g)
     res = torch.randn(M, N, device=DEV, generator=g)
-    plan = fast_ops.gemm_plan(M, N, K, fast_ops.device_state(DEV).sm_count)
+    sms = fast_ops.device_state(DEV).sm_count
+    plan, choice = fast_ops.gemm_plan(M, N, K, sms), fast_ops.gemm_choice(M, N, K, sms)
+    plans = [plan]
     if M >= 1024:
-        assert plan[1] >= 256, f"this shape is meant to take the persistent kernel, the plan is {plan}"
+        assert 256 <= plan[1] <= 512, f"this shape is meant to take the persistent kernel, the plan is {plan}"
+        plans.append((0, 1024 + 2 * 192, 1, 0, 0))
+    if M >= 2048:
+        assert choice[1] >= 1280, f"this shape is meant to run on pairs of SMs, the choice is {choice}"
     exact = x.double() @ w.double().T
     cond = (x.float().abs() @ w.float().abs().T + 1.0).double()
-    got = fast_ops.gemm_tc(x, w, bias, None, torch.float32)
-    assert ((got.double() - (exact + bias.double())).abs() / cond).max().item() < 2e-6
-    r2 = res.clone()
-    fast_ops.gemm_tc(x, w, None, r2, torch.float32, out=r2)
-    assert ((r2.double() - (exact + res.double())).abs() / cond).max().item() < 2e-6
+    for p in [p for p in plans if p != choice] + [choice]:
+        got = fast_ops.gemm_tc(x, w, bias, None, torch.float32, plan=p)
+        assert ((got.double() - (exact + bias.double())).abs() / cond).max().item() < 2e-6, p
+        r2 = res.clone()
+        fast_ops.gemm_tc(x, w, None, r2, torch.float32, out=r2, plan=p)
+        assert ((r2.double() - (exact + res.double())).abs() / cond).max().item() < 2e-6, p
+    assert torch.equal(fast_ops.gemm_tc(x, w, bias, None, torch.float32), got)          # (without a plan: the choice, which came last)
     assert fast_ops.device_state(DEV).status.item() == 0
