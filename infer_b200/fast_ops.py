@@ -457,6 +457,21 @@ def _prefill_plan(sm_count: int, n_heads: int, head_dim: int, lens, max_ctx_len:
     return best[1], best[2]
 
 
+@functools.lru_cache(maxsize=None)
+def _build_prefill_forms(head_dim: int) -> None:
+    """Both forms of the tcgen05 prefill kernel for a head size, built beside each other at the first use of either: which one a step takes
+    follows from its sizes, and a server would stop for the compiler again when the other one's turn comes."""
+    from concurrent.futures import ThreadPoolExecutor
+    from .csrc.build import compile_module
+    with ThreadPoolExecutor(max_workers=2) as pool:
+        list(pool.map(lambda d: compile_module("attn_tc", d), ({"IB_HEAD_DIM": head_dim}, {"IB_HEAD_DIM": head_dim, "IB_ATTN_BN": 128})))
+
+
+def _prefill_fn(name: str, argtypes, defines):
+    _build_prefill_forms(defines["IB_HEAD_DIM"])
+    return _fn("attn_tc", name, argtypes, defines)
+
+
 def attention_fast(q: torch.Tensor, k_cache: torch.Tensor, v_cache: torch.Tensor, block_table: torch.Tensor,
                    seg_start: torch.Tensor, seg_pos0: torch.Tensor, n_heads: int, n_kv: int, head_dim: int,
                    window: Optional[int], scale: float, has_decode: bool, max_q_len: int, max_ctx_len: int,
@@ -491,7 +506,7 @@ def attention_fast(q: torch.Tensor, k_cache: torch.Tensor, v_cache: torch.Tensor
         n_prefill = S - (n_decode or 0)
         defines, split = prefill_plan(st.sm_count, n_heads, head_dim, seg_lens or [max_q_len] * n_prefill, max_ctx_len, window)
         split = split if tc_split is None else tc_split
-        g = _fn("attn_tc", "ib_attention_prefill_tc", [c_void_p] * 5 + [c_int] + [c_void_p] * 2 + [c_int, c_int64] + [c_int] * 5 +
+        g = _prefill_fn("ib_attention_prefill_tc", [c_void_p] * 5 + [c_int] + [c_void_p] * 2 + [c_int, c_int64] + [c_int] * 5 +
                 [c_float, c_int64, c_int] + [c_void_p] * 2 + [c_int, c_void_p, c_int64, c_void_p, c_int64, c_int], defines)
         # (without the lengths every segment that may have two or more tokens counts as the longest one)
         query_tiles = prefill_query_tiles(seg_lens or [max_q_len] * max(1, n_prefill))
@@ -549,8 +564,8 @@ def attention_prefill_biased(q, k_cache, v_cache, block_table, step, n_heads, n_
     kept = keep_first > 0 or slopes is not None                 # (the entry point that takes them; the other is unchanged)
     sig = [c_void_p] * 5 + [c_int] + [c_void_p] * 2 + [c_int, c_int64] + [c_int] * 5 + [c_float, c_int64, c_int] + [c_void_p] * 2 + \
           [c_int, c_void_p, c_int64, c_void_p, c_int64, c_int, c_void_p, c_int, c_void_p]
-    g = _fn("attn_tc", "ib_attention_prefill_tc_kept" if kept else "ib_attention_prefill_tc_biased", sig + ([c_int, c_void_p] if kept else []),
-            defines)
+    g = _prefill_fn("ib_attention_prefill_tc_kept" if kept else "ib_attention_prefill_tc_biased", sig + ([c_int, c_void_p] if kept else []),
+                    defines)
     args = [q.data_ptr(), k_cache.data_ptr(), v_cache.data_ptr(), out.data_ptr(), block_table.data_ptr(), block_table.shape[1],
             step.seg_start.data_ptr(), step.seg_pos0.data_ptr(), S, T, n_heads, n_kv, head_dim, page_size, int(window or 0), float(scale),
             n_pages, int(step.max_q_len), st.status.data_ptr(), _stream(), int(split), _ptr(tc_ws), 0 if tc_ws is None else tc_ws.numel(),

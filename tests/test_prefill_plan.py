@@ -54,3 +54,18 @@ def test_scratch_of_ragged_portions_stays_within_its_limit(heads, lens, ctx):
     assert st.n == heads * sum(-(-n // 128) for n in lens)
     assert st.floats == st.n * max(parts, 2) * (128 * 128 + 256)
     assert parts == 1 or st.floats <= fast_ops.PREFILL_PARTS_MAX_FLOATS
+
+
+@pytest.mark.parametrize("head_dim", [64, 128])
+def test_both_forms_are_built_at_the_first_use_of_either(head_dim, monkeypatch):
+    from infer_b200 import fast_ops
+    from infer_b200.csrc import build
+    compiled, loaded = [], []
+    monkeypatch.setattr(build, "compile_module", lambda module, defines=None, verbose=False: compiled.append((module, dict(defines))))
+    monkeypatch.setattr(fast_ops, "_fn", lambda module, name, argtypes, defines=None: loaded.append(defines))
+    fast_ops._build_prefill_forms.cache_clear()
+    for _ in range(2):
+        fast_ops._prefill_fn("ib_attention_prefill_tc", [], {"IB_HEAD_DIM": head_dim})
+    assert sorted(len(d) for m, d in compiled if m == "attn_tc" and d["IB_HEAD_DIM"] == head_dim) == [1, 2] and len(compiled) == 2
+    assert loaded == [{"IB_HEAD_DIM": head_dim}] * 2
+    fast_ops._build_prefill_forms.cache_clear()
