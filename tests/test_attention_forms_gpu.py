@@ -54,3 +54,57 @@ def test_scratch_of_ragged_portions(lens, end, parts, monkeypatch):
         assert (run(parts, [max(lens)]).float() - whole.float()).abs().max() < 1e-2
     assert int(st._counters.abs().sum()) == 0
     assert st.status.item() == 0
+
+
+# ------------------------------------------------------------------------------------------------ the two forms of the kernel
+
+@pytest.fixture(params=[64, 128], ids=["64 keys", "128 keys"])
+def form(request, monkeypatch):
+    """The kernel that walks over keys 64 or 128 at a time, whatever the plan would take; how often it was asked for."""
+    from infer_b200 import fast_ops
+    plan, asked = fast_ops.prefill_plan, []
+
+    def pinned(sm_count, n_heads, head_dim, *more):
+        asked.append(head_dim)
+        return {"IB_HEAD_DIM": head_dim, "IB_ATTN_BN": 128} if request.param == 128 else {"IB_HEAD_DIM": head_dim}, plan(sm_count, n_heads, head_dim, *more)[1]
+    monkeypatch.setattr(fast_ops, "prefill_plan", pinned)
+    yield request.param
+    assert asked
+
+
+LAYOUTS = [(12, 2, 128), (14, 2, 64)]
+
+
+@pytest.mark.parametrize("heads,kv,hd", LAYOUTS)
+@pytest.mark.parametrize("window", [None, 1, 40, 64, 65, 129, 300])
+def test_both_forms_with_windows(form, heads, kv, hd, window):
+    """Query tiles and contexts that end on, before and behind the edges of key tiles of either size; windows likewise."""
+    from test_attention_gpu import _run
+    _run(heads, kv, hd, window, [(0, 2), (0, 63), (0, 64), (0, 65), (0, 128), (1, 128), (64, 129), (127, 257), (300, 17), (5, 1), (63, 2)])
+
+
+@pytest.mark.parametrize("split", [1, 2, 3, 4])
+@pytest.mark.parametrize("heads,kv,hd", LAYOUTS)
+def test_both_forms_with_shared_query_tiles(form, heads, kv, hd, split):
+    """1 to 17 tiles of 128 keys and twice as many of 64, whole and in parts, twice; with a window that cuts a part's first tile."""
+    from infer_b200 import fast_ops
+    from test_attention_gpu import _run
+    segs = [(0, 1100), (1900, 200), (1, 1), (1530, 2), (500, 1)]
+    first = _run(heads, kv, hd, None, segs, 2, seed=5, tc_split=split)
+    assert torch.equal(first, _run(heads, kv, hd, None, segs, 2, seed=5, tc_split=split, count_decode=True))
+    assert int(fast_ops.device_state(DEV)._counters.abs().sum()) == 0
+    _run(heads, kv, hd, 1200, [(700, 900), (2000, 130)], seed=6, tc_split=split)
+
+
+@pytest.mark.parametrize("window", [None, 33, 130, 300])
+@pytest.mark.parametrize("sizes", [(4, 2, 64), (8, 1, 128)])
+def test_both_forms_with_distance_bias_and_sink(form, sizes, window):
+    import test_fozerax_kernels_gpu as t
+    t.test_tensor_core_attention_with_distance_bias_and_sink(sizes, window)
+
+
+@pytest.mark.parametrize("window,keep", [(None, 0), (150, 40), (128, 3), (300, 200), (40, 130), (520, 1)])
+@pytest.mark.parametrize("sizes", [(4, 2, 64), (2, 1, 128)])
+def test_both_forms_with_slopes_and_kept_first_keys(form, sizes, window, keep):
+    import test_biravik_kernels_gpu as t
+    t.test_prompt_portions_on_the_tensor_core_kernel_with_slopes_and_kept_first_keys(sizes, window, keep)
