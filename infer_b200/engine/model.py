@@ -58,21 +58,21 @@ class Model:
         """Every part, block and product of the model with its attributes, in a fixed order, whatever it sits in (attributes, lists,
         dicts): [object, None, None, object, attribute name, value, ...] (one list: tens of thousands of tuples would be the garbage
         collector's)."""
-        found, seen = [], set()
-
-        def visit(obj):
-            if isinstance(obj, dict):
-                obj = list(obj.values())
-            if isinstance(obj, (list, tuple)):
-                for v in obj:
-                    visit(v)
-            elif isinstance(obj, Watched) and id(obj) not in seen:
-                seen.add(id(obj))
+        # (a list of what is left to visit, not a function that calls itself: such a closure is a cycle, and would keep the weights that it
+        # has listed alive until the next collection)
+        found, seen, left = [], set(), [*self.all_parts(), *self.blocks]
+        while left:
+            obj = left.pop()
+            if not isinstance(obj, (dict, list, tuple, Watched)) or id(obj) in seen:
+                continue
+            seen.add(id(obj))
+            if isinstance(obj, Watched):
                 found.extend((obj, None, None))
                 for name, value in vars(obj).items():
                     found.extend((obj, name, value))
-                    visit(value)
-        visit([*self.all_parts(), *self.blocks])
+                    left.append(value)
+            else:
+                left.extend(obj.values() if isinstance(obj, dict) else obj)
         return found
 
     def built_in(self) -> bool:

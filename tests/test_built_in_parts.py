@@ -1,5 +1,8 @@
 """Which models count as made of the package's own parts only (the 32-bit path captures the steps of those): parts anywhere inside other
 parts are looked at, and methods that were replaced on an instance or a class count as foreign."""
+import gc
+import weakref
+
 import pytest
 
 import infer_b200.models  # noqa: F401  (registers the architectures)
@@ -73,4 +76,26 @@ def test_a_method_replaced_on_a_class_or_a_block(monkeypatch):
 def test_parts_that_know_each_other():
     a, b = _bare(Attention), _bare(Attention)
     a.other, b.other = b, a
+    assert _model(a).built_in()
+
+
+def test_looking_at_the_parts_keeps_none_of_them():
+    """A model's weights go with the model, without waiting for a collection."""
+    collecting = gc.isenabled()
+    gc.disable()
+    try:
+        model = _model(_sides(_bare(Attention)))
+        part = weakref.ref(model.blocks[0].mixer.sides["second"])
+        assert model.built_in() and len(model.made_of()) > 3
+        del model
+        assert part() is None
+    finally:
+        if collecting:
+            gc.enable()
+
+
+def test_containers_that_hold_themselves():
+    a = _bare(Attention)
+    a.more = [a]
+    a.more.append(a.more)
     assert _model(a).built_in()
