@@ -25,7 +25,7 @@ from .. import ops
 from ..cache.manager import CacheManager
 from ..config.registry import load_config
 from ..config.specs import ModelSpec
-from ..parts.base import CHANGES
+from ..parts.base import CHANGES, watch
 from ..runtime import Runtime, parse_dtype
 from ..weights.binder import load_weights
 from .model import Model
@@ -196,7 +196,7 @@ class Engine:
         self._portion_runs: Dict[tuple, _PortionRun] = {}
         self._ms_per_launch = float("inf")                # the fastest eager run's host time per launch
         self._graph_pool = None
-        self._made_of, self._changes_seen = None, -1
+        self._made_of, self._seen = None, ()
         self._look_at_parts()
 
     # ------------------------------------------------------------------ construction helpers
@@ -224,10 +224,14 @@ class Engine:
     def _look_at_parts(self) -> None:
         """32-bit path: captured steps go when an attribute of a part was replaced since they were made (a method, a matrix, a whole
         part), and while one of the parts is not the package's own every step runs eagerly, as it would without graphs."""
-        if not (self._may_use_graphs and self._copy_results) or self._changes_seen == CHANGES[0]:
+        if not (self._may_use_graphs and self._copy_results):
             return
-        self._changes_seen = CHANGES[0]
+        seen = (CHANGES[0], self.model, *self.model.blocks)
+        if seen == self._seen:
+            return
+        self._seen = seen
         before, self._made_of = self._made_of, self.model.made_of()
+        watch(self._made_of[::3])
         if before is None or len(before) != len(self._made_of) or any(x is not y for x, y in zip(before, self._made_of)):
             self._graphs.clear()
             self._portion_runs.clear()

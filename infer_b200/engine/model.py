@@ -19,7 +19,7 @@ from ..runtime import Runtime
 from ..weights.binder import check_weights
 
 
-class Model:
+class Model(Watched):
     def __init__(self, spec: ModelSpec, weights: Mapping[str, torch.Tensor], runtime: Runtime):
         spec.validate()
         check_weights(weights, spec)
@@ -55,12 +55,12 @@ class Model:
         return all(getattr(p, "graph_safe", True) for p in self.all_parts())
 
     def made_of(self) -> list:
-        """Every part, block and product of the model with its attributes, in a fixed order, whatever it sits in (attributes, lists,
+        """The model, and every part, block and product of it, with its attributes, in a fixed order, whatever it sits in (attributes, lists,
         dicts): [object, None, None, object, attribute name, value, ...] (one list: tens of thousands of tuples would be the garbage
         collector's)."""
-        # (a list of what is left to visit, not a function that calls itself: such a closure is a cycle, and would keep the weights that it
-        # has listed alive until the next collection)
-        found, seen, left = [], set(), [*self.all_parts(), *self.blocks]
+        # (A list of what is left to visit, not a function that calls itself: such a closure is a cycle, and would keep the weights that it
+        # has listed alive until the next collection.)
+        found, seen, left = [], set(), [self]
         while left:
             obj = left.pop()
             if not isinstance(obj, (dict, list, tuple, Watched)) or id(obj) in seen:
@@ -69,8 +69,9 @@ class Model:
             if isinstance(obj, Watched):
                 found.extend((obj, None, None))
                 for name, value in vars(obj).items():
-                    found.extend((obj, name, value))
-                    left.append(value)
+                    if name != "_watched":
+                        found.extend((obj, name, value))
+                        left.append(value)
             else:
                 left.extend(obj.values() if isinstance(obj, dict) else obj)
         return found

@@ -62,22 +62,32 @@ class CompositeNeed:
 
 # ----------------------------------------------------------------------------- interfaces
 
-# How many attributes were set on or taken from any ``Watched`` object (in a list: an attribute of the class would empty Python's
-# method caches of all parts each time).
+# How often an attribute was set on or taken from an object that is being watched (in a list: an attribute of the class would empty
+# Python's method caches of all parts each time).
 CHANGES = [0]
 
 
 class Watched:
-    """What a model is made of: whoever keeps something made from such objects (a captured step) sees by ``CHANGES`` that none has
-    changed since."""
+    """What a model is made of. Whoever keeps something made from such objects (a captured step) has them watched, and sees by
+    ``CHANGES`` that none has changed since. Until somebody watches, and for objects that nobody does, nothing is counted."""
 
-    def __setattr__(self, name, value):
-        CHANGES[0] += 1
-        object.__setattr__(self, name, value)
 
-    def __delattr__(self, name):
+def _set(self, name, value):
+    if "_watched" in self.__dict__:
         CHANGES[0] += 1
-        object.__delattr__(self, name)
+    object.__setattr__(self, name, value)
+
+
+def _delete(self, name):
+    if "_watched" in self.__dict__:
+        CHANGES[0] += 1
+    object.__delattr__(self, name)
+
+
+def watch(objects) -> None:
+    Watched.__setattr__, Watched.__delattr__ = _set, _delete
+    for obj in objects:
+        obj.__dict__["_watched"] = True
 
 
 class Part(Watched):

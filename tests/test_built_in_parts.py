@@ -8,7 +8,7 @@ import pytest
 import infer_b200.models  # noqa: F401  (registers the architectures)
 from infer_b200.engine.model import Model
 from infer_b200.parts.attention import Attention
-from infer_b200.parts.base import Block, Mixer
+from infer_b200.parts.base import CHANGES, Block, Mixer, watch
 from infer_b200.parts.linear import Linear
 from infer_b200.parts.rmsnorm import RMSNorm
 from infer_b200.parts.side_by_side import SideBySide
@@ -32,6 +32,7 @@ def _bare(cls, **attributes):
 
 def _model(mixer, block_class=Block):
     model = Model.__new__(Model)
+    model.spec = model.rt = None
     model.embedding = model.head = model.final_norm = _bare(RMSNorm)
     model.stream = None
     model.blocks = [block_class(norm=_bare(RMSNorm), mixer=mixer)]
@@ -99,3 +100,19 @@ def test_containers_that_hold_themselves():
     a.more = [a]
     a.more.append(a.more)
     assert _model(a).built_in()
+
+
+def test_only_what_is_watched_is_counted():
+    """The parts of other models, a model that is being built and one whose steps nobody keeps cost and count nothing."""
+    model, other = _model(_sides(_bare(Attention))), _model(_bare(Attention))
+    before = model.made_of()
+    watch(before[::3])
+    n = CHANGES[0]
+    other.blocks[0].mixer.scale = 2.0
+    _model(_bare(Attention, qkv=_bare(Linear)))
+    assert CHANGES[0] == n and len(model.made_of()) == len(before)
+    model.blocks[0].mixer.sides["second"].scale = 2.0
+    model.blocks[0].extra = 1
+    del model.blocks[0].extra
+    model.final_norm = _bare(RMSNorm)
+    assert CHANGES[0] == n + 4

@@ -220,6 +220,8 @@ def test_float32_steps_see_what_was_replaced():
         assert len(calls) == before + 5
         eng.model.head.linear.weight = eng.model.head.linear.weight * 2.0
         some(6)
+        eng.model.blocks[0], eng.model.blocks[2] = eng.model.blocks[2], eng.model.blocks[0]
+        some(6)
         eng.end_request("r")
         return outs
     eager, captured = _engine("b", torch.float32, cuda_graphs=False), _engine("b", torch.float32)
