@@ -235,7 +235,7 @@ class Engine:
         if before is None or len(before) != len(self._made_of) or any(x is not y for x, y in zip(before, self._made_of)):
             self._graphs.clear()
             self._portion_runs.clear()
-            self.use_graphs = self.model.built_in()
+            self.use_graphs = self.model.built_in(self._made_of)
 
     def _build_context(self, entries: Sequence[StepEntry], graphs: bool = False, sample=None):
         """Packs the step's integers on the host and places them on the device. With ``graphs`` and a decode-only

@@ -76,9 +76,9 @@ class Model(Watched):
                 left.extend(obj.values() if isinstance(obj, dict) else obj)
         return found
 
-    def built_in(self) -> bool:
+    def built_in(self, made_of=None) -> bool:
         """True if every part, the parts inside parts, every block and product are this package's own, and so are their methods: none
-        was replaced, neither on an instance nor on its class."""
+        was replaced, neither on an instance nor on its class. ``made_of``: what ``made_of()`` gave, if that is at hand."""
         own = __name__.split(".")[0]
 
         def ours(x) -> bool:
@@ -86,7 +86,7 @@ class Model(Watched):
 
         def own_class(cls) -> bool:
             return all(ours(c) and all(ours(f) for f in vars(c).values() if isinstance(f, FunctionType)) for c in cls.__mro__ if c is not object)
-        made_of = self.made_of()
+        made_of = self.made_of() if made_of is None else made_of
         return (all(own_class(c) for c in {type(o) for o in made_of[::3]})
                 and not any(callable(v) and name is not None and hasattr(type(o), name) and not ours(v)
                             for o, name, v in zip(made_of[::3], made_of[1::3], made_of[2::3])))
