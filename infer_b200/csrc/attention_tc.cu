@@ -32,9 +32,9 @@
 // P V, store P): neither two threads per row nor a second MMA-issuing thread shortened it, and with one CTA an SM the tensor
 // cores wait meanwhile. So two CTAs share an SM (112 KB of shared memory and half of the tensor memory each), which is what
 // tiles of 64 keys are for. One CTA alone walks faster in tiles of 128 (-DIB_ATTN_BN=128; 2.3 us against 3.2 per 128 keys):
-// where few long query tiles all run at once, the host takes that form. Measured, 128 -> 64 keys, heads of 128: 12 heads,
-// ten segments of 200 tokens 21.4 -> 12.5 us, 4,096 tokens behind 11,777 687 -> 635; 28 heads, 2,048 tokens 77.5 -> 62.3, 4,096
-// behind 11,777 1,593 -> 1,265 (644 TFLOP/s). Query tiles start heaviest first.
+// where few long query tiles all run at once, the host takes that form. Measured, whole query tiles, 128 -> 64 keys, heads of 128:
+// 12 heads, 512 tokens 12.8 -> 15.3 us, 2,048 36.3 -> 52.9, ten segments of 200 18.5 -> 12.5, 4,096 tokens behind 11,777 619 -> 635 (471
+// in three parts); 28 heads, 2,048 tokens 68.3 -> 62.0, 4,096 behind 11,777 1,418 -> 1,261 (644 TFLOP/s). Query tiles start heaviest first.
 // Every mbarrier wait is bounded; one that runs out raises the status word, and the CTA drains its copies,
 // frees its tensor memory and returns.
 #include <algorithm>

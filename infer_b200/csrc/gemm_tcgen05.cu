@@ -5,8 +5,9 @@
 // Structure of one CTA (192 threads, one 128 x BN output tile, BN in {16, 32, 64, 128}; 256 with K slices):
 //   warp 0      one lane issues TMA loads (cp.async.bulk.tensor.2d, 128-byte swizzle) of 128 x 64 and BN x 64
 //               operand tiles into a ring of shared-memory stages, each guarded by a full/empty mbarrier pair;
-//   warp 1      allocates BN TMEM columns; one lane issues tcgen05.mma (M=128, N=BN, K=16, kind::f16) four times
-//               per stage, then tcgen05.commit to hand the stage back, and at the end to signal the epilogue;
+//   warp 1      allocates BN TMEM columns; the warp walks over the stages, one elected lane issues tcgen05.mma (M=128,
+//               N=BN, K=16, kind::f16) four times per stage, then tcgen05.commit to hand the stage back, and at the end
+//               to signal the epilogue;
 //   warps 2-5   read the accumulator with tcgen05.ld (each warp its 32 TMEM lanes = 32 tile rows), apply the
 //               epilogue (bias, residual, conversion) and store to global memory.
 //
@@ -23,8 +24,9 @@
 // A long K on few tiles (a 512-token portion of a prompt against a down matrix) takes 128 x 256 tiles with 2, 4 or 8
 // K slices as a cluster: 128 KB of float tile do not fit behind the ring, so the slices' columns are received in the
 // operand ring itself, once a cluster barrier has told every slice that the others' MMAs are done.
-// For many tokens a persistent kernel (further down) walks over tiles with two accumulators in tensor memory.
-// ib_gemm_tc_plan chooses among these ways with a time model fitted to measurements.
+// For many tokens a persistent kernel (further down) walks over tiles with two accumulators in tensor memory, on one SM a
+// tile or on pairs of SMs. ib_gemm_tc_plan chooses among the ways of single SMs with a time model fitted to measurements,
+// ib_gemm_tc_pairs says where pairs are faster than what it chose.
 // What is read once per step (the weights' tiles) is loaded with the L2 evict-first policy.
 // In the swapped mapping the ring takes up to eight stages (the CTA has the SM to itself and all of its weights
 // should be in flight) and the weights' first stages are requested before the kernel waits for its predecessor.
@@ -1280,8 +1282,9 @@ IB_EXPORT int ib_gemm_tc_plan(int64_t M, int64_t N, int64_t K, int sm_count, int
 IB_EXPORT int ib_gemm_tc_pairs(int64_t M, int64_t N, int64_t K, int sm_count, int swap, int bn, int s, int64_t workspace_floats) {
     // Pairs of SMs on tiles of 256 rows, where a model like the planner's says so. In its unit (0.38 us) a k-block takes a pair
     // 0.50 + width / 655 (0.264 us at width 128, 0.338 at 256) and an SM by itself 0.74 + width / 790 (0.364 at 176, 0.403 at 256: the way from L2 is the bound, and a pair's tile takes a third less through it), beside 20 units a launch
-    // for the pairs, 16 alone. Measured against the other plans at 2,048 rows: gate/up 75.5 and 85.2 us, down 46.6 and 56.3 at 1,536
-    // features, 348 and 392, 210 and 270 at 3,584; one round of short tiles (2048 features, K = 1536: 14.1 and 13.8) stays as it is.
+    // for the pairs, 16 alone. Measured against the other plans at 2,048 rows: gate/up 75.9 and 83.9 us, down 47.1 and 57.2 at 1,536
+    // features, 349 and 385, 207 and 249 at 3,584; at 512 rows and 3,584 features o 22.5 and 29.6, q/k/v 19.4 and 24.8, gate/up 99 and 108;
+    // one round of short tiles (2048 features, K = 1536: 14.1 and 13.9) stays as it is.
     static const bool pairs_on = [] { const char* e = getenv("INFER_B200_GEMM_PAIRS"); return !(e && e[0] == '0'); }();
     if (swap || !pairs_on || sm_count < 2 || workspace_floats > 0) return 0;
     const int kb_total = int((K + BK - 1) / BK);

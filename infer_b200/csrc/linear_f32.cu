@@ -13,7 +13,7 @@
 // Where the caller says that no kernel still running writes w (a loaded weight), the ring's first weights are requested before
 // the kernel waits for its predecessor.
 //
-// (17920 x 1536: 1 row 19 us = 5.8 TB/s, 3 rows 30, 8 rows 43, bound by the reads of x from shared memory; 1536 x 8960: 15, 25, 34.
+// (17920 x 1536: 1 row 20 us = 5.5 TB/s, 3 rows 31, 8 rows 44, bound by the reads of x from shared memory; 1536 x 8960: 17, 25, 35.
 // A single token's step of the 1.5B sizes on tiles of 64 x 64 with scalar reads and no copies in flight took 55.6 ms, its products now 2.)
 //
 // More rows, `tile32_kernel`: bound by the FMA units, which run at 57 % (512 rows, 17920 x 1536: 670 us = 42 TFLOP/s; scalar FMAs
@@ -275,7 +275,7 @@ int dispatch(const Args& a, int kind, int sms, cudaStream_t stream) {
     if (kind == 0) {
         if (a.M <= 8) {
             // 16 features a CTA share a row of x among twice as many threads; 8 where those CTAs leave SMs idle (N = 1536, K = 8960:
-            // one row 15.0 against 16.0 us, 8 rows 34.0 against 35.8; with 3 rows 24.8 either way, N = 2048, K = 1536: 4.9 and 5.0)
+            // 8 rows 34.5 against 36.4 us, one row 17.3 to 17.7 either way; with 3 rows 25.4 either way, N = 2048, K = 1536: 5.0 and 5.1)
             kind = (a.N + 15) / 16 >= 2LL * sms || (a.M > 1 && a.M <= 4) ? 1 : 2;
         } else {
             // The larger a thread's share the fewer shared-memory reads per FMA, but a CTA alone on its SM is bound by its own

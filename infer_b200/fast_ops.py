@@ -143,7 +143,8 @@ def gemm_tc(x: torch.Tensor, w: torch.Tensor, bias: Optional[torch.Tensor] = Non
             out_dtype: torch.dtype = torch.bfloat16, out: Optional[torch.Tensor] = None, plan=None,
             swiglu: bool = False) -> Optional[torch.Tensor]:
     """out = x @ w.T (+ bias) (+ residual) on the tcgen05 tensor cores; None if the sizes are refused.
-    x [M, K], w [N, K] bfloat16; bias float32 [N]; residual float32 [M, N] (may be `out`). With ``swiglu`` the
+    x [M, K], w [N, K] bfloat16; bias float32 [N]; residual float32 [M, N] (may be `out`). ``w`` is a loaded weight: no kernel
+    that may still be running writes it (it may be read before this kernel's predecessor has ended). With ``swiglu`` the
     rows of w are gate/up features interleaved in blocks of 8 and the result is silu(gate) * up, [M, N/2]."""
     _check(x, "x", torch.bfloat16)
     _check(w, "w", torch.bfloat16)
@@ -363,11 +364,9 @@ ATTENTION_TC_PART_MIN_TILES = 4
 
 
 def prefill_split(sm_count: int, n_heads: int, n_prefill: int, max_q_len: int, max_ctx_len: int, window: Optional[int]) -> int:
-    """Into how many parts the tcgen05 prefill kernel may cut the keys of a query tile. One CTA serves 128 queries of a
-    head and walks over their keys in tiles of 128; it has an SM to itself, and starting and finishing a CTA costs
-    about as much as three key tiles. So keys are shared only while all CTAs still run at once (a portion behind a
-    long context on few heads: 48 CTAs of 36 key tiles become 144 of 12); with more CTAs than SMs the extra starts
-    cost more than the evening-out gains (measured at 2,048 tokens on 12 heads: 38.5 us whole, 42 us shared)."""
+    """A first guess at how many parts the tcgen05 prefill kernel may cut the keys of a query tile into, counted in tiles of 128 keys:
+    as many as let all CTAs run at once with one an SM (a portion behind a long context on few heads: 48 CTAs of 36 key tiles become
+    144 of 12). ``_prefill_plan`` compares it with a simulated layout; it stands where key ranges are short or CTAs many."""
     if n_prefill <= 0 or max_q_len <= 1:
         return 1
     ctx0 = max_ctx_len - max_q_len
@@ -424,12 +423,12 @@ def prefill_plan(sm_count: int, n_heads: int, head_dim: int, seg_lens, max_ctx_l
 @functools.lru_cache(maxsize=4096)
 def _prefill_plan(sm_count: int, n_heads: int, head_dim: int, lens, max_ctx_len: int, window: Optional[int]):
     """Alone on its SM a CTA is bound by its own chain, 2.3 us per 128 keys against 3.2 per 2 x 64: 128 keys where the query tiles
-    are long (512 keys and more) and all run at once. Measured with 12 heads (192 CTAs at 2,048 tokens): 512 tokens 13.4 us with
-    128 keys and 15.9 with 64, 2,048 tokens 36 and 42, ten segments of 200 tokens 21 and 12.5; with 28 heads 2,048 tokens 77 and 62,
-    4,096 behind 11,777 1,593 and 1,257. Then the CTAs are laid onto the SMs in the order they start, for every number of parts:
+    are long (512 keys and more) and all run at once. Measured with 12 heads (192 CTAs at 2,048 tokens): 512 tokens 12.8 us with
+    128 keys and 15.3 with 64, 2,048 tokens 36.3 and 52.9, ten segments of 200 tokens 18.5 and 12.5; with 28 heads 2,048 tokens 68.3
+    and 62.0, 4,096 behind 11,777 1,418 and 1,261. Then the CTAs are laid onto the SMs in the order they start, for every number of parts:
     in units of 1.75 us a CTA takes one per 64 keys and 4 to start and end (1.3 per 128 keys and 3), 3 more where parts meet. A
     long second round that is nearly empty is what parts avoid: 12 heads, 4,096 tokens behind 11,777 (384 CTAs on 296 places)
-    632 us whole, 471 in three parts; 1,024 behind 8,192 145 and 89; 28 heads, 2,048 behind 8,192 436 and 402."""
+    635 us whole, 471 in three parts; 1,024 behind 8,192 215 (145 with 128 keys) and 87; 28 heads, 2,048 behind 8,192 437 and 402."""
     n64, n128 = [], []                                           # keys of every query tile, in tiles of 64 and 128
     for n in lens:
         for q_first in range(max_ctx_len - n, max_ctx_len, 128):
