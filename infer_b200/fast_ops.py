@@ -386,6 +386,7 @@ def prefill_split(sm_count: int, n_heads: int, n_prefill: int, max_q_len: int, m
 
 PREFILL_PARTS_MAX_FLOATS = 24 << 20      # of scratch that sharing query tiles may take (96 MB)
 PREFILL_SIMULATED_CTAS = 1024            # beyond that many CTAs they even out by themselves
+PREFILL_IDLE_CTA = 0.0029                # units of 1.75 us: a CTA that finds nothing to do takes 5 ns of the launch
 
 
 def prefill_query_tiles(seg_lens) -> int:
@@ -416,19 +417,21 @@ def prefill_plan(sm_count: int, n_heads: int, head_dim: int, seg_lens, max_ctx_l
     """(compile-time sizes of the tcgen05 prefill kernel, into how many parts it may cut the keys of a query tile). The kernel
     walks over keys 64 at a time with two CTAs an SM, whose softmax and products overlap, or 128 at a time with one. Counted for
     portions that end at max_ctx_len, which is all that a captured step knows; any answer is correct."""
-    form, split = _prefill_plan(sm_count, n_heads, head_dim, tuple(n for n in seg_lens if n > 1) or (1,), max_ctx_len, window)
+    form, split = _prefill_plan(sm_count, n_heads, head_dim, tuple(n for n in seg_lens if n > 1) or (1,), max_ctx_len, window, len(seg_lens))
     return ({"IB_HEAD_DIM": head_dim, "IB_ATTN_BN": 128} if form == 128 else {"IB_HEAD_DIM": head_dim}), split
 
 
 @functools.lru_cache(maxsize=4096)
-def _prefill_plan(sm_count: int, n_heads: int, head_dim: int, lens, max_ctx_len: int, window: Optional[int]):
+def _prefill_plan(sm_count: int, n_heads: int, head_dim: int, lens, max_ctx_len: int, window: Optional[int], n_segments: int):
     """Alone on its SM a CTA is bound by its own chain, 2.3 us per 128 keys against 3.2 per 2 x 64: 128 keys where the query tiles
     are long (512 keys and more) and all run at once. Measured with 12 heads (192 CTAs at 2,048 tokens): 512 tokens 12.8 us with
     128 keys and 15.3 with 64, 2,048 tokens 36.3 and 52.9, ten segments of 200 tokens 18.5 and 12.5; with 28 heads 2,048 tokens 68.3
     and 62.0, 4,096 behind 11,777 1,418 and 1,261. Then the CTAs are laid onto the SMs in the order they start, for every number of parts:
     in units of 1.75 us a CTA takes one per 64 keys and 4 to start and end (1.3 per 128 keys and 3), 3 more where parts meet. A
     long second round that is nearly empty is what parts avoid: 12 heads, 4,096 tokens behind 11,777 (384 CTAs on 296 places)
-    635 us whole, 471 in three parts; 1,024 behind 8,192 215 (145 with 128 keys) and 87; 28 heads, 2,048 behind 8,192 437 and 402."""
+    635 us whole, 471 in three parts; 1,024 behind 8,192 215 (145 with 128 keys) and 87; 28 heads, 2,048 behind 8,192 437 and 402. The grid has as many CTAs for every
+    segment, one-token ones among them, as for the longest, and parts multiply those that find nothing to do: beside 63 one-token segments
+    the last case takes 579 us whole and 829 in three parts, 12 heads with 1,024 behind 8,192 231 and 178."""
     n64, n128 = [], []                                           # keys of every query tile, in tiles of 64 and 128
     for n in lens:
         for q_first in range(max_ctx_len - n, max_ctx_len, 128):
@@ -447,7 +450,8 @@ def _prefill_plan(sm_count: int, n_heads: int, head_dim: int, lens, max_ctx_len:
         for n in sorted(tiles, reverse=True):
             k = max(1, min(parts, n // ATTENTION_TC_PART_MIN_TILES))
             jobs += [per_tile * -(-n // k) + start + (3.0 if k > 1 else 0.0)] * (n_heads * k)
-        return _makespan(jobs, slots)
+        idle = n_heads * -(-max(lens) // 128) * parts * n_segments - len(jobs)
+        return _makespan(jobs, slots) + PREFILL_IDLE_CTA * idle
     now = estimate(n128, split, 1.3, 3.0, sm_count) if form == 128 else estimate(n64, split, 1.0, 4.0, 2 * sm_count)
     best = (0.96 * now, form, split)
     for parts in range(1, ATTENTION_TC_MAX_SPLIT + 1):

@@ -69,3 +69,14 @@ def test_both_forms_are_built_at_the_first_use_of_either(head_dim, monkeypatch):
     assert sorted(len(d) for m, d in compiled if m == "attn_tc" and d["IB_HEAD_DIM"] == head_dim) == [1, 2] and len(compiled) == 2
     assert loaded == [{"IB_HEAD_DIM": head_dim}] * 2
     fast_ops._build_prefill_forms.cache_clear()
+
+
+@pytest.mark.parametrize("heads,n,before,singles,parts", [
+    (28, 2048, 8192, 0, 3), (28, 2048, 8192, 31, 1), (28, 2048, 8192, 63, 1),        # measured: 402 us, then 614 and 829 in three parts, 579 whole
+    (28, 512, 2048, 63, 1),                                                         # 113 us in two parts, 94 whole
+    (12, 1024, 8192, 0, 3), (12, 1024, 8192, 31, 3), (12, 1024, 8192, 63, 3),        # 178 us in three parts, 231 whole
+    (12, 512, 4096, 63, 3),                                                         # 82 and 90
+])
+def test_parts_count_the_ctas_that_one_token_segments_leave_idle(heads, n, before, singles, parts):
+    from infer_b200 import fast_ops
+    assert fast_ops.prefill_plan(SMS, heads, 128, [1] * singles + [n], n + before, None)[1] == parts
