@@ -437,9 +437,9 @@ class Engine:
         return out
 
     def _capture(self, ctx: StepContext):
-        """The step as a CUDA graph: (graph, its output), or None if there is no memory for it. Capturing only records, so nothing needs to have ended on the
-        device; ``torch.cuda.graph`` waits for it, collects garbage and gives the allocator's free memory back to the
-        driver, which costs milliseconds to hundreds of them. That is the second way, where memory is short."""
+        """The step as a CUDA graph: (graph, its output), or None if there is no memory for it. Capturing only records, so nothing
+        needs to have ended on the device; ``torch.cuda.graph`` waits for it, collects garbage and gives the allocator's free
+        memory back to the driver, which costs milliseconds to hundreds of them. That is the second way, where memory is short."""
         with _CAPTURING:
             return self._capture_alone(ctx)
 
