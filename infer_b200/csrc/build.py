@@ -30,6 +30,7 @@ NVCC_FLAGS = ["-gencode", "arch=compute_100a,code=sm_100a", "-lineinfo", "-O3", 
 MODULES: Dict[str, str] = {
     "plain": "plain_ops.cu",
     "lin32": "linear_f32.cu",    # the matrix product of the 32-bit path
+    "lin32_tc": "linear_f32_tc.cu",     # the same for large matrices, on the tensor cores
     "seq": "seq_ops.cu",         # filters over time, pair rotation, gated recurrence, side-by-side sublayers
     "mix": "mix_ops.cu",         # norms on sublayer results, decayed and delta-rule recurrences, routers, row norms of q and k
     "latent": "latent_ops.cu",   # attention through low-rank latents, layer norm, sigmoid router, capped logits
