@@ -251,6 +251,17 @@ def linear(x, weight, bias, residual, out_dtype, out, swiglu=False):
     return gemm_tc(x, weight, bias, residual, out_dtype, out, swiglu=swiglu)
 
 
+def linear_f32_tc(x: torch.Tensor, w: torch.Tensor, bias: Optional[torch.Tensor], residual: Optional[torch.Tensor], out: torch.Tensor,
+                  w_ready: bool) -> torch.Tensor:
+    """The 32-bit path's product by a large matrix (``ops.linear_plain`` has looked at the operands): each float as three bfloat16 numbers
+    on the tensor cores."""
+    st = device_state(x.device)
+    f = _fn("lin32_tc", "ib_linear_f32_tc", [c_void_p] * 5 + [c_int64] * 3 + [c_int] * 2 + [c_void_p] * 2)
+    _call(f, x.data_ptr(), w.data_ptr(), _ptr(bias), _ptr(residual), out.data_ptr(), x.shape[0], w.shape[0], x.shape[1], st.sm_count,
+          int(w_ready), st.status.data_ptr(), _stream())
+    return out
+
+
 GROUPED_FROM = 256            # tokens from which a routed feed-forward's rows are worth grouping by expert
 
 

@@ -8,6 +8,7 @@ from __future__ import annotations
 
 import collections
 import ctypes
+import functools
 import os
 from typing import Optional
 
@@ -128,11 +129,16 @@ def rmsnorm(x: torch.Tensor, weight: torch.Tensor, eps: float, out_dtype: torch.
     return out
 
 
+@functools.lru_cache(maxsize=None)
+def _f32_on_tensor_cores(N: int, K: int) -> bool:
+    return bool(_fn("lin32_tc", "ib_linear_f32_tc_takes", [c_int64, c_int64])(N, K))
+
+
 def linear_plain(x: torch.Tensor, w: torch.Tensor, bias: Optional[torch.Tensor] = None,
                  residual: Optional[torch.Tensor] = None, out_dtype: Optional[torch.dtype] = None,
                  out: Optional[torch.Tensor] = None, kind: int = 0, w_ready: bool = False) -> torch.Tensor:
-    """out = x @ w.T (+ bias) (+ residual) with float accumulation in an order that K alone fixes. kind: which of the
-    float32 kernels (0 = by the sizes; every one gives the same bits). w_ready: no kernel that may still be running writes
+    """out = x @ w.T (+ bias) (+ residual) with float accumulation in an order that N and K alone fix. kind: which of the
+    float32 kernels (0 = by the sizes; 1 to 5, which large matrices do not take by themselves, all give the same bits). w_ready: no kernel that may still be running writes
     ``w`` (a loaded weight), so that it may be read while the kernels before this one drain."""
     _check(x, "x")
     _check(w, "w", x.dtype)
@@ -150,6 +156,9 @@ def linear_plain(x: torch.Tensor, w: torch.Tensor, bias: Optional[torch.Tensor] 
     else:
         _check(out, "out", out_dtype, (M, N))
     if x.dtype == torch.float32 and out_dtype == torch.float32:
+        if kind == 0 and _f32_on_tensor_cores(N, K):
+            from . import fast_ops
+            return fast_ops.linear_f32_tc(x, w, bias, residual, out, w_ready)
         f = _fn("lin32", "ib_linear_f32", [c_void_p] * 5 + [c_int64] * 3 + [c_int, c_int, c_int, c_void_p])
         _call(f, x.data_ptr(), w.data_ptr(), _ptr(bias), _ptr(residual), out.data_ptr(), M, N, K, int(kind), 0, int(w_ready), _stream())
         return out
