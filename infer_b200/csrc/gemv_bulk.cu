@@ -53,6 +53,7 @@ constexpr int RING_BYTES = 2 * ROWS * (KC_MAX * 2 + 64);
 constexpr int NW_BYTES = KC_MAX * 4;         // the fused norm's weight, behind the ring
 constexpr uint32_t SPIN_LIMIT = 1u << 22;
 constexpr int STATUS_TIMEOUT = 104;
+constexpr int PART_FLOATS = 2 * 8 * ROWS; // a tile's sums in the workspace
 
 __device__ __forceinline__ uint32_t smem_u32(const void* p) { return uint32_t(__cvta_generic_to_shared(p)); }
 __device__ __forceinline__ void mbar_init(uint32_t bar, uint32_t count) {
@@ -130,11 +131,15 @@ struct GemvParams {
                               //    copies (up to 8 rows of activations; measured: q/k/v 4.1 -> 3.2 us)
     int kc;                   // elements of K per stage and row: a multiple of 64, at most KC_MAX
     int ns;                   // stages in the ring: 2 .. NS_MAX, ns * ROWS * (kc * 2 + 64) <= RING_BYTES
-    int64_t tiles;
+    int tiles;
+    int n_stages, per_cta;    // stages of a tile's K, and of a CTA of its cluster
     int groups;               // tile walkers in the grid (grid = groups * cluster); a walker takes every groups-th tile
     int* status;
-    const void* prefetch;     // weights of a later kernel to pull into L2 meanwhile (or null)
-    int64_t prefetch_bytes;
+    // even: the stages of all tiles, tile after tile, are dealt out in equal runs, one a CTA (run + 1 stages to the first `longer`
+    // CTAs, `run` to the others); a tile that several CTAs share is put together by the one that completes its count
+    int even, run, longer;
+    float* parts;             // [grid][2][PART_FLOATS]: sums of the tiles that a CTA begins and ends inside
+    unsigned int* arrived;    // [tiles] stages summed so far, zero between calls
 };
 
 template <int NT, int EPI, typename TOut, bool NWS>
@@ -146,6 +151,7 @@ bulk_gemv_kernel(const GemvParams p) {
     __shared__ float part[NT][8][ROWS];                  // this CTA's sum; read by the cluster's first CTA
     __shared__ float sumsq[WARPS][NT * 8];               // the warps' shares of a row's sum of squares (fused norm)
     __shared__ int failed;
+    __shared__ int last_here;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int g = lane >> 2, t = lane & 3;
     const int cluster = p.cluster;
@@ -156,12 +162,15 @@ bulk_gemv_kernel(const GemvParams p) {
     const int PITCH = KC * 2 + 64;                       // bytes between rows of a stage: consecutive rows start 16 banks apart
     const int STAGE_BYTES = ROWS * PITCH;
     // This CTA's slice of K, in stages of KC elements.
-    const int64_t total_stages = (K + KC - 1) / KC;
-    const int64_t per_cta = (total_stages + cluster - 1) / cluster;
-    const int64_t s_begin = min(total_stages, rank * per_cta), s_end = min(total_stages, s_begin + per_cta);
-    const int spt = int(s_end - s_begin);                // stages per tile
-    const int64_t my_tiles = group < p.tiles ? (p.tiles - group + p.groups - 1) / p.groups : 0;
-    const int64_t n_iter = my_tiles * spt;
+    const int total_stages = p.n_stages;
+    const int s_begin = min(total_stages, rank * p.per_cta), s_end = min(total_stages, s_begin + p.per_cta);
+    const int spt = s_end - s_begin;                     // stages per tile
+    const int run0 = int(blockIdx.x) * p.run + min(int(blockIdx.x), p.longer);          // (even) the CTA's first stage
+    const int my_tiles = group < p.tiles ? (p.tiles - group + p.groups - 1) / p.groups : 0;
+    const int n_iter = p.even ? p.run + (int(blockIdx.x) < p.longer ? 1 : 0) : my_tiles * spt;
+    const int tile0 = p.even ? run0 / total_stages : group;
+    const int st0 = p.even ? run0 - tile0 * total_stages : 0;
+    const int tile_step = p.even ? 1 : p.groups;
     const uint32_t stage0 = smem_u32(stages), bar0 = smem_u32(bars);
     auto full_bar = [&](int s) { return bar0 + 8u * s; };
     auto empty_bar = [&](int s) { return bar0 + 8u * (NS_MAX + s); };
@@ -174,7 +183,8 @@ bulk_gemv_kernel(const GemvParams p) {
     }
     // Rows beyond N (last tile only) are never copied: start from zeros. A stage that held an earlier tile's rows is
     // harmless there, because those rows' results are not stored.
-    if (N % ROWS != 0 && (p.tiles - 1 - group) % p.groups == 0) {     // this CTA takes the last, partial tile
+    // this CTA takes (part of) the last, partial tile
+    if (N % ROWS != 0 && (p.even ? run0 + n_iter > (p.tiles - 1) * total_stages : (p.tiles - 1 - group) % p.groups == 0)) {
         for (int i = threadIdx.x; i < RING_BYTES / 16; i += THREADS) reinterpret_cast<uint4*>(stages)[i] = make_uint4(0u, 0u, 0u, 0u);
         asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
     }
@@ -184,11 +194,11 @@ bulk_gemv_kernel(const GemvParams p) {
         // ---------------------------------------------------------------- producer: lane r copies row r of every stage
         // (ring slot, its use count, stage within the tile and tile are carried along: 64-bit divisions by run-time
         // values would cost more per stage than the copies)
-        int s = 0, st = 0;
+        int s = 0, st = st0;
         uint32_t round = 0;
-        int64_t tile = group;
+        int tile = tile0;
         const uint64_t once = policy_evict_first();
-        for (int64_t i = 0; i < n_iter; i++) {
+        for (int i = 0; i < n_iter; i++) {
             if (i == 1 && p.gate_ring) {
                 // With every SM's ring being filled at once, activations requested after the dependency wait would
                 // queue behind megabytes of weights and the consumers would start microseconds late: the second slot
@@ -204,8 +214,8 @@ bulk_gemv_kernel(const GemvParams p) {
                 ok = __shfl_sync(0xffffffffu, ok, 0);
                 if (!ok) { if (lane == 0) { atomicExch(p.status, STATUS_TIMEOUT); failed = 1; } break; }
             }
-            const int64_t n0 = tile * ROWS;
-            const int64_t k0 = (s_begin + st) * KC;
+            const int64_t n0 = int64_t(tile) * ROWS;
+            const int64_t k0 = int64_t(s_begin + st) * KC;
             const int live_rows = int(min(int64_t(ROWS), N - n0));
             const uint32_t bytes = uint32_t(min(int64_t(KC), K - k0) * 2);
             if (lane == 0) mbar_expect_tx(full_bar(s), bytes * uint32_t(live_rows));
@@ -213,10 +223,9 @@ bulk_gemv_kernel(const GemvParams p) {
             if (lane < live_rows) bulk_load(stage0 + s * STAGE_BYTES + lane * PITCH, p.w + (n0 + lane) * K + k0, bytes, full_bar(s), once);
             if (i == NS - 1 || i == n_iter - 1) ib::pdl_launch_dependents();     // the first ring is on its way
             if (++s == NS) { s = 0; round++; }
-            if (++st == spt) { st = 0; tile += p.groups; }
+            if (++st == spt) { st = 0; tile += tile_step; }
         }
         if (n_iter == 0) ib::pdl_launch_dependents();
-        ib::l2_prefetch_share(p.prefetch, p.prefetch_bytes, blockIdx.x, gridDim.x);
         if (cluster > 1) {                               // the cluster barriers below count every thread
             cg::cluster_group cl = cg::this_cluster();
             cl.sync();
@@ -358,11 +367,11 @@ bulk_gemv_kernel(const GemvParams p) {
     }
 
     IB_GT(2);
-    int s = 0, st = 0;
+    int s = 0, st = st0, st_from = st0;
     uint32_t round = 0;
-    int64_t tile = group;
-    for (int64_t i = 0; i < n_iter; i++) {
-        const int64_t k0 = (s_begin + st) * KC;
+    int tile = tile0;
+    for (int i = 0; i < n_iter; i++) {
+        const int64_t k0 = int64_t(s_begin + st) * KC;
         IB_GT(4 + 4 * int(i));
         if (!hoist) {
             // activations of this warp's chunks: independent of the weights, so they are loaded before the wait
@@ -396,13 +405,14 @@ bulk_gemv_kernel(const GemvParams p) {
         if (lane == 0) mbar_arrive(empty_bar(s));
         IB_GT(6 + 4 * int(i));
         if (++s == NS) { s = 0; round++; }
-        if (++st != spt) continue;
-        st = 0;
+        if (++st != spt && !(p.even && i == n_iter - 1)) continue;
+        const int summed = st - st_from;                 // stages of this tile that this CTA has summed
+        st = st_from = 0;
 
         // ---------------------------------------------------------------- the tile is complete
-        const int64_t this_tile = tile;
-        tile += p.groups;
-        const int64_t n0 = this_tile * ROWS;
+        const int this_tile = tile;
+        tile += tile_step;
+        const int64_t n0 = int64_t(this_tile) * ROWS;
         asm volatile("bar.sync 1, 256;" ::: "memory");   // the previous tile's sums have been read (consumers only)
 #pragma unroll
         for (int nt = 0; nt < NT; nt++) {
@@ -419,6 +429,29 @@ bulk_gemv_kernel(const GemvParams p) {
             for (int wi = 0; wi < WARPS; wi++) v += red[wi][ant][col][r];
         }
         bool writer = true;
+        if (p.even && summed != spt) {
+            // A part of a tile. Its sums go to the workspace; the CTA that completes the tile's count adds all parts in
+            // ascending order of K, so that the result does not depend on which one that is.
+            if (active) __stcg(p.parts + (int(blockIdx.x) * 2 + (this_tile == tile0 ? 0 : 1)) * PART_FLOATS + threadIdx.x, v);
+            __threadfence();
+            asm volatile("bar.sync 1, 256;" ::: "memory");
+            if (threadIdx.x == 0) {
+                last_here = atomicAdd(p.arrived + this_tile, unsigned(summed)) + unsigned(summed) == unsigned(spt);
+                if (last_here) p.arrived[this_tile] = 0u;
+                __threadfence();
+            }
+            asm volatile("bar.sync 1, 256;" ::: "memory");
+            writer = last_here != 0;
+            if (writer && active) {
+                const int u0 = this_tile * total_stages, border = p.longer * (p.run + 1);
+                int c = u0 < border ? u0 / (p.run + 1) : p.longer + (u0 - border) / p.run;      // the CTA whose run holds stage u0
+                int begin = c * p.run + min(c, p.longer);
+                // (a part is its CTA's first tile's, unless the run begins before this tile)
+                v = 0.0f;
+                for (; begin < u0 + total_stages; begin += p.run + (c < p.longer ? 1 : 0), c++)
+                    v += __ldcg(p.parts + (c * 2 + (begin < u0 ? 1 : 0)) * PART_FLOATS + threadIdx.x);
+            }
+        }
         if (cluster > 1) {
             cg::cluster_group cl = cg::this_cluster();
             if (active) part[ant][col][r] = v;
@@ -440,7 +473,7 @@ bulk_gemv_kernel(const GemvParams p) {
         if constexpr (EPI == 2) {
             if (r < 8) {
                 const float gate = v, up = part[ant][col][r + 8];
-                const int64_t f = this_tile * 8 + r;
+                const int64_t f = int64_t(this_tile) * 8 + r;
                 if (f < N / 2) out[int64_t(m) * (N / 2) + f] = ib::from_f32<TOut>(gate / (1.0f + expf(-gate)) * up);
             }
         } else {
@@ -502,7 +535,8 @@ IB_EXPORT int ib_linear_skinny_bulk_limits(int* max_rows, int* max_fused_norm_k)
 
 IB_EXPORT int ib_linear_skinny_bulk(const void* x, const float* norm_w, float norm_eps, const void* w, const float* bias, const float* residual, void* out,
                                     int64_t M, int64_t N, int64_t K, int out_dtype, int epi, int cluster, int sm_count,
-                                    int* status, const void* prefetch, int64_t prefetch_bytes, cudaStream_t stream) {
+                                    int* status, float* parts, int64_t n_parts, unsigned int* arrived, int64_t n_arrived, int even,
+                                    cudaStream_t stream) {
     if (M <= 0 || N <= 0) return IB_OK;
     if (M > 16) return ib::fail(IB_ERR_ARG, "linear_skinny_bulk: at most 16 rows, got %lld", (long long)M);
     if (K <= 0 || K % 8) return ib::fail(IB_ERR_ARG, "linear_skinny_bulk: K = %lld must be a positive multiple of 8", (long long)K);
@@ -526,22 +560,34 @@ IB_EXPORT int ib_linear_skinny_bulk(const void* x, const float* norm_w, float no
         while (cluster < 8 && tiles * cluster < 2LL * sms && n_stages >= 6 * cluster) cluster *= 2;
     }
     if (cluster != 1 && cluster != 2 && cluster != 4 && cluster != 8) return ib::fail(IB_ERR_ARG, "linear_skinny_bulk: cluster must be 1, 2, 4 or 8");
+    // even < 0: chosen here; 0: never; else the number of stages that a tile's K is cut into
+    const int64_t places = int64_t(IB_GEMV_CTAS_PER_SM) * sms;
+    const bool can = !norm_w && tiles * 64 < (1LL << 30) && parts && arrived && n_arrived >= tiles && n_parts >= 2 * places * PART_FLOATS;
+    if (!can) even = 0;
+    if (even < 0) even = 0;
+    if (even > 0) { n_stages = even; cluster = 1; }
     n_stages = (n_stages + cluster - 1) / cluster * cluster;     // the same number of stages for every CTA of a cluster
     const int kc = int(((K + n_stages - 1) / n_stages + 63) / 64 * 64);
     int ns = RING_BYTES / (ROWS * (kc * 2 + 64));
     if (ns > NS_MAX) ns = NS_MAX;
     GemvParams p;
     p.x = (const bf16*)x; p.norm_w = norm_w; p.eps = norm_eps; p.w = (const bf16*)w; p.bias = bias; p.residual = residual; p.out = out;
-    p.M = int(M); p.N = N; p.K = K; p.cluster = cluster; p.status = status; p.tiles = tiles; p.kc = kc; p.ns = ns;
+    p.M = int(M); p.N = N; p.K = K; p.cluster = cluster; p.status = status; p.tiles = int(tiles); p.kc = kc; p.ns = ns;
+    p.n_stages = int((K + kc - 1) / kc); p.per_cta = (p.n_stages + cluster - 1) / cluster;
     // gate the ring's second slot where the whole GPU's rings fill at once (a CTA per half SM) and a tile is one stage
     p.gate_ring = (n_stages == 1 && cluster == 1 && tiles >= 2LL * sms) ? 1 : 0;
     p.nw_smem = norm_w ? 1 : 0;
-    p.prefetch = prefetch; p.prefetch_bytes = prefetch_bytes & ~int64_t(15);
     // Two CTAs fit an SM; with more tiles than that, a CTA walks over several and its ring never drains between them.
-    constexpr int64_t PER_SM = IB_GEMV_CTAS_PER_SM;
-    int64_t groups = cluster > 1 ? tiles : (tiles < PER_SM * sms ? tiles : PER_SM * sms);
-    p.groups = int(groups);
-    const int grid_ctas = int(groups) * cluster;
+    p.groups = int(cluster > 1 || tiles < places ? tiles : places);
+    int grid_ctas = p.groups * cluster;
+    p.even = even > 0;
+    p.run = p.longer = 0;
+    if (p.even) {
+        const int64_t units = tiles * p.n_stages;
+        grid_ctas = int(units < places ? units : places);
+        p.run = int(units / grid_ctas); p.longer = int(units % grid_ctas);
+    }
+    p.parts = parts; p.arrived = arrived;
     if (M <= 8) return launch<1>(p, out_dtype, epi, grid_ctas, stream);
     return launch<2>(p, out_dtype, epi, grid_ctas, stream);
 }
