@@ -443,6 +443,146 @@ attention_kernel(const T* __restrict__ q, const T* __restrict__ k_cache, const T
     if (tid + AT < v_dim) o[tid + AT] = ib::from_f32<T>(acc1 * inv);
 }
 
+// The same for steps of a few tokens, float: the same arithmetic in the same order, hence the same bits, but a tile's keys and
+// values come through shared memory by asynchronous copies, two tiles of keys and one of values ahead, so that a
+// block waits for memory once and not a dozen times a tile. 200 KB a block at head size 128: one block an SM, which is why it
+// is for as few blocks as run in a round or two.
+__device__ __forceinline__ void copy16_async(uint32_t dst, const void* src, bool ok) {
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(src), "r"(ok ? 16 : 0) : "memory");
+}
+
+__global__ void __launch_bounds__(AT)
+attention_few_kernel(const float* __restrict__ q, const float* k_cache, const float* v_cache,
+                     const int* __restrict__ block_table, int64_t max_blocks, const int* __restrict__ token_seg,
+                     const int* __restrict__ positions, float* __restrict__ out, int n_heads, int n_kv, int head_dim, int v_dim,
+                     int page_size, int window, float scale, int64_t n_pages, int* status,
+                     const float* __restrict__ dist_bias, int bias_len, const float* __restrict__ sink,
+                     const int* __restrict__ single_only, int keep_first, const float* __restrict__ slopes) {
+    ib::pdl_launch_dependents();                           // the successor may request its weights meanwhile
+    ib::pdl_wait();
+    if (single_only) {
+        const int sg = token_seg[blockIdx.x];
+        if (single_only[sg + 1] - single_only[sg] > 1) return;
+    }
+    extern __shared__ __align__(16) float smem[];
+    const int k_pitch = head_dim + 4;                      // floats between keys: eight threads reading eight keys meet eight banks
+    float* keys = smem;                                    // [2][AT][k_pitch]
+    float* values = keys + 2 * AT * k_pitch;               // [AT][v_dim]
+    float* qs = values + AT * v_dim;                       // [head_dim]
+    float* ps = qs + head_dim;                             // [AT]
+    __shared__ int64_t rowoff[2][AT];                      // row of each key in the pages, -1: not seen or not there
+    __shared__ float red[32];
+
+    const int64_t t = blockIdx.x;
+    const int h = blockIdx.y;
+    const int g = h / (n_heads / n_kv);
+    const int tid = threadIdx.x;
+    const int pos = positions[t];
+    const int lo = window > 0 ? max(0, pos - window + 1) : 0;
+    const int keep_end = min(keep_first, lo);
+    const float slope = slopes ? slopes[h] : 0.0f;
+    const int* table = block_table + int64_t(token_seg[t]) * max_blocks;
+    // the tile after `tile` of which something is seen (beyond pos: there is none)
+    auto next = [&](int tile) {
+        tile += AT;
+        return tile >= keep_end && tile + AT <= lo ? (lo / AT) * AT : tile;
+    };
+    auto find = [&](int tile, int buf) {
+        const int j = tile + tid;
+        int64_t row = -1;
+        if (j <= pos && (j >= lo || j < keep_end)) {
+            const int page = table[j / page_size];
+            if (page < 0 || page >= n_pages) {
+                if (status) atomicExch(status, 3);
+            } else {
+                row = (int64_t(page) * n_kv + g) * page_size + j % page_size;
+            }
+        }
+        rowoff[buf][tid] = row;
+    };
+    auto copy = [&](float* dst, int pitch, const float* src, int dim, int buf) {
+        const int units = dim / 4;
+        const uint32_t base = uint32_t(__cvta_generic_to_shared(dst));
+        for (int i = tid; i < AT * units; i += AT) {
+            const int key = i / units, u = i - key * units;
+            const int64_t row = rowoff[buf][key];
+            copy16_async(base + uint32_t(key * pitch + u * 4) * 4u, src + (row < 0 ? 0 : row) * dim + u * 4, row >= 0);
+        }
+    };
+    auto commit = [] { asm volatile("cp.async.commit_group;" ::: "memory"); };
+
+    int tile = keep_end > 0 ? 0 : (lo / AT) * AT, ahead = next(tile), buf = 0;
+    find(tile, 0);
+    if (ahead <= pos) find(ahead, 1);
+    for (int d = tid; d < head_dim; d += AT) qs[d] = q[(t * n_heads + h) * head_dim + d];
+    __syncthreads();
+    copy(keys, k_pitch, k_cache, head_dim, 0);
+    commit();
+    copy(values, v_dim, v_cache, v_dim, 0);
+    commit();
+    if (ahead <= pos) copy(keys + AT * k_pitch, k_pitch, k_cache, head_dim, 1);
+    commit();
+    float m = -INFINITY, l = 0.0f, acc0 = 0.0f, acc1 = 0.0f;
+    if (sink) {
+        m = sink[h];
+        l = 1.0f;
+    }
+    for (; tile <= pos; buf ^= 1) {
+        asm volatile("cp.async.wait_group 2;" ::: "memory");           // this tile's keys (its values and the next keys may be on their way)
+        __syncthreads();
+        const int j = tile + tid;
+        const bool valid = j <= pos && (j >= lo || j < keep_end);
+        float s = -INFINITY;
+        if (valid && rowoff[buf][tid] >= 0) {
+            const float4* k4 = reinterpret_cast<const float4*>(keys + (buf * AT + tid) * k_pitch);
+            const float4* q4 = reinterpret_cast<const float4*>(qs);
+            float dot = 0.0f;
+#pragma unroll 8
+            for (int c = 0; c < head_dim / 4; c++) {
+                const float4 a = q4[c], b = k4[c];
+                dot = fmaf(a.x, b.x, dot); dot = fmaf(a.y, b.y, dot); dot = fmaf(a.z, b.z, dot); dot = fmaf(a.w, b.w, dot);
+            }
+            s = dot * scale;
+            if (dist_bias) s += dist_bias[int64_t(min(pos - j, bias_len - 1)) * n_heads + h];
+            if (slopes) s = fmaf(-slope, float(pos - j), s);
+        }
+        const float tile_max = ib::block_max(s, red);
+        const float m_new = fmaxf(m, tile_max);
+        const float p = valid && s > -INFINITY ? expf(s - m_new) : 0.0f;
+        ps[tid] = p;
+        const float tile_sum = ib::block_sum(p, red);
+        const float corr = m == -INFINITY ? 0.0f : expf(m - m_new);
+        l = l * corr + tile_sum;
+        acc0 *= corr;
+        acc1 *= corr;
+        asm volatile("cp.async.wait_group 1;" ::: "memory");           // this tile's values
+        __syncthreads();
+        const int jj0 = (tile < keep_end ? tile : max(lo, tile)) - tile, jj1 = min(pos, tile + AT - 1) - tile;
+        const float *v0 = values + (tid < v_dim ? tid : 0), *v1 = values + (tid + AT < v_dim ? tid + AT : 0);
+#pragma unroll 16
+        for (int jj = jj0; jj <= jj1; jj++) {
+            acc0 = fmaf(ps[jj], v0[jj * v_dim], acc0);                 // (unseen keys: zeros times zeros)
+            if (v_dim > AT) acc1 = fmaf(ps[jj], v1[jj * v_dim], acc1);
+        }
+        m = m_new;
+        __syncthreads();                                               // keys, values and rows of this tile have been read
+        const int after = next(ahead);
+        if (ahead <= pos) copy(values, v_dim, v_cache, v_dim, buf ^ 1);
+        commit();
+        if (after <= pos) find(after, buf);
+        __syncthreads();
+        if (after <= pos) copy(keys + buf * AT * k_pitch, k_pitch, k_cache, head_dim, buf);
+        commit();
+        tile = ahead;
+        ahead = after;
+    }
+    asm volatile("cp.async.wait_group 0;" ::: "memory");
+    const float inv = l > 0.0f ? 1.0f / l : 0.0f;
+    float* o = out + (t * n_heads + h) * v_dim;
+    if (tid < v_dim) o[tid] = acc0 * inv;
+    if (tid + AT < v_dim) o[tid + AT] = acc1 * inv;
+}
+
 // ------------------------------------------------------------------------------------------------
 // SwiGLU: out[t, i] = silu(gate) * up, silu(g) = g / (1 + exp(-g)); input rows are [gate | up], or with
 // `interleave8` blocks of 16: gate features 8b..8b+7, then up features 8b..8b+7.
@@ -655,6 +795,9 @@ sample_filtered_kernel(const float* __restrict__ logits, int64_t vocab, const fl
     }
 }
 
+constexpr int64_t FEW_BLOCKS = 296;                       // (two rounds over 148 SMs)
+constexpr size_t FEW_SMEM = 224 * 1024;
+
 inline unsigned blocks_for(int64_t n, int threads) { return unsigned((n + threads - 1) / threads); }
 
 }  // namespace
@@ -760,7 +903,16 @@ IB_EXPORT int ib_attention_plain(const void* q, const void* k_cache, const void*
     if (n_heads > 65535) return ib::fail(IB_ERR_ARG, "ib_attention_plain: too many heads");
     const dim3 grid{unsigned(n_tokens), unsigned(n_heads), 1u};
     const size_t smem = size_t(((head_dim + 1) & ~1) + AT) * sizeof(float) + AT * sizeof(int64_t) + 8;
-    if (dtype == IB_F32)
+    // A few tokens, whose blocks run in a round or two (see the kernel); rows that can be copied in 16-byte pieces, and that fit.
+    const size_t few = size_t(2 * AT * (head_dim + 4) + AT * v_dim + head_dim + AT) * sizeof(float);
+    if (dtype == IB_F32 && n_tokens * n_heads <= FEW_BLOCKS && head_dim % 4 == 0 && v_dim % 4 == 0 && few <= FEW_SMEM &&
+        ((uintptr_t(k_cache) | uintptr_t(v_cache)) & 15) == 0) {
+        static ib::PerDevice allowed;
+        if (const int rc = ib::allow_smem(allowed, "attention_few", attention_few_kernel, FEW_SMEM)) return rc;
+        IB_LAUNCH(attention_few_kernel, grid, AT, few, (const float*)q, (const float*)k_cache, (const float*)v_cache,
+            block_table, max_blocks, token_seg, positions, (float*)out, n_heads, n_kv, head_dim, v_dim, page_size, window, scale, n_pages, status,
+            dist_bias, bias_len, sink, single_only, window > 0 && keep_first > 0 ? keep_first : 0, slopes);
+    } else if (dtype == IB_F32)
         IB_LAUNCH(attention_kernel<float>, grid, AT, smem, (const float*)q, (const float*)k_cache, (const float*)v_cache,
             block_table, max_blocks, token_seg, positions, (float*)out, n_heads, n_kv, head_dim, v_dim, page_size, window, scale, n_pages, status,
             dist_bias, bias_len, sink, single_only, window > 0 && keep_first > 0 ? keep_first : 0, slopes);
