@@ -563,11 +563,21 @@ IB_EXPORT int ib_linear_skinny_bulk(const void* x, const float* norm_w, float no
     // even < 0: chosen here; 0: never; else the number of stages that a tile's K is cut into
     const int64_t places = int64_t(IB_GEMV_CTAS_PER_SM) * sms;
     const bool can = !norm_w && tiles * 64 < (1LL << 30) && parts && arrived && n_arrived >= tiles && n_parts >= 2 * places * PART_FLOATS;
-    if (!can) even = 0;
-    if (even < 0) even = 0;
-    if (even > 0) { n_stages = even; cluster = 1; }
+    auto stage_of = [&](int64_t n) { return ((K + n - 1) / n + 63) / 64 * 64; };       // elements of K in each of n equal stages
+    auto rounds = [&](int64_t work) { return (work + places - 1) / places; };
+    const int64_t least = n_stages;                              // as few stages as the ring allows
     n_stages = (n_stages + cluster - 1) / cluster * cluster;     // the same number of stages for every CTA of a cluster
-    const int kc = int(((K + n_stages - 1) / n_stages + 63) / 64 * 64);
+    if (!can) even = 0;
+    if (even < 0) {
+        // Equal runs where whole tiles would give some CTA at least 4,000 elements of K more (of 16 rows): the parts' meeting costs what
+        // reading those does. us with whole tiles -> with runs at 8 rows, and elements saved: 5120 x 13824 34.1 -> 26.9 (12,288),
+        // 3584 x 18944 31.8 -> 27.1 (5,888), 2560 x 9728 17.7 -> 14.6 (4,096), 6400 x 8192 23.6 -> 22.7 (4,224), but 5120 x 5120
+        // 14.8 -> 15.8 (3,840), 4960 x 4096 11.2 -> 13.2 (2,816), 1536 x 8960 8.0 -> 9.3 (1,536).
+        const int64_t whole = rounds(tiles * cluster) * (n_stages / cluster) * stage_of(n_stages);
+        even = whole - rounds(tiles * least) * stage_of(least) >= 4000 ? int(least) : 0;
+    }
+    if (even > 0) { n_stages = even; cluster = 1; }
+    const int kc = int(stage_of(n_stages));
     int ns = RING_BYTES / (ROWS * (kc * 2 + 64));
     if (ns > NS_MAX) ns = NS_MAX;
     GemvParams p;

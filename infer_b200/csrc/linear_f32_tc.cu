@@ -13,9 +13,10 @@
 // weigh 2^-8, run over a group of such blocks. Groups (at most 8, from N and K alone) are added in ascending order. A result
 // does not depend on how many rows x has, nor on which CTA forms which group: a row's bits are the same in every batch.
 //
-// A CTA (512 threads, one an SM) forms 128 features x NT tokens (features on the tensor memory's 128 lanes). Its warps load a
-// block of 64 elements of K into registers two blocks ahead, cut and store it as six swizzled operand tiles, the first warp
-// issues the block's 16 MMAs, and meanwhile all add up the accumulator of the block before. A few rows (NT = 16) are bound by
+// A CTA (544 threads, one an SM) forms 128 features x NT tokens (features on the tensor memory's 128 lanes). Sixteen warps load a
+// block of 64 elements of K into registers a block or two ahead, cut and store it as six swizzled operand tiles, and add up the
+// accumulator of the block before, while the seventeenth warp issues the block's 16 MMAs. The sixteen warps' instructions bound
+// it as much as anything: pairs of floats go through packed arithmetic, and addresses advance by addition. A few rows (NT = 16) are bound by
 // the reads of w; 64 rows and more by shared memory's bandwidth (per block 72 KB stored and 112 KB read by the MMAs
 // against 768 cycles of the tensor pipe).
 // Where the tiles are fewer than the SMs, the groups of a tile go to the CTAs of a cluster: each pushes its groups' sums to
@@ -30,20 +31,20 @@ namespace {
 using namespace ib::tc;
 
 constexpr int BM = 128, BK = 64;                 // features of a tile, elements of K in a block
-constexpr int WARPS = 16, THREADS = WARPS * 32;
+constexpr int WARPS = 16, WORKERS = WARPS * 32, THREADS = WORKERS + 32;
 constexpr int MAX_GROUPS = 8;
 constexpr int A_BYTES = BM * BK * 2;
 constexpr int SMEM_MOST = 226 * 1024;
 constexpr int STATUS_TIMEOUT = 131;
-constexpr int DEPTH = 2;                         // blocks requested ahead
 
 template <int NT> struct Cfg {
     static constexpr int B_BYTES = NT * BK * 2;
     static constexpr int STAGE_BYTES = 3 * A_BYTES + 3 * B_BYTES;
     static constexpr int TMEM_COLS = NT >= 64 ? 512 : (NT >= 32 ? 256 : 128);    // six accumulators of NT columns
     static constexpr int COLS = NT / 4;          // columns of a warp
-    static constexpr int A_UNITS = BM * BK / 4 / THREADS;                        // 16-byte units of w a thread and block
-    static constexpr int B_UNITS = (NT * BK / 4 + THREADS - 1) / THREADS;        // ... of x (NT = 16: half of the threads)
+    static constexpr int A_UNITS = BM * BK / 4 / WORKERS;                        // 16-byte units of w a thread and block
+    static constexpr int B_UNITS = (NT * BK / 4 + WORKERS - 1) / WORKERS;        // ... of x (NT = 16: half of the threads)
+    static constexpr int DEPTH = NT >= 64 ? 1 : 2;                               // blocks requested ahead
 };
 
 template <int N> __device__ __forceinline__ void tmem_ld(uint32_t taddr, float* v);
@@ -70,26 +71,25 @@ template <> __device__ __forceinline__ void tmem_ld<16>(uint32_t taddr, float* v
     for (int j = 0; j < 16; j++) v[j] = __uint_as_float(r[j]);
 }
 
-// Four elements of a row from k on; past its end others of the row, which `cleared` takes out (a load without a condition is in
-// flight until its value is used). VEC: 16-byte aligned, K a multiple of 4. ONCE: w, which is read once a step.
+// Four elements of a row, the first of them at `at`. VEC: 16-byte aligned. ONCE: w, which is read once a step.
 template <bool VEC, bool ONCE>
-__device__ __forceinline__ float4 load_unit(const float* row, int64_t k, int64_t K) {
+__device__ __forceinline__ float4 load_unit(const float* at) {
     float4 v;
     if constexpr (VEC) {
-        const float* at = row + (k < K ? k : K - 4);
         if constexpr (ONCE) asm volatile("ld.global.L1::no_allocate.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "l"(at));
         else v = *reinterpret_cast<const float4*>(at);
     } else {
-        v.x = row[k < K ? k : K - 1]; v.y = row[k + 1 < K ? k + 1 : K - 1];
-        v.z = row[k + 2 < K ? k + 2 : K - 1]; v.w = row[k + 3 < K ? k + 3 : K - 1];
+        v.x = at[0]; v.y = at[1]; v.z = at[2]; v.w = at[3];
     }
     return v;
 }
-__device__ __forceinline__ float4 cleared(float4 v, int64_t k, int64_t K) {
-    if (k >= K) v.x = 0.0f;
-    if (k + 1 >= K) v.y = 0.0f;
-    if (k + 2 >= K) v.z = 0.0f;
-    if (k + 3 >= K) v.w = 0.0f;
+// The same where only `n` of the four (or none) are in the row: zeros for the others.
+__device__ __forceinline__ float4 load_some(const float* at, int n) {
+    float4 v = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+    if (n > 0) v.x = at[0];
+    if (n > 1) v.y = at[1];
+    if (n > 2) v.z = at[2];
+    if (n > 3) v.w = at[3];
     return v;
 }
 
@@ -98,8 +98,18 @@ __device__ __forceinline__ uint32_t round2(float lo, float hi) {
     __nv_bfloat162 v = __floats2bfloat162_rn(lo, hi);
     return *reinterpret_cast<uint32_t*>(&v);
 }
-__device__ __forceinline__ float low_half(uint32_t v) { return __uint_as_float(v << 16); }
-__device__ __forceinline__ float high_half(uint32_t v) { return __uint_as_float(v & 0xffff0000u); }
+// Two floats side by side in 64 bits, for the packed forms of the arithmetic.
+using pair = unsigned long long;
+__device__ __forceinline__ pair pack(uint32_t lo, uint32_t hi) { return (pair(hi) << 32) | lo; }
+// (v - h) 256, exactly: h is v rounded to bfloat16 (two of them in 32 bits).
+__device__ __forceinline__ void rest(float& a, float& b, uint32_t h) {
+    constexpr pair MINUS = 0xbf800000bf800000ull, SCALE = 0x4380000043800000ull;
+    pair v = pack(__float_as_uint(a), __float_as_uint(b));
+    asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(v) : "l"(pack(h << 16, h & 0xffff0000u)), "l"(MINUS));
+    asm("mul.rn.f32x2 %0, %0, %1;" : "+l"(v) : "l"(SCALE));
+    a = __uint_as_float(uint32_t(v));
+    b = __uint_as_float(uint32_t(v >> 32));
+}
 
 // The three parts of four elements, eight bytes each, `part` bytes apart.
 __device__ __forceinline__ void store_parts(uint8_t* at, uint32_t part, float4 v) {
@@ -109,10 +119,7 @@ __device__ __forceinline__ void store_parts(uint8_t* at, uint32_t part, float4 v
         p.x = round2(v.x, v.y);
         p.y = round2(v.z, v.w);
         *reinterpret_cast<uint2*>(at + i * part) = p;
-        if (i < 2) {
-            v.x = (v.x - low_half(p.x)) * 256.0f; v.y = (v.y - high_half(p.x)) * 256.0f;
-            v.z = (v.z - low_half(p.y)) * 256.0f; v.w = (v.w - high_half(p.y)) * 256.0f;
-        }
+        if (i < 2) { rest(v.x, v.y, p.x); rest(v.z, v.w, p.y); }
     }
 }
 
@@ -151,7 +158,8 @@ linear32_tc_kernel(const Params p) {
     __shared__ __align__(8) uint64_t bars[4];    // full[2], done[2]
     __shared__ uint32_t slot, failed;
     uint8_t* stages = smem_raw + ((1024u - (smem_u32(smem_raw) & 1023u)) & 1023u);
-    uint8_t* recv = stages + 2 * C::STAGE_BYTES;              // [group][own column][128 features] where a tile is shared
+    // [own column][128 features] the groups' sum so far, or, where a tile is shared, [group][own column][128 features] each group's
+    float* recv = reinterpret_cast<float*>(stages + 2 * C::STAGE_BYTES);
     const int tid = threadIdx.x, warp = __shfl_sync(0xffffffffu, int(threadIdx.x >> 5), 0), lane = threadIdx.x & 31;
     const int rank = blockIdx.x;                              // in the cluster
     const int64_t n0 = int64_t(blockIdx.y) * BM, m0 = int64_t(blockIdx.z) * NT;
@@ -167,32 +175,45 @@ linear32_tc_kernel(const Params p) {
         failed = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
-    if (warp == 0) {
+    if (warp == WARPS) {
         tmem_alloc(smem_u32(&slot), C::TMEM_COLS);
         tmem_relinquish();
     }
 
-    const int unit = tid & 15, row0 = tid >> 4;               // unit u of rows row0, row0 + 32, ...
-    constexpr int ROW_STEP = THREADS / 16;
-    const bool has_x = NT * 16 >= THREADS || tid < NT * 16;
-    float4 wq[DEPTH][C::A_UNITS], xq[DEPTH][C::B_UNITS];
-    // (rows past the last one are read from it: what they lead to is not stored)
+    // Unit `unit` of rows row0, row0 + 32, ... of either operand; the pointers advance with the blocks. (In place of rows past the
+    // last one others are read: what they lead to is not stored.)
+    const int unit = tid & 15, row0 = tid >> 4;
+    constexpr int ROW_STEP = WORKERS / 16;
+    const bool worker = warp < WARPS, has_x = worker && (NT * 16 >= WORKERS || tid < NT * 16);
+    float4 wq[C::DEPTH][C::A_UNITS], xq[C::DEPTH][C::B_UNITS];
+    const int64_t k_first = int64_t(b0) * BK + unit * 4, w_step = ROW_STEP * p.K;
+    const float* pw = p.w + min(n0 + row0, p.N - 1) * p.K + k_first;
+    const float* px = p.x + min(m0 + row0, p.M - 1) * p.K + k_first;
+    const int w_rows = int(min(int64_t(BM), p.N - n0)) - row0, x_rows = int(min(int64_t(NT), p.M - m0)) - row0;      // from row0 on
+    const int whole = int(min(int64_t(nb), p.K / BK - b0));   // blocks that lie inside K
+    const int tail = int(p.K - p.K / BK * BK) - unit * 4;     // elements of this unit in the block that does not
     auto load_w = [&](int b, int d) {
-        const int64_t k = int64_t(b0 + b) * BK + unit * 4;
 #pragma unroll
-        for (int i = 0; i < C::A_UNITS; i++) wq[d][i] = load_unit<VEC, true>(p.w + min(n0 + row0 + i * ROW_STEP, p.N - 1) * p.K, k, p.K);
+        for (int i = 0; i < C::A_UNITS; i++) {
+            const float* at = pw + (i * ROW_STEP < w_rows ? i * w_step : 0);
+            wq[d][i] = b < whole ? load_unit<VEC, true>(at) : load_some(at, tail);
+        }
+        pw += BK;
     };
     auto load_x = [&](int b, int d) {
-        const int64_t k = int64_t(b0 + b) * BK + unit * 4;
-        if (has_x) {
 #pragma unroll
-            for (int i = 0; i < C::B_UNITS; i++) xq[d][i] = load_unit<VEC, false>(p.x + min(m0 + row0 + i * ROW_STEP, p.M - 1) * p.K, k, p.K);
+        for (int i = 0; i < C::B_UNITS; i++) {
+            const float* at = px + (i * ROW_STEP < x_rows ? i * w_step : 0);
+            if (has_x) xq[d][i] = b < whole ? load_unit<VEC, false>(at) : load_some(at, tail);
         }
+        px += BK;
     };
     if (!p.w_ready) ib::pdl_wait();
+    if (worker) {
 #pragma unroll
-    for (int d = 0; d < DEPTH; d++)
-        if (d < nb) load_w(d, d);
+        for (int d = 0; d < C::DEPTH; d++)
+            if (d < nb) load_w(d, d);
+    }
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
@@ -200,165 +221,148 @@ linear32_tc_kernel(const Params p) {
     if (p.share > 1) asm volatile("barrier.cluster.arrive.relaxed.aligned;" ::: "memory");
     const uint32_t tmem = slot;
     ib::pdl_wait();
+    if (worker) {
 #pragma unroll
-    for (int d = 0; d < DEPTH; d++)
-        if (d < nb) load_x(d, d);
+        for (int d = 0; d < C::DEPTH; d++)
+            if (d < nb) load_x(d, d);
+    }
     if (p.share > 1) asm volatile("barrier.cluster.wait.aligned;" ::: "memory");
 
-    const bool leader = elect_one();
     const uint32_t lanes = tmem + (uint32_t((warp & 3) * 32) << 16) + uint32_t(warp >> 2) * C::COLS;
     const int row = (warp & 3) * 32 + lane, col0 = (warp >> 2) * C::COLS;              // this thread's feature and first token
     const int own_cols = NT / p.share;                        // columns that a CTA of the cluster adds and stores
-    float acc[C::COLS], total[C::COLS];
+    float acc[C::COLS];
 #pragma unroll
-    for (int j = 0; j < C::COLS; j++) acc[j] = total[j] = 0.0f;
-    int g = g_begin, g_last = first_block(g_begin + 1) - b0;  // the group that is being added up; the first block of the next one
-    int mma_g = g_begin, mma_last = g_last;                   // the same for the MMAs, which are a block ahead
-    bool fresh = true;                                        // the next block's MMAs are their group's first
+    for (int j = 0; j < C::COLS; j++) acc[j] = 0.0f;
+    int g = g_begin, g_last = first_block(g_begin + 1) - b0;  // the group at hand; the first block of the next one
     bool ok = true;
-    // the first warp: block b's MMAs, once every warp has stored its part of the operands
-    auto multiply = [&](int b) {
+    if (warp == WARPS) {
+        // ------------------------------------------------------------------------------------------------ MMA issuer
         constexpr uint32_t one = make_idesc(NT, false), two = make_idesc(2 * NT, false);
-        if (b == mma_last) { mma_g++; mma_last = first_block(mma_g + 1) - b0; fresh = true; }
-        if (!mbar_wait_each(full(b), uint32_t(b >> 1) & 1u)) { ok = false; return; }
-        tc_fence_after();
-        const uint32_t a = smem_u32(stages) + uint32_t(b & 1) * C::STAGE_BYTES, x = a + 3 * A_BYTES;
-        const uint32_t c0 = tmem + uint32_t(b & 1) * NT, c12 = tmem + uint32_t(2 + 2 * ((mma_g - g_begin) & 1)) * NT;
-        const uint64_t w1 = make_desc(a, 16, 1024), w2 = make_desc(a + A_BYTES, 16, 1024), w3 = make_desc(a + 2 * A_BYTES, 16, 1024);
-        const uint64_t x1 = make_desc(x, 16, 1024), x2 = make_desc(x + C::B_BYTES, 16, 1024);
-        if (leader) {
+        const bool leader = elect_one();
+        bool fresh = true;                                    // the next block's MMAs are their group's first
+        for (int b = 0; b < nb; b++) {
+            if (b == g_last) { g++; g_last = first_block(g + 1) - b0; fresh = true; }
+            if (!mbar_wait_each(full(b), uint32_t(b >> 1) & 1u)) { ok = false; break; }
+            tc_fence_after();
+            const uint32_t a = smem_u32(stages) + uint32_t(b & 1) * C::STAGE_BYTES, x = a + 3 * A_BYTES;
+            const uint32_t c0 = tmem + uint32_t(b & 1) * NT, c12 = tmem + uint32_t(2 + 2 * ((g - g_begin) & 1)) * NT;
+            const uint64_t w1 = make_desc(a, 16, 1024), w2 = make_desc(a + A_BYTES, 16, 1024), w3 = make_desc(a + 2 * A_BYTES, 16, 1024);
+            const uint64_t x1 = make_desc(x, 16, 1024), x2 = make_desc(x + C::B_BYTES, 16, 1024);
+            if (leader) {
 #pragma unroll
-            for (int k = 0; k < BK / 16; k++) {
-                const uint64_t o = uint64_t(2 * k);           // 16 elements = 32 bytes = 2 units of the address field
-                umma_f16(c0, w1 + o, x1 + o, one, k > 0);
-                umma_f16(c12, w1 + o, x2 + o, two, (!fresh || k > 0) ? 1u : 0u);
-                umma_f16(c12, w2 + o, x1 + o, two, 1u);
-                umma_f16(c12 + NT, w3 + o, x1 + o, one, 1u);
-            }
-            umma_commit(done(b));
-        }
-        __syncwarp();
-        fresh = false;
-    };
-    // adds what block b left in its accumulator; at the end of a group also the two of the group
-    auto add_up = [&](int b) {
-        if (!mbar_wait_warp(done(b), uint32_t(b >> 1) & 1u)) { ok = false; return; }
-        tc_fence_after();
-        float v[C::COLS];
-        tmem_ld<C::COLS>(lanes + uint32_t(b & 1) * NT, v);
-#pragma unroll
-        for (int j = 0; j < C::COLS; j++) acc[j] += v[j];
-        if (b + 1 == g_last) {
-            float u[C::COLS];
-            const uint32_t c12 = lanes + uint32_t(2 + 2 * ((g - g_begin) & 1)) * NT;
-            tmem_ld<C::COLS>(c12, v);
-            tmem_ld<C::COLS>(c12 + NT, u);
-            int owner = col0 / own_cols, own = col0 - owner * own_cols;
-#pragma unroll
-            for (int j = 0; j < C::COLS; j++) {
-                const float sum = acc[j] + fmaf(u[j], 1.0f / 65536.0f, v[j] * (1.0f / 256.0f));
-                if (p.share > 1) {
-                    const uint32_t at = map_cluster(smem_u32(recv) + uint32_t((g * own_cols + own) * BM + row) * 4u, uint32_t(owner));
-                    asm volatile("st.shared::cluster.f32 [%0], %1;" ::"r"(at), "f"(sum) : "memory");
-                    if (++own == own_cols) { own = 0; owner++; }
-                } else {
-                    total[j] += sum;
+                for (int k = 0; k < BK / 16; k++) {
+                    const uint64_t o = uint64_t(2 * k);       // 16 elements = 32 bytes = 2 units of the address field
+                    umma_f16(c0, w1 + o, x1 + o, one, k > 0);
+                    umma_f16(c12, w1 + o, x2 + o, two, (!fresh || k > 0) ? 1u : 0u);
+                    umma_f16(c12, w2 + o, x1 + o, two, 1u);
+                    umma_f16(c12 + NT, w3 + o, x1 + o, one, 1u);
                 }
-                acc[j] = 0.0f;
+                umma_commit(done(b));
             }
-            g++;
-            g_last = first_block(g + 1) - b0;
+            __syncwarp();
+            fresh = false;
         }
-        tc_fence_before();
-    };
-    auto step = [&](int b, int d) {
-        // (the stage is free: its last MMAs, block b - 2's, were waited for when that block was added up)
-        uint8_t* stage = stages + (b & 1) * C::STAGE_BYTES;
-        auto place = [&](int r) { return uint32_t(r) * 128u + ((uint32_t(unit >> 1) ^ uint32_t(r & 7)) << 4) + uint32_t(unit & 1) * 8u; };
-        const int64_t k = int64_t(b0 + b) * BK + unit * 4;
-        if (int64_t(b0 + b + 1) * BK > p.K) {
+    } else {
+        // ------------------------------------------------------------------------------------------------ workers
+        const uint32_t place = uint32_t(row0) * 128u + ((uint32_t(unit >> 1) ^ uint32_t(row0 & 7)) << 4) + uint32_t(unit & 1) * 8u;   // (32 rows on: the same pattern)
+        // adds what block b left in its accumulator; at the end of a group also the two of the group
+        auto add_up = [&](int b) {
+            if (!mbar_wait_warp(done(b), uint32_t(b >> 1) & 1u)) { ok = false; return; }
+            tc_fence_after();
+            float v[C::COLS];
+            tmem_ld<C::COLS>(lanes + uint32_t(b & 1) * NT, v);
 #pragma unroll
-            for (int i = 0; i < C::A_UNITS; i++) wq[d][i] = cleared(wq[d][i], k, p.K);
+            for (int j = 0; j < C::COLS; j++) acc[j] += v[j];
+            if (b + 1 == g_last) {
+                float u[C::COLS];
+                const uint32_t c12 = lanes + uint32_t(2 + 2 * ((g - g_begin) & 1)) * NT;
+                tmem_ld<C::COLS>(c12, v);
+                tmem_ld<C::COLS>(c12 + NT, u);
+                int owner = col0 / own_cols, own = col0 - owner * own_cols;
 #pragma unroll
-            for (int i = 0; i < C::B_UNITS; i++) xq[d][i] = cleared(xq[d][i], k, p.K);
+                for (int j = 0; j < C::COLS; j++) {
+                    const float sum = acc[j] + fmaf(u[j], 1.0f / 65536.0f, v[j] * (1.0f / 256.0f));
+                    if (p.share > 1) {
+                        const uint32_t at = map_cluster(smem_u32(recv) + uint32_t((g * own_cols + own) * BM + row) * 4u, uint32_t(owner));
+                        asm volatile("st.shared::cluster.f32 [%0], %1;" ::"r"(at), "f"(sum) : "memory");
+                        if (++own == own_cols) { own = 0; owner++; }
+                    } else {
+                        float* at = recv + (col0 + j) * BM + row;
+                        *at = g > 0 ? *at + sum : sum;
+                    }
+                    acc[j] = 0.0f;
+                }
+                g++;
+                g_last = first_block(g + 1) - b0;
+            }
+            tc_fence_before();
+        };
+        auto step = [&](int b, int d) {
+            // (the stage is free: its last MMAs, block b - 2's, were waited for when that block was added up)
+            uint8_t* at = stages + (b & 1) * C::STAGE_BYTES + place;
+#pragma unroll
+            for (int i = 0; i < C::A_UNITS; i++) store_parts(at + i * (ROW_STEP * 128), A_BYTES, wq[d][i]);
+            if (has_x) {
+#pragma unroll
+                for (int i = 0; i < C::B_UNITS; i++) store_parts(at + 3 * A_BYTES + i * (ROW_STEP * 128), C::B_BYTES, xq[d][i]);
+            }
+            fence_proxy_async();
+            __syncwarp();
+            if (lane == 0) mbar_arrive(full(b));
+            if (b + C::DEPTH < nb) { load_w(b + C::DEPTH, d); load_x(b + C::DEPTH, d); }
+            if (b > 0) add_up(b - 1);
+        };
+        for (int b = 0; b < nb && ok; b += C::DEPTH) {
+#pragma unroll
+            for (int d = 0; d < C::DEPTH; d++)
+                if (b + d < nb && ok) step(b + d, d);
         }
-#pragma unroll
-        for (int i = 0; i < C::A_UNITS; i++) store_parts(stage + place(row0 + i * ROW_STEP), A_BYTES, wq[d][i]);
-        if (has_x) {
-#pragma unroll
-            for (int i = 0; i < C::B_UNITS; i++) store_parts(stage + 3 * A_BYTES + place(row0 + i * ROW_STEP), C::B_BYTES, xq[d][i]);
-        }
-        fence_proxy_async();
-        tc_fence_before();
-        __syncwarp();
-        if (lane == 0) mbar_arrive(full(b));
-        if (b + DEPTH < nb) { load_w(b + DEPTH, d); load_x(b + DEPTH, d); }
-        if (warp == 0) multiply(b);
-        if (b > 0 && ok) add_up(b - 1);
-    };
-    for (int b = 0; b < nb && ok; b += DEPTH) {
-#pragma unroll
-        for (int d = 0; d < DEPTH; d++)
-            if (b + d < nb && ok) step(b + d, d);
+        ib::pdl_launch_dependents();
+        if (ok) add_up(nb - 1);
     }
-    ib::pdl_launch_dependents();
-    if (ok) add_up(nb - 1);
     if (!ok && lane == 0) { atomicExch(p.status, STATUS_TIMEOUT); *reinterpret_cast<volatile uint32_t*>(&failed) = 1; }
 
-    auto finish = [&](float v, int64_t m, int64_t n, float bias, float res) {
-        if (!isfinite(v)) v = plain_product(p.x + m * p.K, p.w + n * p.K, p.K);
-        if (p.bias) v += bias;
-        if (p.residual) v += res;
-        p.out[m * p.N + n] = v;
-    };
-    if (p.share > 1) {
-        // feature tid & 127 of own columns tid / 128, + 4, ...; what is added to the sums is requested before the barrier
-        constexpr int MOST = 4;                               // (a CTA owns at most 16 columns)
-        const int64_t n = n0 + (tid & (BM - 1));
-        const bool n_ok = n < p.N;
-        const float bias = p.bias && n_ok ? p.bias[n] : 0.0f;
-        float res[MOST];
+    // Feature tid & 127 of own columns tid / 128, + 4, ..., four columns at a time; what is added to the first four's sums is requested
+    // before the barrier.
+    const int64_t n = n0 + (tid & (BM - 1));
+    const bool storing = worker && n < p.N;
+    const float bias = storing && p.bias ? p.bias[n] : 0.0f;
+    const int slots = p.share > 1 ? p.groups : 1;
+    float res[4];
+    auto request = [&](int c0) {
 #pragma unroll
-        for (int i = 0; i < MOST; i++) {
-            const int c = (tid >> 7) + 4 * i;
+        for (int i = 0; i < 4; i++) {
+            const int c = c0 + (tid >> 7) + 4 * i;
             const int64_t m = m0 + rank * own_cols + c;
-            res[i] = p.residual && n_ok && c < own_cols && m < p.M ? p.residual[m * p.N + n] : 0.0f;
+            res[i] = storing && p.residual && c < own_cols && m < p.M ? p.residual[m * p.N + n] : 0.0f;
         }
-        __syncwarp();
-        asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
-        if (n_ok && !*reinterpret_cast<volatile uint32_t*>(&failed)) {
-            const float* sums = reinterpret_cast<const float*>(recv);
+    };
+    request(0);
+    __syncwarp();
+    if (p.share > 1) asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+    else __syncthreads();
+    if (storing && !*reinterpret_cast<volatile uint32_t*>(&failed)) {
+        for (int c0 = 0; c0 < own_cols; c0 += 16) {
+            if (c0) request(c0);
 #pragma unroll
-            for (int i = 0; i < MOST; i++) {
-                const int c = (tid >> 7) + 4 * i;
+            for (int i = 0; i < 4; i++) {
+                const int c = c0 + (tid >> 7) + 4 * i;
                 const int64_t m = m0 + rank * own_cols + c;
                 if (c < own_cols && m < p.M) {
                     float v = 0.0f;
-                    for (int h = 0; h < p.groups; h++) v += sums[(h * own_cols + c) * BM + (tid & (BM - 1))];
-                    finish(v, m, n, bias, res[i]);
+                    for (int h = 0; h < slots; h++) v += recv[(h * own_cols + c) * BM + (tid & (BM - 1))];
+                    if (!isfinite(v)) v = plain_product(p.x + m * p.K, p.w + n * p.K, p.K);
+                    if (p.bias) v += bias;
+                    if (p.residual) v += res[i];
+                    p.out[m * p.N + n] = v;
                 }
-            }
-        }
-    } else {
-        const int64_t n = n0 + row;
-        if (n < p.N && !*reinterpret_cast<volatile uint32_t*>(&failed)) {
-            const float bias = p.bias ? p.bias[n] : 0.0f;
-            float res[C::COLS];
-#pragma unroll
-            for (int j = 0; j < C::COLS; j++) {
-                const int64_t m = m0 + col0 + j;
-                res[j] = p.residual && m < p.M ? p.residual[m * p.N + n] : 0.0f;
-            }
-#pragma unroll
-            for (int j = 0; j < C::COLS; j++) {
-                const int64_t m = m0 + col0 + j;
-                if (m < p.M) finish(total[j], m, n, bias, res[j]);
             }
         }
     }
     tc_fence_before();
     __syncthreads();
-    if (warp == 0) {
+    if (warp == WARPS) {
         tc_fence_after();
         tmem_dealloc(tmem, C::TMEM_COLS);
     }
@@ -376,7 +380,7 @@ int group_count(int64_t N, int64_t blocks, int sms) {
 }
 
 int smem_bytes(int nt, int groups, int share) {
-    const int recv = share > 1 ? nt * BM * 4 * groups / share : 0;
+    const int recv = nt * BM * 4 * (share > 1 ? groups : 1) / share;
     return 2 * 3 * (A_BYTES + nt * BK * 2) + 1024 + recv;
 }
 
@@ -387,12 +391,14 @@ Plan make_plan(int64_t M, int64_t N, int64_t K, int sms) {
     q.nt = M <= 16 ? 16 : (M <= 32 ? 32 : 64);
     const int64_t tiles = ((N + BM - 1) / BM) * ((M + q.nt - 1) / q.nt);
     // How many CTAs share a tile: the number whose rounds over the SMs take least, a CTA's start and end counted as four blocks
-    // and the cluster's meeting as two more. (A CTA stores at most 16 columns, and holds every group's sums of those.)
+    // and the cluster's meeting as two more. (A CTA of a cluster holds every group's sums of its columns.)
     q.share = 1;
     int64_t best = 0;
     for (int z = 1; z <= q.groups; z *= 2) {
-        if (z > 1 && (q.nt / z > 16 || smem_bytes(q.nt, q.groups, z) > SMEM_MOST)) continue;
-        const int64_t rounds = (tiles * z + sms - 1) / sms;
+        if (smem_bytes(q.nt, q.groups, z) > SMEM_MOST) continue;
+        // (of the SMs, clusters of four and eight cannot use a seventh)
+        const int64_t at_once = z == 1 ? sms : (z == 2 ? sms - 4 : (sms - sms / 7) / z * z);
+        const int64_t rounds = (tiles * z + at_once - 1) / at_once;
         const int64_t cost = rounds * ((blocks + z - 1) / z + 4 + (z > 1 ? 2 : 0));
         if (best == 0 || cost < best) { best = cost; q.share = z; }
     }
