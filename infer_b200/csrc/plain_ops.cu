@@ -443,44 +443,46 @@ attention_kernel(const T* __restrict__ q, const T* __restrict__ k_cache, const T
     if (tid + AT < v_dim) o[tid + AT] = ib::from_f32<T>(acc1 * inv);
 }
 
-// The same for steps of a few tokens, float: the same arithmetic in the same order, hence the same bits, but a tile's keys and
-// values come through shared memory by asynchronous copies, two tiles of keys and one of values ahead, so that a
-// block waits for memory once and not a dozen times a tile. 200 KB a block at head size 128: one block an SM, which is why it
-// is for as few blocks as run in a round or two.
+// The same for float pages with rows of whole 16-byte pieces: the same arithmetic in the same order, hence the same bits, but a
+// tile's keys and values come through shared memory by asynchronous copies, two tiles of keys and one of values ahead, so that a
+// block waits for memory once and not a dozen times a tile. A block of S x 128 threads takes S x H heads of a kv head's group, which
+// read them together, each 128 threads H of the heads. 200 KB at head size 128: one block an SM. Steps of a few tokens take a
+// head a block, which then still all run at once.
 __device__ __forceinline__ void copy16_async(uint32_t dst, const void* src, bool ok) {
     asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(src), "r"(ok ? 16 : 0) : "memory");
 }
 
-__global__ void __launch_bounds__(AT)
-attention_few_kernel(const float* __restrict__ q, const float* k_cache, const float* v_cache,
-                     const int* __restrict__ block_table, int64_t max_blocks, const int* __restrict__ token_seg,
-                     const int* __restrict__ positions, float* __restrict__ out, int n_heads, int n_kv, int head_dim, int v_dim,
-                     int page_size, int window, float scale, int64_t n_pages, int* status,
-                     const float* __restrict__ dist_bias, int bias_len, const float* __restrict__ sink,
-                     const int* __restrict__ single_only, int keep_first, const float* __restrict__ slopes) {
+template <int H, int S>
+__global__ void __launch_bounds__(AT * S, 1)
+attention_staged_kernel(const float* __restrict__ q, const float* k_cache, const float* v_cache,
+                        const int* __restrict__ block_table, int64_t max_blocks, const int* __restrict__ token_seg,
+                        const int* __restrict__ positions, float* __restrict__ out, int n_heads, int n_kv, int head_dim, int v_dim,
+                        int page_size, int window, float scale, int64_t n_pages, int* status,
+                        const float* __restrict__ dist_bias, int bias_len, const float* __restrict__ sink,
+                        const int* __restrict__ single_only, int keep_first, const float* __restrict__ slopes) {
     ib::pdl_launch_dependents();                           // the successor may request its weights meanwhile
     ib::pdl_wait();
     if (single_only) {
         const int sg = token_seg[blockIdx.x];
         if (single_only[sg + 1] - single_only[sg] > 1) return;
     }
+    constexpr int WARPS = AT / 32 * S;
     extern __shared__ __align__(16) float smem[];
     const int k_pitch = head_dim + 4;                      // floats between keys: eight threads reading eight keys meet eight banks
     float* keys = smem;                                    // [2][AT][k_pitch]
     float* values = keys + 2 * AT * k_pitch;               // [AT][v_dim]
-    float* qs = values + AT * v_dim;                       // [head_dim]
-    float* ps = qs + head_dim;                             // [AT]
-    __shared__ int64_t rowoff[2][AT];                      // row of each key in the pages, -1: not seen or not there
-    __shared__ float red[32];
+    float* qs = values + AT * v_dim;                       // [S * H][head_dim]
+    float* ps = qs + S * H * head_dim;                     // [S][AT][H] probabilities
+    __shared__ int64_t rows[2][AT];                        // row of each key in the pages, -1: not seen or not there
+    __shared__ float red[2][S][H][AT / 32];
 
     const int64_t t = blockIdx.x;
-    const int h = blockIdx.y;
-    const int g = h / (n_heads / n_kv);
-    const int tid = threadIdx.x;
+    const int sub = S == 1 ? 0 : int(threadIdx.x) / AT, tid = int(threadIdx.x) - sub * AT, warp = tid >> 5, lane = tid & 31;
+    const int h_block = blockIdx.y * (S * H), h0 = h_block + sub * H;
+    const int g = h_block / (n_heads / n_kv);
     const int pos = positions[t];
     const int lo = window > 0 ? max(0, pos - window + 1) : 0;
     const int keep_end = min(keep_first, lo);
-    const float slope = slopes ? slopes[h] : 0.0f;
     const int* table = block_table + int64_t(token_seg[t]) * max_blocks;
     // the tile after `tile` of which something is seen (beyond pos: there is none)
     auto next = [&](int tile) {
@@ -488,6 +490,7 @@ attention_few_kernel(const float* __restrict__ q, const float* k_cache, const fl
         return tile >= keep_end && tile + AT <= lo ? (lo / AT) * AT : tile;
     };
     auto find = [&](int tile, int buf) {
+        if (sub > 0) return;
         const int j = tile + tid;
         int64_t row = -1;
         if (j <= pos && (j >= lo || j < keep_end)) {
@@ -498,23 +501,30 @@ attention_few_kernel(const float* __restrict__ q, const float* k_cache, const fl
                 row = (int64_t(page) * n_kv + g) * page_size + j % page_size;
             }
         }
-        rowoff[buf][tid] = row;
+        rows[buf][tid] = row;
     };
+    // a warp copies whole rows, its lanes their 16-byte pieces; zeros where there is no row
     auto copy = [&](float* dst, int pitch, const float* src, int dim, int buf) {
-        const int units = dim / 4;
-        const uint32_t base = uint32_t(__cvta_generic_to_shared(dst));
-        for (int i = tid; i < AT * units; i += AT) {
-            const int key = i / units, u = i - key * units;
-            const int64_t row = rowoff[buf][key];
-            copy16_async(base + uint32_t(key * pitch + u * 4) * 4u, src + (row < 0 ? 0 : row) * dim + u * 4, row >= 0);
+        const int wid = int(threadIdx.x) >> 5;
+        for (int u = lane * 4; u < dim; u += 128) {
+            uint32_t to = uint32_t(__cvta_generic_to_shared(dst)) + uint32_t(wid * pitch + u) * 4u;
+#pragma unroll 4
+            for (int key = wid; key < AT; key += WARPS, to += uint32_t(WARPS * pitch) * 4u) {
+                const int64_t row = rows[buf][key];
+                copy16_async(to, src + (row < 0 ? 0 : row) * dim + u, row >= 0);
+            }
         }
     };
     auto commit = [] { asm volatile("cp.async.commit_group;" ::: "memory"); };
+    auto meet = [&] {                                      // the threads of these heads
+        if constexpr (S == 1) __syncthreads();
+        else asm volatile("bar.sync %0, 128;" ::"r"(1 + sub) : "memory");
+    };
 
     int tile = keep_end > 0 ? 0 : (lo / AT) * AT, ahead = next(tile), buf = 0;
     find(tile, 0);
     if (ahead <= pos) find(ahead, 1);
-    for (int d = tid; d < head_dim; d += AT) qs[d] = q[(t * n_heads + h) * head_dim + d];
+    for (int d = threadIdx.x; d < S * H * head_dim; d += AT * S) qs[d] = q[(t * n_heads + h_block) * head_dim + d];
     __syncthreads();
     copy(keys, k_pitch, k_cache, head_dim, 0);
     commit();
@@ -522,49 +532,87 @@ attention_few_kernel(const float* __restrict__ q, const float* k_cache, const fl
     commit();
     if (ahead <= pos) copy(keys + AT * k_pitch, k_pitch, k_cache, head_dim, 1);
     commit();
-    float m = -INFINITY, l = 0.0f, acc0 = 0.0f, acc1 = 0.0f;
-    if (sink) {
-        m = sink[h];
-        l = 1.0f;
+    float m[H], l[H], acc0[H], acc1[H];
+#pragma unroll
+    for (int h = 0; h < H; h++) {
+        m[h] = sink ? sink[h0 + h] : -INFINITY;            // the running maximum starts at the sink's logit, the sum at exp(0)
+        l[h] = sink ? 1.0f : 0.0f;
+        acc0[h] = acc1[h] = 0.0f;
     }
     for (; tile <= pos; buf ^= 1) {
         asm volatile("cp.async.wait_group 2;" ::: "memory");           // this tile's keys (its values and the next keys may be on their way)
         __syncthreads();
         const int j = tile + tid;
-        const bool valid = j <= pos && (j >= lo || j < keep_end);
-        float s = -INFINITY;
-        if (valid && rowoff[buf][tid] >= 0) {
+        float s[H];
+#pragma unroll
+        for (int h = 0; h < H; h++) s[h] = -INFINITY;
+        if (rows[buf][tid] >= 0) {
             const float4* k4 = reinterpret_cast<const float4*>(keys + (buf * AT + tid) * k_pitch);
-            const float4* q4 = reinterpret_cast<const float4*>(qs);
-            float dot = 0.0f;
+            const float4* q4 = reinterpret_cast<const float4*>(qs + sub * H * head_dim);
+            float dot[H];
+#pragma unroll
+            for (int h = 0; h < H; h++) dot[h] = 0.0f;
 #pragma unroll 8
             for (int c = 0; c < head_dim / 4; c++) {
-                const float4 a = q4[c], b = k4[c];
-                dot = fmaf(a.x, b.x, dot); dot = fmaf(a.y, b.y, dot); dot = fmaf(a.z, b.z, dot); dot = fmaf(a.w, b.w, dot);
+                const float4 b = k4[c];
+#pragma unroll
+                for (int h = 0; h < H; h++) {
+                    const float4 a = q4[h * (head_dim / 4) + c];
+                    dot[h] = fmaf(a.x, b.x, dot[h]); dot[h] = fmaf(a.y, b.y, dot[h]);
+                    dot[h] = fmaf(a.z, b.z, dot[h]); dot[h] = fmaf(a.w, b.w, dot[h]);
+                }
             }
-            s = dot * scale;
-            if (dist_bias) s += dist_bias[int64_t(min(pos - j, bias_len - 1)) * n_heads + h];
-            if (slopes) s = fmaf(-slope, float(pos - j), s);
+#pragma unroll
+            for (int h = 0; h < H; h++) {
+                s[h] = dot[h] * scale;
+                if (dist_bias) s[h] += dist_bias[int64_t(min(pos - j, bias_len - 1)) * n_heads + h0 + h];
+                if (slopes) s[h] = fmaf(-slopes[h0 + h], float(pos - j), s[h]);
+            }
         }
-        const float tile_max = ib::block_max(s, red);
-        const float m_new = fmaxf(m, tile_max);
-        const float p = valid && s > -INFINITY ? expf(s - m_new) : 0.0f;
-        ps[tid] = p;
-        const float tile_sum = ib::block_sum(p, red);
-        const float corr = m == -INFINITY ? 0.0f : expf(m - m_new);
-        l = l * corr + tile_sum;
-        acc0 *= corr;
-        acc1 *= corr;
+#pragma unroll
+        for (int h = 0; h < H; h++) {
+            const float w = ib::warp_max(s[h]);
+            if (lane == 0) red[0][sub][h][warp] = w;
+        }
+        meet();
+        float corr[H];
+#pragma unroll
+        for (int h = 0; h < H; h++) {
+            const float* r = red[0][sub][h];
+            const float m_new = fmaxf(m[h], fmaxf(fmaxf(r[0], r[1]), fmaxf(r[2], r[3])));
+            const float p = s[h] > -INFINITY ? expf(s[h] - m_new) : 0.0f;
+            ps[(sub * AT + tid) * H + h] = p;
+            corr[h] = m[h] == -INFINITY ? 0.0f : expf(m[h] - m_new);
+            m[h] = m_new;
+            const float w = ib::warp_sum(p);
+            if (lane == 0) red[1][sub][h][warp] = w;
+        }
         asm volatile("cp.async.wait_group 1;" ::: "memory");           // this tile's values
         __syncthreads();
+#pragma unroll
+        for (int h = 0; h < H; h++) {
+            const float* r = red[1][sub][h];                           // (added as ib::block_sum adds the warps' sums)
+            l[h] = l[h] * corr[h] + ((r[0] + r[2]) + (r[1] + r[3]));
+            acc0[h] *= corr[h];
+            acc1[h] *= corr[h];
+        }
         const int jj0 = (tile < keep_end ? tile : max(lo, tile)) - tile, jj1 = min(pos, tile + AT - 1) - tile;
         const float *v0 = values + (tid < v_dim ? tid : 0), *v1 = values + (tid + AT < v_dim ? tid + AT : 0);
+        const float* pj = ps + sub * AT * H;
 #pragma unroll 16
-        for (int jj = jj0; jj <= jj1; jj++) {
-            acc0 = fmaf(ps[jj], v0[jj * v_dim], acc0);                 // (unseen keys: zeros times zeros)
-            if (v_dim > AT) acc1 = fmaf(ps[jj], v1[jj * v_dim], acc1);
+        for (int jj = jj0; jj <= jj1; jj++) {                          // (unseen keys between: zeros times zeros)
+            const float a = v0[jj * v_dim];
+#pragma unroll
+            for (int h = 0; h < H; h++) acc0[h] = fmaf(pj[jj * H + h], a, acc0[h]);
         }
-        m = m_new;
+        if (v_dim > AT) {
+#pragma unroll 16
+            for (int jj = jj0; jj <= jj1; jj++) {
+                const float a = v1[jj * v_dim];
+#pragma unroll
+                for (int h = 0; h < H; h++) acc1[h] = fmaf(pj[jj * H + h], a, acc1[h]);
+            }
+        }
         __syncthreads();                                               // keys, values and rows of this tile have been read
         const int after = next(ahead);
         if (ahead <= pos) copy(values, v_dim, v_cache, v_dim, buf ^ 1);
@@ -577,10 +625,13 @@ attention_few_kernel(const float* __restrict__ q, const float* k_cache, const fl
         ahead = after;
     }
     asm volatile("cp.async.wait_group 0;" ::: "memory");
-    const float inv = l > 0.0f ? 1.0f / l : 0.0f;
-    float* o = out + (t * n_heads + h) * v_dim;
-    if (tid < v_dim) o[tid] = acc0 * inv;
-    if (tid + AT < v_dim) o[tid + AT] = acc1 * inv;
+#pragma unroll
+    for (int h = 0; h < H; h++) {
+        const float inv = l[h] > 0.0f ? 1.0f / l[h] : 0.0f;
+        float* o = out + (t * n_heads + h0 + h) * v_dim;
+        if (tid < v_dim) o[tid] = acc0[h] * inv;
+        if (tid + AT < v_dim) o[tid + AT] = acc1[h] * inv;
+    }
 }
 
 // ------------------------------------------------------------------------------------------------
@@ -795,8 +846,8 @@ sample_filtered_kernel(const float* __restrict__ logits, int64_t vocab, const fl
     }
 }
 
-constexpr int64_t FEW_BLOCKS = 296;                       // (two rounds over 148 SMs)
-constexpr size_t FEW_SMEM = 224 * 1024;
+constexpr int64_t ONE_ROUND = 148;                        // blocks of the staged attention that run at once
+constexpr size_t STAGED_SMEM = 224 * 1024;
 
 inline unsigned blocks_for(int64_t n, int threads) { return unsigned((n + threads - 1) / threads); }
 
@@ -903,16 +954,45 @@ IB_EXPORT int ib_attention_plain(const void* q, const void* k_cache, const void*
     if (n_heads > 65535) return ib::fail(IB_ERR_ARG, "ib_attention_plain: too many heads");
     const dim3 grid{unsigned(n_tokens), unsigned(n_heads), 1u};
     const size_t smem = size_t(((head_dim + 1) & ~1) + AT) * sizeof(float) + AT * sizeof(int64_t) + 8;
-    // A few tokens, whose blocks run in a round or two (see the kernel); rows that can be copied in 16-byte pieces, and that fit.
-    const size_t few = size_t(2 * AT * (head_dim + 4) + AT * v_dim + head_dim + AT) * sizeof(float);
-    if (dtype == IB_F32 && n_tokens * n_heads <= FEW_BLOCKS && head_dim % 4 == 0 && v_dim % 4 == 0 && few <= FEW_SMEM &&
-        ((uintptr_t(k_cache) | uintptr_t(v_cache)) & 15) == 0) {
-        static ib::PerDevice allowed;
-        if (const int rc = ib::allow_smem(allowed, "attention_few", attention_few_kernel, FEW_SMEM)) return rc;
-        IB_LAUNCH(attention_few_kernel, grid, AT, few, (const float*)q, (const float*)k_cache, (const float*)v_cache,
-            block_table, max_blocks, token_seg, positions, (float*)out, n_heads, n_kv, head_dim, v_dim, page_size, window, scale, n_pages, status,
-            dist_bias, bias_len, sink, single_only, window > 0 && keep_first > 0 ? keep_first : 0, slopes);
-    } else if (dtype == IB_F32)
+    if (dtype == IB_F32 && head_dim % 4 == 0 && v_dim % 4 == 0 && ((uintptr_t(k_cache) | uintptr_t(v_cache)) & 15) == 0) {
+        // Heads a block: the fewest that share keys and whose blocks run at once, else the most; two rather than one. us for 3, 24, 100 and
+        // 512 tokens of 12 heads on 2 at up to 300 keys (one query head and tile after the other: 25, 31, 95, 344): one head 16, 31, 130, 516;
+        // two 15, 15, 67, 243; three 17, 17, 47, 187; six 19, 19, 35, 108. Blocks that mostly find nothing to do are the other kernel's.
+        const int group = n_heads / n_kv;
+        int heads = 0;
+        for (const int code : {12, 11, 13, 22, 15, 23, 17}) {
+            const int n = code / 10 * (code % 10);
+            if (group % n) continue;
+            if (n_tokens * (n_heads / n) <= ONE_ROUND) { heads = code; break; }
+            if (n > 1 && !single_only) heads = code;
+        }
+        if (heads == 0 && n_tokens * n_heads <= 2 * ONE_ROUND) heads = 11;
+        const int taken = heads / 10 * (heads % 10);
+        const size_t need = (size_t(2 * AT) * (head_dim + 4) + size_t(AT) * v_dim + size_t(taken) * (head_dim + AT)) * sizeof(float);
+        if (heads > 0 && need <= STAGED_SMEM) {
+            const dim3 staged{unsigned(n_tokens), unsigned(n_heads / taken), 1u};
+#define IB_STAGED(H_, S_)                                                                                                      \
+    case H_ * 10 + S_: {                                                                                                       \
+        static ib::PerDevice allowed;                                                                                          \
+        if (const int rc = ib::allow_smem(allowed, "attention_staged", attention_staged_kernel<H_, S_>, STAGED_SMEM)) return rc;   \
+        return ib::launch("attention_staged", attention_staged_kernel<H_, S_>, staged, dim3(AT * S_), need, stream, 1u, (const float*)q,  \
+                          (const float*)k_cache, (const float*)v_cache, block_table, max_blocks, token_seg, positions, (float*)out, n_heads,   \
+                          n_kv, head_dim, v_dim, page_size, window, scale, n_pages, status, dist_bias, bias_len, sink, single_only,  \
+                          window > 0 && keep_first > 0 ? keep_first : 0, slopes);                                              \
+    }
+            switch (heads) {
+                IB_STAGED(1, 1)
+                IB_STAGED(1, 2)
+                IB_STAGED(1, 3)
+                IB_STAGED(1, 5)
+                IB_STAGED(1, 7)
+                IB_STAGED(2, 2)
+                IB_STAGED(2, 3)
+            }
+#undef IB_STAGED
+        }
+    }
+    if (dtype == IB_F32)
         IB_LAUNCH(attention_kernel<float>, grid, AT, smem, (const float*)q, (const float*)k_cache, (const float*)v_cache,
             block_table, max_blocks, token_seg, positions, (float*)out, n_heads, n_kv, head_dim, v_dim, page_size, window, scale, n_pages, status,
             dist_bias, bias_len, sink, single_only, window > 0 && keep_first > 0 ? keep_first : 0, slopes);
