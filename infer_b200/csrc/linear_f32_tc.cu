@@ -77,7 +77,7 @@ __device__ __forceinline__ float4 load_unit(const float* at) {
     float4 v;
     if constexpr (VEC) {
         if constexpr (ONCE) asm volatile("ld.global.L1::no_allocate.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "l"(at));
-        else v = *reinterpret_cast<const float4*>(at);
+        else asm volatile("ld.global.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "l"(at));
     } else {
         v.x = at[0]; v.y = at[1]; v.z = at[2]; v.w = at[3];
     }
@@ -162,7 +162,8 @@ linear32_tc_kernel(const Params p) {
     float* recv = reinterpret_cast<float*>(stages + 2 * C::STAGE_BYTES);
     const int tid = threadIdx.x, warp = __shfl_sync(0xffffffffu, int(threadIdx.x >> 5), 0), lane = threadIdx.x & 31;
     const int rank = blockIdx.x;                              // in the cluster
-    const int64_t n0 = int64_t(blockIdx.y) * BM, m0 = int64_t(blockIdx.z) * NT;
+    // (the last tile of features is a whole one too: what it shares with the one before, it does not store)
+    const int64_t n_first = int64_t(blockIdx.y) * BM, n0 = min(n_first, p.N - BM), m0 = int64_t(blockIdx.z) * NT;
     const int g_begin = rank * p.per_cta, g_end = g_begin + p.per_cta;
     auto first_block = [&](int g) { return int(int64_t(g) * p.blocks / p.groups); };
     const int b0 = first_block(g_begin), nb = first_block(g_end) - b0;
@@ -180,31 +181,39 @@ linear32_tc_kernel(const Params p) {
         tmem_relinquish();
     }
 
-    // Unit `unit` of rows row0, row0 + 32, ... of either operand; the pointers advance with the blocks. (In place of rows past the
+    // Unit `unit` of rows row0, row0 + 32, ... of either operand; the pointers advance with the blocks. (In place of rows past x's
     // last one others are read: what they lead to is not stored.)
-    const int unit = tid & 15, row0 = tid >> 4;
+    const int unit = tid & 15, row0 = (tid >> 4) & 31;
     constexpr int ROW_STEP = WORKERS / 16;
     const bool worker = warp < WARPS, has_x = worker && (NT * 16 >= WORKERS || tid < NT * 16);
     float4 wq[C::DEPTH][C::A_UNITS], xq[C::DEPTH][C::B_UNITS];
-    const int64_t k_first = int64_t(b0) * BK + unit * 4, w_step = ROW_STEP * p.K;
-    const float* pw = p.w + min(n0 + row0, p.N - 1) * p.K + k_first;
+    const int64_t k_first = int64_t(b0) * BK + unit * 4, step = ROW_STEP * p.K;
+    const float* pw = p.w + (n0 + row0) * p.K + k_first;
     const float* px = p.x + min(m0 + row0, p.M - 1) * p.K + k_first;
-    const int w_rows = int(min(int64_t(BM), p.N - n0)) - row0, x_rows = int(min(int64_t(NT), p.M - m0)) - row0;      // from row0 on
+    const int64_t x_step = m0 + row0 + ROW_STEP < p.M ? step : 0;
     const int whole = int(min(int64_t(nb), p.K / BK - b0));   // blocks that lie inside K
     const int tail = int(p.K - p.K / BK * BK) - unit * 4;     // elements of this unit in the block that does not
     auto load_w = [&](int b, int d) {
+        const float* at = pw;
+        if (b < whole) {
 #pragma unroll
-        for (int i = 0; i < C::A_UNITS; i++) {
-            const float* at = pw + (i * ROW_STEP < w_rows ? i * w_step : 0);
-            wq[d][i] = b < whole ? load_unit<VEC, true>(at) : load_some(at, tail);
+            for (int i = 0; i < C::A_UNITS; i++, at += step) wq[d][i] = load_unit<VEC, true>(at);
+        } else {
+#pragma unroll
+            for (int i = 0; i < C::A_UNITS; i++, at += step) wq[d][i] = load_some(at, tail);
         }
         pw += BK;
     };
     auto load_x = [&](int b, int d) {
+        if (has_x) {
+            const float* at = px;
+            if (b < whole) {
 #pragma unroll
-        for (int i = 0; i < C::B_UNITS; i++) {
-            const float* at = px + (i * ROW_STEP < x_rows ? i * w_step : 0);
-            if (has_x) xq[d][i] = b < whole ? load_unit<VEC, false>(at) : load_some(at, tail);
+                for (int i = 0; i < C::B_UNITS; i++, at += x_step) xq[d][i] = load_unit<VEC, false>(at);
+            } else {
+#pragma unroll
+                for (int i = 0; i < C::B_UNITS; i++, at += x_step) xq[d][i] = load_some(at, tail);
+            }
         }
         px += BK;
     };
@@ -298,25 +307,44 @@ linear32_tc_kernel(const Params p) {
             }
             tc_fence_before();
         };
-        auto step = [&](int b, int d) {
+        auto next_block = [&](int b, int d) {
             // (the stage is free: its last MMAs, block b - 2's, were waited for when that block was added up)
             uint8_t* at = stages + (b & 1) * C::STAGE_BYTES + place;
+            if (b + C::DEPTH < whole) {
+                // a unit's registers take the next load as soon as it is stored: that load has the whole of a block's time
+                const float *from = pw, *from_x = px;
 #pragma unroll
-            for (int i = 0; i < C::A_UNITS; i++) store_parts(at + i * (ROW_STEP * 128), A_BYTES, wq[d][i]);
-            if (has_x) {
+                for (int i = 0; i < C::A_UNITS; i++, from += step) {
+                    store_parts(at + i * (ROW_STEP * 128), A_BYTES, wq[d][i]);
+                    wq[d][i] = load_unit<VEC, true>(from);
+                }
+                if (has_x) {
 #pragma unroll
-                for (int i = 0; i < C::B_UNITS; i++) store_parts(at + 3 * A_BYTES + i * (ROW_STEP * 128), C::B_BYTES, xq[d][i]);
+                    for (int i = 0; i < C::B_UNITS; i++, from_x += x_step) {
+                        store_parts(at + 3 * A_BYTES + i * (ROW_STEP * 128), C::B_BYTES, xq[d][i]);
+                        xq[d][i] = load_unit<VEC, false>(from_x);
+                    }
+                }
+                pw += BK;
+                px += BK;
+            } else {
+#pragma unroll
+                for (int i = 0; i < C::A_UNITS; i++) store_parts(at + i * (ROW_STEP * 128), A_BYTES, wq[d][i]);
+                if (has_x) {
+#pragma unroll
+                    for (int i = 0; i < C::B_UNITS; i++) store_parts(at + 3 * A_BYTES + i * (ROW_STEP * 128), C::B_BYTES, xq[d][i]);
+                }
+                if (b + C::DEPTH < nb) { load_w(b + C::DEPTH, d); load_x(b + C::DEPTH, d); }
             }
             fence_proxy_async();
             __syncwarp();
             if (lane == 0) mbar_arrive(full(b));
-            if (b + C::DEPTH < nb) { load_w(b + C::DEPTH, d); load_x(b + C::DEPTH, d); }
             if (b > 0) add_up(b - 1);
         };
         for (int b = 0; b < nb && ok; b += C::DEPTH) {
 #pragma unroll
             for (int d = 0; d < C::DEPTH; d++)
-                if (b + d < nb && ok) step(b + d, d);
+                if (b + d < nb && ok) next_block(b + d, d);
         }
         ib::pdl_launch_dependents();
         if (ok) add_up(nb - 1);
@@ -326,7 +354,7 @@ linear32_tc_kernel(const Params p) {
     // Feature tid & 127 of own columns tid / 128, + 4, ..., four columns at a time; what is added to the first four's sums is requested
     // before the barrier.
     const int64_t n = n0 + (tid & (BM - 1));
-    const bool storing = worker && n < p.N;
+    const bool storing = worker && n >= n_first;
     const float bias = storing && p.bias ? p.bias[n] : 0.0f;
     const int slots = p.share > 1 ? p.groups : 1;
     float res[4];
