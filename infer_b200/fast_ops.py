@@ -232,27 +232,24 @@ def linear_skinny(x: torch.Tensor, w: torch.Tensor, bias: Optional[torch.Tensor]
     return out
 
 
-# Rows up to which a product takes the streaming kernel. From 9 on it needs two 8-row MMA tiles per weight fragment, mma.sync bounds it and
-# its registers spill: the four products and two norms of a layer of 1536 features at 12 rows took 39 us, on the tcgen05 kernel 36.5.
-SKINNY_ROWS = 8
-
-
 def linear(x, weight, bias, residual, out_dtype, out, swiglu=False):
-    """The bfloat16 matrix product of the serving path: the streaming kernel for up to 8 rows, the tcgen05 kernel
-    above that (the streaming one where it refuses up to 16); None if neither takes the shape. x may be a DeferredNorm (the float32 residual stream plus the norm
+    """The bfloat16 matrix product of the serving path: the streaming kernel for up to 16 rows, the tcgen05 kernel
+    above that; None if neither takes the shape. x may be a DeferredNorm (the float32 residual stream plus the norm
     that is still to be applied): the streaming kernel then normalises inside, anything else materialises it."""
     from .parts.base import DeferredNorm
     if isinstance(x, DeferredNorm):
-        if weight.dtype == torch.bfloat16 and x.h.shape[0] <= SKINNY_ROWS:
+        if weight.dtype == torch.bfloat16 and x.h.shape[0] <= skinny_limits()[0]:
             y = linear_skinny(x.h, weight, bias, residual, out_dtype, out, swiglu, 0, x.norm.weight, x.norm.eps)
             if y is not None:
                 return y
         x = x.materialize()
     if x.dtype != torch.bfloat16:
         return None
-    first, second = (linear_skinny, gemm_tc) if x.shape[0] <= SKINNY_ROWS else (gemm_tc, linear_skinny)
-    y = first(x, weight, bias, residual, out_dtype, out, swiglu=swiglu)
-    return y if y is not None else second(x, weight, bias, residual, out_dtype, out, swiglu=swiglu)
+    if x.shape[0] <= skinny_limits()[0]:
+        y = linear_skinny(x, weight, bias, residual, out_dtype, out, swiglu)
+        if y is not None:
+            return y
+    return gemm_tc(x, weight, bias, residual, out_dtype, out, swiglu=swiglu)
 
 
 def linear_f32_tc(x: torch.Tensor, w: torch.Tensor, bias: Optional[torch.Tensor], residual: Optional[torch.Tensor], out: torch.Tensor,

@@ -56,10 +56,10 @@ def _side_streams(device):
 
 def normed_input(norm, consumer, h):
     """norm(h), or, for as few rows as the streaming product takes and a consumer that can normalise inside its
-    first kernel, the norm deferred."""
+    first kernel, the norm deferred. How many rows that is, is the kernel library's answer, not a constant here."""
     if consumer.accepts_deferred_norm and getattr(norm, "fusable", False) and norm.rt.fast("norm"):
         from .. import fast_ops
-        if h.shape[0] <= fast_ops.SKINNY_ROWS:
+        if h.shape[0] <= fast_ops.skinny_limits()[0]:
             return DeferredNorm(norm, h)
     return norm.forward(h)
 
