@@ -115,6 +115,13 @@ __device__ long long ib_gemv_trace[64];
 #define IB_GT(k) do {} while (0)
 #endif
 
+// How a matrix is dealt out to the CTAs of a grid (a part of GemvParams by itself: what the product that follows will ask for first).
+struct Deal {
+    const bf16* w;
+    int64_t N, K;
+    int tiles, cluster, kc, ns, n_stages, per_cta, groups, even, run, longer, grid;
+};
+
 struct GemvParams {
     const bf16* x;            // [M, K]; or, with norm_w, float rows that are RMS-normalised first (K <= KC_MAX)
     const float* norm_w;      // [K] or null
@@ -140,9 +147,11 @@ struct GemvParams {
     int even, run, longer;
     float* parts;             // [grid][2][PART_FLOATS]: sums of the tiles that a CTA begins and ends inside
     unsigned int* arrived;    // [tiles] stages summed so far, zero between calls
+    Deal next;                // grid 0: none
 };
 
-template <int NT, int EPI, typename TOut, bool NWS>
+// EVEN: equal runs of stages (p.even); a kernel of its own, since what it needs costs the other registers that it has not got.
+template <int NT, int EPI, typename TOut, bool NWS, bool EVEN>
 __global__ void __launch_bounds__(THREADS, 2)
 bulk_gemv_kernel(const GemvParams p) {
     extern __shared__ __align__(128) uint8_t stages[];   // [ns][ROWS][pitch]
@@ -165,12 +174,12 @@ bulk_gemv_kernel(const GemvParams p) {
     const int total_stages = p.n_stages;
     const int s_begin = min(total_stages, rank * p.per_cta), s_end = min(total_stages, s_begin + p.per_cta);
     const int spt = s_end - s_begin;                     // stages per tile
-    const int run0 = int(blockIdx.x) * p.run + min(int(blockIdx.x), p.longer);          // (even) the CTA's first stage
+    const int run0 = EVEN ? int(blockIdx.x) * p.run + min(int(blockIdx.x), p.longer) : 0;          // the CTA's first stage
     const int my_tiles = group < p.tiles ? (p.tiles - group + p.groups - 1) / p.groups : 0;
-    const int n_iter = p.even ? p.run + (int(blockIdx.x) < p.longer ? 1 : 0) : my_tiles * spt;
-    const int tile0 = p.even ? run0 / total_stages : group;
-    const int st0 = p.even ? run0 - tile0 * total_stages : 0;
-    const int tile_step = p.even ? 1 : p.groups;
+    const int n_iter = EVEN ? p.run + (int(blockIdx.x) < p.longer ? 1 : 0) : my_tiles * spt;
+    const int tile0 = EVEN ? run0 / total_stages : group;
+    const int st0 = EVEN ? run0 - tile0 * total_stages : 0;
+    const int tile_step = EVEN ? 1 : p.groups;
     const uint32_t stage0 = smem_u32(stages), bar0 = smem_u32(bars);
     auto full_bar = [&](int s) { return bar0 + 8u * s; };
     auto empty_bar = [&](int s) { return bar0 + 8u * (NS_MAX + s); };
@@ -184,7 +193,7 @@ bulk_gemv_kernel(const GemvParams p) {
     // Rows beyond N (last tile only) are never copied: start from zeros. A stage that held an earlier tile's rows is
     // harmless there, because those rows' results are not stored.
     // this CTA takes (part of) the last, partial tile
-    if (N % ROWS != 0 && (p.even ? run0 + n_iter > (p.tiles - 1) * total_stages : (p.tiles - 1 - group) % p.groups == 0)) {
+    if (N % ROWS != 0 && (EVEN ? run0 + n_iter > (p.tiles - 1) * total_stages : (p.tiles - 1 - group) % p.groups == 0)) {
         for (int i = threadIdx.x; i < RING_BYTES / 16; i += THREADS) reinterpret_cast<uint4*>(stages)[i] = make_uint4(0u, 0u, 0u, 0u);
         asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
     }
@@ -226,6 +235,23 @@ bulk_gemv_kernel(const GemvParams p) {
             if (++st == spt) { st = 0; tile += tile_step; }
         }
         if (n_iter == 0) ib::pdl_launch_dependents();
+        // This CTA has asked for all of its own: what CTAs of the product that follows will ask for first (their rings) goes into L2 while
+        // the rest of this kernel and the change to the next leave the memory idle. Layer of 1536 features, gate/up before down:
+        // 31.1 -> 29.9 us at one row, 32.7 -> 31.7 at eight.
+        const Deal& q = p.next;
+        if constexpr (EPI == 2)
+        for (int v = blockIdx.x; v < q.grid; v += gridDim.x) {
+            const int vrank = v % q.cluster, vgroup = v / q.cluster, v0 = v * q.run + min(v, q.longer);
+            const int vbegin = q.even ? 0 : min(q.n_stages, vrank * q.per_cta), vend = q.even ? q.n_stages : min(q.n_stages, vbegin + q.per_cta);
+            int vtile = q.even ? v0 / q.n_stages : vgroup, vst = q.even ? v0 - vtile * q.n_stages : vbegin;
+            for (int i = 0; i < q.ns && vtile < q.tiles && vst < vend; i++) {
+                const int64_t row = int64_t(vtile) * ROWS + lane, k = int64_t(vst) * q.kc;
+                if (lane < ROWS && row < q.N)
+                    asm volatile("cp.async.bulk.prefetch.L2.global.L2::cache_hint [%0], %1, %2;"
+                                 ::"l"(q.w + row * q.K + k), "r"(uint32_t(min(int64_t(q.kc), q.K - k) * 2)), "l"(once) : "memory");
+                if (++vst == vend) { vst = vbegin; vtile += q.even ? 1 : q.groups; }
+            }
+        }
         if (cluster > 1) {                               // the cluster barriers below count every thread
             cg::cluster_group cl = cg::this_cluster();
             cl.sync();
@@ -405,7 +431,7 @@ bulk_gemv_kernel(const GemvParams p) {
         if (lane == 0) mbar_arrive(empty_bar(s));
         IB_GT(6 + 4 * int(i));
         if (++s == NS) { s = 0; round++; }
-        if (++st != spt && !(p.even && i == n_iter - 1)) continue;
+        if (++st != spt && !(EVEN && i == n_iter - 1)) continue;
         const int summed = st - st_from;                 // stages of this tile that this CTA has summed
         st = st_from = 0;
 
@@ -429,7 +455,7 @@ bulk_gemv_kernel(const GemvParams p) {
             for (int wi = 0; wi < WARPS; wi++) v += red[wi][ant][col][r];
         }
         bool writer = true;
-        if (p.even && summed != spt) {
+        if (EVEN && summed != spt) {
             // A part of a tile. Its sums go to the workspace; the CTA that completes the tile's count adds all parts in
             // ascending order of K, so that the result does not depend on which one that is.
             if (active) __stcg(p.parts + (int(blockIdx.x) * 2 + (this_tile == tile0 ? 0 : 1)) * PART_FLOATS + threadIdx.x, v);
@@ -452,7 +478,7 @@ bulk_gemv_kernel(const GemvParams p) {
                     v += __ldcg(p.parts + (c * 2 + (begin < u0 ? 1 : 0)) * PART_FLOATS + threadIdx.x);
             }
         }
-        if (cluster > 1) {
+        if (!EVEN && cluster > 1) {
             cg::cluster_group cl = cg::this_cluster();
             if (active) part[ant][col][r] = v;
             cl.sync();
@@ -492,17 +518,18 @@ int launch(const GemvParams& p, int out_dtype, int epi, int grid_ctas, cudaStrea
     const dim3 grid{unsigned(grid_ctas), 1u, 1u};
     const dim3 block{THREADS, 1u, 1u};
     const unsigned cl = unsigned(p.cluster);
-#define IB_GEMV_LAUNCH_(EPI_, T_, NWS_)                                                                            \
+#define IB_GEMV_LAUNCH_(EPI_, T_, NWS_, EVEN_)                                                                     \
     do {                                                                                                           \
         static ib::PerDevice allowed;                                                                              \
-        if (const int rc = ib::allow_smem(allowed, "linear_skinny_bulk", bulk_gemv_kernel<NT, EPI_, T_, NWS_>, RING_BYTES + NW_BYTES)) return rc; \
-        return ib::launch("linear_skinny_bulk", bulk_gemv_kernel<NT, EPI_, T_, NWS_>, grid, block,                 \
+        if (const int rc = ib::allow_smem(allowed, "linear_skinny_bulk", bulk_gemv_kernel<NT, EPI_, T_, NWS_, EVEN_>, RING_BYTES + NW_BYTES)) return rc; \
+        return ib::launch("linear_skinny_bulk", bulk_gemv_kernel<NT, EPI_, T_, NWS_, EVEN_>, grid, block,          \
                           size_t(RING_BYTES) + (NWS_ ? size_t(NW_BYTES) : 0), stream, cl, p);                      \
     } while (0)
 #define IB_GEMV_LAUNCH(EPI_, T_)                                                                                   \
     do {                                                                                                           \
-        if (NT == 1 && p.norm_w && p.nw_smem) IB_GEMV_LAUNCH_(EPI_, T_, true);                                     \
-        IB_GEMV_LAUNCH_(EPI_, T_, false);                                                                          \
+        if (p.even) IB_GEMV_LAUNCH_(EPI_, T_, false, true);                                                        \
+        if (NT == 1 && p.norm_w && p.nw_smem) IB_GEMV_LAUNCH_(EPI_, T_, true, false);                              \
+        IB_GEMV_LAUNCH_(EPI_, T_, false, false);                                                                   \
     } while (0)
     if (epi == 2) {
         if (out_dtype != IB_BF16) return ib::fail(IB_ERR_ARG, "linear_skinny_bulk: the SwiGLU epilogue writes bfloat16");
@@ -519,12 +546,58 @@ int launch(const GemvParams& p, int out_dtype, int epi, int grid_ctas, cudaStrea
     return ib::fail(IB_ERR_ARG, "linear_skinny_bulk: unknown output dtype %d", out_dtype);
 }
 
+// K of a tile in as few stages as the ring allows (a whole row for K up to KC_MAX), since the cost of a stage (its copies, the barrier
+// round trip) does not depend on its size. cluster 0: chosen here. even < 0: chosen here (where `can`), 0: never, else the number
+// of stages that a tile's K is cut into.
+Deal deal_out(const bf16* w, int64_t N, int64_t K, int cluster, int even, bool can, int sms) {
+    Deal d = {};
+    d.w = w; d.N = N; d.K = K;
+    const int64_t tiles = (N + ROWS - 1) / ROWS, places = int64_t(IB_GEMV_CTAS_PER_SM) * sms;
+    const int64_t least = (K + KC_MAX - 1) / KC_MAX;
+    if (cluster == 0) {
+        // Share a tile among CTAs while the tiles alone leave SMs idle and every CTA keeps at least three stages of K
+        // (measured on B200 for K = 8960: 10.8 us alone, 8.9 us in pairs, 14.4 us in fours; clusters of three or six
+        // run slower still).
+        cluster = 1;
+        while (cluster < 8 && tiles * cluster < 2LL * sms && least >= 6 * cluster) cluster *= 2;
+    }
+    auto stage_of = [&](int64_t n) { return ((K + n - 1) / n + 63) / 64 * 64; };       // elements of K in each of n equal stages
+    auto rounds = [&](int64_t work) { return (work + places - 1) / places; };
+    int64_t n_stages = (least + cluster - 1) / cluster * cluster;                      // the same number of stages for every CTA of a cluster
+    if (!can) even = 0;
+    if (even < 0) {
+        // Equal runs where whole tiles would give some CTA at least 4,000 elements of K more (of 16 rows): the parts' meeting costs what
+        // reading those does. us with whole tiles -> with runs at 8 rows, and elements saved: 5120 x 13824 34.1 -> 26.9 (12,288),
+        // 3584 x 18944 31.8 -> 27.1 (5,888), 2560 x 9728 17.7 -> 14.6 (4,096), 6400 x 8192 23.6 -> 22.7 (4,224), but 5120 x 5120
+        // 14.8 -> 15.8 (3,840), 4960 x 4096 11.2 -> 13.2 (2,816), 1536 x 8960 8.0 -> 9.3 (1,536).
+        const int64_t whole = rounds(tiles * cluster) * (n_stages / cluster) * stage_of(n_stages);
+        even = whole - rounds(tiles * least) * stage_of(least) >= 4000 ? int(least) : 0;
+    }
+    if (even > 0) { n_stages = even; cluster = 1; }
+    d.tiles = int(tiles); d.cluster = cluster; d.even = even > 0;
+    d.kc = int(stage_of(n_stages));
+    d.ns = RING_BYTES / (ROWS * (d.kc * 2 + 64));
+    if (d.ns > NS_MAX) d.ns = NS_MAX;
+    d.n_stages = int((K + d.kc - 1) / d.kc);
+    d.per_cta = (d.n_stages + cluster - 1) / cluster;
+    // Two CTAs fit an SM; with more tiles than that, a CTA walks over several and its ring never drains between them.
+    d.groups = int(cluster > 1 || tiles < places ? tiles : places);
+    d.grid = d.groups * cluster;
+    if (d.even) {
+        const int64_t units = tiles * d.n_stages;
+        d.grid = int(units < places ? units : places);
+        d.run = int(units / d.grid); d.longer = int(units % d.grid);
+    }
+    return d;
+}
+
 }  // namespace
 
 // x: bfloat16 [M, K]; with norm_w (float [K]) x is float [M, K] and is RMS-normalised (eps norm_eps) on the way in,
 // each CTA once for all its tiles (K <= 1536). epi: 0 = (+ bias), 1 = (+ bias) + residual -> float, 2 = SwiGLU over rows interleaved by 8 ->
 // bfloat16 [M, N/2]. cluster: CTAs that share a tile's K range (1, 2, 4 or 8); 0 lets the kernel choose from N, K and
-// sm_count. status: one int in device memory, raised if a bounded wait runs out.
+// sm_count. status: one int in device memory, raised if a bounded wait runs out. next_w [next_N, next_K]: the matrix of the product that
+// follows on the stream, or null (a hint).
 // What this kernel takes: the most rows of activations, and the longest row that the fused RMSNorm prologue
 // normalises in registers. Callers plan with these figures instead of carrying copies of them.
 IB_EXPORT int ib_linear_skinny_bulk_limits(int* max_rows, int* max_fused_norm_k) {
@@ -536,7 +609,7 @@ IB_EXPORT int ib_linear_skinny_bulk_limits(int* max_rows, int* max_fused_norm_k)
 IB_EXPORT int ib_linear_skinny_bulk(const void* x, const float* norm_w, float norm_eps, const void* w, const float* bias, const float* residual, void* out,
                                     int64_t M, int64_t N, int64_t K, int out_dtype, int epi, int cluster, int sm_count,
                                     int* status, float* parts, int64_t n_parts, unsigned int* arrived, int64_t n_arrived, int even,
-                                    cudaStream_t stream) {
+                                    const void* next_w, int64_t next_N, int64_t next_K, cudaStream_t stream) {
     if (M <= 0 || N <= 0) return IB_OK;
     if (M > 16) return ib::fail(IB_ERR_ARG, "linear_skinny_bulk: at most 16 rows, got %lld", (long long)M);
     if (K <= 0 || K % 8) return ib::fail(IB_ERR_ARG, "linear_skinny_bulk: K = %lld must be a positive multiple of 8", (long long)K);
@@ -549,55 +622,26 @@ IB_EXPORT int ib_linear_skinny_bulk(const void* x, const float* norm_w, float no
     const int64_t tiles = (N + ROWS - 1) / ROWS;
     if (tiles > 0x7fffffffLL / 8) return ib::fail(IB_ERR_ARG, "linear_skinny_bulk: N too large");
     const int sms = sm_count > 0 ? sm_count : 148;
-    // A stage holds ROWS rows of kc elements: K in as few equal stages as the ring allows (a whole row for K up to
-    // KC_MAX), since the cost of a stage (its copies, the barrier round trip) does not depend on its size.
-    int64_t n_stages = (K + KC_MAX - 1) / KC_MAX;
-    if (cluster == 0) {
-        // Share a tile among CTAs while the tiles alone leave SMs idle and every CTA keeps at least three stages of K
-        // (measured on B200 for K = 8960: 10.8 us alone, 8.9 us in pairs, 14.4 us in fours; clusters of three or six
-        // run slower still).
-        cluster = 1;
-        while (cluster < 8 && tiles * cluster < 2LL * sms && n_stages >= 6 * cluster) cluster *= 2;
-    }
-    if (cluster != 1 && cluster != 2 && cluster != 4 && cluster != 8) return ib::fail(IB_ERR_ARG, "linear_skinny_bulk: cluster must be 1, 2, 4 or 8");
-    // even < 0: chosen here; 0: never; else the number of stages that a tile's K is cut into
-    const int64_t places = int64_t(IB_GEMV_CTAS_PER_SM) * sms;
-    const bool can = !norm_w && tiles * 64 < (1LL << 30) && parts && arrived && n_arrived >= tiles && n_parts >= 2 * places * PART_FLOATS;
-    auto stage_of = [&](int64_t n) { return ((K + n - 1) / n + 63) / 64 * 64; };       // elements of K in each of n equal stages
-    auto rounds = [&](int64_t work) { return (work + places - 1) / places; };
-    const int64_t least = n_stages;                              // as few stages as the ring allows
-    n_stages = (n_stages + cluster - 1) / cluster * cluster;     // the same number of stages for every CTA of a cluster
-    if (!can) even = 0;
-    if (even < 0) {
-        // Equal runs where whole tiles would give some CTA at least 4,000 elements of K more (of 16 rows): the parts' meeting costs what
-        // reading those does. us with whole tiles -> with runs at 8 rows, and elements saved: 5120 x 13824 34.1 -> 26.9 (12,288),
-        // 3584 x 18944 31.8 -> 27.1 (5,888), 2560 x 9728 17.7 -> 14.6 (4,096), 6400 x 8192 23.6 -> 22.7 (4,224), but 5120 x 5120
-        // 14.8 -> 15.8 (3,840), 4960 x 4096 11.2 -> 13.2 (2,816), 1536 x 8960 8.0 -> 9.3 (1,536).
-        const int64_t whole = rounds(tiles * cluster) * (n_stages / cluster) * stage_of(n_stages);
-        even = whole - rounds(tiles * least) * stage_of(least) >= 4000 ? int(least) : 0;
-    }
-    if (even > 0) { n_stages = even; cluster = 1; }
-    const int kc = int(stage_of(n_stages));
-    int ns = RING_BYTES / (ROWS * (kc * 2 + 64));
-    if (ns > NS_MAX) ns = NS_MAX;
+    if (cluster != 0 && cluster != 1 && cluster != 2 && cluster != 4 && cluster != 8) return ib::fail(IB_ERR_ARG, "linear_skinny_bulk: cluster must be 1, 2, 4 or 8");
+    auto can_share = [&](int64_t n) {                            // tiles among CTAs through the workspace
+        const int64_t t = (n + ROWS - 1) / ROWS;
+        return t * 64 < (1LL << 30) && parts && arrived && n_arrived >= t && n_parts >= 2LL * IB_GEMV_CTAS_PER_SM * sms * PART_FLOATS;
+    };
+    const Deal d = deal_out((const bf16*)w, N, K, cluster, even, !norm_w && can_share(N), sms);
     GemvParams p;
     p.x = (const bf16*)x; p.norm_w = norm_w; p.eps = norm_eps; p.w = (const bf16*)w; p.bias = bias; p.residual = residual; p.out = out;
-    p.M = int(M); p.N = N; p.K = K; p.cluster = cluster; p.status = status; p.tiles = int(tiles); p.kc = kc; p.ns = ns;
-    p.n_stages = int((K + kc - 1) / kc); p.per_cta = (p.n_stages + cluster - 1) / cluster;
+    p.M = int(M); p.N = N; p.K = K; p.cluster = d.cluster; p.status = status; p.tiles = d.tiles; p.kc = d.kc; p.ns = d.ns;
+    p.n_stages = d.n_stages; p.per_cta = d.per_cta;
     // gate the ring's second slot where the whole GPU's rings fill at once (a CTA per half SM) and a tile is one stage
-    p.gate_ring = (n_stages == 1 && cluster == 1 && tiles >= 2LL * sms) ? 1 : 0;
+    p.gate_ring = (d.n_stages == 1 && d.cluster == 1 && tiles >= 2LL * sms) ? 1 : 0;
     p.nw_smem = norm_w ? 1 : 0;
-    // Two CTAs fit an SM; with more tiles than that, a CTA walks over several and its ring never drains between them.
-    p.groups = int(cluster > 1 || tiles < places ? tiles : places);
-    int grid_ctas = p.groups * cluster;
-    p.even = even > 0;
-    p.run = p.longer = 0;
-    if (p.even) {
-        const int64_t units = tiles * p.n_stages;
-        grid_ctas = int(units < places ? units : places);
-        p.run = int(units / grid_ctas); p.longer = int(units % grid_ctas);
-    }
+    p.groups = d.groups;
+    p.even = d.even; p.run = d.run; p.longer = d.longer;
     p.parts = parts; p.arrived = arrived;
+    p.next = Deal{};
+    if (next_w && next_N > 0 && next_K > 0 && next_K % 8 == 0 && !(uintptr_t(next_w) & 15) && next_N < (1LL << 30))
+        p.next = deal_out((const bf16*)next_w, next_N, next_K, 0, -1, can_share(next_N), sms);
+    const int grid_ctas = d.grid;
     if (M <= 8) return launch<1>(p, out_dtype, epi, grid_ctas, stream);
     return launch<2>(p, out_dtype, epi, grid_ctas, stream);
 }
