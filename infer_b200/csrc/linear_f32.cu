@@ -1,4 +1,5 @@
-// Matrix product of the true 32-bit path: out[m, n] = sum_k x[m, k] * w[n, k] (+ bias[n]) (+ residual[m, n]), all float.
+// Matrix product of the true 32-bit path: out[m, n] = sum_k x[m, k] * w[n, k] (+ bias[n]) (+ residual[m, n]), all float, for matrices of fewer
+// than 1024 features or columns (larger ones: linear_f32_tc.cu; the figures below are of those, from before).
 //
 // The order of every sum is fixed by K alone, so that a row of the result has the same bits in every batch, whichever
 // kernel below computes it: K is cut into blocks of 32; within a block the even and the odd k are two fused

@@ -12,6 +12,10 @@
 // first accumulator starts anew every 64 elements of K and is added to a float in registers; the other two, whose errors
 // weigh 2^-8, run over a group of such blocks. Groups (at most 8, from N and K alone) are added in ascending order. A result
 // does not depend on how many rows x has, nor on which CTA forms which group: a row's bits are the same in every batch.
+// Error against 64 bits (norm over norm, normal operands): 0.94e-7 at K = 1024, 1.2e-7 at 8960, where multiply-adds have 1.3e-7 and 3.1e-7.
+// us on multiply-adds -> here: 512 rows, 17920 x 1536 671 -> 272, 1536 x 8960 441 -> 165; 16 rows 55 -> 31 and 118 -> 23; 3 rows 31 -> 29
+// and 25 -> 23; one row 20 -> 29 and 18 -> 22. (A row's bits must not depend on the batch, so one row comes here too.) The line at
+// 1024 x 1024: below it the tiles leave most SMs idle.
 //
 // A CTA (544 threads, one an SM) forms 128 features x NT tokens (features on the tensor memory's 128 lanes). Sixteen warps load a
 // block of 64 elements of K into registers a block or two ahead, cut and store it as six swizzled operand tiles, and add up the
