@@ -115,10 +115,8 @@ __device__ long long ib_gemv_trace[64];
 #define IB_GT(k) do {} while (0)
 #endif
 
-// How a matrix is dealt out to the CTAs of a grid (a part of GemvParams by itself: what the product that follows will ask for first).
+// How a matrix is dealt out to the CTAs of a grid.
 struct Deal {
-    const bf16* w;
-    int64_t N, K;
     int tiles, cluster, kc, ns, n_stages, per_cta, groups, even, run, longer, grid;
 };
 
@@ -147,7 +145,6 @@ struct GemvParams {
     int even, run, longer;
     float* parts;             // [grid][2][PART_FLOATS]: sums of the tiles that a CTA begins and ends inside
     unsigned int* arrived;    // [tiles] stages summed so far, zero between calls
-    Deal next;                // grid 0: none
 };
 
 // EVEN: equal runs of stages (p.even); a kernel of its own, since what it needs costs the other registers that it has not got.
@@ -235,23 +232,6 @@ bulk_gemv_kernel(const GemvParams p) {
             if (++st == spt) { st = 0; tile += tile_step; }
         }
         if (n_iter == 0) ib::pdl_launch_dependents();
-        // This CTA has asked for all of its own: what CTAs of the product that follows will ask for first (their rings) goes into L2 while
-        // the rest of this kernel and the change to the next leave the memory idle. Layer of 1536 features, gate/up before down:
-        // 31.1 -> 29.9 us at one row, 32.7 -> 31.7 at eight.
-        const Deal& q = p.next;
-        if constexpr (EPI == 2)
-        for (int v = blockIdx.x; v < q.grid; v += gridDim.x) {
-            const int vrank = v % q.cluster, vgroup = v / q.cluster, v0 = v * q.run + min(v, q.longer);
-            const int vbegin = q.even ? 0 : min(q.n_stages, vrank * q.per_cta), vend = q.even ? q.n_stages : min(q.n_stages, vbegin + q.per_cta);
-            int vtile = q.even ? v0 / q.n_stages : vgroup, vst = q.even ? v0 - vtile * q.n_stages : vbegin;
-            for (int i = 0; i < q.ns && vtile < q.tiles && vst < vend; i++) {
-                const int64_t row = int64_t(vtile) * ROWS + lane, k = int64_t(vst) * q.kc;
-                if (lane < ROWS && row < q.N)
-                    asm volatile("cp.async.bulk.prefetch.L2.global.L2::cache_hint [%0], %1, %2;"
-                                 ::"l"(q.w + row * q.K + k), "r"(uint32_t(min(int64_t(q.kc), q.K - k) * 2)), "l"(once) : "memory");
-                if (++vst == vend) { vst = vbegin; vtile += q.even ? 1 : q.groups; }
-            }
-        }
         if (cluster > 1) {                               // the cluster barriers below count every thread
             cg::cluster_group cl = cg::this_cluster();
             cl.sync();
@@ -549,9 +529,8 @@ int launch(const GemvParams& p, int out_dtype, int epi, int grid_ctas, cudaStrea
 // K of a tile in as few stages as the ring allows (a whole row for K up to KC_MAX), since the cost of a stage (its copies, the barrier
 // round trip) does not depend on its size. cluster 0: chosen here. even < 0: chosen here (where `can`), 0: never, else the number
 // of stages that a tile's K is cut into.
-Deal deal_out(const bf16* w, int64_t N, int64_t K, int cluster, int even, bool can, int sms) {
+Deal deal_out(int64_t N, int64_t K, int cluster, int even, bool can, int sms) {
     Deal d = {};
-    d.w = w; d.N = N; d.K = K;
     const int64_t tiles = (N + ROWS - 1) / ROWS, places = int64_t(IB_GEMV_CTAS_PER_SM) * sms;
     const int64_t least = (K + KC_MAX - 1) / KC_MAX;
     if (cluster == 0) {
@@ -596,8 +575,7 @@ Deal deal_out(const bf16* w, int64_t N, int64_t K, int cluster, int even, bool c
 // x: bfloat16 [M, K]; with norm_w (float [K]) x is float [M, K] and is RMS-normalised (eps norm_eps) on the way in,
 // each CTA once for all its tiles (K <= 1536). epi: 0 = (+ bias), 1 = (+ bias) + residual -> float, 2 = SwiGLU over rows interleaved by 8 ->
 // bfloat16 [M, N/2]. cluster: CTAs that share a tile's K range (1, 2, 4 or 8); 0 lets the kernel choose from N, K and
-// sm_count. status: one int in device memory, raised if a bounded wait runs out. next_w [next_N, next_K]: the matrix of the product that
-// follows on the stream, or null (a hint).
+// sm_count. status: one int in device memory, raised if a bounded wait runs out.
 // What this kernel takes: the most rows of activations, and the longest row that the fused RMSNorm prologue
 // normalises in registers. Callers plan with these figures instead of carrying copies of them.
 IB_EXPORT int ib_linear_skinny_bulk_limits(int* max_rows, int* max_fused_norm_k) {
@@ -609,7 +587,7 @@ IB_EXPORT int ib_linear_skinny_bulk_limits(int* max_rows, int* max_fused_norm_k)
 IB_EXPORT int ib_linear_skinny_bulk(const void* x, const float* norm_w, float norm_eps, const void* w, const float* bias, const float* residual, void* out,
                                     int64_t M, int64_t N, int64_t K, int out_dtype, int epi, int cluster, int sm_count,
                                     int* status, float* parts, int64_t n_parts, unsigned int* arrived, int64_t n_arrived, int even,
-                                    const void* next_w, int64_t next_N, int64_t next_K, cudaStream_t stream) {
+                                    cudaStream_t stream) {
     if (M <= 0 || N <= 0) return IB_OK;
     if (M > 16) return ib::fail(IB_ERR_ARG, "linear_skinny_bulk: at most 16 rows, got %lld", (long long)M);
     if (K <= 0 || K % 8) return ib::fail(IB_ERR_ARG, "linear_skinny_bulk: K = %lld must be a positive multiple of 8", (long long)K);
@@ -623,11 +601,10 @@ IB_EXPORT int ib_linear_skinny_bulk(const void* x, const float* norm_w, float no
     if (tiles > 0x7fffffffLL / 8) return ib::fail(IB_ERR_ARG, "linear_skinny_bulk: N too large");
     const int sms = sm_count > 0 ? sm_count : 148;
     if (cluster != 0 && cluster != 1 && cluster != 2 && cluster != 4 && cluster != 8) return ib::fail(IB_ERR_ARG, "linear_skinny_bulk: cluster must be 1, 2, 4 or 8");
-    auto can_share = [&](int64_t n) {                            // tiles among CTAs through the workspace
-        const int64_t t = (n + ROWS - 1) / ROWS;
-        return t * 64 < (1LL << 30) && parts && arrived && n_arrived >= t && n_parts >= 2LL * IB_GEMV_CTAS_PER_SM * sms * PART_FLOATS;
-    };
-    const Deal d = deal_out((const bf16*)w, N, K, cluster, even, !norm_w && can_share(N), sms);
+    // tiles shared by CTAs: with a workspace, and stages that an int counts
+    const bool can = !norm_w && tiles * 64 < (1LL << 30) && K < (1LL << 16) && parts && arrived && n_arrived >= tiles &&
+                     n_parts >= 2LL * IB_GEMV_CTAS_PER_SM * sms * PART_FLOATS;
+    const Deal d = deal_out(N, K, cluster, even, can, sms);
     GemvParams p;
     p.x = (const bf16*)x; p.norm_w = norm_w; p.eps = norm_eps; p.w = (const bf16*)w; p.bias = bias; p.residual = residual; p.out = out;
     p.M = int(M); p.N = N; p.K = K; p.cluster = d.cluster; p.status = status; p.tiles = d.tiles; p.kc = d.kc; p.ns = d.ns;
@@ -638,9 +615,6 @@ IB_EXPORT int ib_linear_skinny_bulk(const void* x, const float* norm_w, float no
     p.groups = d.groups;
     p.even = d.even; p.run = d.run; p.longer = d.longer;
     p.parts = parts; p.arrived = arrived;
-    p.next = Deal{};
-    if (next_w && next_N > 0 && next_K > 0 && next_K % 8 == 0 && !(uintptr_t(next_w) & 15) && next_N < (1LL << 30))
-        p.next = deal_out((const bf16*)next_w, next_N, next_K, 0, -1, can_share(next_N), sms);
     const int grid_ctas = d.grid;
     if (M <= 8) return launch<1>(p, out_dtype, epi, grid_ctas, stream);
     return launch<2>(p, out_dtype, epi, grid_ctas, stream);

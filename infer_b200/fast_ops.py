@@ -194,13 +194,12 @@ def skinny_limits():
 def linear_skinny(x: torch.Tensor, w: torch.Tensor, bias: Optional[torch.Tensor] = None,
                   residual: Optional[torch.Tensor] = None, out_dtype: torch.dtype = torch.bfloat16,
                   out: Optional[torch.Tensor] = None, swiglu: bool = False, cluster: int = 0,
-                  norm_weight: Optional[torch.Tensor] = None, norm_eps: float = 0.0, even: int = -1, then: Optional[torch.Tensor] = None) -> Optional[torch.Tensor]:
+                  norm_weight: Optional[torch.Tensor] = None, norm_eps: float = 0.0, even: int = -1) -> Optional[torch.Tensor]:
     """The decode kernel: x [M <= 16, K] against w [N, K], weights streamed once; same epilogues as gemm_tc.
     With ``norm_weight`` x is the float32 residual stream and is RMS-normalised inside the kernel (rows up to
     ``skinny_limits()[1]`` long).
     cluster: CTAs sharing one tile's K range (0 = chosen by the kernel). even: the number of stages that a tile's K is cut into where equal
-    runs of stages are dealt out (-1 = chosen by the kernel, 0 = never). then: the matrix of the product that follows directly, whose
-    first rows the kernel asks L2 to fetch at its end."""
+    runs of stages are dealt out (-1 = chosen by the kernel, 0 = never)."""
     fused = norm_weight is not None
     _check(x, "x", torch.float32 if fused else torch.bfloat16)
     _check(w, "w", torch.bfloat16)
@@ -228,28 +227,27 @@ def linear_skinny(x: torch.Tensor, w: torch.Tensor, bias: Optional[torch.Tensor]
     st = device_state(x.device)
     epi = 2 if swiglu else (1 if residual is not None else 0)
     f = _fn("gemvb", "ib_linear_skinny_bulk", [c_void_p, c_void_p, c_float] + [c_void_p] * 4 + [c_int64] * 3 + [c_int] * 4 +
-            [c_void_p] * 2 + [c_int64, c_void_p, c_int64, c_int, c_void_p, c_int64, c_int64, c_void_p])
-    hint = (then.data_ptr(), then.shape[0], then.shape[1]) if then is not None and then.dtype == torch.bfloat16 and then.is_contiguous() else (None, 0, 0)
+            [c_void_p] * 2 + [c_int64, c_void_p, c_int64, c_int, c_void_p])
     _call(f, x.data_ptr(), _ptr(norm_weight), float(norm_eps), w.data_ptr(), _ptr(bias), _ptr(residual), out.data_ptr(),
-          M, N, K, dtype_code(out_dtype), epi, int(cluster), st.sm_count, st.status.data_ptr(), st.parts.data_ptr(), st.parts.numel(), st._counters.data_ptr(), st._counters.numel(), int(even), *hint, _stream())
+          M, N, K, dtype_code(out_dtype), epi, int(cluster), st.sm_count, st.status.data_ptr(), st.parts.data_ptr(), st.parts.numel(), st._counters.data_ptr(), st._counters.numel(), int(even), _stream())
     return out
 
 
-def linear(x, weight, bias, residual, out_dtype, out, swiglu=False, then=None):
+def linear(x, weight, bias, residual, out_dtype, out, swiglu=False):
     """The bfloat16 matrix product of the serving path: the streaming kernel for up to 16 rows, the tcgen05 kernel
     above that; None if neither takes the shape. x may be a DeferredNorm (the float32 residual stream plus the norm
     that is still to be applied): the streaming kernel then normalises inside, anything else materialises it."""
     from .parts.base import DeferredNorm
     if isinstance(x, DeferredNorm):
         if weight.dtype == torch.bfloat16 and x.h.shape[0] <= skinny_limits()[0]:
-            y = linear_skinny(x.h, weight, bias, residual, out_dtype, out, swiglu, 0, x.norm.weight, x.norm.eps, then=then)
+            y = linear_skinny(x.h, weight, bias, residual, out_dtype, out, swiglu, 0, x.norm.weight, x.norm.eps)
             if y is not None:
                 return y
         x = x.materialize()
     if x.dtype != torch.bfloat16:
         return None
     if x.shape[0] <= skinny_limits()[0]:
-        y = linear_skinny(x, weight, bias, residual, out_dtype, out, swiglu, then=then)
+        y = linear_skinny(x, weight, bias, residual, out_dtype, out, swiglu)
         if y is not None:
             return y
     return gemm_tc(x, weight, bias, residual, out_dtype, out, swiglu=swiglu)
@@ -705,6 +703,6 @@ def attention(q, cache, table, step, n_heads, n_kv, head_dim, window, scale):
                           scale, n_decode > 0, step.max_q_len, step.max_ctx_len, n_decode, seg_lens=step.seg_lens)
 
 
-def gate_up_swiglu(x, gate_up_weight, then=None):
+def gate_up_swiglu(x, gate_up_weight):
     """silu(x Wg^T) * (x Wu^T) in one kernel; gate_up_weight rows interleaved in blocks of 8."""
-    return linear(x, gate_up_weight, None, None, torch.bfloat16, None, swiglu=True, then=then)
+    return linear(x, gate_up_weight, None, None, torch.bfloat16, None, swiglu=True)

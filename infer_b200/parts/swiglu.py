@@ -44,7 +44,7 @@ class SwiGLU(FeedForward):
         act = None
         if self.interleaved and self.rt.fast("swiglu") and self.rt.fast("linear"):
             from .. import fast_ops
-            act = fast_ops.gate_up_swiglu(x, self.gate_up.weight, self.down.weight)
+            act = fast_ops.gate_up_swiglu(x, self.gate_up.weight)
         if act is None:
             act = ops.swiglu(self.gate_up(x), self.interleaved)      # Linear materialises a deferred norm
         return self.down(act, residual=residual)
