@@ -53,7 +53,6 @@ constexpr int RING_BYTES = 2 * ROWS * (KC_MAX * 2 + 64);
 constexpr int NW_BYTES = KC_MAX * 4;         // the fused norm's weight, behind the ring
 constexpr uint32_t SPIN_LIMIT = 1u << 22;
 constexpr int STATUS_TIMEOUT = 104;
-constexpr int PART_FLOATS = 2 * 8 * ROWS; // a tile's sums in the workspace
 
 __device__ __forceinline__ uint32_t smem_u32(const void* p) { return uint32_t(__cvta_generic_to_shared(p)); }
 __device__ __forceinline__ void mbar_init(uint32_t bar, uint32_t count) {
@@ -115,11 +114,6 @@ __device__ long long ib_gemv_trace[64];
 #define IB_GT(k) do {} while (0)
 #endif
 
-// How a matrix is dealt out to the CTAs of a grid.
-struct Deal {
-    int tiles, cluster, kc, ns, n_stages, per_cta, groups, even, run, longer, grid;
-};
-
 struct GemvParams {
     const bf16* x;            // [M, K]; or, with norm_w, float rows that are RMS-normalised first (K <= KC_MAX)
     const float* norm_w;      // [K] or null
@@ -136,19 +130,12 @@ struct GemvParams {
                               //    copies (up to 8 rows of activations; measured: q/k/v 4.1 -> 3.2 us)
     int kc;                   // elements of K per stage and row: a multiple of 64, at most KC_MAX
     int ns;                   // stages in the ring: 2 .. NS_MAX, ns * ROWS * (kc * 2 + 64) <= RING_BYTES
-    int tiles;
-    int n_stages, per_cta;    // stages of a tile's K, and of a CTA of its cluster
+    int64_t tiles;
     int groups;               // tile walkers in the grid (grid = groups * cluster); a walker takes every groups-th tile
     int* status;
-    // even: the stages of all tiles, tile after tile, are dealt out in equal runs, one a CTA (run + 1 stages to the first `longer`
-    // CTAs, `run` to the others); a tile that several CTAs share is put together by the one that completes its count
-    int even, run, longer;
-    float* parts;             // [grid][2][PART_FLOATS]: sums of the tiles that a CTA begins and ends inside
-    unsigned int* arrived;    // [tiles] stages summed so far, zero between calls
 };
 
-// EVEN: equal runs of stages (p.even); a kernel of its own, since what it needs costs the other registers that it has not got.
-template <int NT, int EPI, typename TOut, bool NWS, bool EVEN>
+template <int NT, int EPI, typename TOut, bool NWS>
 __global__ void __launch_bounds__(THREADS, 2)
 bulk_gemv_kernel(const GemvParams p) {
     extern __shared__ __align__(128) uint8_t stages[];   // [ns][ROWS][pitch]
@@ -157,7 +144,6 @@ bulk_gemv_kernel(const GemvParams p) {
     __shared__ float part[NT][8][ROWS];                  // this CTA's sum; read by the cluster's first CTA
     __shared__ float sumsq[WARPS][NT * 8];               // the warps' shares of a row's sum of squares (fused norm)
     __shared__ int failed;
-    __shared__ int last_here;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int g = lane >> 2, t = lane & 3;
     const int cluster = p.cluster;
@@ -168,15 +154,12 @@ bulk_gemv_kernel(const GemvParams p) {
     const int PITCH = KC * 2 + 64;                       // bytes between rows of a stage: consecutive rows start 16 banks apart
     const int STAGE_BYTES = ROWS * PITCH;
     // This CTA's slice of K, in stages of KC elements.
-    const int total_stages = p.n_stages;
-    const int s_begin = min(total_stages, rank * p.per_cta), s_end = min(total_stages, s_begin + p.per_cta);
-    const int spt = s_end - s_begin;                     // stages per tile
-    const int run0 = EVEN ? int(blockIdx.x) * p.run + min(int(blockIdx.x), p.longer) : 0;          // the CTA's first stage
-    const int my_tiles = group < p.tiles ? (p.tiles - group + p.groups - 1) / p.groups : 0;
-    const int n_iter = EVEN ? p.run + (int(blockIdx.x) < p.longer ? 1 : 0) : my_tiles * spt;
-    const int tile0 = EVEN ? run0 / total_stages : group;
-    const int st0 = EVEN ? run0 - tile0 * total_stages : 0;
-    const int tile_step = EVEN ? 1 : p.groups;
+    const int64_t total_stages = (K + KC - 1) / KC;
+    const int64_t per_cta = (total_stages + cluster - 1) / cluster;
+    const int64_t s_begin = min(total_stages, rank * per_cta), s_end = min(total_stages, s_begin + per_cta);
+    const int spt = int(s_end - s_begin);                // stages per tile
+    const int64_t my_tiles = group < p.tiles ? (p.tiles - group + p.groups - 1) / p.groups : 0;
+    const int64_t n_iter = my_tiles * spt;
     const uint32_t stage0 = smem_u32(stages), bar0 = smem_u32(bars);
     auto full_bar = [&](int s) { return bar0 + 8u * s; };
     auto empty_bar = [&](int s) { return bar0 + 8u * (NS_MAX + s); };
@@ -189,8 +172,7 @@ bulk_gemv_kernel(const GemvParams p) {
     }
     // Rows beyond N (last tile only) are never copied: start from zeros. A stage that held an earlier tile's rows is
     // harmless there, because those rows' results are not stored.
-    // this CTA takes (part of) the last, partial tile
-    if (N % ROWS != 0 && (EVEN ? run0 + n_iter > (p.tiles - 1) * total_stages : (p.tiles - 1 - group) % p.groups == 0)) {
+    if (N % ROWS != 0 && (p.tiles - 1 - group) % p.groups == 0) {     // this CTA takes the last, partial tile
         for (int i = threadIdx.x; i < RING_BYTES / 16; i += THREADS) reinterpret_cast<uint4*>(stages)[i] = make_uint4(0u, 0u, 0u, 0u);
         asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
     }
@@ -200,11 +182,11 @@ bulk_gemv_kernel(const GemvParams p) {
         // ---------------------------------------------------------------- producer: lane r copies row r of every stage
         // (ring slot, its use count, stage within the tile and tile are carried along: 64-bit divisions by run-time
         // values would cost more per stage than the copies)
-        int s = 0, st = st0;
+        int s = 0, st = 0;
         uint32_t round = 0;
-        int tile = tile0;
+        int64_t tile = group;
         const uint64_t once = policy_evict_first();
-        for (int i = 0; i < n_iter; i++) {
+        for (int64_t i = 0; i < n_iter; i++) {
             if (i == 1 && p.gate_ring) {
                 // With every SM's ring being filled at once, activations requested after the dependency wait would
                 // queue behind megabytes of weights and the consumers would start microseconds late: the second slot
@@ -220,8 +202,8 @@ bulk_gemv_kernel(const GemvParams p) {
                 ok = __shfl_sync(0xffffffffu, ok, 0);
                 if (!ok) { if (lane == 0) { atomicExch(p.status, STATUS_TIMEOUT); failed = 1; } break; }
             }
-            const int64_t n0 = int64_t(tile) * ROWS;
-            const int64_t k0 = int64_t(s_begin + st) * KC;
+            const int64_t n0 = tile * ROWS;
+            const int64_t k0 = (s_begin + st) * KC;
             const int live_rows = int(min(int64_t(ROWS), N - n0));
             const uint32_t bytes = uint32_t(min(int64_t(KC), K - k0) * 2);
             if (lane == 0) mbar_expect_tx(full_bar(s), bytes * uint32_t(live_rows));
@@ -229,7 +211,7 @@ bulk_gemv_kernel(const GemvParams p) {
             if (lane < live_rows) bulk_load(stage0 + s * STAGE_BYTES + lane * PITCH, p.w + (n0 + lane) * K + k0, bytes, full_bar(s), once);
             if (i == NS - 1 || i == n_iter - 1) ib::pdl_launch_dependents();     // the first ring is on its way
             if (++s == NS) { s = 0; round++; }
-            if (++st == spt) { st = 0; tile += tile_step; }
+            if (++st == spt) { st = 0; tile += p.groups; }
         }
         if (n_iter == 0) ib::pdl_launch_dependents();
         if (cluster > 1) {                               // the cluster barriers below count every thread
@@ -373,11 +355,11 @@ bulk_gemv_kernel(const GemvParams p) {
     }
 
     IB_GT(2);
-    int s = 0, st = st0, st_from = st0;
+    int s = 0, st = 0;
     uint32_t round = 0;
-    int tile = tile0;
-    for (int i = 0; i < n_iter; i++) {
-        const int64_t k0 = int64_t(s_begin + st) * KC;
+    int64_t tile = group;
+    for (int64_t i = 0; i < n_iter; i++) {
+        const int64_t k0 = (s_begin + st) * KC;
         IB_GT(4 + 4 * int(i));
         if (!hoist) {
             // activations of this warp's chunks: independent of the weights, so they are loaded before the wait
@@ -411,14 +393,13 @@ bulk_gemv_kernel(const GemvParams p) {
         if (lane == 0) mbar_arrive(empty_bar(s));
         IB_GT(6 + 4 * int(i));
         if (++s == NS) { s = 0; round++; }
-        if (++st != spt && !(EVEN && i == n_iter - 1)) continue;
-        const int summed = st - st_from;                 // stages of this tile that this CTA has summed
-        st = st_from = 0;
+        if (++st != spt) continue;
+        st = 0;
 
         // ---------------------------------------------------------------- the tile is complete
-        const int this_tile = tile;
-        tile += tile_step;
-        const int64_t n0 = int64_t(this_tile) * ROWS;
+        const int64_t this_tile = tile;
+        tile += p.groups;
+        const int64_t n0 = this_tile * ROWS;
         asm volatile("bar.sync 1, 256;" ::: "memory");   // the previous tile's sums have been read (consumers only)
 #pragma unroll
         for (int nt = 0; nt < NT; nt++) {
@@ -435,30 +416,7 @@ bulk_gemv_kernel(const GemvParams p) {
             for (int wi = 0; wi < WARPS; wi++) v += red[wi][ant][col][r];
         }
         bool writer = true;
-        if (EVEN && summed != spt) {
-            // A part of a tile. Its sums go to the workspace; the CTA that completes the tile's count adds all parts in
-            // ascending order of K, so that the result does not depend on which one that is.
-            if (active) __stcg(p.parts + (int(blockIdx.x) * 2 + (this_tile == tile0 ? 0 : 1)) * PART_FLOATS + threadIdx.x, v);
-            __threadfence();
-            asm volatile("bar.sync 1, 256;" ::: "memory");
-            if (threadIdx.x == 0) {
-                last_here = atomicAdd(p.arrived + this_tile, unsigned(summed)) + unsigned(summed) == unsigned(spt);
-                if (last_here) p.arrived[this_tile] = 0u;
-                __threadfence();
-            }
-            asm volatile("bar.sync 1, 256;" ::: "memory");
-            writer = last_here != 0;
-            if (writer && active) {
-                const int u0 = this_tile * total_stages, border = p.longer * (p.run + 1);
-                int c = u0 < border ? u0 / (p.run + 1) : p.longer + (u0 - border) / p.run;      // the CTA whose run holds stage u0
-                int begin = c * p.run + min(c, p.longer);
-                // (a part is its CTA's first tile's, unless the run begins before this tile)
-                v = 0.0f;
-                for (; begin < u0 + total_stages; begin += p.run + (c < p.longer ? 1 : 0), c++)
-                    v += __ldcg(p.parts + (c * 2 + (begin < u0 ? 1 : 0)) * PART_FLOATS + threadIdx.x);
-            }
-        }
-        if (!EVEN && cluster > 1) {
+        if (cluster > 1) {
             cg::cluster_group cl = cg::this_cluster();
             if (active) part[ant][col][r] = v;
             cl.sync();
@@ -479,7 +437,7 @@ bulk_gemv_kernel(const GemvParams p) {
         if constexpr (EPI == 2) {
             if (r < 8) {
                 const float gate = v, up = part[ant][col][r + 8];
-                const int64_t f = int64_t(this_tile) * 8 + r;
+                const int64_t f = this_tile * 8 + r;
                 if (f < N / 2) out[int64_t(m) * (N / 2) + f] = ib::from_f32<TOut>(gate / (1.0f + expf(-gate)) * up);
             }
         } else {
@@ -498,18 +456,17 @@ int launch(const GemvParams& p, int out_dtype, int epi, int grid_ctas, cudaStrea
     const dim3 grid{unsigned(grid_ctas), 1u, 1u};
     const dim3 block{THREADS, 1u, 1u};
     const unsigned cl = unsigned(p.cluster);
-#define IB_GEMV_LAUNCH_(EPI_, T_, NWS_, EVEN_)                                                                     \
+#define IB_GEMV_LAUNCH_(EPI_, T_, NWS_)                                                                            \
     do {                                                                                                           \
         static ib::PerDevice allowed;                                                                              \
-        if (const int rc = ib::allow_smem(allowed, "linear_skinny_bulk", bulk_gemv_kernel<NT, EPI_, T_, NWS_, EVEN_>, RING_BYTES + NW_BYTES)) return rc; \
-        return ib::launch("linear_skinny_bulk", bulk_gemv_kernel<NT, EPI_, T_, NWS_, EVEN_>, grid, block,          \
+        if (const int rc = ib::allow_smem(allowed, "linear_skinny_bulk", bulk_gemv_kernel<NT, EPI_, T_, NWS_>, RING_BYTES + NW_BYTES)) return rc; \
+        return ib::launch("linear_skinny_bulk", bulk_gemv_kernel<NT, EPI_, T_, NWS_>, grid, block,                 \
                           size_t(RING_BYTES) + (NWS_ ? size_t(NW_BYTES) : 0), stream, cl, p);                      \
     } while (0)
 #define IB_GEMV_LAUNCH(EPI_, T_)                                                                                   \
     do {                                                                                                           \
-        if (p.even) IB_GEMV_LAUNCH_(EPI_, T_, false, true);                                                        \
-        if (NT == 1 && p.norm_w && p.nw_smem) IB_GEMV_LAUNCH_(EPI_, T_, true, false);                              \
-        IB_GEMV_LAUNCH_(EPI_, T_, false, false);                                                                   \
+        if (NT == 1 && p.norm_w && p.nw_smem) IB_GEMV_LAUNCH_(EPI_, T_, true);                                     \
+        IB_GEMV_LAUNCH_(EPI_, T_, false);                                                                          \
     } while (0)
     if (epi == 2) {
         if (out_dtype != IB_BF16) return ib::fail(IB_ERR_ARG, "linear_skinny_bulk: the SwiGLU epilogue writes bfloat16");
@@ -524,50 +481,6 @@ int launch(const GemvParams& p, int out_dtype, int epi, int grid_ctas, cudaStrea
 #undef IB_GEMV_LAUNCH
 #undef IB_GEMV_LAUNCH_
     return ib::fail(IB_ERR_ARG, "linear_skinny_bulk: unknown output dtype %d", out_dtype);
-}
-
-// K of a tile in as few stages as the ring allows (a whole row for K up to KC_MAX), since the cost of a stage (its copies, the barrier
-// round trip) does not depend on its size. cluster 0: chosen here. even < 0: chosen here (where `can`), 0: never, else the number
-// of stages that a tile's K is cut into.
-Deal deal_out(int64_t N, int64_t K, int cluster, int even, bool can, int sms) {
-    Deal d = {};
-    const int64_t tiles = (N + ROWS - 1) / ROWS, places = int64_t(IB_GEMV_CTAS_PER_SM) * sms;
-    const int64_t least = (K + KC_MAX - 1) / KC_MAX;
-    if (cluster == 0) {
-        // Share a tile among CTAs while the tiles alone leave SMs idle and every CTA keeps at least three stages of K
-        // (measured on B200 for K = 8960: 10.8 us alone, 8.9 us in pairs, 14.4 us in fours; clusters of three or six
-        // run slower still).
-        cluster = 1;
-        while (cluster < 8 && tiles * cluster < 2LL * sms && least >= 6 * cluster) cluster *= 2;
-    }
-    auto stage_of = [&](int64_t n) { return ((K + n - 1) / n + 63) / 64 * 64; };       // elements of K in each of n equal stages
-    auto rounds = [&](int64_t work) { return (work + places - 1) / places; };
-    int64_t n_stages = (least + cluster - 1) / cluster * cluster;                      // the same number of stages for every CTA of a cluster
-    if (!can) even = 0;
-    if (even < 0) {
-        // Equal runs where whole tiles would give some CTA at least 4,000 elements of K more (of 16 rows): the parts' meeting costs what
-        // reading those does. us with whole tiles -> with runs at 8 rows, and elements saved: 5120 x 13824 34.1 -> 26.9 (12,288),
-        // 3584 x 18944 31.8 -> 27.1 (5,888), 2560 x 9728 17.7 -> 14.6 (4,096), 6400 x 8192 23.6 -> 22.7 (4,224), but 5120 x 5120
-        // 14.8 -> 15.8 (3,840), 4960 x 4096 11.2 -> 13.2 (2,816), 1536 x 8960 8.0 -> 9.3 (1,536).
-        const int64_t whole = rounds(tiles * cluster) * (n_stages / cluster) * stage_of(n_stages);
-        even = whole - rounds(tiles * least) * stage_of(least) >= 4000 ? int(least) : 0;
-    }
-    if (even > 0) { n_stages = even; cluster = 1; }
-    d.tiles = int(tiles); d.cluster = cluster; d.even = even > 0;
-    d.kc = int(stage_of(n_stages));
-    d.ns = RING_BYTES / (ROWS * (d.kc * 2 + 64));
-    if (d.ns > NS_MAX) d.ns = NS_MAX;
-    d.n_stages = int((K + d.kc - 1) / d.kc);
-    d.per_cta = (d.n_stages + cluster - 1) / cluster;
-    // Two CTAs fit an SM; with more tiles than that, a CTA walks over several and its ring never drains between them.
-    d.groups = int(cluster > 1 || tiles < places ? tiles : places);
-    d.grid = d.groups * cluster;
-    if (d.even) {
-        const int64_t units = tiles * d.n_stages;
-        d.grid = int(units < places ? units : places);
-        d.run = int(units / d.grid); d.longer = int(units % d.grid);
-    }
-    return d;
 }
 
 }  // namespace
@@ -586,8 +499,7 @@ IB_EXPORT int ib_linear_skinny_bulk_limits(int* max_rows, int* max_fused_norm_k)
 
 IB_EXPORT int ib_linear_skinny_bulk(const void* x, const float* norm_w, float norm_eps, const void* w, const float* bias, const float* residual, void* out,
                                     int64_t M, int64_t N, int64_t K, int out_dtype, int epi, int cluster, int sm_count,
-                                    int* status, float* parts, int64_t n_parts, unsigned int* arrived, int64_t n_arrived, int even,
-                                    cudaStream_t stream) {
+                                    int* status, cudaStream_t stream) {
     if (M <= 0 || N <= 0) return IB_OK;
     if (M > 16) return ib::fail(IB_ERR_ARG, "linear_skinny_bulk: at most 16 rows, got %lld", (long long)M);
     if (K <= 0 || K % 8) return ib::fail(IB_ERR_ARG, "linear_skinny_bulk: K = %lld must be a positive multiple of 8", (long long)K);
@@ -600,22 +512,32 @@ IB_EXPORT int ib_linear_skinny_bulk(const void* x, const float* norm_w, float no
     const int64_t tiles = (N + ROWS - 1) / ROWS;
     if (tiles > 0x7fffffffLL / 8) return ib::fail(IB_ERR_ARG, "linear_skinny_bulk: N too large");
     const int sms = sm_count > 0 ? sm_count : 148;
-    if (cluster != 0 && cluster != 1 && cluster != 2 && cluster != 4 && cluster != 8) return ib::fail(IB_ERR_ARG, "linear_skinny_bulk: cluster must be 1, 2, 4 or 8");
-    // tiles shared by CTAs: with a workspace, and stages that an int counts
-    const bool can = !norm_w && tiles * 64 < (1LL << 30) && K < (1LL << 16) && parts && arrived && n_arrived >= tiles &&
-                     n_parts >= 2LL * IB_GEMV_CTAS_PER_SM * sms * PART_FLOATS;
-    const Deal d = deal_out(N, K, cluster, even, can, sms);
+    // A stage holds ROWS rows of kc elements: K in as few equal stages as the ring allows (a whole row for K up to
+    // KC_MAX), since the cost of a stage (its copies, the barrier round trip) does not depend on its size.
+    int64_t n_stages = (K + KC_MAX - 1) / KC_MAX;
+    if (cluster == 0) {
+        // Share a tile among CTAs while the tiles alone leave SMs idle and every CTA keeps at least three stages of K
+        // (measured on B200 for K = 8960: 10.8 us alone, 8.9 us in pairs, 14.4 us in fours; clusters of three or six
+        // run slower still).
+        cluster = 1;
+        while (cluster < 8 && tiles * cluster < 2LL * sms && n_stages >= 6 * cluster) cluster *= 2;
+    }
+    if (cluster != 1 && cluster != 2 && cluster != 4 && cluster != 8) return ib::fail(IB_ERR_ARG, "linear_skinny_bulk: cluster must be 1, 2, 4 or 8");
+    n_stages = (n_stages + cluster - 1) / cluster * cluster;     // the same number of stages for every CTA of a cluster
+    const int kc = int(((K + n_stages - 1) / n_stages + 63) / 64 * 64);
+    int ns = RING_BYTES / (ROWS * (kc * 2 + 64));
+    if (ns > NS_MAX) ns = NS_MAX;
     GemvParams p;
     p.x = (const bf16*)x; p.norm_w = norm_w; p.eps = norm_eps; p.w = (const bf16*)w; p.bias = bias; p.residual = residual; p.out = out;
-    p.M = int(M); p.N = N; p.K = K; p.cluster = d.cluster; p.status = status; p.tiles = d.tiles; p.kc = d.kc; p.ns = d.ns;
-    p.n_stages = d.n_stages; p.per_cta = d.per_cta;
+    p.M = int(M); p.N = N; p.K = K; p.cluster = cluster; p.status = status; p.tiles = tiles; p.kc = kc; p.ns = ns;
     // gate the ring's second slot where the whole GPU's rings fill at once (a CTA per half SM) and a tile is one stage
-    p.gate_ring = (d.n_stages == 1 && d.cluster == 1 && tiles >= 2LL * sms) ? 1 : 0;
+    p.gate_ring = (n_stages == 1 && cluster == 1 && tiles >= 2LL * sms) ? 1 : 0;
     p.nw_smem = norm_w ? 1 : 0;
-    p.groups = d.groups;
-    p.even = d.even; p.run = d.run; p.longer = d.longer;
-    p.parts = parts; p.arrived = arrived;
-    const int grid_ctas = d.grid;
+    // Two CTAs fit an SM; with more tiles than that, a CTA walks over several and its ring never drains between them.
+    constexpr int64_t PER_SM = IB_GEMV_CTAS_PER_SM;
+    int64_t groups = cluster > 1 ? tiles : (tiles < PER_SM * sms ? tiles : PER_SM * sms);
+    p.groups = int(groups);
+    const int grid_ctas = int(groups) * cluster;
     if (M <= 8) return launch<1>(p, out_dtype, epi, grid_ctas, stream);
     return launch<2>(p, out_dtype, epi, grid_ctas, stream);
 }

@@ -30,7 +30,6 @@ class DeviceState:
         self._workspace = torch.empty(0, dtype=torch.float32, device=device)
         self._counters = torch.zeros(4096, dtype=torch.int32, device=device)
         self._retired = []
-        self.parts = torch.empty(2 * 2 * 256 * self.sm_count, dtype=torch.float32, device=device)     # the streaming product's shared tiles
 
     def workspace(self, n_floats: int) -> torch.Tensor:
         if self._workspace.numel() < n_floats:
@@ -194,12 +193,11 @@ def skinny_limits():
 def linear_skinny(x: torch.Tensor, w: torch.Tensor, bias: Optional[torch.Tensor] = None,
                   residual: Optional[torch.Tensor] = None, out_dtype: torch.dtype = torch.bfloat16,
                   out: Optional[torch.Tensor] = None, swiglu: bool = False, cluster: int = 0,
-                  norm_weight: Optional[torch.Tensor] = None, norm_eps: float = 0.0, even: int = -1) -> Optional[torch.Tensor]:
+                  norm_weight: Optional[torch.Tensor] = None, norm_eps: float = 0.0) -> Optional[torch.Tensor]:
     """The decode kernel: x [M <= 16, K] against w [N, K], weights streamed once; same epilogues as gemm_tc.
     With ``norm_weight`` x is the float32 residual stream and is RMS-normalised inside the kernel (rows up to
     ``skinny_limits()[1]`` long).
-    cluster: CTAs sharing one tile's K range (0 = chosen by the kernel). even: the number of stages that a tile's K is cut into where equal
-    runs of stages are dealt out (-1 = chosen by the kernel, 0 = never)."""
+    cluster: CTAs sharing one tile's K range (0 = chosen by the kernel). The kernel needs no scratch: calls may run on any streams at once."""
     fused = norm_weight is not None
     _check(x, "x", torch.float32 if fused else torch.bfloat16)
     _check(w, "w", torch.bfloat16)
@@ -227,9 +225,9 @@ def linear_skinny(x: torch.Tensor, w: torch.Tensor, bias: Optional[torch.Tensor]
     st = device_state(x.device)
     epi = 2 if swiglu else (1 if residual is not None else 0)
     f = _fn("gemvb", "ib_linear_skinny_bulk", [c_void_p, c_void_p, c_float] + [c_void_p] * 4 + [c_int64] * 3 + [c_int] * 4 +
-            [c_void_p] * 2 + [c_int64, c_void_p, c_int64, c_int, c_void_p])
+            [c_void_p] * 2)
     _call(f, x.data_ptr(), _ptr(norm_weight), float(norm_eps), w.data_ptr(), _ptr(bias), _ptr(residual), out.data_ptr(),
-          M, N, K, dtype_code(out_dtype), epi, int(cluster), st.sm_count, st.status.data_ptr(), st.parts.data_ptr(), st.parts.numel(), st._counters.data_ptr(), st._counters.numel(), int(even), _stream())
+          M, N, K, dtype_code(out_dtype), epi, int(cluster), st.sm_count, st.status.data_ptr(), _stream())
     return out
 
 
