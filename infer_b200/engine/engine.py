@@ -575,10 +575,11 @@ class Engine:
         return StepResult(out, ran)
 
     def check_status(self) -> None:
-        """Synchronises and raises if a kernel met a page index or token id out of range."""
+        """Synchronises and raises if a kernel met a page index or token id out of range, or gave up a wait. The engine can be used on."""
         code = int(self.status.item())
         if code:
-            self.status.zero_()
+            from ..fast_ops import clear_failure
+            clear_failure(self.rt.device)
             what = {1: "a token id outside the table", 2: "a cache write through an invalid page",
                     3: "a cache read through an invalid page", 101: "a tensor-core GEMM's copy wait ran out",
                     102: "a tensor-core GEMM's operand wait ran out", 103: "a tensor-core GEMM's accumulator wait ran out",

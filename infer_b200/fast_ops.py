@@ -4,7 +4,7 @@ when the kernel does not take the shape, in which case the caller uses the plain
 Kernels that need scratch memory (split-K partial tiles, flash-decoding partial results) share one
 workspace per device, allocated once and grown on demand; calls on one stream run in order, so they
 may share it (a registered side stream has its own).  One status word per device collects failures that kernels report (a page index out of
-range, a bounded wait that ran out).
+range, a bounded wait that ran out); ``clear_failure`` takes it back, and with it the counts that a kernel which gave up has left.
 """
 from __future__ import annotations
 
@@ -46,6 +46,12 @@ class DeviceState:
             self._retired.append(self._counters)
             self._counters = torch.zeros(max(n, 4096), dtype=torch.int32, device=self.device)
         return self._counters
+
+    def clear_counts(self) -> None:
+        """Zeroes the counters, those that captured graphs may still point at among them, where they lie."""
+        for t in [self._counters] + self._retired:
+            if t.dtype == torch.int32:
+                t.zero_()
 
 
 _STATES: Dict[torch.device, DeviceState] = {}
@@ -90,6 +96,19 @@ def register_side_stream(stream: "torch.cuda.Stream") -> None:
         st = DeviceState(device)
         st.status = device_state(device).status
         _SIDE_STATES[key] = st
+
+
+def clear_failure(device) -> None:
+    """Makes a device usable again after a kernel has raised its status word: a kernel whose wait ran out leaves its tiles' counts short, and
+    the next one that counts on them would add sums that are not there yet, or none. Waits for the device before and after."""
+    device = torch.device(device)
+    if device.index is None:
+        device = torch.device("cuda", torch.cuda.current_device())
+    torch.cuda.synchronize(device)
+    for st in [s for d, s in _STATES.items() if d == device] + [s for (d, _), s in _SIDE_STATES.items() if d == device]:
+        st.status.zero_()
+        st.clear_counts()
+    torch.cuda.synchronize(device)
 
 
 def device_state(device) -> DeviceState:
