@@ -937,6 +937,14 @@ IB_EXPORT int ib_rope_kv_write(const void* qkv, const float* cos_t, const float*
 
 // The largest head size the plain attention kernel takes (parts ask at construction, so that a configuration the
 // kernels cannot serve is refused when the model is built, not at its first step).
+// What this thread may call while a stream is being captured (cudaStreamCaptureMode); returns what it was, or an error code below zero.
+IB_EXPORT int ib_thread_capture_mode(int mode) {
+    cudaStreamCaptureMode m = cudaStreamCaptureMode(mode);
+    const cudaError_t e = cudaThreadExchangeStreamCaptureMode(&m);
+    if (e != cudaSuccess) return ib::fail(IB_ERR_CUDA, "thread_capture_mode: %s", cudaGetErrorString(e));
+    return int(m);
+}
+
 IB_EXPORT int ib_attention_plain_max_head_dim() { return 2 * AT; }
 
 IB_EXPORT int ib_attention_plain(const void* q, const void* k_cache, const void* v_cache, const int* block_table,

@@ -12,6 +12,7 @@ import ctypes
 import functools
 import heapq
 import os
+import threading
 from typing import Dict, Optional
 
 import torch
@@ -20,16 +21,36 @@ from . import ops
 from .ops import KernelError, _call, _check, _fn, _ptr, _stream, c_float, c_int, c_int64, c_void_p, dtype_code
 
 
+def _stream_without_capture(device) -> "torch.cuda.Stream":
+    """A stream that nothing is being captured on (torch's streams come round again: a new one may be one that a caller captures on)."""
+    for _ in range(64):
+        stream = torch.cuda.Stream(device)
+        with torch.cuda.stream(stream):
+            if not torch.cuda.is_current_stream_capturing():
+                return stream
+    raise KernelError("every stream of the device is being captured")
+
+
 class DeviceState:
-    """Per-device scratch shared by the fast kernels."""
+    """Per-device scratch shared by the fast kernels. It may come into being in the middle of a capture: its words are zeroed on a stream of
+    its own, before any caller has them, since a zeroing that a graph records is none until the first replay and one too many in
+    each replay after it."""
 
     def __init__(self, device: torch.device):
         self.device = device
-        self.status = torch.zeros(1, dtype=torch.int32, device=device)
         self.sm_count = torch.cuda.get_device_properties(device).multi_processor_count
-        self._workspace = torch.empty(0, dtype=torch.float32, device=device)
-        self._counters = torch.zeros(4096, dtype=torch.int32, device=device)
         self._retired = []
+        mode = _fn("plain", "ib_thread_capture_mode", [c_int])
+        before = mode(2)                               # (relaxed: a capture elsewhere does not forbid this thread to zero and to wait)
+        try:
+            with torch.cuda.stream(_stream_without_capture(device)):
+                self.status = torch.zeros(1, dtype=torch.int32, device=device)
+                self._workspace = torch.empty(0, dtype=torch.float32, device=device)
+                self._counters = torch.zeros(4096, dtype=torch.int32, device=device)
+                torch.cuda.current_stream(device).synchronize()
+        finally:
+            if before >= 0:
+                mode(before)
 
     def workspace(self, n_floats: int) -> torch.Tensor:
         if self._workspace.numel() < n_floats:
@@ -55,6 +76,7 @@ class DeviceState:
 
 
 _STATES: Dict[torch.device, DeviceState] = {}
+_STATES_LOCK = threading.Lock()
 _SIDE_STATES: Dict[tuple, DeviceState] = {}        # (device, raw handle of a registered side stream) -> its scratch
 
 
@@ -121,7 +143,10 @@ def device_state(device) -> DeviceState:
             return side
     st = _STATES.get(device)
     if st is None:
-        st = _STATES[device] = DeviceState(device)
+        with _STATES_LOCK:                             # (one status word per device, whichever threads ask first)
+            st = _STATES.get(device)
+            if st is None:
+                st = _STATES[device] = DeviceState(device)
     return st
 
 

@@ -42,3 +42,27 @@ def test_counts_are_cleared_with_the_status_word():
     eng.add_request("r")
     assert torch.isfinite(eng.step([StepEntry("r", H.random_ids(cfg, 8, 1), [7])])).all()
     eng.check_status()
+
+
+@pytest.mark.parametrize("mode", ["global", "thread_local", "relaxed"])
+def test_a_device_first_met_inside_a_capture(monkeypatch, mode):
+    """The status word and the counters are there, and zero, before the first replay, and no replay touches them."""
+    from infer_b200 import fast_ops, ops
+    x, w = torch.randn(3, 1536, device=DEV), torch.randn(1536, 1536, device=DEV)
+    want = ops.linear_plain(x, w)
+    torch.cuda.synchronize()
+    monkeypatch.setattr(fast_ops, "_STATES", {})
+    graph, out = torch.cuda.CUDAGraph(), torch.empty_like(want)
+    with torch.cuda.graph(graph, capture_error_mode=mode):
+        ops.linear_plain(x, w, out=out)
+    assert len(fast_ops._STATES) == 1
+    st = fast_ops.device_state(DEV)
+    assert int(st.status) == 0 and not st._counters.any()
+    st.status.fill_(7)
+    st._counters.fill_(2)
+    for _ in range(2):
+        out.zero_()
+        graph.replay()
+        torch.cuda.synchronize()
+        assert torch.equal(out, want)
+    assert int(st.status) == 7 and int(st._counters.min()) == 2
