@@ -143,16 +143,43 @@ __device__ __forceinline__ uint32_t map_cluster(uint32_t local_smem, uint32_t ra
     return remote;
 }
 
-// One result by plain multiply-adds.
-__device__ __noinline__ float plain_product(const float* x, const float* w, int64_t K) {
+// One result by plain multiply-adds, in the order of linear_f32.cu: blocks of 32 elements of K, even and odd k apart, then the blocks' sums
+// in ascending order. A warp takes 16 blocks at a time through its shared memory (two lanes a block, blocks 34 floats apart: no two lanes
+// meet in a bank). Every lane has the result.
+constexpr int PLAIN_BLOCKS = 16, PLAIN_PITCH = 34, PLAIN_FLOATS = 2 * PLAIN_BLOCKS * PLAIN_PITCH;
+__device__ __forceinline__ float plain_product(const float* x, const float* w, int64_t K, float* mem, int lane) {
     float total = 0.0f;
-    for (int64_t k0 = 0; k0 < K; k0 += 32) {
-        float block = 0.0f;
-        for (int64_t k = k0; k < K && k < k0 + 32; k++) block = fmaf(x[k], w[k], block);
-        total += block;
+    float* mem_x = mem + PLAIN_BLOCKS * PLAIN_PITCH;
+    for (int64_t k0 = 0; k0 < K; k0 += PLAIN_BLOCKS * 32) {
+        __syncwarp();                                         // the blocks before have been read
+#pragma unroll
+        for (int b = 0; b < PLAIN_BLOCKS; b++) {
+            const int64_t k = k0 + b * 32 + lane;
+            mem[b * PLAIN_PITCH + lane] = k < K ? w[k] : 0.0f;
+            mem_x[b * PLAIN_PITCH + lane] = k < K ? x[k] : 0.0f;
+        }
+        __syncwarp();
+        const int at = (lane >> 1) * PLAIN_PITCH + (lane & 1);
+        float sum = 0.0f;
+#pragma unroll
+        for (int j = 0; j < 32; j += 2) sum = fmaf(mem[at + j], mem_x[at + j], sum);
+        sum += __shfl_xor_sync(0xffffffffu, sum, 1);
+        if (__any_sync(0xffffffffu, isnan(sum))) return __int_as_float(0x7fffffff);
+#pragma unroll
+        for (int b = 0; b < PLAIN_BLOCKS; b++) total += __shfl_sync(0xffffffffu, sum, 2 * b);
     }
     return total;
 }
+
+// Whether a row holds a NaN (asked by a whole warp).
+__device__ __forceinline__ bool has_nan(const float* row, int64_t K, int lane) {
+    bool found = false;
+#pragma unroll 8
+    for (int64_t k = lane; k < K; k += 32) found |= isnan(row[k]);
+    return __any_sync(0xffffffffu, found) != 0;
+}
+
+static_assert(WARPS * PLAIN_FLOATS * 4 <= 2 * Cfg<16>::STAGE_BYTES, "the warps' blocks lie in the operand stages");
 
 template <int NT, bool VEC>
 __global__ void __launch_bounds__(THREADS, 1)
@@ -160,7 +187,7 @@ linear32_tc_kernel(const Params p) {
     using C = Cfg<NT>;
     extern __shared__ uint8_t smem_raw[];
     __shared__ __align__(8) uint64_t bars[4];    // full[2], done[2]
-    __shared__ uint32_t slot, failed;
+    __shared__ uint32_t slot, failed, again;
     uint8_t* stages = smem_raw + ((1024u - (smem_u32(smem_raw) & 1023u)) & 1023u);
     // [own column][128 features] the groups' sum so far, or, where a tile is shared, [group][own column][128 features] each group's
     float* recv = reinterpret_cast<float*>(stages + 2 * C::STAGE_BYTES);
@@ -177,7 +204,7 @@ linear32_tc_kernel(const Params p) {
 
     if (tid == 0) {
         for (int i = 0; i < 2; i++) { mbar_init(full(i), WARPS); mbar_init(done(i), 1); }
-        failed = 0;
+        failed = again = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
     if (warp == WARPS) {
@@ -384,7 +411,10 @@ linear32_tc_kernel(const Params p) {
                 if (c < own_cols && m < p.M) {
                     float v = 0.0f;
                     for (int h = 0; h < slots; h++) v += recv[(h * own_cols + c) * BM + (tid & (BM - 1))];
-                    if (!isfinite(v)) v = plain_product(p.x + m * p.K, p.w + n * p.K, p.K);
+                    if (!isfinite(v)) {
+                        *reinterpret_cast<volatile uint32_t*>(&again) = 1;
+                        continue;
+                    }
                     if (p.bias) v += bias;
                     if (p.residual) v += res[i];
                     p.out[m * p.N + n] = v;
@@ -397,6 +427,41 @@ linear32_tc_kernel(const Params p) {
     if (warp == WARPS) {
         tc_fence_after();
         tmem_dealloc(tmem, C::TMEM_COLS);
+    } else if (*reinterpret_cast<volatile uint32_t*>(&again)) {
+        // Results that are not finite, by multiply-adds: a warp takes 8 of the 128 features of every column, so that a column whose
+        // token holds a NaN or an infinity is spread over all warps; where it holds a NaN, all of the column's results are known at once.
+        // (One row that holds a NaN or an infinity, calls by themselves: 17920 x 1536, 1, 16 and 512 rows 45 and 69, 46 and 68, 292 and 320 us,
+        // all finite 44, 43, 285; 1536 x 8960, 16 rows 43 and 192 against 34. A thread for each of them took 204, 204, 456 and 827.)
+        const int f = warp * (BM / WARPS) + (lane & 7);
+        const int64_t nf = n0 + f;
+        float* mem = reinterpret_cast<float*>(stages) + warp * PLAIN_FLOATS;           // (every MMA that read the stages has been waited for)
+        for (int c0 = 0; c0 < own_cols; c0 += 4) {
+            const int c = c0 + (lane >> 3);
+            const int64_t m = m0 + rank * own_cols + c;
+            float v = 0.0f;
+            if (c < own_cols && m < p.M && nf >= n_first)
+                for (int h = 0; h < slots; h++) v += recv[(h * own_cols + c) * BM + f];
+            const bool mine = !isfinite(v);
+            const uint32_t todo = __ballot_sync(0xffffffffu, mine);
+            for (int q = 0; q < 4; q++) {
+                uint32_t here = (todo >> (8 * q)) & 0xffu;
+                const float* row = p.x + (m0 + rank * own_cols + c0 + q) * p.K;
+                if ((here & (here - 1)) && has_nan(row, p.K, lane)) {
+                    if (mine && (lane >> 3) == q) v = __int_as_float(0x7fffffff);
+                    continue;
+                }
+                for (; here; here &= here - 1) {
+                    const int j = __ffs(here) - 1;
+                    const float total = plain_product(row, p.w + (n0 + warp * (BM / WARPS) + j) * p.K, p.K, mem, lane);
+                    if (lane == 8 * q + j) v = total;
+                }
+            }
+            if (mine) {
+                if (p.bias) v += p.bias[nf];
+                if (p.residual) v += p.residual[m * p.N + nf];
+                p.out[m * p.N + nf] = v;
+            }
+        }
     }
 }
 

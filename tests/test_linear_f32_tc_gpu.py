@@ -89,3 +89,27 @@ def test_captured():
         graph.replay()
         torch.cuda.synchronize()
         assert torch.equal(out, want)
+
+
+# one group, clusters of two and of eight, the last tile of features a repeat of the one before; every tile of tokens
+@pytest.mark.parametrize("N,K", [(19000, 1088), (2048, 1536), (1025, 1031), (1536, 8960)])
+@pytest.mark.parametrize("M", [1, 5, 20, 70])
+def test_not_finite_has_the_bits_of_the_multiply_adds(M, N, K):
+    """Rows with a NaN, infinities of one and of both signs, elements that are beyond every bfloat16 number (their results are finite or overflow);
+    with bias and with the residual in place."""
+    from infer_b200 import ops
+    x, w, b, r = _operands(M, N, K, M + N)
+    clean = ops.linear_plain(x, w, b, r)
+    x[0, K - 1] = float("nan")
+    if M > 1:
+        x[1, 3], x[2, 7], x[2, 900], x[3, 40:60] = float("inf"), float("inf"), -float("inf"), 3.4e38
+    w[N - 1, 5], w[130, 0], w[700, 1] = float("nan"), -float("inf"), 3.4028e38
+    got, plain = ops.linear_plain(x, w), ops.linear_plain(x, w, kind=3)
+    assert torch.equal(torch.isnan(got), torch.isnan(plain))
+    again = (x.abs().nan_to_num(4e38).amax(1) > 3e38)[:, None] | (w.abs().nan_to_num(4e38).amax(1) > 3e38)[None, :]
+    assert torch.equal(torch.where(again, got, 0.0).nan_to_num(), torch.where(again, plain, 0.0).nan_to_num())
+    full, own = ops.linear_plain(x, w, b, r), r.clone()
+    assert torch.equal(torch.nan_to_num(full), torch.nan_to_num((got + b) + r))
+    assert torch.equal(torch.nan_to_num(ops.linear_plain(x, w, b, own, out=own)), torch.nan_to_num(full)) and torch.equal(torch.isnan(own), torch.isnan(full))
+    kept = [n for n in range(N) if n not in (N - 1, 130, 700)]
+    assert torch.equal(full[4:, kept], clean[4:, kept])
