@@ -503,13 +503,16 @@ attention_staged_kernel(const float* __restrict__ q, const float* k_cache, const
         }
         rows[buf][tid] = row;
     };
-    // a warp copies whole rows, its lanes their 16-byte pieces; zeros where there is no row
-    auto copy = [&](float* dst, int pitch, const float* src, int dim, int buf) {
+    // the keys of a tile that are looked at: from the first to the last one seen
+    auto first_of = [&](int tile) { return (tile < keep_end ? tile : max(lo, tile)) - tile; };
+    auto last_of = [&](int tile) { return min(pos, tile + AT - 1) - tile; };
+    // a warp copies whole rows from `first` to `last`, its lanes their 16-byte pieces; zeros where there is no row
+    auto copy = [&](float* dst, int pitch, const float* src, int dim, int buf, int first, int last) {
         const int wid = int(threadIdx.x) >> 5;
         for (int u = lane * 4; u < dim; u += 128) {
-            uint32_t to = uint32_t(__cvta_generic_to_shared(dst)) + uint32_t(wid * pitch + u) * 4u;
+            uint32_t to = uint32_t(__cvta_generic_to_shared(dst)) + uint32_t((first + wid) * pitch + u) * 4u;
 #pragma unroll 4
-            for (int key = wid; key < AT; key += WARPS, to += uint32_t(WARPS * pitch) * 4u) {
+            for (int key = first + wid; key <= last; key += WARPS, to += uint32_t(WARPS * pitch) * 4u) {
                 const int64_t row = rows[buf][key];
                 copy16_async(to, src + (row < 0 ? 0 : row) * dim + u, row >= 0);
             }
@@ -526,11 +529,11 @@ attention_staged_kernel(const float* __restrict__ q, const float* k_cache, const
     if (ahead <= pos) find(ahead, 1);
     for (int d = threadIdx.x; d < S * H * head_dim; d += AT * S) qs[d] = q[(t * n_heads + h_block) * head_dim + d];
     __syncthreads();
-    copy(keys, k_pitch, k_cache, head_dim, 0);
+    copy(keys, k_pitch, k_cache, head_dim, 0, first_of(tile), last_of(tile));      // (all of a short context: what is not looked at is not copied)
     commit();
-    copy(values, v_dim, v_cache, v_dim, 0);
+    copy(values, v_dim, v_cache, v_dim, 0, first_of(tile), last_of(tile));
     commit();
-    if (ahead <= pos) copy(keys + AT * k_pitch, k_pitch, k_cache, head_dim, 1);
+    if (ahead <= pos) copy(keys + AT * k_pitch, k_pitch, k_cache, head_dim, 1, 0, AT - 1);
     commit();
     float m[H], l[H], acc0[H], acc1[H];
 #pragma unroll
@@ -596,7 +599,7 @@ attention_staged_kernel(const float* __restrict__ q, const float* k_cache, const
             acc0[h] *= corr[h];
             acc1[h] *= corr[h];
         }
-        const int jj0 = (tile < keep_end ? tile : max(lo, tile)) - tile, jj1 = min(pos, tile + AT - 1) - tile;
+        const int jj0 = first_of(tile), jj1 = last_of(tile);
         const float *v0 = values + (tid < v_dim ? tid : 0), *v1 = values + (tid + AT < v_dim ? tid + AT : 0);
         const float* pj = ps + sub * AT * H;
 #pragma unroll 16
@@ -613,13 +616,14 @@ attention_staged_kernel(const float* __restrict__ q, const float* k_cache, const
                 for (int h = 0; h < H; h++) acc1[h] = fmaf(pj[jj * H + h], a, acc1[h]);
             }
         }
+        if (ahead > pos) break;
         __syncthreads();                                               // keys, values and rows of this tile have been read
         const int after = next(ahead);
-        if (ahead <= pos) copy(values, v_dim, v_cache, v_dim, buf ^ 1);
+        copy(values, v_dim, v_cache, v_dim, buf ^ 1, 0, AT - 1);
         commit();
         if (after <= pos) find(after, buf);
         __syncthreads();
-        if (after <= pos) copy(keys + buf * AT * k_pitch, k_pitch, k_cache, head_dim, buf);
+        if (after <= pos) copy(keys + buf * AT * k_pitch, k_pitch, k_cache, head_dim, buf, 0, AT - 1);
         commit();
         tile = ahead;
         ahead = after;
