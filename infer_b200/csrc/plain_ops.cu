@@ -850,8 +850,39 @@ sample_filtered_kernel(const float* __restrict__ logits, int64_t vocab, const fl
     }
 }
 
-constexpr int64_t ONE_ROUND = 148;                        // blocks of the staged attention that run at once
 constexpr size_t STAGED_SMEM = 224 * 1024;
+inline size_t staged_smem(int heads, int head_dim, int v_dim) {
+    return (size_t(2 * AT) * (head_dim + 4) + size_t(AT) * v_dim + size_t(heads) * (head_dim + AT)) * sizeof(float);
+}
+
+// Heads that a block of the staged attention takes, as 10 H + S, or 0: the other kernel. Of the numbers whose queries and probabilities
+// fit beside the keys, the fewest that share keys and whose blocks run at once (one an SM), else the most; two rather than one. us for 3, 24,
+// 100 and 512 tokens of 12 heads on 2 at up to 300 keys (one query head and tile after the other: 25, 31, 95, 344): one head 16, 31, 130, 516;
+// two 15, 15, 67, 243; three 17, 17, 47, 187; six 19, 19, 35, 108. Blocks that mostly find nothing to do are the other kernel's.
+// Two rounds of one head a block, 16 tokens of 16 heads of 128: 6.5 us at 8 keys, 8.0 at 40, 28 at 300, 85 at 1,000 (the other kernel 5.9, 8.0, 32, 123). Three of
+// six heads of 144, 512 tokens: 287 us (325), 4,258 -> 3,540 behind 4,000 keys; 64 tokens at 8 keys 9.1 (7.7).
+int staged_heads(int64_t n_tokens, int n_heads, int n_kv, int head_dim, int v_dim, bool single_only, int64_t sms) {
+    const int group = n_heads / n_kv;
+    int heads = 0;
+    for (const int code : {12, 11, 13, 22, 15, 23, 17}) {
+        const int n = code / 10 * (code % 10);
+        if (group % n || staged_smem(n, head_dim, v_dim) > STAGED_SMEM) continue;
+        if (n_tokens * (n_heads / n) <= sms) return code;
+        if (n > 1 && !single_only) heads = code;
+    }
+    if (heads == 0 && staged_smem(1, head_dim, v_dim) <= STAGED_SMEM && n_tokens * n_heads <= 2 * sms) heads = 11;
+    return heads;
+}
+
+inline int64_t sm_count() {
+    static ib::PerDevice kept;
+    const int device = ib::current_device();
+    const int n = kept.get(device, [&] {
+        int v = 0;
+        return device >= 0 && cudaDeviceGetAttribute(&v, cudaDevAttrMultiProcessorCount, device) == cudaSuccess ? v : 0;
+    });
+    return n > 0 ? n : 148;
+}
 
 inline unsigned blocks_for(int64_t n, int threads) { return unsigned((n + threads - 1) / threads); }
 
@@ -949,6 +980,11 @@ IB_EXPORT int ib_thread_capture_mode(int mode) {
     return int(m);
 }
 
+// What staged_heads chooses on a device of `sms` SMs.
+IB_EXPORT int ib_attention_plain_heads(int64_t n_tokens, int n_heads, int n_kv, int head_dim, int v_dim, int single_only, int64_t sms) {
+    return staged_heads(n_tokens, n_heads, n_kv, head_dim, v_dim, single_only != 0, sms);
+}
+
 IB_EXPORT int ib_attention_plain_max_head_dim() { return 2 * AT; }
 
 IB_EXPORT int ib_attention_plain(const void* q, const void* k_cache, const void* v_cache, const int* block_table,
@@ -967,27 +1003,15 @@ IB_EXPORT int ib_attention_plain(const void* q, const void* k_cache, const void*
     const dim3 grid{unsigned(n_tokens), unsigned(n_heads), 1u};
     const size_t smem = size_t(((head_dim + 1) & ~1) + AT) * sizeof(float) + AT * sizeof(int64_t) + 8;
     if (dtype == IB_F32 && head_dim % 4 == 0 && v_dim % 4 == 0 && ((uintptr_t(k_cache) | uintptr_t(v_cache)) & 15) == 0) {
-        // Heads a block: the fewest that share keys and whose blocks run at once, else the most; two rather than one. us for 3, 24, 100 and
-        // 512 tokens of 12 heads on 2 at up to 300 keys (one query head and tile after the other: 25, 31, 95, 344): one head 16, 31, 130, 516;
-        // two 15, 15, 67, 243; three 17, 17, 47, 187; six 19, 19, 35, 108. Blocks that mostly find nothing to do are the other kernel's.
-        const int group = n_heads / n_kv;
-        int heads = 0;
-        for (const int code : {12, 11, 13, 22, 15, 23, 17}) {
-            const int n = code / 10 * (code % 10);
-            if (group % n) continue;
-            if (n_tokens * (n_heads / n) <= ONE_ROUND) { heads = code; break; }
-            if (n > 1 && !single_only) heads = code;
-        }
-        if (heads == 0 && n_tokens * n_heads <= 2 * ONE_ROUND) heads = 11;
-        const int taken = heads / 10 * (heads % 10);
-        const size_t need = (size_t(2 * AT) * (head_dim + 4) + size_t(AT) * v_dim + size_t(taken) * (head_dim + AT)) * sizeof(float);
-        if (heads > 0 && need <= STAGED_SMEM) {
+        const int heads = staged_heads(n_tokens, n_heads, n_kv, head_dim, v_dim, single_only != nullptr, sm_count());
+        if (heads > 0) {
+            const int taken = heads / 10 * (heads % 10);
             const dim3 staged{unsigned(n_tokens), unsigned(n_heads / taken), 1u};
 #define IB_STAGED(H_, S_)                                                                                                      \
     case H_ * 10 + S_: {                                                                                                       \
         static ib::PerDevice allowed;                                                                                          \
         if (const int rc = ib::allow_smem(allowed, "attention_staged", attention_staged_kernel<H_, S_>, STAGED_SMEM)) return rc;   \
-        return ib::launch("attention_staged", attention_staged_kernel<H_, S_>, staged, dim3(AT * S_), need, stream, 1u, (const float*)q,  \
+        return ib::launch("attention_staged", attention_staged_kernel<H_, S_>, staged, dim3(AT * S_), staged_smem(taken, head_dim, v_dim), stream, 1u, (const float*)q,  \
                           (const float*)k_cache, (const float*)v_cache, block_table, max_blocks, token_seg, positions, (float*)out, n_heads,   \
                           n_kv, head_dim, v_dim, page_size, window, scale, n_pages, status, dist_bias, bias_len, sink, single_only,  \
                           window > 0 && keep_first > 0 ? keep_first : 0, slopes);                                              \

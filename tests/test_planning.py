@@ -100,3 +100,24 @@ def test_every_plan_that_the_no_alloc_entry_point_accepts_fits_its_array():
             if ws <= room_floats and counters <= 4096:
                 reached += 1                                          # accepted: it fits by the same comparison
     assert reached > 0
+
+
+def _staged_heads(tokens, heads, kv, hd, vd=None, single_only=0, sms=SMS):
+    from infer_b200 import ops
+    from infer_b200.csrc.build import BuildError
+    try:
+        f = ops._fn("plain", "ib_attention_plain_heads", [ops.c_int64] + [ops.c_int] * 5 + [ops.c_int64])
+    except BuildError as e:
+        pytest.skip(f"the library that holds the planner cannot be compiled here: {str(e)[:80]}")
+    return f(tokens, heads, kv, hd, vd or hd, single_only, sms)
+
+
+def test_heads_that_a_block_of_the_float_attention_takes():
+    # 10 H + S: two heads that share keys where their blocks run at once, then the fewest that do, else the most
+    assert [_staged_heads(n, 12, 2, 128) for n in (1, 24, 25, 37, 512)] == [12, 12, 13, 13, 23]
+    assert _staged_heads(24, 12, 2, 128, sms=132) == 13                       # (on the device at hand, not on one of 148 SMs)
+    # six heads' queries do not fit beside keys of 144 floats, three do; nothing fits beside keys of 200
+    assert _staged_heads(512, 12, 2, 144) == 13 and _staged_heads(512, 6, 2, 200) == 0
+    # a head by itself: up to two rounds; blocks that mostly find nothing to do are the other kernel's beyond one
+    assert [_staged_heads(n, 4, 4, 64) for n in (37, 74, 75)] == [11, 11, 0]
+    assert [_staged_heads(n, 12, 2, 128, single_only=1) for n in (24, 75)] == [12, 0]
