@@ -5,7 +5,7 @@
 // bytes as possible are in flight per SM without costing registers or issue slots.
 //
 // A tile is 16 output features. For small N a thread-block cluster of up to 8 CTAs owns a tile and each CTA takes
-// a slice of K; for large N the grid is three CTAs per SM and a CTA walks over many tiles, its copy ring running ahead
+// a slice of K; for large N the grid is two CTAs per SM and a CTA walks over many tiles, its copy ring running ahead
 // into the next tile while the current one is reduced. A producer warp streams the tile's rows into a ring of shared-memory stages with bulk
 // asynchronous copies (cp.async.bulk, one per row and stage, completion counted on an mbarrier); eight consumer
 // warps wait for a stage, read weight fragments from it with conflict-free 16-byte loads, multiply them with the

@@ -1,5 +1,5 @@
 // Matrix product of the true 32-bit path: out[m, n] = sum_k x[m, k] * w[n, k] (+ bias[n]) (+ residual[m, n]), all float, for matrices of fewer
-// than 1024 features or columns (larger ones: linear_f32_tc.cu; the figures below are of those, from before).
+// than 1024 features or columns (larger ones: linear_f32_tc.cu, unless a caller names a kernel of this file).
 //
 // The order of every sum is fixed by K alone, so that a row of the result has the same bits in every batch, whichever
 // kernel below computes it: K is cut into blocks of 32; within a block the even and the odd k are two fused
@@ -276,14 +276,18 @@ int dispatch(const Args& a, int kind, int sms, cudaStream_t stream) {
     if (kind == 0) {
         if (a.M <= 8) {
             // 16 features a CTA share a row of x among twice as many threads; 8 where those CTAs leave SMs idle (N = 1536, K = 8960:
-            // 8 rows 34.5 against 36.4 us, one row 17.3 to 17.7 either way; with 3 rows 25.4 either way, N = 2048, K = 1536: 5.0 and 5.1)
+            // 8 rows 34.5 against 36.4 us, one row 17.3 to 17.7 either way; with 3 rows 25.4 either way, N = 2048, K = 1536: 5.0 and 5.1).
+            // Of the sizes that come here, with 16 and with 8 features: 896 x 896 one row 2.5 and 2.7, 3 rows 3.4 and 3.3, 8 rows 4.7 and 4.2;
+            // 896 x 4864 9.1 and 9.2, 13.5 and 12.5, 19.6 and 16.7; 9728 x 896 8.5 and 8.6, 14.2 and 13.6, 19.4 and 17.4
             kind = (a.N + 15) / 16 >= 2LL * sms || (a.M > 1 && a.M <= 4) ? 1 : 2;
         } else {
             // The larger a thread's share the fewer shared-memory reads per FMA, but a CTA alone on its SM is bound by its own
             // chain (1.07 us per 32 elements of K with 8 x 4 results a thread, 0.66 with 4 x 4, 0.43 with 4 x 2): 64 x 64 and
             // 32 x 64 need about one and a half CTAs an SM (512 rows, N = 1536: 192 and 384 tiles, 94 and 77 us; 256 rows: 192
             // tiles of 32 x 64 take 54 us, 384 of 32 x 32 48), and 64-row tiles win by 8 % where they pad no more rows
-            // (N = 17920: 87 rows 175 against 147 us, 128 rows 177 against 194).
+            // (N = 17920: 87 rows 175 against 147 us, 128 rows 177 against 194). Of the sizes that come here, 64 x 64, 32 x 64 and 32 x 32:
+            // 896 x 4864 9 rows 158, 98 and 64 us, 512 rows 165, 166 and 193, 2,048 rows 552, 530 and 595; 9728 x 896 64 rows 57, 47 and 46,
+            // 128 rows 80, 74 and 79, 2,048 rows 805, 895 and 1,103: the choice is within 9 % of the best
             const int64_t big = ((a.M + 63) / 64) * ((a.N + 63) / 64), mid = ((a.M + 31) / 32) * ((a.N + 63) / 64);
             const bool pads = (a.M + 63) / 64 * 64 * 100 > (a.M + 31) / 32 * 32 * 108;
             kind = big * 5 >= 8LL * sms && !pads ? 3 : (mid * 2 >= 3LL * sms ? 4 : 5);

@@ -4,25 +4,32 @@
 // Every float is cut into three bfloat16 numbers, v = v1 + v2 2^-8 + v3 2^-16 (each the rounding of what the ones before it
 // leave; three times eight bits hold a float's 24), on its way from global to shared memory, and a product becomes six of
 // the tensor cores': w1 x1 in one accumulator, w1 x2 + w2 x1 in a second (weight 2^-8) and w1 x3 + w2 x2 + w3 x1 in a third
-// (2^-16). What is left out (w2 x3, w3 x2, w3 x3) is below 2^-26 of a product. The powers of two keep the small parts out of
-// the subnormal range. A result that is not finite (an operand that is not, or too large a sum or part) is computed again by
-// plain multiply-adds, so that infinities and NaN come out as they do there.
+// (2^-16). What is left out is w2 x3 + w3 x2 (and w3 x3, below 2^-33): |v2| 2^-8 is at most 2^-8 of v and |v3| 2^-16 at most 2^-17 (both
+// where v is just above a power of two), hence below 2^-24 of a product, for random operands mostly below 2^-26. The powers of two keep the
+// small parts out of the subnormal range. A result that is not finite (an operand that is not, or too large a sum or part) is computed again
+// by plain multiply-adds, so that infinities and NaN come out as they do there.
 //
 // The tensor core's additions do not round as a float addition does, so few of them follow one another where it counts: the
 // first accumulator starts anew every 64 elements of K and is added to a float in registers; the other two, whose errors
-// weigh 2^-8, run over a group of such blocks. Groups (at most 8, from N and K alone) are added in ascending order. A result
-// does not depend on how many rows x has, nor on which CTA forms which group: a row's bits are the same in every batch.
-// Error against 64 bits (norm over norm, normal operands): 0.94e-7 at K = 1024, 1.2e-7 at 8960, where multiply-adds have 1.3e-7 and 3.1e-7.
-// us on multiply-adds -> here: 512 rows, 17920 x 1536 671 -> 272, 1536 x 8960 441 -> 165; 16 rows 55 -> 31 and 118 -> 23; 3 rows 31 -> 29
-// and 25 -> 23; one row 20 -> 29 and 18 -> 22. (A row's bits must not depend on the batch, so one row comes here too.) The line at
-// 1024 x 1024: below it the tiles leave most SMs idle.
+// weigh 2^-8, run over a group of such blocks. Groups (at most 8, from N, K and the device's SMs) are added in ascending order. A result
+// does not depend on how many rows x has, nor on which CTA forms which group: on one device a row's bits are the same in every batch.
+// Error against 64 bits (norm over norm), multiply-adds in brackets: normal operands 0.94e-7 (1.3e-7) at K = 1024, 1.2e-7 (3.1e-7) at 8960.
+// The tensor core truncates, so operands of one sign have errors of one sign, -0.7e-7 on average (1e-10), in norm 0.92e-7 (0.90e-7) at
+// K = 1024 and 0.95e-7 (2.6e-7) at 8960; scales e^(3 normal) apart -3.3e-7 (-0.1e-7), 2.0e-7 (0.7e-7) and 1.7e-7 (5.9e-7); normal w and
+// widely scaled x 1.4e-7 (1.2e-7) and 1.2e-7 (4.0e-7). Closer than multiply-adds from K = 3584 on, whatever the operands; below, on those
+// that a model has.
+// us on multiply-adds -> here: 512 rows, 17920 x 1536 669 -> 267, 1536 x 8960 440 -> 165; 16 rows 54 -> 28 and 117 -> 21; 3 rows 30 -> 27
+// and 24 -> 21. One and two rows lose: 18.7 -> 27.4, 16.8 -> 20.9, 2048 x 1536 4.3 -> 9.1, 4608 x 3584 11.9 -> 29.9, 151936 x 1536 129 -> 230.
+// (A row's bits must not depend on the batch, so they come here too: what prompts gain is 2 to 6 times that.) The line at 1024 x 1024: below
+// it the tiles leave most SMs idle.
 //
 // A CTA (544 threads, one an SM) forms 128 features x NT tokens (features on the tensor memory's 128 lanes). Sixteen warps load a
 // block of 64 elements of K into registers a block or two ahead, cut and store it as six swizzled operand tiles, and add up the
 // accumulator of the block before, while the seventeenth warp issues the block's 16 MMAs. The sixteen warps' instructions bound
 // it as much as anything: pairs of floats go through packed arithmetic, and addresses advance by addition. A few rows (NT = 16) are bound by
-// the reads of w; 64 rows and more by shared memory's bandwidth (per block 72 KB stored and 112 KB read by the MMAs
-// against 768 cycles of the tensor pipe).
+// the chain of a block (loads, cutting, a fence, the MMAs, adding up: 1.1 us, also where w came through a ring of asynchronous copies and
+// where a tile had half the features: 17920 x 1536 at one row 32 us that way), 64 rows and more by the workers' instructions beside shared
+// memory's bandwidth (per block 72 KB stored and 112 KB read by the MMAs against 768 cycles of the tensor pipe).
 // Where the tiles are fewer than the SMs, the groups of a tile go to the CTAs of a cluster: each pushes its groups' sums to
 // the CTAs that own their columns, through distributed shared memory, and after one cluster barrier the owners add them.
 #include "common.cuh"

@@ -583,6 +583,8 @@ class Engine:
             what = {1: "a token id outside the table", 2: "a cache write through an invalid page",
                     3: "a cache read through an invalid page", 101: "a tensor-core GEMM's copy wait ran out",
                     102: "a tensor-core GEMM's operand wait ran out", 103: "a tensor-core GEMM's accumulator wait ran out",
+                    104: "the streaming product's wait ran out", 106: "the prefill attention's wait ran out",
+                    107: "the score attention's wait ran out", 131: "the 32-bit tensor-core product's wait ran out",
                     108: "the prefill attention's shared memory does not start on a 1024-byte boundary",
                     }.get(code, f"code {code}")
             raise RuntimeError(f"device status word was raised: {what}")

@@ -137,7 +137,7 @@ def _f32_on_tensor_cores(N: int, K: int) -> bool:
 def linear_plain(x: torch.Tensor, w: torch.Tensor, bias: Optional[torch.Tensor] = None,
                  residual: Optional[torch.Tensor] = None, out_dtype: Optional[torch.dtype] = None,
                  out: Optional[torch.Tensor] = None, kind: int = 0, w_ready: bool = False) -> torch.Tensor:
-    """out = x @ w.T (+ bias) (+ residual) with float accumulation in an order that N and K alone fix. kind: which of the
+    """out = x @ w.T (+ bias) (+ residual) with float accumulation in an order that N, K and the device fix (never the number of rows). kind: which of the
     float32 kernels (0 = by the sizes; 1 to 5, which large matrices do not take by themselves, all give the same bits). w_ready: no kernel that may still be running writes
     ``w`` (a loaded weight), so that it may be read while the kernels before this one drain."""
     _check(x, "x")

@@ -3,7 +3,8 @@
 ``dtype`` is the compute dtype of the whole model: ``torch.bfloat16`` is the serving path
 (bfloat16 matrices, activations and cache; float32 residual stream, norms, softmax, rotation and
 logits), ``torch.float32`` is the true 32-bit path (every tensor float32; products of
-large matrices from three bfloat16 parts of each float, no less exact than float multiply-adds).
+large matrices from three bfloat16 parts of each float, which hold all of its 24 bits: on operands like a model's as
+close to 64 bits as float multiply-adds or closer).
 
 ``kernels`` chooses, per operation, between the fast kernel ("auto": the fast kernel where it
 accepts the shape, else the plain one) and the plain kernel ("plain").  Tests use it to check one
