@@ -76,3 +76,30 @@ def test_a_page_that_is_not_there():
     assert int(status) == 3 and torch.isfinite(got).all()
     fine = ops.attention_plain(q[1:].contiguous(), kc, kc, table[1:].contiguous(), seg[:1], pos[1:].contiguous(), 2, 1, 64, None, 0.1)
     assert torch.equal(got[1:], fine)
+
+
+@pytest.mark.parametrize("window,keep,extra", [(None, 0, ""), (50, 7, "sink")])
+def test_as_many_heads_together_as_fit(window, keep, extra):
+    """Six query heads of 144 floats do not fit beside their keys: three do."""
+    test_heads_together(12, 2, 144, 144, window, keep, extra)
+
+
+@pytest.mark.parametrize("nh,nkv,hd", [(4, 4, 64), (12, 2, 128), (14, 2, 64)])
+def test_a_few_keys(nh, nkv, hd):
+    """Contexts of one tile: only the keys that a token sees are copied. What shared memory held before is not looked at."""
+    from infer_b200 import ops
+    gen = torch.Generator(device=DEV).manual_seed(nh + hd)
+    rand = lambda *s: torch.randn(*s, generator=gen, device=DEV)  # noqa: E731
+    T = 24
+    kc, vc = rand(T * 8, nkv, 16, hd), rand(T * 8, nkv, 16, hd)
+    table = torch.randperm(T * 8, generator=gen, device=DEV).view(T, 8).int().contiguous()
+    q, seg = rand(T, nh * hd), torch.arange(T, device=DEV).int()
+    pos = torch.tensor([0, 1, 2, 3, 6, 7, 8, 14, 15, 16, 17, 30, 31, 32, 33, 63, 64, 65, 100, 120, 125, 126, 127, 5], device=DEV).int()
+    bad_k, bad_v = torch.full_like(kc, float("nan")), torch.full_like(vc, float("nan"))
+    for window, keep in ((None, 0), (10, 0), (10, 3)):
+        # NaN first, so that keys that are not there would show
+        ops.attention_plain(q, bad_k, bad_v, table, seg, pos, nh, nkv, hd, None, 0.1)
+        got = ops.attention_plain(q, kc, vc, table, seg, pos, nh, nkv, hd, window, 0.1, keep_first=keep)
+        want = _oracle(q, kc, vc, table, seg, pos, nh, nkv, window, 0.1, keep, None, None, None)
+        # hd products and a sum over up to 128 keys, in float
+        assert (got.double() - want).abs().max() <= 300 * 2.0 ** -24 * max(1.0, want.abs().max().item())

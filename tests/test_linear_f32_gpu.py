@@ -43,3 +43,19 @@ def test_a_matrix_that_the_kernel_before_has_just_written(M, N, K):
         again = torch.full_like(w, float("nan"))
         assert torch.equal(ops.linear_plain(x, ops.linear_plain(a, b, out=again)), want)
     assert torch.equal(ops.linear_plain(x, w, w_ready=True), want)
+
+
+# (the matrices above of 1024 x 1024 and more go to the tensor cores by themselves: here the kernels of this file are named, or the matrix is smaller)
+@pytest.mark.parametrize("M,N,K,kind", [(1, 2048, 1536, 1), (8, 2048, 1536, 2), (9, 2048, 1536, 3), (40, 2048, 1536, 4), (9, 2048, 1536, 5), (9, 900, 1536, 0), (70, 1100, 900, 0)])
+def test_every_kernel_waits_for_the_matrix_that_the_kernel_before_writes(M, N, K, kind):
+    from infer_b200 import ops
+    gen = torch.Generator(device=DEV).manual_seed(M + N + K)
+    x, a, b = (torch.randn(n, k, generator=gen, device=DEV) for n, k in ((M, K), (N, 1000), (K, 1000)))
+    w = ops.linear_plain(a, b)
+    torch.cuda.synchronize()
+    want = ops.linear_plain(x, w, kind=kind)
+    torch.cuda.synchronize()
+    for _ in range(20):
+        again = torch.full_like(w, float("nan"))
+        assert torch.equal(ops.linear_plain(x, ops.linear_plain(a, b, out=again), kind=kind), want)
+    assert torch.equal(ops.linear_plain(x, w, w_ready=True, kind=kind), want)

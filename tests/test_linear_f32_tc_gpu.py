@@ -113,3 +113,37 @@ def test_not_finite_has_the_bits_of_the_multiply_adds(M, N, K):
     assert torch.equal(torch.nan_to_num(ops.linear_plain(x, w, b, own, out=own)), torch.nan_to_num(full)) and torch.equal(torch.isnan(own), torch.isnan(full))
     kept = [n for n in range(N) if n not in (N - 1, 130, 700)]
     assert torch.equal(full[4:, kept], clean[4:, kept])
+
+
+def _values(kind, gen, *shape):
+    r = torch.randn(*shape, generator=gen, device=DEV)
+    if kind == "positive":
+        return r.abs()
+    if kind in ("wide", "wide positive"):
+        r = r * torch.exp(3.0 * torch.randn(*shape, generator=gen, device=DEV))
+        return r.abs() if kind == "wide positive" else r
+    if kind == "outliers":
+        r[:, ::97] *= 300.0
+    if kind == "one value":
+        r.fill_(1.0038986)                                        # the largest parts: 2^-8 and 2^-17 of the value are left to the second and third
+    return r
+
+
+@pytest.mark.parametrize("kx,kw", [("normal", "normal"), ("outliers", "normal"), ("wide", "normal"), ("wide", "wide"), ("positive", "positive"),
+                                   ("wide positive", "wide positive"), ("one value", "one value")])
+@pytest.mark.parametrize("N,K", [(1024, 1024), (17920, 1536), (1536, 8960)])
+def test_other_operands(N, K, kx, kw):
+    """The error's bound holds for operands of one sign, for widely scaled ones and for those of which most is left out; a mean of errors of one
+    sign is at most half of what the additions can lose; from K = 3584 on no set of operands is further off than on multiply-adds."""
+    from infer_b200 import ops
+    gen = torch.Generator(device=DEV).manual_seed(N + K)
+    x, w = _values(kx, gen, 40, K), _values(kw, gen, N, K)
+    exact, size = x.double() @ w.double().T, x.double().abs() @ w.double().abs().T
+    off = ops.linear_plain(x, w).double() - exact
+    units = 8 + K / 64 + 8 + K / 8 * 2 / 256 + 3                   # as in test_product
+    assert (off.abs() / size).max() <= units * 2.0 ** -24
+    # four additions a block, each loses up to two units, one on average; what is left out: one more
+    assert abs((off / size).mean().item()) <= (8 / 2 + 1 + 1) * 2.0 ** -24
+    plain = ops.linear_plain(x, w, kind=3).double() - exact
+    if K >= 3584:
+        assert off.norm() <= plain.norm() * 1.001
