@@ -114,6 +114,11 @@ __device__ long long ib_gemv_trace[64];
 #define IB_GT(k) do {} while (0)
 #endif
 
+// How a matrix is dealt out to the CTAs of a grid.
+struct Deal {
+    int tiles, cluster, kc, ns, n_stages, per_cta, groups;
+};
+
 struct GemvParams {
     const bf16* x;            // [M, K]; or, with norm_w, float rows that are RMS-normalised first (K <= KC_MAX)
     const float* norm_w;      // [K] or null
@@ -130,7 +135,8 @@ struct GemvParams {
                               //    copies (up to 8 rows of activations; measured: q/k/v 4.1 -> 3.2 us)
     int kc;                   // elements of K per stage and row: a multiple of 64, at most KC_MAX
     int ns;                   // stages in the ring: 2 .. NS_MAX, ns * ROWS * (kc * 2 + 64) <= RING_BYTES
-    int64_t tiles;
+    int tiles;
+    int n_stages, per_cta;    // stages of a tile's K, and of a CTA of its cluster
     int groups;               // tile walkers in the grid (grid = groups * cluster); a walker takes every groups-th tile
     int* status;
 };
@@ -154,12 +160,11 @@ bulk_gemv_kernel(const GemvParams p) {
     const int PITCH = KC * 2 + 64;                       // bytes between rows of a stage: consecutive rows start 16 banks apart
     const int STAGE_BYTES = ROWS * PITCH;
     // This CTA's slice of K, in stages of KC elements.
-    const int64_t total_stages = (K + KC - 1) / KC;
-    const int64_t per_cta = (total_stages + cluster - 1) / cluster;
-    const int64_t s_begin = min(total_stages, rank * per_cta), s_end = min(total_stages, s_begin + per_cta);
-    const int spt = int(s_end - s_begin);                // stages per tile
-    const int64_t my_tiles = group < p.tiles ? (p.tiles - group + p.groups - 1) / p.groups : 0;
-    const int64_t n_iter = my_tiles * spt;
+    const int total_stages = p.n_stages;
+    const int s_begin = min(total_stages, rank * p.per_cta), s_end = min(total_stages, s_begin + p.per_cta);
+    const int spt = s_end - s_begin;                     // stages per tile
+    const int my_tiles = group < p.tiles ? (p.tiles - group + p.groups - 1) / p.groups : 0;
+    const int n_iter = my_tiles * spt;
     const uint32_t stage0 = smem_u32(stages), bar0 = smem_u32(bars);
     auto full_bar = [&](int s) { return bar0 + 8u * s; };
     auto empty_bar = [&](int s) { return bar0 + 8u * (NS_MAX + s); };
@@ -184,9 +189,9 @@ bulk_gemv_kernel(const GemvParams p) {
         // values would cost more per stage than the copies)
         int s = 0, st = 0;
         uint32_t round = 0;
-        int64_t tile = group;
+        int tile = group;
         const uint64_t once = policy_evict_first();
-        for (int64_t i = 0; i < n_iter; i++) {
+        for (int i = 0; i < n_iter; i++) {
             if (i == 1 && p.gate_ring) {
                 // With every SM's ring being filled at once, activations requested after the dependency wait would
                 // queue behind megabytes of weights and the consumers would start microseconds late: the second slot
@@ -202,8 +207,8 @@ bulk_gemv_kernel(const GemvParams p) {
                 ok = __shfl_sync(0xffffffffu, ok, 0);
                 if (!ok) { if (lane == 0) { atomicExch(p.status, STATUS_TIMEOUT); failed = 1; } break; }
             }
-            const int64_t n0 = tile * ROWS;
-            const int64_t k0 = (s_begin + st) * KC;
+            const int64_t n0 = int64_t(tile) * ROWS;
+            const int64_t k0 = int64_t(s_begin + st) * KC;
             const int live_rows = int(min(int64_t(ROWS), N - n0));
             const uint32_t bytes = uint32_t(min(int64_t(KC), K - k0) * 2);
             if (lane == 0) mbar_expect_tx(full_bar(s), bytes * uint32_t(live_rows));
@@ -357,9 +362,9 @@ bulk_gemv_kernel(const GemvParams p) {
     IB_GT(2);
     int s = 0, st = 0;
     uint32_t round = 0;
-    int64_t tile = group;
-    for (int64_t i = 0; i < n_iter; i++) {
-        const int64_t k0 = (s_begin + st) * KC;
+    int tile = group;
+    for (int i = 0; i < n_iter; i++) {
+        const int64_t k0 = int64_t(s_begin + st) * KC;
         IB_GT(4 + 4 * int(i));
         if (!hoist) {
             // activations of this warp's chunks: independent of the weights, so they are loaded before the wait
@@ -397,9 +402,9 @@ bulk_gemv_kernel(const GemvParams p) {
         st = 0;
 
         // ---------------------------------------------------------------- the tile is complete
-        const int64_t this_tile = tile;
+        const int this_tile = tile;
         tile += p.groups;
-        const int64_t n0 = this_tile * ROWS;
+        const int64_t n0 = int64_t(this_tile) * ROWS;
         asm volatile("bar.sync 1, 256;" ::: "memory");   // the previous tile's sums have been read (consumers only)
 #pragma unroll
         for (int nt = 0; nt < NT; nt++) {
@@ -437,7 +442,7 @@ bulk_gemv_kernel(const GemvParams p) {
         if constexpr (EPI == 2) {
             if (r < 8) {
                 const float gate = v, up = part[ant][col][r + 8];
-                const int64_t f = this_tile * 8 + r;
+                const int64_t f = int64_t(this_tile) * 8 + r;
                 if (f < N / 2) out[int64_t(m) * (N / 2) + f] = ib::from_f32<TOut>(gate / (1.0f + expf(-gate)) * up);
             }
         } else {
@@ -483,6 +488,31 @@ int launch(const GemvParams& p, int out_dtype, int epi, int grid_ctas, cudaStrea
     return ib::fail(IB_ERR_ARG, "linear_skinny_bulk: unknown output dtype %d", out_dtype);
 }
 
+// K of a tile in as few equal stages as the ring allows (a whole row for K up to KC_MAX), since the cost of a stage (its copies, the barrier
+// round trip) does not depend on its size. cluster 0: chosen here.
+Deal deal_out(int64_t tiles, int64_t K, int cluster, int sms) {
+    Deal d = {};
+    int64_t n_stages = (K + KC_MAX - 1) / KC_MAX;
+    if (cluster == 0) {
+        // Share a tile among CTAs while the tiles alone leave SMs idle and every CTA keeps at least three stages of K
+        // (measured on B200 for K = 8960: 10.8 us alone, 8.9 us in pairs, 14.4 us in fours; clusters of three or six
+        // run slower still).
+        cluster = 1;
+        while (cluster < 8 && tiles * cluster < 2LL * sms && n_stages >= 6 * cluster) cluster *= 2;
+    }
+    n_stages = (n_stages + cluster - 1) / cluster * cluster;     // the same number of stages for every CTA of a cluster
+    d.tiles = int(tiles); d.cluster = cluster;
+    d.kc = int(((K + n_stages - 1) / n_stages + 63) / 64 * 64);
+    d.ns = RING_BYTES / (ROWS * (d.kc * 2 + 64));
+    if (d.ns > NS_MAX) d.ns = NS_MAX;
+    d.n_stages = int((K + d.kc - 1) / d.kc);
+    d.per_cta = (d.n_stages + cluster - 1) / cluster;
+    // Two CTAs fit an SM; with more tiles than that, a CTA walks over several and its ring never drains between them.
+    const int64_t places = int64_t(IB_GEMV_CTAS_PER_SM) * sms;
+    d.groups = int(cluster > 1 || tiles < places ? tiles : places);
+    return d;
+}
+
 }  // namespace
 
 // x: bfloat16 [M, K]; with norm_w (float [K]) x is float [M, K] and is RMS-normalised (eps norm_eps) on the way in,
@@ -512,32 +542,17 @@ IB_EXPORT int ib_linear_skinny_bulk(const void* x, const float* norm_w, float no
     const int64_t tiles = (N + ROWS - 1) / ROWS;
     if (tiles > 0x7fffffffLL / 8) return ib::fail(IB_ERR_ARG, "linear_skinny_bulk: N too large");
     const int sms = sm_count > 0 ? sm_count : 148;
-    // A stage holds ROWS rows of kc elements: K in as few equal stages as the ring allows (a whole row for K up to
-    // KC_MAX), since the cost of a stage (its copies, the barrier round trip) does not depend on its size.
-    int64_t n_stages = (K + KC_MAX - 1) / KC_MAX;
-    if (cluster == 0) {
-        // Share a tile among CTAs while the tiles alone leave SMs idle and every CTA keeps at least three stages of K
-        // (measured on B200 for K = 8960: 10.8 us alone, 8.9 us in pairs, 14.4 us in fours; clusters of three or six
-        // run slower still).
-        cluster = 1;
-        while (cluster < 8 && tiles * cluster < 2LL * sms && n_stages >= 6 * cluster) cluster *= 2;
-    }
-    if (cluster != 1 && cluster != 2 && cluster != 4 && cluster != 8) return ib::fail(IB_ERR_ARG, "linear_skinny_bulk: cluster must be 1, 2, 4 or 8");
-    n_stages = (n_stages + cluster - 1) / cluster * cluster;     // the same number of stages for every CTA of a cluster
-    const int kc = int(((K + n_stages - 1) / n_stages + 63) / 64 * 64);
-    int ns = RING_BYTES / (ROWS * (kc * 2 + 64));
-    if (ns > NS_MAX) ns = NS_MAX;
+    if (cluster != 0 && cluster != 1 && cluster != 2 && cluster != 4 && cluster != 8) return ib::fail(IB_ERR_ARG, "linear_skinny_bulk: cluster must be 1, 2, 4 or 8");
+    const Deal d = deal_out(tiles, K, cluster, sms);
     GemvParams p;
     p.x = (const bf16*)x; p.norm_w = norm_w; p.eps = norm_eps; p.w = (const bf16*)w; p.bias = bias; p.residual = residual; p.out = out;
-    p.M = int(M); p.N = N; p.K = K; p.cluster = cluster; p.status = status; p.tiles = tiles; p.kc = kc; p.ns = ns;
+    p.M = int(M); p.N = N; p.K = K; p.cluster = d.cluster; p.status = status; p.tiles = d.tiles; p.kc = d.kc; p.ns = d.ns;
+    p.n_stages = d.n_stages; p.per_cta = d.per_cta;
     // gate the ring's second slot where the whole GPU's rings fill at once (a CTA per half SM) and a tile is one stage
-    p.gate_ring = (n_stages == 1 && cluster == 1 && tiles >= 2LL * sms) ? 1 : 0;
+    p.gate_ring = (d.n_stages == 1 && d.cluster == 1 && tiles >= 2LL * sms) ? 1 : 0;
     p.nw_smem = norm_w ? 1 : 0;
-    // Two CTAs fit an SM; with more tiles than that, a CTA walks over several and its ring never drains between them.
-    constexpr int64_t PER_SM = IB_GEMV_CTAS_PER_SM;
-    int64_t groups = cluster > 1 ? tiles : (tiles < PER_SM * sms ? tiles : PER_SM * sms);
-    p.groups = int(groups);
-    const int grid_ctas = int(groups) * cluster;
+    p.groups = d.groups;
+    const int grid_ctas = d.groups * d.cluster;
     if (M <= 8) return launch<1>(p, out_dtype, epi, grid_ctas, stream);
     return launch<2>(p, out_dtype, epi, grid_ctas, stream);
 }
