@@ -27,8 +27,8 @@
 // block of 64 elements of K into registers a block or two ahead, cut and store it as six swizzled operand tiles, and add up the
 // accumulator of the block before, while the seventeenth warp issues the block's 16 MMAs. The sixteen warps' instructions bound
 // it as much as anything: pairs of floats go through packed arithmetic, and addresses advance by addition. A few rows (NT = 16) are bound by
-// the chain of a block (loads, cutting, a fence, the MMAs, adding up: 1.1 us, also where w came through a ring of asynchronous copies and
-// where a tile had half the features: 17920 x 1536 at one row 32 us that way), 64 rows and more by the workers' instructions beside shared
+// the chain of a worker's round (cut, fence, arrive, see that the MMAs of the block before are done, add: 1,770 cycles, also where w came through
+// a ring of asynchronous copies and where a tile had half the features: 17920 x 1536 at one row 32 us that way), 64 rows and more by the workers' instructions beside shared
 // memory's bandwidth (per block 72 KB stored and 112 KB read by the MMAs against 768 cycles of the tensor pipe).
 // Where the tiles are fewer than the SMs, the groups of a tile go to the CTAs of a cluster: each pushes its groups' sums to
 // the CTAs that own their columns, through distributed shared memory, and after one cluster barrier the owners add them.
