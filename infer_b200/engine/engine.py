@@ -579,7 +579,8 @@ class Engine:
         code = int(self.status.item())
         if code:
             from ..fast_ops import clear_failure
-            clear_failure(self.rt.device)
+            with _CAPTURING:                                # (it waits for the whole device: not while another engine captures)
+                clear_failure(self.rt.device)
             what = {1: "a token id outside the table", 2: "a cache write through an invalid page",
                     3: "a cache read through an invalid page", 101: "a tensor-core GEMM's copy wait ran out",
                     102: "a tensor-core GEMM's operand wait ran out", 103: "a tensor-core GEMM's accumulator wait ran out",
